@@ -214,6 +214,10 @@ int qb_attn_decode(qb_ctx* ctx, void* stream, const float* q, const void* kc, co
                    float* part_acc, float* out, void* mix_f16);
 int qb_attn_dec_splits(int keys);
 int qb_attn_dec_splits_sm(int keys, int sms);
+/* The splits that a launch of qb_attn_decode with this max_keys provides for: the most of any key count up to it (a
+ * longer range has longer splits: on 148 SMs 3000 keys are 24 splits, 4400 keys 23). A captured launch serves every step
+ * with the same value. */
+int qb_attn_dec_grid(int max_keys, int sms);
 /* qb_attn_prefill  attn_prefill + attn_combine_tiles (+ to_xin when mix_f16 != NULL), kernels/attn.cuh:327-349,351-520,
  *                  as Attn::run launches them (src/cuda/qwen/attn.rs:338-368): ntile tiles (ptile: first token,
  *                  count; at most 64 / 6 = 10 consecutive tokens of one segment each), max_keys = tile_max_pos + 1.

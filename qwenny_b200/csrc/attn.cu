@@ -875,6 +875,8 @@ int qb_attn_prep(qb_ctx* ctx, void* stream, const float* part, int splits, int n
 int qb_attn_dec_splits(int keys) { return keys > 0 ? dec_splits(keys, DSPLITS) : 0; }
 int qb_attn_dec_splits_sm(int keys, int sms) { return keys > 0 && sms > 0 ? dec_splits(keys, dsplits_for(sms)) : 0; }
 
+int qb_attn_dec_grid(int max_keys, int sms) { return max_keys > 0 && sms > 0 ? dec_splits_upto(max_keys, dsplits_for(sms)) : 0; }
+
 // ndseg short segments (dseg: first index into dtok, token count; at most 8 tokens each), ndec = their tokens in
 // all, dmax = the longest segment's tokens, max_keys = the largest key count among them (sizes the grid).
 int qb_attn_decode(qb_ctx* ctx, void* stream, const float* q, const void* kc, const void* vc, const float* ks,
@@ -886,7 +888,7 @@ int qb_attn_decode(qb_ctx* ctx, void* stream, const float* q, const void* kc, co
         max_keys > cap)
         return QB_ERR_ARG;
     const int dsplits = dsplits_for(ctx->sms);
-    const int z = dec_splits(max_keys, dsplits), rt = (dmax * GROUP + 15) / 16;
+    const int z = dec_splits_upto(max_keys, dsplits), rt = (dmax * GROUP + 15) / 16;
     cudaStream_t st = (cudaStream_t)stream;
     dim3 grid(ndseg, NKV, z);
     // a step has at most 64 decode tokens: whatever lies 64 positions or more before a segment's last key is from

@@ -32,6 +32,13 @@ __host__ __device__ inline int dec_chunk(int keys, int dsplits) {
     return max(64, ((range_end + dsplits - 1) / dsplits + 63) / 64 * 64);
 }
 __host__ __device__ inline int dec_splits(int keys, int dsplits) { int c = dec_chunk(keys, dsplits); return (keys + c - 1) / c; }
+// The most splits of any key count up to `most`: not dec_splits(most), because a longer range has longer splits (148 SMs: 3000
+// keys are 24 splits of 128, 4400 keys 23 of 192).
+__host__ inline int dec_splits_upto(int most, int dsplits) {
+    int z = dec_splits(most, dsplits);
+    for (int e = 2048; e < most; e += 2048) z = max(z, dec_splits(e, dsplits));
+    return z;
+}
 // the most key splits of a decode token on a part with `sms` SMs: one block per SM over the kv heads, at most 64
 __host__ inline int dsplits_for(int sms) { return max(1, min(64, sms / NKV)); }
 

@@ -254,3 +254,29 @@ def test_attn_prefill_pairs_and_segment_boundaries(ctx, ref):
     assert np.array_equal(mix.cpu().numpy(), a.astype(np.float16))
     want = R.attn_decode(q.numpy(), gate.numpy(), *[t.numpy() for t in cache], st["tok_slot"], st["tok_pos"], cap)
     assert close(a, want).all()
+
+
+@pytest.mark.parametrize("rows", [1, 4, 8])
+def test_attn_decode_of_a_ragged_batch(ctx, rows):
+    """A batch of ragged sequences gives each token the bits that its sequence alone gives, and the oracle's values: also where
+    a shorter sequence has more key splits than the longest (3000 keys: 24 splits, 4400: 23 on 148 SMs)."""
+    g = synth.gen(151 + rows)
+    cap, ends = 4480, [1, 63, 64, 500, 1025, 2047, 2049, 3000, 4400]
+    cache = make_cache(len(ends), cap, g, 0)
+    toks = [(0, s, max(0, e - rows) + i) for s, e in enumerate(ends) for i in range(rows)]
+    n = len(toks)
+    q = torch.randn(n, R.NH, R.HD, generator=g) * QSCALE
+    gate = torch.sigmoid(torch.randn(n, R.MIX, generator=g))
+    st = R.build_step(toks, list(range(n)), max_dec=n)
+    assert st["ndec"] == n
+    dc = [t.cuda() for t in cache]
+    full = run_decode(ctx, q.cuda(), gate.cuda(), dc, st, ref_cuda.upload_step(st), cap, n)
+    torch.cuda.synchronize()
+    assert ctx.device_error() == 0
+    for s in range(len(ends)):
+        a, e = s * rows, (s + 1) * rows
+        st1 = R.build_step(toks[a:e], list(range(rows)))
+        one = run_decode(ctx, q[a:e].cuda().contiguous(), gate[a:e].cuda().contiguous(), dc, st1, ref_cuda.upload_step(st1), cap, rows)
+        assert torch.equal(one, full[a:e])
+    want = R.attn_decode(q.numpy(), gate.numpy(), *[t.numpy() for t in cache], st["tok_slot"], st["tok_pos"], cap)
+    assert close(full.cpu().numpy(), want).all()

@@ -173,3 +173,15 @@ def test_host_bookkeeping_selftests():
     from qwenny_b200._lib import lib
     assert lib().qb_graph_cache_selftest() == 0
     assert lib().qb_attr_cache_selftest() == 0
+
+
+def test_decode_attention_grid_holds_every_split():
+    """The key splits that a launch provides for cover those of every key count up to its largest (the split size grows
+    in steps of 2048 keys, so a shorter sequence may have more splits than the longest of the step)."""
+    from qwenny_b200._lib import lib
+    grid = lib().qb_attn_dec_grid
+    for sms in (148, 132, 16, 4):
+        most = 0
+        for keys in range(1, 40000, 61):
+            most = max(most, lib().qb_attn_dec_splits_sm(keys, sms))
+            assert most <= grid(keys, sms) <= 64
