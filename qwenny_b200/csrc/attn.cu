@@ -414,13 +414,21 @@ attn_decode_kernel(const float* q, const uint8_t* kc, const uint8_t* vc, const f
 }
 
 // ------------------------------------------------------------------------------------------------ decode attention
+// 2^x, results below 2^-126 as 0 (exp2f spends three more instructions on those; P is rounded to f16 next)
+__device__ __forceinline__ float exp2_ftz(float x) {
+    float y;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+
 // Block (short segment, kv head, key split) of the decode / verify attention: 2 to 4 QUADS of four compute warps and a
 // copy warp. The keys and values of the split arrive in 64-key stages through a ring fed by bulk copies; the quads
 // take the stages in turn. Inside a quad the work of a stage is dealt so that no byte is converted twice:
 //   scores   warp w multiplies all the rows (RT tiles of 16 (token, head) rows) by the keys 16 w .. 16 w + 15 of the
 //            stage over the whole head dimension: one conversion of a key serves every row tile;
 //   softmax  the four warps agree on the rows' running maxima through shared memory, so that all of them scale by the
-//            same power of two, and exchange their 16-key slices of P (as f16 mma fragments) and of the row sums;
+//            same power of two, and exchange their 16-key slices of P (as f16 mma fragments); a lane keeps the sums of its
+//            own keys to the end;
 //   values   warp w accumulates the output dims 64 w .. 64 w + 63 over all 64 keys of the stage (for every row tile),
 //            so the output accumulators of a row are spread over four warps (RT x 32 registers each).
 // The int8 codes go to the tensor cores as 1152 + q halves (one prmt per pair) and the offset is folded out through the
@@ -650,7 +658,7 @@ attn_dec4_kernel(const float* q, const uint8_t* kc, const uint8_t* vc, const flo
 #pragma unroll
                     for (int e = 0; e < 2; e++) {
                         const float sv = v[rt][nn][2 * h2 + e];
-                        const float pp = sv == -INFINITY ? 0.f : exp2f(sv - m[rt][h2]);
+                        const float pp = sv == -INFINITY ? 0.f : exp2_ftz(sv - m[rt][h2]);
                         sum[h2] += pp;
                         pv[nn][2 * h2 + e] = pp * vsc[nn][e];
                     }
@@ -662,31 +670,16 @@ attn_dec4_kernel(const float* q, const uint8_t* kc, const uint8_t* vc, const flo
             __half2 h0, h1, h2v, h3;
             *(uint32_t*)&h0 = pa.x; *(uint32_t*)&h1 = pa.y; *(uint32_t*)&h2v = pa.z; *(uint32_t*)&h3 = pa.w;
             const float2 f0 = __half22float2(h0), f1 = __half22float2(h1), f2 = __half22float2(h2v), f3 = __half22float2(h3);
-            float pr[2] = {f0.x + f0.y + f2.x + f2.y, f1.x + f1.y + f3.x + f3.y};
+            const float pr[2] = {f0.x + f0.y + f2.x + f2.y, f1.x + f1.y + f3.x + f3.y};
+            // a lane sums its own keys; lanes and warps are added up once, after the last stage (added up in every stage the
+            // shuffles and the exchange were some 700 of a stage's 6100 cycles)
 #pragma unroll
             for (int h2 = 0; h2 < 2; h2++) {
-                sum[h2] += __shfl_xor_sync(0xffffffffu, sum[h2], 1);
-                sum[h2] += __shfl_xor_sync(0xffffffffu, sum[h2], 2);
-                pr[h2] += __shfl_xor_sync(0xffffffffu, pr[h2], 1);
-                pr[h2] += __shfl_xor_sync(0xffffffffu, pr[h2], 2);
-                if (t4 == 0) xsum[(w * RT + rt) * 16 + r + 8 * h2] = make_float2(sum[h2], pr[h2]);
+                l[rt][h2] = l[rt][h2] * corr[rt][h2] + sum[h2];
+                ps[rt][h2] = ps[rt][h2] * corr[rt][h2] + pr[h2];
             }
         }
         named_bar_sync(2 + quad, 128);
-#pragma unroll
-        for (int rt = 0; rt < RT; rt++)
-#pragma unroll
-            for (int h2 = 0; h2 < 2; h2++) {
-                float sl2 = 0.f, sp2 = 0.f;
-#pragma unroll
-                for (int ww = 0; ww < 4; ww++) {  // in warp order: the same sum in all four warps
-                    const float2 x = xsum[(ww * RT + rt) * 16 + r + 8 * h2];
-                    sl2 += x.x;
-                    sp2 += x.y;
-                }
-                l[rt][h2] = l[rt][h2] * corr[rt][h2] + sl2;
-                ps[rt][h2] = ps[rt][h2] * corr[rt][h2] + sp2;
-            }
         if (__any_sync(0xffffffffu, grew)) {
 #pragma unroll
             for (int rt = 0; rt < RT; rt++)
@@ -765,11 +758,28 @@ attn_dec4_kernel(const float* q, const uint8_t* kc, const uint8_t* vc, const flo
         named_bar_sync(1, NCW);
     }
     if (quad != 0) return;
+    // the rows' sums: over a row's four lanes, then over the four warps in order
 #pragma unroll
     for (int rt = 0; rt < RT; rt++)
 #pragma unroll
         for (int h2 = 0; h2 < 2; h2++) {
-            const float L = l[rt][h2], P = ps[rt][h2];   // already whole-row sums, the same in the four warps
+            float a = l[rt][h2], b = ps[rt][h2];
+            a += __shfl_xor_sync(0xffffffffu, a, 1); b += __shfl_xor_sync(0xffffffffu, b, 1);
+            a += __shfl_xor_sync(0xffffffffu, a, 2); b += __shfl_xor_sync(0xffffffffu, b, 2);
+            if (t4 == 0) xsum[(w * RT + rt) * 16 + r + 8 * h2] = make_float2(a, b);
+        }
+    named_bar_sync(2, 128);
+#pragma unroll
+    for (int rt = 0; rt < RT; rt++)
+#pragma unroll
+        for (int h2 = 0; h2 < 2; h2++) {
+            float L = 0.f, P = 0.f;
+#pragma unroll
+            for (int ww = 0; ww < 4; ww++) {
+                const float2 x = xsum[(ww * RT + rt) * 16 + r + 8 * h2];
+                L += x.x;
+                P += x.y;
+            }
             const int row = rt * 16 + r + 8 * h2, tok = row / GROUP;
             if (tok >= nt) continue;
             const int i = first + tok, t = dtok[i], head = g * GROUP + row % GROUP;
