@@ -15,8 +15,8 @@ struct qb_ctx {
     int* counters = nullptr;
     size_t ncounters = 0;
     int* err = nullptr;  // device word
-    float* tc_part = nullptr;   // partial tiles of the tensor-core W4A16 product's stream-K shares (sms x 2 x 256 KB), taken with its first call
-    int* tc_tickets = nullptr;  // its per-tile tickets (QB_TC_TICKETS, zero between launches)
+    float* tc_part = nullptr;   // partial tiles of the tensor-core W4A16 product's stream-K shares (sms x 256 KB), taken with its first call
+    int* tc_tickets = nullptr;  // its tickets, two per tile (QB_TC_TICKETS, zero between launches)
     float* delta_tp = nullptr;  // scratch of the chunked delta rule (T, P, log decays per chunk and value head), taken by
                                 // the first prompt-sized DeltaNet step
     // measurement override of the GEMV plan (0: built-in choice)
@@ -30,7 +30,7 @@ struct qb_ctx {
     long long* trace = nullptr;  // measurement: per-block timestamps of the next products
 };
 
-constexpr int QB_TC_TICKETS = 1 << 16;  // tiles of one tensor-core W4A16 product (256 outputs x 256 tokens each)
+constexpr int QB_TC_TICKETS = 1 << 17;  // two per tile of a tensor-core W4A16 product (256 outputs x 256 tokens each)
 #define QB_CUDA(x)                         \
     do {                                   \
         cudaError_t e_ = (x);              \
@@ -71,3 +71,5 @@ int qb_attn_prefill_tc_launch(qb_ctx* ctx, cudaStream_t st, const float* q, cons
 // S carries the offsets' table after the scales) for more than 16 rows
 int qb_gemm_tc_launch(qb_ctx* ctx, cudaStream_t st, const void* X, const void* B, void* Y, const void* S, int m, int n,
                       int k, int row0, int epi, int zp);
+// the scratch of the two products on pairs of blocks (partial tiles, tickets), taken with the first one
+int qb_tc_scratch(qb_ctx* ctx);

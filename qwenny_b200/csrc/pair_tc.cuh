@@ -1,0 +1,117 @@
+// What the W4A16 products on pairs of blocks (tcgen05 cta_group::2) share: descriptors, the product / commit / tensor-memory
+// wrappers, barriers across the pair, the exact unpacking of a Marlin word, and the dealing of (tile, k block) lists.
+#pragma once
+#include <cuda.h>
+#include "common.cuh"
+
+namespace qb {
+namespace tc {
+
+// instruction descriptor of tcgen05.mma kind::f16, M = 256 (a pair of blocks), N = n: D f32 (bits 4-5 = 1), A and B f16
+// (0), both K-major (0), N >> 3 at bits 17-22, M >> 4 at bits 24-28
+__device__ __forceinline__ uint32_t idesc_pair(int n) { return (1u << 4) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(256 >> 4) << 24); }
+
+// shared-memory matrix descriptor of a K-major operand with the 128-byte swizzle: start address >> 4, leading byte
+// offset 1 (unused with a swizzle), stride byte offset 1024 >> 4 (between 8-row groups), descriptor version 1
+// (bit 46), layout type 2 = SWIZZLE_128B (bits 61-63)
+__device__ __forceinline__ uint64_t smem_desc(uint32_t addr) {
+    return (uint64_t)((addr >> 4) & 0x3FFF) | (1ull << 16) | (64ull << 32) | (1ull << 46) | (2ull << 61);
+}
+
+__device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, int x, int y, uint64_t* bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];\n" ::
+            "r"(smem_u32(dst)), "l"(map), "r"(x), "r"(y), "r"(smem_u32(bar))
+        : "memory");
+}
+// four products over consecutive 16-wide steps of k: A 8 tensor-memory columns, B 32 bytes of its 128-byte rows further
+// each time; the first overwrites the accumulator where `accumulate` is 0
+__device__ __forceinline__ void umma2_ts4(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t id, uint32_t accumulate) {
+    asm volatile(
+        "{\n"
+        ".reg .pred p, t;\n"
+        ".reg .b32 a1;\n"
+        ".reg .b64 b1;\n"
+        "setp.ne.b32 p, %4, 0;\n"
+        "setp.eq.b32 t, 0, 0;\n"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n"
+        "add.u32 a1, %1, 8;\n"
+        "add.u64 b1, %2, 2;\n"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], [a1], b1, %3, t;\n"
+        "add.u32 a1, %1, 16;\n"
+        "add.u64 b1, %2, 4;\n"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], [a1], b1, %3, t;\n"
+        "add.u32 a1, %1, 24;\n"
+        "add.u64 b1, %2, 6;\n"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], [a1], b1, %3, t;\n"
+        "}\n" ::"r"(d_tmem), "r"(a_tmem), "l"(bdesc), "r"(id), "r"(accumulate)
+        : "memory");
+}
+// arrives on the barrier at this offset in both blocks of the pair once the products issued so far have completed
+__device__ __forceinline__ void umma2_commit(uint64_t* bar) {
+    asm volatile(
+        "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n" ::"r"(smem_u32(bar)),
+        "h"((uint16_t)3)
+        : "memory");
+}
+// arrive on the first block's barrier. The scopes are the default ones: what is handed over lives in tensor memory
+// (tcgen05.wait::st and fence::before_thread_sync come first) or was written for the tensor core's async proxy (a TMA copy, or
+// stores behind fence.proxy.async); a release at cluster scope here costs a memory barrier of about a microsecond per
+// stage and warp, which made the product 1.7 times slower.
+__device__ __forceinline__ void mbar_arrive_at(uint32_t addr) {
+    asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];\n" ::"r"(addr) : "memory");
+}
+// a 16 x 16 block of halves per k16 step, four steps: lane (g, t) holds rows g and g + 8 of column pairs t and t + 4 of each
+__device__ __forceinline__ void tmem_st_16x128_x8(uint32_t taddr, const uint32_t* r) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.16x128b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};\n" ::"r"(taddr), "r"(r[0]),
+        "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]),
+        "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
+        : "memory");
+}
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t* r) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+        : "r"(taddr));
+}
+// the share of pair b of a grid of g pairs: iterations [share_start(b), share_start(b + 1))
+__device__ __forceinline__ long long share_start(long long iters, int g, int b) { return iters * b / g; }
+__device__ __forceinline__ int share_of(long long iters, int g, long long it) {
+    int b = (int)(it * g / iters);
+    while (b + 1 < g && share_start(iters, g, b + 1) <= it) b++;
+    while (b > 0 && share_start(iters, g, b) > it) b--;
+    return b;
+}
+
+// A pair's work as a list of segments (tile, k blocks [kb0, kb1)); every role of both blocks walks the same list.
+// SHARES: equal contiguous shares of the (tile, k block) list; otherwise pair b takes the whole tiles b, b + grid, ...
+template <bool SHARES>
+struct Walk {
+    long long iters;
+    int tiles, nkb, G, b, j = 0;
+    long long it, it1;
+    __device__ Walk(long long iters_, int tiles_, int nkb_, int G_, int b_) : iters(iters_), tiles(tiles_), nkb(nkb_), G(G_), b(b_) {
+        it = SHARES ? share_start(iters, G, b) : 0;
+        it1 = SHARES ? share_start(iters, G, b + 1) : 0;
+    }
+    __device__ bool next(int& tile, int& kb0, int& kb1) {
+        if (!SHARES) {
+            tile = j * G + b; kb0 = 0; kb1 = nkb; j++;
+            return tile < tiles;
+        }
+        if (it >= it1) return false;
+        tile = (int)(it / nkb); kb0 = (int)(it % nkb); kb1 = (int)min((long long)nkb, kb0 + (it1 - it));
+        it += kb1 - kb0;
+        return true;
+    }
+    // the pairs that hold the parts of a tile cut by this walk: the first one and how many
+    __device__ void parts_of(int tile, int& first, int& parts) const {
+        first = share_of(iters, G, (long long)tile * nkb);
+        parts = share_of(iters, G, (long long)(tile + 1) * nkb - 1) - first + 1;
+    }
+};
+
+}  // namespace tc
+}  // namespace qb

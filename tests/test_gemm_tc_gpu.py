@@ -94,3 +94,22 @@ def test_shares_of_the_tile_list_repeat_and_agree_with_whole_tiles(ctx, m, rows,
     an, cn = a.float().cpu().numpy(), c.float().cpu().numpy()
     assert close(an, want.astype(np.float32)).all() and close(cn, want.astype(np.float32)).all()
     assert np.abs(an - cn).max() <= (2e-3 if silu else 2e-4) * max(1.0, np.abs(want).max())
+
+
+@pytest.mark.parametrize("m", [65, 97, 256, 257, 333])
+def test_token_tile_widths_and_zero_points(ctx, m):
+    """The tile's width follows the row count (96, 128, 256, 2 x 160, 2 x 192 tokens); zero-point matrices take the same path."""
+    g = synth.gen(700 + m)
+    x = synth.activations(m, 384, g)
+    codes, sc = synth.int4_matrix(512, 384, g)
+    zeros = np.random.default_rng(m).integers(4, 13, (512, 3)).astype(np.uint8)
+    words, s16 = host.pack_marlin(codes, sc, zeros=zeros)
+    q, s = R.unpack_marlin(words, s16[:3])
+    off = R.unpack_marlin(words, s16[3:])[1]
+    dev = lambda a: torch.from_numpy(a).cuda()
+    sd = dev(s16.view(np.int16)).view(torch.float16)
+    y = ctx.marlin_gemm(dev(x), dev(words.view(np.int32)), sd, zp=True)
+    torch.cuda.synchronize()
+    assert ctx.device_error() == 0
+    want = R.marlin_gemm(x, R.dequant_z(q, s, off))
+    assert np.abs(y.cpu().numpy() - want).max() < 1e-5 * np.abs(want).max()
