@@ -9,9 +9,11 @@
 // {2t, 2t + 1, 2t + 8, 2t + 9} of a 16 x 16 block, which is exactly what a lane of tcgen05.st.16x128b writes, so the
 // dequantised halves go from registers to tensor memory without touching shared memory. What that buys: the form that
 // wrote them to shared memory (one block per tile, two M = 128 halves re-reading the X tile) moved 169 KB through an SM's
-// shared memory per 1024 cycles of products and was bound by it (tensor pipe 65 % active); this one moves 40 KB per 512.
+// shared memory per 1024 cycles of products and was bound by it (tensor pipe 65 % active); this one moves 80 KB per
+// 1024. A stage is 128 of k because the issuing threads are the next limit: a wait, a commit and their like cost 180 cycles per
+// stage beside 65 per product, and the copying lane 70 per copy (64 of k per stage: 600 cycles of the 512 at N = 256).
 //
-// The work is the list of (tile, k block of 64) pairs, tile after tile. Where whole tiles would leave the last wave
+// The work is the list of (tile, k block of 128) pairs, tile after tile. Where whole tiles would leave the last wave
 // mostly empty, a persistent grid of one pair per two SMs deals the list out in equal contiguous shares (stream-K): a
 // pair that ends or starts inside a tile writes that tile's partial accumulators to scratch and takes a ticket; the
 // tile's last arriver adds the parts in pair order and runs the epilogue, nobody waits. Otherwise a pair is a tile.
@@ -20,8 +22,8 @@
 //               w = f16((q - 8) s), kernels/marlin.cuh:100-124), tcgen05.st into the stage's 32 columns; then they run
 //               the epilogue: tcgen05.ld of the accumulators, Y [token][output] f32, or silu(gate) * up as f16 for
 //               the interleaved SwiGLU matrices (or the partial tile)
-//   warp 8      copies, one lane: the X half tile (tensor map, 128-byte swizzle), the 4 KB of words (tensor map), the
-//               group scales; full/empty mbarriers, a ring of 8 stages
+//   warp 8      copies, one lane: the X half tile (tensor map, 128-byte swizzle), the 8 KB of words (tensor map), the
+//               group's scales; full/empty mbarriers, a ring of 4 stages
 //   warp 9      of the pair's first block: one lane issues the products (K = 16 each), tcgen05.commit hands the stage
 //               back in both blocks when they have read it
 #include "launch.h"
@@ -35,10 +37,11 @@ enum { EPI_PLAIN_TC = 0, EPI_SILU_TC = 1 };
 constexpr int BO = 256;             // outputs per pair of blocks
 constexpr int BH = BO / 2;          // outputs per block: the 128 lanes of its tensor memory
 constexpr int BT = 256;             // most tokens per tile (the product's N); a launch takes the width that divides its rows
-constexpr int BK = 64;              // k per stage: one 128-byte swizzle row of f16
-constexpr int NSTAGE = 8;           // ring depth, in shared memory and in tensor memory (8 x 32 columns + 256 = 512)
-constexpr int X_BYTES = BT / 2 * BK * 2;    // 16 KB: this block's half of the tokens
-constexpr int W_BYTES = BH * BK / 2;        // 4 KB of Marlin words
+constexpr int BK = 128;             // k per stage: two 128-byte swizzle rows of f16, one group of scales
+constexpr int NSTAGE = 4;           // ring depth, in shared memory and in tensor memory (4 x 64 columns + 256 = 512)
+constexpr int XH_BYTES = BT / 2 * 64 * 2;   // 16 KB: this block's half of the tokens, 64 of k
+constexpr int X_BYTES = 2 * XH_BYTES;
+constexpr int W_BYTES = BH * BK / 2;        // 8 KB of Marlin words
 constexpr int S_BYTES = 512;                // 128 f16 scales, then (zero-point matrices) their offsets (8 - z) * scale
 constexpr int SMEM_BYTES = NSTAGE * (X_BYTES + W_BYTES + S_BYTES) + 1024 /* barriers, tmem address */ + 1024 /* alignment slack */;
 constexpr int DQ_WARPS = 8, DQ_GROUPS = DQ_WARPS / 4;  // a group of four warps dequantises a stage; the groups take turns
@@ -122,10 +125,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
                     }
                     mbar_expect_tx(&full[s], bytes);
                     tma_load_2d(smem + s * X_BYTES, &xmap, kb * BK, tok0, &full[s]);
+                    tma_load_2d(smem + s * X_BYTES + XH_BYTES, &xmap, kb * BK + 64, tok0, &full[s]);
                     tma_load_2d(wsmem + s * W_BYTES, &wmap, n0, kb * (BK / 16), &full[s]);
-                    bulk_g2s(ssmem + s * S_BYTES, a.S + (size_t)(kb / 2) * a.N + n0, BH * 2, &full[s], pol);
+                    bulk_g2s(ssmem + s * S_BYTES, a.S + (size_t)kb * a.N + n0, BH * 2, &full[s], pol);
                     if (a.zp)
-                        bulk_g2s(ssmem + s * S_BYTES + BH * 2, a.S + (size_t)(a.K / 128 + kb / 2) * a.N + n0, BH * 2, &full[s], pol);
+                        bulk_g2s(ssmem + s * S_BYTES + BH * 2, a.S + (size_t)(a.K / 128 + kb) * a.N + n0, BH * 2, &full[s], pol);
                 }
             }
             if (!ok) atomicExch(a.err, 5);
@@ -150,24 +154,25 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
                     if (dead && lane == 0) atomicExch(a.err, 6);
                 }
                 asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");  // (the slot's earlier products have read it)
-                // words [k16 4][c64 2][lane 32] x 4 blocks; this warp's: c64 q / 2, blocks 2 (q % 2) + b
+                // words [k16 8][c64 2][lane 32] x 4 blocks; this warp's: c64 q / 2, blocks 2 (q % 2) + b
                 const uint8_t* wp = wsmem + s * W_BYTES + (q >> 1) * 512 + lane * 16 + (q & 1) * 8;
-                uint2 w[4];
+                uint2 w[8];
 #pragma unroll
-                for (int j = 0; j < 4; j++) w[j] = *(const uint2*)(wp + j * 1024);
+                for (int j = 0; j < 8; j++) w[j] = *(const uint2*)(wp + j * 1024);
                 // scales of outputs 16 b + g + 8 i of a c64 at 8 g + 2 b + i
                 const __half* sp = (const __half*)(ssmem + s * S_BYTES) + (q >> 1) * 64 + 8 * g + 4 * (q & 1);
                 const uint2 s4 = *(const uint2*)sp;
                 uint2 z4 = make_uint2(0u, 0u);  // the offsets (0: the symmetric form)
                 if (a.zp) z4 = *(const uint2*)(sp + BH);
 #pragma unroll
-                for (int b = 0; b < 2; b++) {
+                for (int bh = 0; bh < 4; bh++) {  // 16-row block b, k half hf of the stage
+                    const int b = bh & 1, hf = bh >> 1;
                     const __half2 sc = *(const __half2*)(b ? &s4.y : &s4.x), zc = *(const __half2*)(b ? &z4.y : &z4.x);
                     const __half2 s0 = __low2half2(sc), s1 = __high2half2(sc), z0 = __low2half2(zc), z1 = __high2half2(zc);
                     uint32_t r[16];
 #pragma unroll
                     for (int j = 0; j < 4; j++) {
-                        const uint32_t qw = b ? w[j].y : w[j].x, q8 = qw >> 8;
+                        const uint32_t qw = b ? w[4 * hf + j].y : w[4 * hf + j].x, q8 = qw >> 8;
                         uint32_t lo0, hi0, lo1, hi1;
                         asm("lop3.b32 %0, %1, 0x000f000f, 0x64006400, 0xea;\n" : "=r"(lo0) : "r"(qw));
                         asm("lop3.b32 %0, %1, 0x00f000f0, 0x54005400, 0xea;\n" : "=r"(hi0) : "r"(qw));
@@ -183,7 +188,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
                         r[4 * j] = *(uint32_t*)&v0; r[4 * j + 1] = *(uint32_t*)&v1;
                         r[4 * j + 2] = *(uint32_t*)&v2; r[4 * j + 3] = *(uint32_t*)&v3;
                     }
-                    tmem_st_16x128_x8(tmem_a + s * A_COLS + quarter + ((uint32_t)(16 * b) << 16), r);
+                    tmem_st_16x128_x8(tmem_a + s * A_COLS + 32 * hf + quarter + ((uint32_t)(16 * b) << 16), r);
                 }
                 asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory");
                 asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
@@ -297,6 +302,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
                     if (!ok) break;
                     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
                     umma2_ts4(tmem, tmem_a + s * A_COLS, smem_desc(xs + s * X_BYTES), id, kb > kb0 ? 1u : 0u);
+                    umma2_ts4(tmem, tmem_a + s * A_COLS + 32, smem_desc(xs + s * X_BYTES + XH_BYTES), id, 1u);
                     umma2_commit(&empty[s]);
                 }
                 if (ok) umma2_commit(done);
@@ -347,12 +353,12 @@ int qb_gemm_tc_launch(qb_ctx* ctx, cudaStream_t st, const void* X, const void* B
     CUtensorMap xmap, wmap;
     const cuuint32_t one[2] = {1, 1};
     const cuuint64_t xd[2] = {(cuuint64_t)k, (cuuint64_t)m}, xs[1] = {(cuuint64_t)k * 2};
-    const cuuint32_t xb[2] = {tc::BK, (cuuint32_t)(bt / 2)};
+    const cuuint32_t xb[2] = {64, (cuuint32_t)(bt / 2)};
     void* base = (void*)((const __half*)X + (size_t)row0 * k);
     if (enc(&xmap, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, base, xd, xs, xb, one, CU_TENSOR_MAP_INTERLEAVE_NONE,
             CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
         return QB_ERR_ARG;
-    // the words: K/16 rows of 2N words = N 8-byte elements; a stage's box: 128 outputs x 4 rows
+    // the words: K/16 rows of 2N words = N 8-byte elements; a stage's box: 128 outputs x 8 rows
     const cuuint64_t wd[2] = {(cuuint64_t)n, (cuuint64_t)(k / 16)}, ws[1] = {(cuuint64_t)n * 8};
     const cuuint32_t wb[2] = {tc::BH, tc::BK / 16};
     if (enc(&wmap, CU_TENSOR_MAP_DATA_TYPE_UINT64, 2, (void*)B, wd, ws, wb, one, CU_TENSOR_MAP_INTERLEAVE_NONE,
