@@ -73,3 +73,6 @@ int qb_gemm_tc_launch(qb_ctx* ctx, cudaStream_t st, const void* X, const void* B
                       int k, int row0, int epi, int zp);
 // the scratch of the two products on pairs of blocks (partial tiles, tickets), taken with the first one
 int qb_tc_scratch(qb_ctx* ctx);
+// the product for 17 .. 64 rows (w4a16_gemm_mid.cu), symmetric matrices; reached through qb_marlin_gemm
+int qb_gemm_mid_launch(qb_ctx* ctx, cudaStream_t st, const void* X, const void* B, void* Y, const void* S, int m, int n, int k,
+                       int row0, int epi, const int* xrows, unsigned long long* keys, int n_valid);

@@ -254,6 +254,17 @@ static int gemm_rows(qb_ctx* ctx, cudaStream_t st, const void* X, const void* B,
 #undef QB_GO
 }
 
+// The product for 17 .. 64 rows needs the pair products' scratch, which the first one allocates. Where that cannot be had (no
+// memory left, a stream being captured) the rows run as 16-row slabs, which need nothing.
+static bool pair_scratch(qb_ctx* ctx, cudaStream_t st) {
+    if (ctx->tc_part) return true;
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) return false;
+    if (qb_tc_scratch(ctx) == QB_OK) return true;
+    (void)cudaGetLastError();
+    return false;
+}
+
 extern "C" int qb_marlin_gemm(qb_ctx* ctx, void* stream, const void* X, const void* B, void* Y, const void* S, int m,
                               int n, int k, int row0, int epi, const int* xrows, unsigned long long* keys,
                               int n_valid) {
@@ -262,12 +273,26 @@ extern "C" int qb_marlin_gemm(qb_ctx* ctx, void* stream, const void* X, const vo
     if (epi == QB_EPI_SILU && (n % 16)) return QB_ERR_ARG;
     if (epi < 0 || epi > QB_EPI_ARGMAX) return QB_ERR_ARG;
     cudaStream_t st = (cudaStream_t)stream;
-    // more than 16 rows: the tensor-core product (plain and SwiGLU epilogues, contiguous rows)
-    if (m > 16 && epi != QB_EPI_ARGMAX && !xrows && !ctx->no_tc)
+    // more than 64 rows, plain and SwiGLU epilogues, contiguous: the prompt-sized tensor-core product
+    if (m > 64 && epi != QB_EPI_ARGMAX && !xrows && !ctx->no_tc)
         return qb_gemm_tc_launch(ctx, st, X, B, Y, S, m, n, k, row0, epi, 0);
-    // otherwise 16-row slabs through the skinny kernel
-    for (int r = 0; r < m; r += 16) {
-        int mm = m - r < 16 ? m - r : 16;
+    // slabs: 17 .. 64 rows through the tensor-core product for a few rows, up to 16 through the skinny kernel. At 16 rows the
+    // skinny kernel takes 22, 11, 31 and 24 us over the layer's four shapes, at 17 the other 28, 20, 48 and 32 (two skinny
+    // slabs 43, 22, 62 and 48); at 64 rows 31, 24, 51 and 36 us, the prompt-sized product at 65 25, 25, 47 and 37. Before,
+    // 17 .. 64 rows padded to 256 tokens took 68, 68, 69 and 89 us, and 40 gathered rows of a 248,320-row output layer
+    // as three 16-row slabs 577 us (320 now).
+    int mm;
+    for (int r = 0; r < m; r += mm) {
+        mm = m - r;
+        if (mm > 16 && !ctx->no_tc && pair_scratch(ctx, st)) {
+            if (mm > 64) mm = 64;
+            int rc = qb_gemm_mid_launch(ctx, st, X, B, Y, S, mm, n, k, xrows ? 0 : row0 + r, epi, xrows ? xrows + r : nullptr,
+                                        keys ? keys + (xrows ? r : 0) : nullptr, n_valid);
+            if (rc) return rc;
+            if (xrows) Y = (char*)Y + (size_t)mm * (epi == QB_EPI_SILU ? n / 2 * 2 : (size_t)n * 4);
+            continue;
+        }
+        if (mm > 16) mm = 16;
         int rc = gemm_rows(ctx, st, X, B, Y, S, mm, n, k, xrows ? 0 : row0 + r, epi, xrows ? xrows + r : nullptr,
                            keys ? keys + (xrows ? r : 0) : nullptr, n_valid);
         if (rc) return rc;

@@ -1,0 +1,406 @@
+// W4A16 product for 17 .. 64 token rows (several sequences' verify steps, short prompt pieces, the output layer over a
+// batch) on the 5th-generation tensor cores: Y = X . W^T with W int4 in Marlin's layout, plain, SwiGLU or argmax epilogue,
+// contiguous or gathered rows.
+//
+// Bound by the weights' way from HBM (0.52 bytes each, read once) as long as the products keep up. A block owns 128 outputs and
+// the weights go from registers to tensor memory in the layout that a Marlin word already has (w4a16_gemm_tc.cu), but
+// not as a pair of blocks: with A in tensor memory a K = 16 product of M = 256 over a pair takes 128 cycles whatever its N,
+// one of M = 128 some 50 cycles for any N up to 64: 400 per 128-wide k block, against 380 for the block's 8 KB at the
+// measured copy bandwidth. (As pairs: 40 rows x 34816 x 5120 in 62 us.) What else differs from the prompt-sized product:
+//   - the weights are the exact integers q - 8; a group of 128 columns is one accumulation, and the drain warps multiply its
+//     f32 sums by the f32 value of the group's scale and add them up in registers (one thread per output, a register
+//     per token): one rounding per group, the arithmetic of the product for up to 16 rows (w4a16_gemv.cuh), where
+//     f16((q - 8) s) would round every weight. Two accumulators take turns, each with an issuing thread of its own (a
+//     wait, eight products and two commits take one thread longer than the products themselves)
+//   - the rows are few: they are loaded per k block into the swizzled layout by cp.async (which also gathers), or by the
+//     tensor map when they are contiguous
+// The (tile, group) list is dealt to one block per SM in equal shares; parts of a cut tile are added by its last arriver in
+// block order (the bits repeat).
+#include "launch.h"
+#include "pair_tc.cuh"
+
+namespace qb {
+namespace mid {
+
+using namespace tc;
+
+constexpr int BH = 128;             // outputs per block
+constexpr int BK = 128;             // k per stage: a group of scales
+constexpr int NSTAGE = 8;           // stages in shared memory (words, X): a copy takes some 2000 cycles, a stage's products 400
+constexpr int NA = 4;               // stages in tensor memory (64 columns each)
+constexpr int NS = 16;              // groups in the ring of scales: those of the ring's stages and of the two being drained
+constexpr int W_BYTES = BH * BK / 2;
+constexpr int DQ_WARPS = 8, DQ_GROUPS = DQ_WARPS / 4;  // a group of four warps unpacks a stage, the groups take turns
+constexpr int X_WARPS = 2;
+constexpr int TMEM_COLS = 512;
+template <int NT>
+struct Cfg {
+    static constexpr int DR_WARPS = 4 * ((NT + 31) / 32);  // a drain warp: 32 outputs x 32 tokens
+    static constexpr int COPY_WARP = DQ_WARPS + DR_WARPS, MMA_WARP = COPY_WARP + 1, X_WARP = COPY_WARP + 3;
+    static constexpr int THREADS = (X_WARP + X_WARPS) * 32;
+    static constexpr int XH = NT * 64 * 2, XB = 2 * XH;  // the tokens, 64 of k; a stage
+    static constexpr int SMEM = NSTAGE * (XB + W_BYTES) + NS * BH * 2 + 1024 + 1024;
+    static_assert(XH % 1024 == 0, "swizzled tiles want 1 KB");
+};
+
+struct Args {
+    const __half* X;
+    const int* xrows;    // gathered rows of X, or null: rows row0 ..
+    const __half* S;     // scales [K/128][N]
+    void* Y;             // plain / argmax: f32 [.][N]; silu: f16 [.][N/2]; rows y0 ..
+    unsigned long long* keys;
+    int m, N, K, row0, y0, n_valid;
+    int* err;
+    float* part;         // [block][2][NT][BH]
+    int* tickets;
+    long long iters;     // tiles x groups
+    int tiles;
+};
+
+template <int NT, int EPI>
+__global__ void __launch_bounds__(Cfg<NT>::THREADS, 1)
+    w4a16_gemm_mid_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap wmap, const Args a) {
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+    using C = Cfg<NT>;
+    constexpr int XB = C::XB, DR_WARPS = C::DR_WARPS, COPY_WARP = C::COPY_WARP, MMA_WARP = C::MMA_WARP, X_WARP = C::X_WARP;
+    uint8_t* wsmem = smem + NSTAGE * XB;
+    __half* ssmem = (__half*)(wsmem + NSTAGE * W_BYTES);
+    uint64_t* full = (uint64_t*)(ssmem + NS * BH);  // a stage's copies landed in this block
+    uint64_t* aready = full + NSTAGE;    // its weights are in tensor memory
+    uint64_t* empty = aready + NSTAGE;   // its products are done
+    uint64_t* sfull = empty + NSTAGE;    // a group's scales landed in this block
+    uint64_t* dfull = sfull + NS;        // a group's accumulator is complete
+    uint64_t* dfree = dfull + 2;         // it has been drained
+    uint32_t* tmem_slot = (uint32_t*)(dfree + 2);
+    int* flag = (int*)(tmem_slot + 1);
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int ngr = a.K / 128;
+    const bool gathered = a.xrows != nullptr;
+    Walk<true> walk(a.iters, a.tiles, ngr, gridDim.x, blockIdx.x);
+    int tile, g0, g1;
+
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < NSTAGE; i++) {
+            mbar_init(&full[i], gathered ? 1 + X_WARPS : 1);
+            mbar_init(&aready[i], 4);
+            mbar_init(&empty[i], 1);
+        }
+        for (int i = 0; i < NS; i++) mbar_init(&sfull[i], 1);
+        for (int i = 0; i < 2; i++) { mbar_init(&dfull[i], 1); mbar_init(&dfree[i], DR_WARPS); }
+        mbar_fence_init();
+    }
+    if (warp == MMA_WARP) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(tmem_slot)),
+                     "r"(TMEM_COLS));
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+    const uint32_t tmem = *tmem_slot, tmem_a = tmem + 256;  // accumulators at columns 0 and 128, weights from 256 on
+    pdl_launch_dependents();
+
+    // every role walks the same segments (tile, groups [g0, g1)); st counts stages, gr groups, from the start
+    if (warp == COPY_WARP) {
+        if (lane == 0) {
+            const uint64_t pol = policy_evict_first();
+            bool ok = true, waited = false;
+            uint32_t st = 0;
+            while (ok && walk.next(tile, g0, g1)) {
+                const int n0 = tile * BH;
+                for (int gi = g0; gi < g1; gi++, st++) {
+                    // (the scales' slot: the group NS before this one was drained long ago: this stage waits for products
+                    // that came after the reuse of its accumulator)
+                    const int s = (int)(st % NSTAGE), sl = (int)(st % NS);
+                    if (st >= NSTAGE) {
+                        ok = mbar_wait(&empty[s], ((st / NSTAGE) - 1) & 1);
+                        if (!ok) break;
+                    }
+                    mbar_expect_tx(&full[s], W_BYTES + (gathered ? 0 : XB));
+                    tma_load_2d(wsmem + s * W_BYTES, &wmap, n0, gi * (BK / 16), &full[s]);
+                    mbar_expect_tx(&sfull[sl], BH * 2);
+                    bulk_g2s(ssmem + sl * BH, a.S + (size_t)gi * a.N + n0, BH * 2, &sfull[sl], pol);
+                    if (!gathered) {
+                        if (!waited) { pdl_wait(); waited = true; }  // the weights above do not depend on the kernel before
+                        tma_load_2d(smem + s * XB, &xmap, gi * BK, 0, &full[s]);
+                        tma_load_2d(smem + s * XB + C::XH, &xmap, gi * BK + 64, 0, &full[s]);
+                    }
+                }
+            }
+            if (!waited) pdl_wait();
+            if (!ok) atomicExch(a.err, 9);
+        }
+        __syncwarp();
+    } else if (warp >= X_WARP) {
+        // ---------------------------------------------------------------- gathered rows: cp.async into the swizzled rows
+        if (gathered) {
+            pdl_wait();
+            constexpr int PER = NT * 16 / (X_WARPS * 32);  // 16-byte chunks per lane and stage
+            static_assert(PER * X_WARPS * 32 == NT * 16, "chunks divide the loading lanes");
+            const int xl = threadIdx.x - X_WARP * 32;
+            const int ch = xl & 15, r0 = xl >> 4;  // this lane: 16-byte chunk ch of rows r0, r0 + 4, ..
+            uint32_t row[PER];
+#pragma unroll
+            for (int i = 0; i < PER; i++) row[i] = (uint32_t)a.xrows[min(4 * i + r0, a.m - 1)];  // (rows past the last are never written)
+            const uint32_t even = (uint32_t)((ch >> 3) * C::XH + r0 * 128 + (((ch & 7) ^ r0) << 4)),
+                           odd = (uint32_t)((ch >> 3) * C::XH + (r0 + 4) * 128 + (((ch & 7) ^ (r0 + 4)) << 4));
+            bool ok = true;
+            uint32_t st = 0;
+            // a stage is handed over once the copies of the two after it are under way
+            auto hand = [&](uint32_t n) {
+                asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&full[n % NSTAGE]);
+            };
+            while (walk.next(tile, g0, g1)) {
+                for (int kb = g0; kb < g1; kb++, st++) {
+                    const int s = (int)(st % NSTAGE);
+                    if (st >= NSTAGE && ok) {
+                        if (lane == 0) ok = mbar_wait(&empty[s], ((st / NSTAGE) - 1) & 1);
+                        ok = __shfl_sync(0xffffffffu, ok, 0);
+                        if (!ok && lane == 0) atomicExch(a.err, 9);
+                    }
+                    if (ok) {
+#pragma unroll
+                        for (int i = 0; i < PER; i++) cp_async16(smem + s * XB + (i >> 1) * 1024 + (i & 1 ? odd : even), a.X + (size_t)row[i] * a.K + kb * BK + ch * 8);
+                    }
+                    cp_async_commit();
+                    if (st > 1) {
+                        asm volatile("cp.async.wait_group 2;\n" ::: "memory");
+                        hand(st - 2);
+                    }
+                }
+            }
+            asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+            if (st > 1) hand(st - 2);
+            if (st > 0) hand(st - 1);
+        }
+    } else if (warp < DQ_WARPS) {
+        // ---------------------------------------------------------------- q - 8 into tensor memory
+        const int q = warp & 3, h = warp >> 2;
+        const uint32_t quarter = (uint32_t)(q * 32) << 16;
+        bool dead = false;
+        uint32_t st = 0;
+        while (walk.next(tile, g0, g1)) {
+            for (int kb = g0; kb < g1; kb++, st++) {
+                if ((int)(st % DQ_GROUPS) != h) continue;
+                const int s = (int)(st % NSTAGE);
+                if (!dead) {
+                    dead = !mbar_wait(&full[s], (st / NSTAGE) & 1);
+                    // (the tensor-memory slot: the products of the stage NA before have read it)
+                    if (!dead && st >= NA) dead = !mbar_wait(&empty[(st - NA) % NSTAGE], ((st - NA) / NSTAGE) & 1);
+                    if (dead && lane == 0) atomicExch(a.err, 10);
+                }
+                asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+                const int sa = (int)(st % NA);
+                const uint8_t* wp = wsmem + s * W_BYTES + (q >> 1) * 512 + lane * 16 + (q & 1) * 8;
+                uint2 w[8];
+#pragma unroll
+                for (int j = 0; j < 8; j++) w[j] = *(const uint2*)(wp + j * 1024);
+#pragma unroll
+                for (int bh = 0; bh < 4; bh++) {  // 16-row block b, k half hf of the stage
+                    const int b = bh & 1, hf = bh >> 1;
+                    uint32_t r[16];
+#pragma unroll
+                    for (int j = 0; j < 4; j++) {
+                        const uint32_t qw = b ? w[4 * hf + j].y : w[4 * hf + j].x, q8 = qw >> 8;
+                        uint32_t lo0, hi0, lo1, hi1;
+                        asm("lop3.b32 %0, %1, 0x000f000f, 0x64006400, 0xea;\n" : "=r"(lo0) : "r"(qw));
+                        asm("lop3.b32 %0, %1, 0x00f000f0, 0x54005400, 0xea;\n" : "=r"(hi0) : "r"(qw));
+                        asm("lop3.b32 %0, %1, 0x000f000f, 0x64006400, 0xea;\n" : "=r"(lo1) : "r"(q8));
+                        asm("lop3.b32 %0, %1, 0x00f000f0, 0x54005400, 0xea;\n" : "=r"(hi1) : "r"(q8));
+                        const uint32_t SUB_LO = 0x64086408u, SUB_HI = 0x54805480u;
+                        __half2 v0 = __hsub2(*(__half2*)&lo0, *(const __half2*)&SUB_LO), v1 = __hsub2(*(__half2*)&lo1, *(const __half2*)&SUB_LO);
+                        __half2 v2 = __hsub2(*(__half2*)&hi0, *(const __half2*)&SUB_HI), v3 = __hsub2(*(__half2*)&hi1, *(const __half2*)&SUB_HI);
+                        r[4 * j] = *(uint32_t*)&v0; r[4 * j + 1] = *(uint32_t*)&v1;
+                        r[4 * j + 2] = *(uint32_t*)&v2; r[4 * j + 3] = *(uint32_t*)&v3;
+                    }
+                    tmem_st_16x128_x8(tmem_a + sa * (BK / 2) + 32 * hf + quarter + ((uint32_t)(16 * b) << 16), r);
+                }
+                asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory");
+                asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&aready[s]);
+            }
+        }
+    } else if (warp < COPY_WARP) {
+        // ---------------------------------------------------------------- drain the groups, then the epilogue
+        const int q = warp & 3, lrow = q * 32 + lane, t0 = (warp - DQ_WARPS) / 4 * 32;  // this warp's outputs and tokens
+        const uint32_t tq = tmem + ((uint32_t)(q * 32) << 16) + t0;
+        bool dead = false;
+        uint32_t gr = 0;
+        unsigned long long best = 0;  // argmax: lane l holds the best key of token t0 + l over this warp's outputs
+        pdl_wait();
+        while (walk.next(tile, g0, g1)) {
+            const int orow = tile * BH + lrow;
+            float acc[32];
+#pragma unroll
+            for (int j = 0; j < 32; j++) acc[j] = 0.f;
+#pragma unroll 1
+            for (int gi = g0; gi < g1; gi++, gr++) {
+                const int p = (int)(gr & 1), sl = (int)(gr % NS);
+                if (!dead) {
+                    dead = !mbar_wait(&sfull[sl], (gr / NS) & 1) || !mbar_wait(&dfull[p], (gr >> 1) & 1);
+                    if (dead && lane == 0) atomicExch(a.err, 11);
+                }
+                asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+                // scale of output 16 b + 8 i + r of a c64 at 8 r + 2 b + i
+                const float sc = __half2float(ssmem[sl * BH + (lrow >> 6) * 64 + 8 * (lrow & 7) + ((lrow & 63) >> 3)]);
+                uint32_t v[32];
+                tmem_ld32(tq + p * 128, v);
+                asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+                asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&dfree[p]);
+#pragma unroll
+                for (int j = 0; j < 32; j++) acc[j] = fmaf(sc, __uint_as_float(v[j]), acc[j]);
+            }
+            bool finish = !dead;
+            if (g0 > 0 || g1 < ngr) {
+                int parts, first;
+                walk.parts_of(tile, first, parts);
+                float* slot = a.part + ((size_t)blockIdx.x * 2 + (g0 == 0 ? 1 : 0)) * (NT * BH) + t0 * BH + lrow;
+#pragma unroll
+                for (int j = 0; j < 32; j++)
+                    if (t0 + j < a.m) slot[j * BH] = acc[j];
+                __threadfence();
+                named_bar_sync(1, DR_WARPS * 32);
+                if (threadIdx.x == DQ_WARPS * 32) {
+                    const int tk = atomicAdd(&a.tickets[tile], 1);
+                    *flag = tk == parts - 1;
+                    if (tk == parts - 1) a.tickets[tile] = 0;
+                }
+                named_bar_sync(1, DR_WARPS * 32);
+                finish = *flag != 0 && !dead;
+                named_bar_sync(1, DR_WARPS * 32);
+                if (finish) {
+                    __threadfence();
+#pragma unroll
+                    for (int j = 0; j < 32; j++) acc[j] = 0.f;
+#pragma unroll 1
+                    for (int pt = 0; pt < parts; pt++) {
+                        const float* o = a.part + ((size_t)(first + pt) * 2 + (pt == 0 ? 1 : 0)) * (NT * BH) + t0 * BH + lrow;
+#pragma unroll
+                        for (int j = 0; j < 32; j++)
+                            if (t0 + j < a.m) acc[j] += __ldcg(o + j * BH);
+                    }
+                }
+            }
+            if (!finish) continue;
+            if (EPI == QB_EPI_SILU) {
+                // packed rows 16 p + i are gate rows, 16 p + 8 + i their up rows, 8 lanes on
+                const bool up_lane = (lane & 8) != 0;
+#pragma unroll
+                for (int j = 0; j < 32; j += 2) {
+                    const float other = __shfl_xor_sync(0xffffffffu, up_lane ? acc[j] : acc[j + 1], 8);
+                    const float gate = up_lane ? other : acc[j], up = up_lane ? acc[j + 1] : other;
+                    const int tok = t0 + j + (up_lane ? 1 : 0);
+                    if (tok < a.m)
+                        ((__half*)a.Y)[(size_t)(a.y0 + tok) * (a.N / 2) + (orow >> 4) * 8 + (orow & 7)] = __float2half_rn(silu(gate) * up);
+                }
+            } else {
+#pragma unroll
+                for (int j = 0; j < 32; j++)
+                    if (t0 + j < a.m) ((float*)a.Y)[(size_t)(a.y0 + t0 + j) * a.N + orow] = acc[j];
+                if (EPI == QB_EPI_ARGMAX) {
+                    const bool valid = orow < a.n_valid;
+                    const unsigned any = __ballot_sync(0xffffffffu, valid);
+                    if (any) {
+#pragma unroll
+                        for (int j = 0; j < 32; j++) {
+                            const unsigned u = valid ? ordered(acc[j]) : 0u, mx = __reduce_max_sync(0xffffffffu, u);
+                            const int at = __ffs(__ballot_sync(0xffffffffu, valid && u == mx)) - 1;
+                            const unsigned long long key =
+                                ((unsigned long long)mx << 32) | (0xffffffffu - (uint32_t)(orow - lane + at));
+                            if (lane == j && key > best) best = key;
+                        }
+                    }
+                }
+            }
+        }
+        if (EPI == QB_EPI_ARGMAX && best && t0 + lane < a.m) atomicMax(a.keys + a.y0 + t0 + lane, best);
+    } else {
+        // ---------------------------------------------------------------- the products: one lane per accumulator
+        if (lane == 0) {
+            const int p = warp - MMA_WARP;
+            bool ok = true;
+            uint32_t st = 0;
+            const uint32_t xs = smem_u32(smem), d = tmem + p * 128;
+            while (ok && walk.next(tile, g0, g1)) {
+                for (int gi = g0; gi < g1; gi++, st++) {
+                    if ((int)(st & 1) != p) continue;
+                    const int s = (int)(st % NSTAGE);
+                    const uint32_t at = tmem_a + (int)(st % NA) * (BK / 2);
+                    if (st >= 2) ok = mbar_wait(&dfree[p], ((st >> 1) - 1) & 1);
+                    ok = ok && mbar_wait(&aready[s], (st / NSTAGE) & 1);
+                    if (!ok) break;
+                    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+                    umma_ts4(d, at, smem_desc(xs + s * XB), idesc(NT), 0u);
+                    umma_ts4(d, at + 32, smem_desc(xs + s * XB + C::XH), idesc(NT), 1u);
+                    umma_commit(&empty[s]);
+                    umma_commit(&dfull[p]);
+                }
+            }
+            if (!ok) atomicExch(a.err, 12);
+        }
+        __syncwarp();
+    }
+
+    asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+    __syncthreads();
+    if (warp == MMA_WARP) {
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(TMEM_COLS));
+    }
+}
+
+template <int NT>
+int go(qb_ctx* ctx, cudaStream_t st, int epi, int G, const CUtensorMap& xmap, const CUtensorMap& wmap, const Args& a) {
+    const dim3 grid(G), block(Cfg<NT>::THREADS);
+    switch (epi) {
+        case QB_EPI_PLAIN: return launch(ctx, w4a16_gemm_mid_kernel<NT, QB_EPI_PLAIN>, grid, block, Cfg<NT>::SMEM, st, xmap, wmap, a);
+        case QB_EPI_SILU: return launch(ctx, w4a16_gemm_mid_kernel<NT, QB_EPI_SILU>, grid, block, Cfg<NT>::SMEM, st, xmap, wmap, a);
+        default: return launch(ctx, w4a16_gemm_mid_kernel<NT, QB_EPI_ARGMAX>, grid, block, Cfg<NT>::SMEM, st, xmap, wmap, a);
+    }
+}
+
+}  // namespace mid
+}  // namespace qb
+
+using namespace qb;
+
+// 1 .. 64 rows of X (row0 .., or xrows[0 .. m)); results at rows y0 .. of Y; keys[y0 .. y0 + m) for the argmax epilogue
+int qb_gemm_mid_launch(qb_ctx* ctx, cudaStream_t st, const void* X, const void* B, void* Y, const void* S, int m, int n, int k,
+                       int row0, int epi, const int* xrows, unsigned long long* keys, int n_valid) {
+    if (n % mid::BH || k % 128 || m < 1 || m > 64) return QB_ERR_ARG;
+    EncodeTiled enc = encode_tiled();
+    if (!enc) return QB_ERR_UNSUPPORTED;
+    const int nt = m <= 32 ? 32 : m <= 48 ? 48 : 64;
+    const int tiles = n / mid::BH;
+    if (tiles > QB_TC_TICKETS) return QB_ERR_ARG;
+    CUtensorMap xmap = {}, wmap;
+    const cuuint32_t one[2] = {1, 1};
+    if (!xrows) {
+        const cuuint64_t xd[2] = {(cuuint64_t)k, (cuuint64_t)m}, xs[1] = {(cuuint64_t)k * 2};
+        const cuuint32_t xb[2] = {64, (cuuint32_t)nt};
+        if (enc(&xmap, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, (void*)((const __half*)X + (size_t)row0 * k), xd, xs, xb, one,
+                CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+            return QB_ERR_ARG;
+    }
+    const cuuint64_t wd[2] = {(cuuint64_t)n, (cuuint64_t)(k / 16)}, ws[1] = {(cuuint64_t)n * 8};
+    const cuuint32_t wb[2] = {mid::BH, mid::BK / 16};
+    if (enc(&wmap, CU_TENSOR_MAP_DATA_TYPE_UINT64, 2, (void*)B, wd, ws, wb, one, CU_TENSOR_MAP_INTERLEAVE_NONE,
+            CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+        return QB_ERR_ARG;
+    if (int rc = qb_tc_scratch(ctx)) return rc;
+    mid::Args a;
+    a.X = (const __half*)X; a.xrows = xrows; a.S = (const __half*)S; a.Y = Y; a.keys = keys; a.m = m; a.N = n; a.K = k;
+    a.row0 = row0; a.y0 = xrows ? 0 : row0; a.n_valid = n_valid; a.err = ctx->err; a.part = ctx->tc_part;
+    a.tickets = ctx->tc_tickets; a.iters = (long long)tiles * (k / 128); a.tiles = tiles;
+    const int G = (int)(a.iters < ctx->sms ? a.iters : ctx->sms);
+    if (nt == 32) return mid::go<32>(ctx, st, epi, G, xmap, wmap, a);
+    if (nt == 48) return mid::go<48>(ctx, st, epi, G, xmap, wmap, a);
+    return mid::go<64>(ctx, st, epi, G, xmap, wmap, a);
+}

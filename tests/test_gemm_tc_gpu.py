@@ -96,6 +96,47 @@ def test_shares_of_the_tile_list_repeat_and_agree_with_whole_tiles(ctx, m, rows,
     assert np.abs(an - cn).max() <= (2e-3 if silu else 2e-4) * max(1.0, np.abs(want).max())
 
 
+@pytest.mark.parametrize("m,rows,cols", [(17, 256, 128), (32, 512, 384), (33, 256, 640), (40, 1024, 2048), (63, 768, 256),
+                                         (64, 2048, 1152), (70, 512, 512), (130, 256, 256)])
+def test_few_rows_gathered_argmax_vs_oracle(ctx, m, rows, cols):
+    """17 .. 64 rows (and slabs of 64 beyond): edges of the token tile, one group of k and many, gathered rows in any order
+    with repeats, the greedy key over part of the outputs. The sums are f32 of exact products, scaled once per group of
+    128: an error of at most k / 16 roundings of partial sums, far below 1e-5 of the largest result here."""
+    x, wdq, xd, wd, sd = make(rows, cols, False, 500 + m, m + 5)
+    order = np.random.default_rng(m).integers(0, m + 5, m).astype(np.int32)
+    valid = rows - 100
+    keys = torch.zeros(m, dtype=torch.int64, device="cuda")
+    y = ctx.marlin_gemm(xd, wd, sd, epi="argmax", xrows=torch.from_numpy(order).cuda(), keys=keys, n_valid=valid)
+    torch.cuda.synchronize()
+    assert ctx.device_error() == 0
+    want = R.marlin_gemm(x[order], wdq)
+    a = y.cpu().numpy()
+    assert np.abs(a - want).max() < 1e-5 * np.abs(want).max()
+    assert (keys.cpu().numpy().view(np.uint64) == R.argmax_keys(a, valid)).all()
+    again = torch.zeros_like(keys)
+    assert torch.equal(y, ctx.marlin_gemm(xd, wd, sd, epi="argmax", xrows=torch.from_numpy(order).cuda(), keys=again, n_valid=valid))
+    assert torch.equal(keys, again)
+
+
+@pytest.mark.parametrize("m,rows,cols", [(17, 256, 128), (40, 1024, 640), (64, 512, 1024)])
+def test_few_rows_contiguous_from_row0(ctx, m, rows, cols):
+    x, wdq, xd, wd, sd = make(rows, cols, True, 600 + m, m + 20)
+    y = torch.zeros(m + 20, rows // 2, dtype=torch.float16, device="cuda")
+    ctx.marlin_gemm(xd, wd, sd, epi="silu", y=y, row0=7, m=m)
+    p = torch.zeros(m + 20, rows, device="cuda")
+    keys = torch.zeros(m + 20, dtype=torch.int64, device="cuda")
+    ctx.marlin_gemm(xd, wd, sd, epi="argmax", y=p, row0=7, m=m, keys=keys)
+    torch.cuda.synchronize()
+    assert ctx.device_error() == 0
+    want = R.marlin_gemm(x[7:7 + m], wdq, "silu").astype(np.float32)
+    a, b = y.float().cpu().numpy(), p.cpu().numpy()
+    # (the f32 sums agree to 1e-5; the f16 result may fall on the neighbouring value)
+    assert np.abs(a[7:7 + m] - want).max() <= 2 ** -10 * np.abs(want).max()
+    assert np.all(a[:7] == 0) and np.all(a[7 + m:] == 0) and np.all(b[:7] == 0) and np.all(b[7 + m:] == 0)
+    got = keys.cpu().numpy().view(np.uint64)
+    assert (got[7:7 + m] == R.argmax_keys(b[7:7 + m], rows)).all() and np.all(got[:7] == 0) and np.all(got[7 + m:] == 0)
+
+
 @pytest.mark.parametrize("m", [65, 97, 256, 257, 333])
 def test_token_tile_widths_and_zero_points(ctx, m):
     """The tile's width follows the row count (96, 128, 256, 2 x 160, 2 x 192 tokens); zero-point matrices take the same path."""
