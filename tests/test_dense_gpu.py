@@ -117,3 +117,20 @@ def test_gemm_f16_in_ba(ctx, ref, n):
     split = ref.gemm_f16_plain(wp, xd, yr, n, K, rows // 16)
     assert split == y.shape[0]
     assert np.allclose(got, yr.sum(0).cpu().numpy(), rtol=1e-4, atol=1e-4)
+
+
+@pytest.mark.parametrize("n,tiles,kper", [(33, 6, 256), (64, 4, 128), (100, 2, 384), (97, 10, 256), (40, 12, 144), (35, 3, 256)])
+def test_gemm_f16_blocks_of_tiles(ctx, n, tiles, kper):
+    """More than 32 tokens: a block takes 2, 4 or 6 tiles (or one when they are odd), ragged token blocks and k splits,
+    gathered rows. f32 sums of exact products over at most 384 columns: 1e-5 of the largest."""
+    g = synth.gen(190 + n)
+    K = 384
+    w = (torch.randn(tiles * 16, K, generator=g) * 0.1).half()
+    x = torch.randn(n + 3, K, generator=g).half()
+    rows = torch.randint(0, n + 3, (n,), generator=g).to(torch.int32)
+    wp = torch.from_numpy(R.pack_f16(w.numpy())).cuda()
+    y = ctx.gemm_f16_plain(wp, x.cuda(), n, K, tiles, kper, xrows=rows.cuda())
+    torch.cuda.synchronize()
+    want = x.double()[rows.long()] @ w.double().T
+    got = y.double().cpu().sum(0)
+    assert y.shape[0] == -(-K // kper) and (got - want).abs().max() < 1e-5 * want.abs().max()
