@@ -3,15 +3,15 @@
 // (kernels/qwen_deltanet.cuh: delta_conv :84-131, delta_rule :172-288, delta_norm :295-315), another algorithm:
 //
 //  delta_prep_kernel        the causal depthwise conv, SiLU, the L2 norms of the q and k heads and the two gates. A
-//                           thread owns ONE channel and slides along 16 tokens with the conv's four inputs in
-//                           registers (each input row is read once, not four times); the 128 channels of a block are
-//                           one q, k or v head, so the head's norm is a block reduction per token.
+//                           lane owns FOUR channels and slides along 8 or 16 tokens with the conv's four inputs in
+//                           registers (each input row is read once, not four times); the 128 channels of a warp are
+//                           one q, k or v head, so the head's norm is a warp reduction per token.
 //  delta_chunk_prep_kernel  the part of the CHUNKED delta rule that does not depend on the state (the WY form the
 //                           reference states for its MLX backend, src/mlx/delta.rs:6-15,85-137; chunks of 64 tokens):
 //                           per chunk and key head K K^T and Q K^T once, then per value head the unit lower triangular
 //                           system's inverse T = (I + A)^-1, A_ij = b_i (k_i . k_j) exp(G_i - G_j), and
 //                           P_ij = (q_i . k_j) exp(G_i - G_j). All chunks of all segments in parallel.
-//  delta_scan_kernel        a block per (half of a value head's columns, value head, segment) carries its 64 x 128 slice
+//  delta_scan_kernel        a block per (48 or 64 of a value head's columns, value head, segment) carries its slice
 //                           of the f32 state in shared memory from chunk to chunk: R = b (V - gam K S^T), D = T R,
 //                           O = gam Q S^T + P D, S' = gam_C S + D^T (k_j exp(G_C - G_j)). The contractions run on the
 //                           tensor cores as 3 x TF32 (every operand split into a TF32 head and tail, three products
@@ -26,81 +26,23 @@
 namespace qb {
 
 // ------------------------------------------------------------------------------------------------ delta_prep
-constexpr int PREP_TOK = 16;  // tokens a block slides along
 
-__device__ __forceinline__ float in_sum(const float* p, int splits, size_t stride, size_t at) {
-    float v = p[at];
-    for (int s = 1; s < splits; s++) v += p[at + s * stride];
-    return v;
-}
-
-// grid (LQKV / 128, ceil(n / PREP_TOK)), block 128: thread c is channel 128 blockIdx.x + c
-__global__ void __launch_bounds__(128)
+// grid (LQKV / 512 + 1, ceil(n / PREP_TOK)), block 128: a warp is one head, a lane four of its channels; the last column of
+// blocks makes the gates. Bound by the rows' way from memory and back (n x 80 KB): every row of the tile is requested
+// before anything is used, 16 bytes per lane, and the head's norm is a warp reduction (2048 tokens: 79 us with a channel
+// per thread, four bytes per request and the gates behind the first head's channels).
+// PREP_TOK: the tokens a block slides along. 8 leave room for five blocks per SM, 16 read less history: the mixer of 40 rows takes
+// 48.0 and 51.2 us with them, of 150 138 and 129, of 333 179 and 174, of 700 245 and 256, of 1300 328 and 338.
+template <int PREP_TOK>
+__global__ void __launch_bounds__(128, PREP_TOK == 8 ? 5 : 4)
 delta_prep_kernel(const float* p, int splits, int n, const float* ba, int ba_splits, const float* cw,
                   const float* a_log, const float* dt_bias, const float* mem, long long sst, float* cv,
                   const int* tok_slot, const int* tok_pos) {
-    __shared__ float ss_part[PREP_TOK][4];
     pdl_launch_dependents();
-    const int head = blockIdx.x, ch = head * 128 + threadIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int tb = blockIdx.y * PREP_TOK, cnt = min(PREP_TOK, n - tb);
-    const float4 taps = ld4(cw + (size_t)ch * CONV_K);
-    pdl_wait();
-    const size_t stride = (size_t)n * DELTA_IN;
-    // every load of the tile first (they are independent), the sliding window after
-    float x[PREP_TOK], y[PREP_TOK];
-    int slots[PREP_TOK], poss[PREP_TOK];
-#pragma unroll
-    for (int i = 0; i < PREP_TOK; i++) {
-        const int t = min(tb + i, n - 1);
-        x[i] = in_sum(p, splits, stride, (size_t)t * DELTA_IN + ch);
-        slots[i] = tok_slot[t];
-        poss[i] = tok_pos[t];
-    }
-    float h0 = 0.f, h1 = 0.f, h2 = 0.f;  // the conv inputs at the three positions before the current token
-    int prev_slot = -1;
-#pragma unroll
-    for (int i = 0; i < PREP_TOK; i++) {
-        y[i] = 0.f;
-        if (i < cnt) {
-            const int t = tb + i, slot = slots[i], pos = poss[i];
-            if (slot != prev_slot) {
-                // a segment starts in this tile (or the tile starts): fetch the history, from the step's own rows of
-                // the same sequence or from the slot's ring
-                auto hist = [&](int back) {
-                    const int qp = pos - back, tt = t - back;
-                    if (qp < 0) return 0.f;
-                    if (tt >= 0 && tok_slot[tt] == slot) return in_sum(p, splits, stride, (size_t)tt * DELTA_IN + ch);
-                    return mem[slot * sst + SLOT_RING + (size_t)(qp & (CR - 1)) * LQKV + ch];
-                };
-                h0 = hist(3); h1 = hist(2); h2 = hist(1);
-                prev_slot = slot;
-            }
-            float a = taps.x * h0;
-            a = fmaf(taps.y, h1, a);
-            a = fmaf(taps.z, h2, a);
-            a = fmaf(taps.w, x[i], a);
-            y[i] = silu(a);
-            h0 = h1; h1 = h2; h2 = x[i];
-        }
-    }
-    if (head < 2 * LK_HEADS) {  // a q or k head: L2 norm over the block's 128 channels, q also / sqrt(128)
-#pragma unroll
-        for (int i = 0; i < PREP_TOK; i++) {
-            float s = warp_sum(y[i] * y[i]);
-            if (lane == 0) ss_part[i][warp] = s;
-        }
-        __syncthreads();
-#pragma unroll
-        for (int i = 0; i < PREP_TOK; i++) {
-            float sc = rsqrtf(((ss_part[i][0] + ss_part[i][1]) + (ss_part[i][2] + ss_part[i][3])) + 1e-6f);
-            if (head < LK_HEADS) sc *= rsqrtf((float)LKD);
-            y[i] *= sc;
-        }
-    }
-#pragma unroll
-    for (int i = 0; i < PREP_TOK; i++)
-        if (i < cnt) cv[(size_t)(tb + i) * CVW + ch] = y[i];
-    if (head == 0) {  // the gates of the tile's tokens: exp(g) and beta per value head
+    if (blockIdx.x == LQKV / 512) {  // the gates of the tile's tokens: exp(g) and beta per value head
+        pdl_wait();
         for (int x = threadIdx.x; x < cnt * LV_HEADS; x += 128) {
             const int t = tb + x / LV_HEADS, v = x % LV_HEADS;
             float b = 0.f, a = 0.f;
@@ -114,6 +56,75 @@ delta_prep_kernel(const float* p, int splits, int n, const float* ba, int ba_spl
             cv[(size_t)t * CVW + LQKV + v] = expf(-expf(a_log[v]) * sp);
             cv[(size_t)t * CVW + LQKV + LV_HEADS + v] = 1.f / (1.f + expf(-b));
         }
+        return;
+    }
+    const int head = blockIdx.x * 4 + warp, ch = head * 128 + lane * 4;
+    float4 taps[4];  // of the lane's four channels
+#pragma unroll
+    for (int c = 0; c < 4; c++) taps[c] = ld4(cw + (size_t)(ch + c) * CONV_K);
+    pdl_wait();
+    const size_t stride = (size_t)n * DELTA_IN;
+    // lane i < PREP_TOK: token tb + i's slot and position; the next three: the slots of the three tokens before the tile
+    const int mt = min(lane < PREP_TOK ? tb + lane : max(tb - PREP_TOK - 3 + lane, 0), n - 1);
+    const int my_slot = tok_slot[mt], my_pos = tok_pos[mt];
+    float4 x[PREP_TOK], h[3];  // h: the conv inputs at the three positions before the current token
+#pragma unroll
+    for (int i = 0; i < 3; i++) h[i] = ld4(p + (size_t)max(tb - 3 + i, 0) * DELTA_IN + ch);
+#pragma unroll
+    for (int i = 0; i < PREP_TOK; i++) x[i] = ld4(p + (size_t)min(tb + i, n - 1) * DELTA_IN + ch);
+    // (the other partial sums in a loop of their own: one inside the row's load makes the loads wait for one another)
+    for (int s = 1; s < splits; s++) {
+        const float* ps = p + s * stride + ch;
+        auto add = [](float4& v, float4 w) { v.x += w.x; v.y += w.y; v.z += w.z; v.w += w.w; };
+#pragma unroll
+        for (int i = 0; i < 3; i++) add(h[i], ld4(ps + (size_t)max(tb - 3 + i, 0) * DELTA_IN));
+#pragma unroll
+        for (int i = 0; i < PREP_TOK; i++) add(x[i], ld4(ps + (size_t)min(tb + i, n - 1) * DELTA_IN));
+    }
+    int prev_slot = -1;
+#pragma unroll
+    for (int i = 0; i < PREP_TOK; i++) {
+        if (i < cnt) {
+            const int t = tb + i, slot = __shfl_sync(0xffffffffu, my_slot, i), pos = __shfl_sync(0xffffffffu, my_pos, i);
+            if (slot != prev_slot) {
+                // a segment starts in this tile (or the tile starts): the history comes from the step's own rows of the same
+                // sequence (at the tile's start those are loaded already), from the slot's ring, or is zero
+                float4 f[3];
+#pragma unroll
+                for (int b = 0; b < 3; b++) {
+                    const int back = 3 - b, qp = pos - back, tt = t - back;
+                    const bool own = i == 0 && tt >= 0 && __shfl_sync(0xffffffffu, my_slot, PREP_TOK + b) == slot;
+                    f[b] = make_float4(0.f, 0.f, 0.f, 0.f);
+                    if (qp >= 0) {
+                        const float* r = mem + slot * sst + SLOT_RING + (size_t)(qp & (CR - 1)) * LQKV + ch;  // (sst may be odd)
+                        if (own) f[b] = h[b];
+                        else f[b] = make_float4(r[0], r[1], r[2], r[3]);
+                    }
+                }
+                h[0] = f[0]; h[1] = f[1]; h[2] = f[2];
+                prev_slot = slot;
+            }
+            const float4 v = x[i];
+            auto conv = [&](float4 w, float a0, float a1, float a2, float a3) {
+                float a = w.x * a0;
+                a = fmaf(w.y, a1, a);
+                a = fmaf(w.z, a2, a);
+                a = fmaf(w.w, a3, a);
+                return silu(a);
+            };
+            float4 y;
+            y.x = conv(taps[0], h[0].x, h[1].x, h[2].x, v.x);
+            y.y = conv(taps[1], h[0].y, h[1].y, h[2].y, v.y);
+            y.z = conv(taps[2], h[0].z, h[1].z, h[2].z, v.z);
+            y.w = conv(taps[3], h[0].w, h[1].w, h[2].w, v.w);
+            h[0] = h[1]; h[1] = h[2]; h[2] = v;
+            if (head < 2 * LK_HEADS) {  // a q or k head: L2 norm over its 128 channels, q also / sqrt(128)
+                float sc = rsqrtf(warp_sum((y.x * y.x + y.y * y.y) + (y.z * y.z + y.w * y.w)) + 1e-6f);
+                if (head < LK_HEADS) sc *= rsqrtf((float)LKD);
+                y.x *= sc; y.y *= sc; y.z *= sc; y.w *= sc;
+            }
+            *(float4*)(cv + (size_t)t * CVW + ch) = y;
+        }
     }
 }
 
@@ -122,7 +133,6 @@ constexpr int CH = 64;                   // tokens per chunk
 constexpr int TP_FLOATS = 2 * CH * CH + CH;  // per (chunk, value head): T, P, the cumulative log decays
 constexpr int KLD = LKD + 4;             // row stride of the q / k / state tiles (floats): fragment loads hit 32 banks
 constexpr int TLD = CH + 4;              // ... of T and P
-constexpr int RLD = 64 + 8;              // ... of R, D and V (read with the token index on the fragment's k side)
 
 // tokens of a segment that run in chunks: whole chunks that end at least KEEP tokens before the segment's end (the
 // checkpoint and the bank of the rollback plan are made in the token form)
@@ -164,17 +174,17 @@ __device__ __forceinline__ void mma3(float* c, const FragA& a, float b0, float b
 // grid (chunks of the longest possible segment, LK_HEADS, segs), block 256. tp: [chunk index][LV_HEADS][TP_FLOATS],
 // chunk index = first token of the chunk / 64 (distinct for disjoint 64-token ranges).
 constexpr int CP_THREADS = 256;
-constexpr int CP_SMEM = (2 * CH * KLD + 2 * CH * (CH + 1) + 6 * CH) * 4;  // 102 KB: two blocks per SM
-static_assert(3 * CH * (CH + 1) <= 2 * CH * KLD, "the three A matrices reuse the q / k tiles");
+constexpr int CP_SMEM = (2 * CH * KLD + 6 * CH) * 4;  // 69 KB: three blocks per SM
+static_assert(4 * CH * (CH + 1) <= 2 * CH * KLD, "the three A matrices and K K^T reuse the q / k tiles");
 
 __global__ void __launch_bounds__(CP_THREADS)
 delta_chunk_prep_kernel(const float* cv, float* tp, const int* seg_start, const int* seg_len) {
     extern __shared__ __align__(16) float cps[];
     float* Ks = cps;                         // [64][KLD]; later A of the three value heads [3][64][65]
     float* Qs = Ks + CH * KLD;
-    float* KK = Qs + CH * KLD;               // [64][65]; later scratch of the inverse
-    float* QK = KK + CH * (CH + 1);
-    float* gs = QK + CH * (CH + 1);          // [3][64] cumulative log decay
+    float* QK = Ks;                          // [64][65] over the q / k tiles, then A over it
+    float* KK = Ks + 3 * CH * (CH + 1);      // [64][65] behind the place of the three A; later scratch of the inverse
+    float* gs = Qs + CH * KLD;               // [3][64] cumulative log decay
     float* bs = gs + 3 * CH;                 // [3][64] beta
     pdl_launch_dependents();
     const int c = blockIdx.x, kh = blockIdx.y, sg = blockIdx.z, tid = threadIdx.x;
@@ -224,6 +234,7 @@ delta_chunk_prep_kernel(const float* cv, float* tp, const int* seg_start, const 
             for (int j = 0; j < 8; j++)
                 if (j < nts) mma3(acc[j], a, br[8 * j * KLD + k0], br[8 * j * KLD + k0 + 4]);
         }
+        __syncthreads();  // every warp is done with the tiles
 #pragma unroll
         for (int j = 0; j < 8; j++) {
             float* d0 = dst + (16 * m + g8) * (CH + 1) + 8 * j + 2 * t4;
@@ -232,15 +243,20 @@ delta_chunk_prep_kernel(const float* cv, float* tp, const int* seg_start, const 
         }
     }
     __syncthreads();
-    // A of the three value heads over the q / k tiles (done with), and P straight to global memory
-    float* As = Ks;
+    // P straight to global memory, then A of the three value heads (over Q K^T, which is done with)
     for (int x = tid; x < 3 * CH * CH; x += CP_THREADS) {
         const int hv = x / (CH * CH), i = (x / CH) % CH, j = x % CH;
         const float dec = j <= i ? expf(gs[hv * CH + i] - gs[hv * CH + j]) : 0.f;
-        As[(hv * CH + i) * (CH + 1) + j] = j < i ? bs[hv * CH + i] * KK[i * (CH + 1) + j] * dec : 0.f;
         float* out = tp + ((size_t)(tok >> 6) * LV_HEADS + kh * G + hv) * TP_FLOATS;
         out[CH * CH + i * CH + j] = j <= i ? QK[i * (CH + 1) + j] * dec : 0.f;
         if (j == 0) out[2 * CH * CH + i] = gs[hv * CH + i];
+    }
+    __syncthreads();
+    float* As = Ks;
+    for (int x = tid; x < 3 * CH * CH; x += CP_THREADS) {
+        const int hv = x / (CH * CH), i = (x / CH) % CH, j = x % CH;
+        As[(hv * CH + i) * (CH + 1) + j] =
+            j < i ? bs[hv * CH + i] * KK[i * (CH + 1) + j] * expf(gs[hv * CH + i] - gs[hv * CH + j]) : 0.f;
     }
     __syncthreads();
     // T = (I + A)^-1, unit lower triangular, IN PLACE over A. The four 16 x 16 diagonal blocks by forward substitution,
@@ -248,7 +264,7 @@ delta_chunk_prep_kernel(const float* cv, float* tp, const int* seg_start, const 
     // 16 -> 32 -> 64: for a block pair [[T11, 0], [T21, T22]] the lower left part is T21 = -T22 (A21 T11), two small
     // products spread over the block (X = A21 T11 goes through scratch, so T21 may overwrite A21).
     float* D0 = KK;                    // [3][4][16][17] the diagonal blocks' inverses
-    float* Xs = KK + 3 * 4 * 16 * 17;  // [3][32][33] scratch of the merges (K K^T and Q K^T are done with)
+    float* Xs = KK;                    // [3][32][33] scratch of the merges, once the diagonal blocks are back in place
     float* Ts = As;
     if (tid < 3 * CH) {
         const int hv = tid / CH, blk = (tid % CH) / 16, b0 = blk * 16, col = tid % 16;
@@ -314,27 +330,37 @@ delta_chunk_prep_kernel(const float* cv, float* tp, const int* seg_start, const 
     }
 }
 
-constexpr int SC_THREADS = 512, SC_COLS = 64;   // threads of a scan block; value columns of its state slice
+// A scan block has COLS of a value head's 128 columns, 8 threads per column. Steps with chunks are bound by the tf32 mma.sync
+// rate of each SM, chunk after chunk: three blocks per head (48, 48 and 32 columns) put one sequence on 144 of 148 SMs where
+// two halves leave 52 idle (2048 tokens: 355 us in halves, 299 us in three parts); the launch takes whichever finishes its
+// waves of blocks first. Steps without chunks (the token form alone) take halves: fewer blocks stage the tokens.
 constexpr int SC_TAIL = 16;                      // tokens staged per round of the token form
+template <int COLS>
 struct ScanSmem {
+    static constexpr int RLD = COLS + 8;  // row stride of R, D and V (read with the token index on the fragment's k side)
     float kq[2 * CH][KLD];     // chunk: k rows 0..63, q rows 64..127; token form: q / k / v of a round
     float t[CH][TLD], pm[CH][TLD];
-    float s[SC_COLS][KLD];     // the state slice [value column][key]
+    float s[COLS][KLD];     // the state slice [value column][key]
     float r[CH][RLD], d[CH][RLD];
     float g[CH], b[CH], gam[CH], dec[CH];
     float te[SC_TAIL], tb[SC_TAIL], tkq[SC_TAIL];
 };
 
-__global__ void __launch_bounds__(SC_THREADS, 1)
+template <int SC_COLS>
+__global__ void __launch_bounds__(SC_COLS * 8, 1)
 delta_scan_kernel(const float* p, int splits, int n, const float* cv, const float* tp, float* mem, long long sst,
                   const int* meta, float* out, const int* seg_start, const int* seg_len, const int* seg_slot,
                   const int* seg_pos0) {
     extern __shared__ __align__(16) uint8_t scan_raw[];
-    ScanSmem& M = *(ScanSmem*)scan_raw;
+    constexpr int SC_THREADS = SC_COLS * 8, NT16 = SC_COLS / 16, RLD = ScanSmem<SC_COLS>::RLD;
+    ScanSmem<SC_COLS>& M = *(ScanSmem<SC_COLS>*)scan_raw;
     pdl_launch_dependents();
     const int vs = blockIdx.x, h = blockIdx.y, sg = blockIdx.z, kh = h / (LV_HEADS / LK_HEADS);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g8 = lane >> 2, t4 = lane & 3;
-    const int lc = tid >> 3, sub = tid & 7, col = vs * SC_COLS + lc;   // token form: 8 lanes per value column
+    const int width = min(SC_COLS, LVD - vs * SC_COLS);   // this block's columns
+    const int lc = tid >> 3, sub = tid & 7;   // token form: 8 lanes per value column
+    const bool mine = lc < width;             // (lanes past the last column follow it and store nothing)
+    const int col = vs * SC_COLS + min(lc, width - 1);
     const int t0 = seg_start[sg], len = seg_len[sg], slot = seg_slot[sg], p0 = seg_pos0[sg];
     const Plan pl = make_plan(meta, slot, p0, len);
     float* sm0 = mem + slot * sst;
@@ -365,7 +391,8 @@ delta_scan_kernel(const float* p, int splits, int n, const float* cv, const floa
     if (l0 > 0) {
         // ================================================================ chunks
         st_rows<8>(&M.s[lc][0], S, sub);
-        const int mq = warp >> 2, nq = warp & 3;   // a warp's 16-row tile and 16-column tile in G1, G2 and G3
+        const int mq = warp / NT16, nq = warp % NT16;   // a warp's 16-row tile and 16-column tile in G1, G2 and G3
+        const bool has = 16 * nq < width;         // the tile has columns
         auto load_q = [&](int tok) {
             for (int x = tid; x < CH * (LKD / 4); x += SC_THREADS) {
                 const int r = x / (LKD / 4), dd = (x % (LKD / 4)) * 4;
@@ -383,7 +410,11 @@ delta_scan_kernel(const float* p, int splits, int n, const float* cv, const floa
             for (int x = tid; x < CH * (CH / 4); x += SC_THREADS) {
                 const int r = x / (CH / 4), dd = (x % (CH / 4)) * 4;
                 cp_async16(&M.t[r][dd], src + r * CH + dd);
-                cp_async16(&M.r[r][dd], cv + (size_t)(tok + r) * CVW + 2 * LK_HEADS * LKD + h * LVD + vs * SC_COLS + dd);
+            }
+            for (int x = tid; x < CH * (SC_COLS / 4); x += SC_THREADS) {
+                const int r = x / (SC_COLS / 4), dd = (x % (SC_COLS / 4)) * 4;
+                if (dd < width)
+                    cp_async16(&M.r[r][dd], cv + (size_t)(tok + r) * CVW + 2 * LK_HEADS * LKD + h * LVD + vs * SC_COLS + dd);
             }
             if (tid < CH / 4) cp_async16(&M.g[tid * 4], src + 2 * CH * CH + tid * 4);
             if (tid >= 32 && tid < 32 + CH) cp_async4(&M.b[tid - 32], cv + (size_t)(tok + tid - 32) * CVW + LQKV + LV_HEADS + h);
@@ -416,7 +447,7 @@ delta_scan_kernel(const float* p, int splits, int n, const float* cv, const floa
                 acck[j][0] = acck[j][1] = acck[j][2] = acck[j][3] = 0.f;
                 acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.f;
             }
-            {
+            if (has) {
                 const float* ak = &M.kq[16 * mq + g8][t4];
                 const float* aq = &M.kq[CH + 16 * mq + g8][t4];
                 const float* br = &M.s[16 * nq + g8][t4];
@@ -440,7 +471,7 @@ delta_scan_kernel(const float* p, int splits, int n, const float* cv, const floa
             }
             __syncthreads();  // gam / dec visible (written above), every warp done with q and with S as an operand
 #pragma unroll
-            for (int hh = 0; hh < 2; hh++) {
+            for (int hh = 0; hh < 2 && has; hh++) {
                 // R = b (V - gam K S^T), over V in place; gam Q S^T stays in the registers until P D joins it
                 const int i = 16 * mq + g8 + 8 * hh;
                 const float bi = M.b[i], gi = M.gam[i];
@@ -457,8 +488,8 @@ delta_scan_kernel(const float* p, int splits, int n, const float* cv, const floa
             cp_async_commit();
             __syncthreads();
             // ---- G2: D = T R, 64 x 64 over the chunk's tokens (T is lower triangular: rows 16 m2 .. stop at 16 m2 + 15)
-            {
-                const int m2 = warp >> 2, np = warp & 3;
+            if (has) {
+                const int m2 = mq, np = nq;
                 float dacc[2][4];
 #pragma unroll
                 for (int j = 0; j < 2; j++) dacc[j][0] = dacc[j][1] = dacc[j][2] = dacc[j][3] = 0.f;
@@ -478,8 +509,8 @@ delta_scan_kernel(const float* p, int splits, int n, const float* cv, const floa
             __syncthreads();
             if (more) load_tv(tok + CH);  // T, R (the value columns' place) and the gates are free: gam and dec hold what
             cp_async_commit();            // the rest of the chunk needs of them
-            // ---- G4: S' = gam_C S + D^T (k_j dec_j), 64 value columns x 128 keys over the chunk's tokens
-            {
+            // ---- G4: S' = gam_C S + D^T (k_j dec_j), the value columns x 128 keys over the chunk's tokens
+            if (16 * (warp >> 2) < width) {
                 const int m4 = warp >> 2, nq = warp & 3;
                 float sacc[4][4];
                 const float gc = M.gam[CH - 1];
@@ -509,7 +540,7 @@ delta_scan_kernel(const float* p, int splits, int n, const float* cv, const floa
             if (more) load_k(tok + CH);   // the k tile is free
             cp_async_commit();
             // ---- G3: O = gam Q S^T + P D (operands rounded to TF32 once), straight to the output rows
-            {
+            if (has) {
                 const float* ar = &M.pm[16 * mq + g8][t4];
                 const float* br = &M.d[t4][16 * nq + g8];
                 for (int k0 = 0; k0 < 16 * (mq + 1); k0 += 8) {
@@ -538,7 +569,7 @@ delta_scan_kernel(const float* p, int splits, int n, const float* cv, const floa
     // ================================================================ the token form: tokens l0 .. len - 1
     float* tq = &M.kq[0][0];                       // [SC_TAIL][128]
     float* tk = tq + SC_TAIL * LKD;                // [SC_TAIL][128]
-    float* tv = tk + SC_TAIL * LKD;                // [SC_TAIL][64]
+    float* tv = tk + SC_TAIL * LKD;                // [SC_TAIL][SC_COLS]
     for (int c0 = l0; c0 < len; c0 += SC_TAIL) {
         const int m = min(SC_TAIL, len - c0);
         __syncthreads();  // the previous round (or the chunks) is done with the staging area
@@ -550,7 +581,8 @@ delta_scan_kernel(const float* p, int splits, int n, const float* cv, const floa
         }
         for (int x = tid; x < m * (SC_COLS / 4); x += SC_THREADS) {
             const int r = x / (SC_COLS / 4), dd = (x % (SC_COLS / 4)) * 4;
-            *(float4*)(tv + r * SC_COLS + dd) = ld4(cv + (size_t)(t0 + c0 + r) * CVW + 2 * LK_HEADS * LKD + h * LVD + vs * SC_COLS + dd);
+            if (dd < width)
+                *(float4*)(tv + r * SC_COLS + dd) = ld4(cv + (size_t)(t0 + c0 + r) * CVW + 2 * LK_HEADS * LKD + h * LVD + vs * SC_COLS + dd);
         }
         if (tid < 2 * m) {
             const int r = tid >> 1, which = tid & 1;
@@ -567,7 +599,7 @@ delta_scan_kernel(const float* p, int splits, int n, const float* cv, const floa
         for (int r = max(0, pl.ck - (p0 + c0)); r < m; r++) {
             float* e = entry(pl.cbuf, p0 + c0 + r);
             if (vs == 0 && h % (LV_HEADS / LK_HEADS) == 0 && tid < LKD) e[kh * LKD + tid] = tk[r * LKD + tid];
-            if (tid >= 128 && tid < 128 + SC_COLS) e[LK_HEADS * LKD + h * LVD + vs * SC_COLS + tid - 128] = tv[r * SC_COLS + tid - 128];
+            if (tid >= 128 && tid < 128 + width) e[LK_HEADS * LKD + h * LVD + vs * SC_COLS + tid - 128] = tv[r * SC_COLS + tid - 128];
             if (vs == 0 && tid == 256) {
                 e[LK_HEADS * LKD + LV_HEADS * LVD + h] = M.te[r];
                 e[LK_HEADS * LKD + LV_HEADS * LVD + LV_HEADS + h] = M.tb[r];
@@ -575,18 +607,18 @@ delta_scan_kernel(const float* p, int splits, int n, const float* cv, const floa
         }
         __syncthreads();
         for (int r = 0; r < m; r++) {
-            if (pl.wck && p0 + c0 + r == pl.ck) st_rows<8>(sbuf(pl.cbuf), S, sub);
+            if (mine && pl.wck && p0 + c0 + r == pl.ck) st_rows<8>(sbuf(pl.cbuf), S, sub);
             float k[RPT], q[RPT];
             ld_rows<8>(k, tk + r * LKD, sub);
             ld_rows<8>(q, tq + r * LKD, sub);
             const float dk = dot_rows<8>(S, k), dq = dot_rows<8>(S, q);
-            const float ex = M.te[r], delta = (tv[r * SC_COLS + lc] - ex * dk) * M.tb[r];
-            if (sub == 0) out[(size_t)(t0 + c0 + r) * MIX + h * LVD + col] = ex * dq + delta * M.tkq[r];
+            const float ex = M.te[r], delta = (tv[r * SC_COLS + col - vs * SC_COLS] - ex * dk) * M.tb[r];
+            if (mine && sub == 0) out[(size_t)(t0 + c0 + r) * MIX + h * LVD + col] = ex * dq + delta * M.tkq[r];
 #pragma unroll
             for (int j = 0; j < RPT; j++) S[j] = ex * S[j] + k[j] * delta;
         }
     }
-    st_rows<8>(sbuf(pl.ebuf), S, sub);
+    if (mine) st_rows<8>(sbuf(pl.ebuf), S, sub);
     // ---- the conv ring: the conv inputs of the segment's last CR tokens, this block's share of the channels (after
     // delta_prep, which read the ring, has finished: it is an earlier kernel of the stream)
     const int nb = gridDim.x * gridDim.y, share = (LQKV + nb - 1) / nb;
@@ -648,8 +680,10 @@ int qb_delta_conv(qb_ctx* ctx, void* stream, const float* p, int splits, int n, 
     if (!ctx || !p || !ba || !cw || !a_log || !dt_bias || !mem || !cv || !tok_slot || !tok_pos || n <= 0 ||
         splits < 1 || ba_splits < 1)
         return QB_ERR_ARG;
-    return launch(ctx, delta_prep_kernel, dim3(LQKV / 128, (n + PREP_TOK - 1) / PREP_TOK), dim3(128), 0,
-                  (cudaStream_t)stream, p, splits, n, ba, ba_splits, cw, a_log, dt_bias, mem, sst, cv, tok_slot, tok_pos);
+    const bool wide = n > 128 && n <= 512;
+    const dim3 grid(LQKV / 512 + 1, wide ? (n + 15) / 16 : (n + 7) / 8);
+    return launch(ctx, wide ? delta_prep_kernel<16> : delta_prep_kernel<8>, grid, dim3(128), 0, (cudaStream_t)stream, p, splits, n, ba,
+                  ba_splits, cw, a_log, dt_bias, mem, sst, cv, tok_slot, tok_pos);
 }
 
 // The scratch of the chunked form (T, P and the log decays of every chunk and value head of a step of up to 2048
@@ -673,8 +707,12 @@ int qb_delta_rule(qb_ctx* ctx, void* stream, const float* p, int splits, int n, 
                         ctx->delta_tp, seg_start, seg_len);
         if (rc) return rc;
     }
-    return launch(ctx, delta_scan_kernel, dim3(LVD / SC_COLS, LV_HEADS, segs), dim3(SC_THREADS), sizeof(ScanSmem), st, p,
-                  splits, n, cv, (const float*)ctx->delta_tp, mem, sst, meta, out, seg_start, seg_len, seg_slot, seg_pos0);
+    auto waves = [&](long long parts) { return (parts * LV_HEADS * segs + ctx->sms - 1) / ctx->sms; };
+    if (chunks > 0 && waves(3) * 48 < waves(2) * 64)
+        return launch(ctx, delta_scan_kernel<48>, dim3(3, LV_HEADS, segs), dim3(48 * 8), sizeof(ScanSmem<48>), st, p, splits, n, cv,
+                      (const float*)ctx->delta_tp, mem, sst, meta, out, seg_start, seg_len, seg_slot, seg_pos0);
+    return launch(ctx, delta_scan_kernel<64>, dim3(2, LV_HEADS, segs), dim3(64 * 8), sizeof(ScanSmem<64>), st, p, splits, n, cv,
+                  (const float*)ctx->delta_tp, mem, sst, meta, out, seg_start, seg_len, seg_slot, seg_pos0);
 }
 
 int qb_delta_norm(qb_ctx* ctx, void* stream, const float* p, int splits, int n, const float* nw, const float* out,

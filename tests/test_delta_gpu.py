@@ -336,3 +336,49 @@ def test_rollback_after_a_chunked_prompt(ctx):
         pos += good
     for i in range(P, T):
         assert torch.equal(outsA[i], outsB[i]), f"position {i}"
+
+
+@pytest.mark.parametrize("splits", [1, 2])
+def test_conv_tiles(ctx, splits):
+    """Segments that start and end anywhere in the conv's tiles, shorter than its history of three, from
+    position 0, from the slot's ring and across tiles, against the oracle (2e-4: the fast exponential of SiLU, as in test_delta_conv)."""
+    g = synth.gen(171 + splits)
+    lens, pos0 = [1, 2, 17, 31, 40, 3], [0, 5, 1, 100, 2, 40]
+    toks = [(0, s, p + i) for s, (n, p) in enumerate(zip(lens, pos0)) for i in range(n)]
+    n = len(toks)
+    conv_w, a_log, dt_bias, _ = weights(g)
+    mem = fresh_mem(len(lens), g) * 100
+    part = torch.randn(splits, n, R.DELTA_IN, generator=g)
+    ba = torch.randn(5, n, 2 * R.LV_HEADS, generator=g)
+    st = R.build_step(toks, [])
+    cv = torch.zeros(n, R.CVW, device="cuda")
+    d = lambda t: t.cuda()
+    ctx.delta_conv(d(part), splits, n, d(ba), 5, d(conv_w), d(a_log), d(dt_bias), d(mem), SST, cv, ref_cuda.upload_step(st))
+    torch.cuda.synchronize()
+    want = R.delta_conv(part.numpy(), ba.numpy(), conv_w.numpy(), a_log.numpy(), dt_bias.numpy(), mem.numpy(), SST,
+                        st["tok_slot"], st["tok_pos"])
+    assert np.allclose(cv.cpu().numpy(), want, rtol=2e-4, atol=1e-5)
+
+
+@pytest.mark.parametrize("lens", [(80,), (79, 150), (300,)])
+def test_chunked_rule_against_the_oracle(ctx, lens):
+    """The scan in parts of 48, 48 and 32 value columns, chunks and the token form after them: outputs and state of one and
+    two segments, from zeros and from a stored state, against the oracle's f64 recurrence."""
+    g = synth.gen(181 + len(lens))
+    toks = [(0, s, 7 * s + i) for s, n in enumerate(lens) for i in range(n)]
+    n = len(toks)
+    st = R.build_step(toks, [])
+    dv = ref_cuda.upload_step(st)
+    mem, meta = fresh_mem(len(lens), g), np.array([[7 * s, 7 * s, 0, 0] for s in range(len(lens))], dtype=np.int32)
+    part = torch.randn(1, n, R.DELTA_IN, generator=g)
+    ba = torch.randn(1, n, 2 * R.LV_HEADS, generator=g)
+    conv_w, a_log, dt_bias, _ = weights(g)
+    cvh = R.delta_conv(part.numpy(), ba.numpy(), conv_w.numpy(), a_log.numpy(), dt_bias.numpy(), mem.numpy(), SST,
+                       st["tok_slot"], st["tok_pos"])
+    dmem, out = mem.cuda(), torch.zeros(n, R.MIX, device="cuda")
+    ctx.delta_rule(part.cuda(), 1, n, torch.from_numpy(cvh).cuda(), dmem, SST, torch.from_numpy(meta).cuda(), out, dv, len(lens))
+    torch.cuda.synchronize()
+    omem = mem.numpy().copy()
+    want = R.delta_rule(part.numpy(), cvh, omem, SST, meta, st["seg_start"], st["seg_len"], st["seg_slot"], st["seg_pos0"])
+    assert close(out.cpu().numpy(), want).all()
+    assert np.abs(dmem.cpu().numpy() - omem).max() < 1e-4
