@@ -936,8 +936,11 @@ int qb_attn_prefill(qb_ctx* ctx, void* stream, const float* q, const void* kc, c
         return QB_ERR_ARG;
     const int z = tile_splits(ntile, max_keys);
     if (z > 1 && (!part_ml || !part_acc)) return QB_ERR_ARG;
-    if (z == 1) {  // many tiles: a pair of tiles per block on tcgen05 (attn_prefill_tc.cu)
-        return qb_attn_prefill_tc_launch(ctx, (cudaStream_t)stream, q, kc, vc, ks, vs, ptile, ntile, tok_slot, tok_pos,
+    if (z == 1) {
+        // many tiles, on tcgen05: four tiles per pair of blocks, or, up to 1664 keys, two per block: a stage of 128 keys and the
+        // pair's set-up cost more there than the faster stages give (100 rows at context 0 40.1 us as blocks, 43.7 as
+        // pairs; 1500 at 100 200 and 210; 2048 at 0 289 and 277; 1024 at 2000 257 and 225; 2048 at 30720 2786 and 2019)
+        return (max_keys <= 1664 ? qb_attn_prefill_short_launch : qb_attn_prefill_tc_launch)(ctx, (cudaStream_t)stream, q, kc, vc, ks, vs, ptile, ntile, tok_slot, tok_pos,
                                          cap, out, mix_f16);
     }
     using C = DecCfg<4, 2, 5>;  // 10 tokens x 6 heads = 60 rows: 4 row tiles; 2 warps each; 5 stages of 32 keys

@@ -67,6 +67,9 @@ int prepare_kernel(int device, const void* kern, int smem);
 int qb_attn_prefill_tc_launch(qb_ctx* ctx, cudaStream_t st, const float* q, const void* kc, const void* vc, const float* ks,
                               const float* vs, const int* ptile, int ntile, const int* tok_slot, const int* tok_pos,
                               int cap, float* out, void* mix_f16);
+int qb_attn_prefill_short_launch(qb_ctx* ctx, cudaStream_t st, const float* q, const void* kc, const void* vc, const float* ks,
+                                 const float* vs, const int* ptile, int ntile, const int* tok_slot, const int* tok_pos,
+                              int cap, float* out, void* mix_f16);  // short contexts (attn_prefill_short.cu)
 // the prompt-sized W4A16 product on tcgen05 (w4a16_gemm_tc.cu); reached through qb_marlin_gemm / qb_marlin_gemm_z (zp:
 // S carries the offsets' table after the scales) for more than 16 rows
 int qb_gemm_tc_launch(qb_ctx* ctx, cudaStream_t st, const void* X, const void* B, void* Y, const void* S, int m, int n,

@@ -256,6 +256,30 @@ def test_attn_prefill_pairs_and_segment_boundaries(ctx, ref):
     assert close(a, want).all()
 
 
+@pytest.mark.parametrize("lens,pos0", [((25, 33, 12, 47), (300, 40, 0, 450)), ((400,), (4003,)), ((10, 30, 10), (5, 64, 127))])
+def test_attn_prefill_runs_of_tiles(ctx, lens, pos0):
+    """A pair of blocks takes four tiles of a step, in passes over runs of one sequence: runs of one to four tiles, ragged
+    last tiles, keys that end on and off a 64-key stage, against the oracle."""
+    g = synth.gen(137 + len(lens))
+    cap = 4480 if pos0[0] > 4000 else 512
+    cache = make_cache(len(lens), cap, g, 0)
+    toks = [(0, s, p + i) for s, (n, p) in enumerate(zip(lens, pos0)) for i in range(n)]
+    n = len(toks)
+    q = torch.randn(n, R.NH, R.HD, generator=g) * QSCALE
+    gate = torch.sigmoid(torch.randn(n, R.MIX, generator=g))
+    st = R.build_step(toks, list(range(n)))
+    assert st["ndec"] == 0
+    mine, mix = run_prefill(ctx, q.cuda(), gate.cuda(), [t.cuda() for t in cache], st, ref_cuda.upload_step(st), cap, n, mix=True)
+    torch.cuda.synchronize()
+    assert ctx.device_error() == 0
+    a = mine.cpu().numpy()
+    assert np.array_equal(mix.cpu().numpy(), a.astype(np.float16))
+    rows = list(range(n)) if cap == 512 else [0, 1, 9, 10, 127, 200, 255, 256, 399]
+    want = R.attn_decode(q.numpy()[rows], gate.numpy()[rows], *[t.numpy() for t in cache], st["tok_slot"][rows],
+                         st["tok_pos"][rows], cap)
+    assert close(a[rows], want).all()
+
+
 @pytest.mark.parametrize("rows", [1, 4, 8])
 def test_attn_decode_of_a_ragged_batch(ctx, rows):
     """A batch of ragged sequences gives each token the bits that its sequence alone gives, and the oracle's values: also where
