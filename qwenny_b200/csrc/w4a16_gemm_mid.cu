@@ -2,16 +2,18 @@
 // batch) on the 5th-generation tensor cores: Y = X . W^T with W int4 in Marlin's layout, plain, SwiGLU or argmax epilogue,
 // contiguous or gathered rows.
 //
-// Bound by the weights' way from HBM (0.52 bytes each, read once) as long as the products keep up. A block owns 128 outputs and
-// the weights go from registers to tensor memory in the layout that a Marlin word already has (w4a16_gemm_tc.cu), but
-// not as a pair of blocks: with A in tensor memory a K = 16 product of M = 256 over a pair takes 128 cycles whatever its N,
-// one of M = 128 some 50 cycles for any N up to 64: 400 per 128-wide k block, against 380 for the block's 8 KB at the
-// measured copy bandwidth. (As pairs: 40 rows x 34816 x 5120 in 62 us.) What else differs from the prompt-sized product:
+// A block owns 128 outputs and the weights go from registers to tensor memory in the layout that a Marlin word already has
+// (w4a16_gemm_tc.cu). The floor is the weights' way from HBM (0.52 bytes each, read once): 380 cycles per block and 128 of
+// k. What bounds it is the products: with A in tensor memory a K = 16 step costs some 128 cycles of a block's time beside
+// the stores of the next weights, whatever N is up to 64 (a probe of such products alone: 47), so a stage takes some 1150 cycles.
+// 40 rows: 16384 x 5120 30.5 us, 5120 x 6144 23.0, 34816 x 5120 47.8 (62 as pairs of blocks), 5120 x 17408 34.5; padded to 256
+// tokens they took 69, 68, 70 and 89. What else differs from the prompt-sized product:
 //   - the weights are the exact integers q - 8; a group of 128 columns is one accumulation, and the drain warps multiply its
 //     f32 sums by the f32 value of the group's scale and add them up in registers (one thread per output, a register
 //     per token): one rounding per group, the arithmetic of the product for up to 16 rows (w4a16_gemv.cuh), where
-//     f16((q - 8) s) would round every weight. Two accumulators take turns, each with an issuing thread of its own (a
-//     wait, eight products and two commits take one thread longer than the products themselves)
+//     f16((q - 8) s) would round every weight. Four accumulators take turns, so that draining one overlaps the next
+//     products (with two the products waited 650 of 1100 cycles per stage for them), and two threads issue (eight products
+//     take one thread some 700 cycles, the waits and commits 300)
 //   - the rows are few: they are loaded per k block into the swizzled layout by cp.async (which also gathers), or by the
 //     tensor map when they are contiguous
 // The (tile, group) list is dealt to one block per SM in equal shares; parts of a cut tile are added by its last arriver in
@@ -28,7 +30,8 @@ constexpr int BH = 128;             // outputs per block
 constexpr int BK = 128;             // k per stage: a group of scales
 constexpr int NSTAGE = 8;           // stages in shared memory (words, X): a copy takes some 2000 cycles, a stage's products 400
 constexpr int NA = 4;               // stages in tensor memory (64 columns each)
-constexpr int NS = 16;              // groups in the ring of scales: those of the ring's stages and of the two being drained
+constexpr int ND = 4;               // accumulators in tensor memory (64 columns each)
+constexpr int NS = 16;              // groups in the ring of scales: those of the ring's stages and of the accumulators being drained
 constexpr int W_BYTES = BH * BK / 2;
 constexpr int DQ_WARPS = 8, DQ_GROUPS = DQ_WARPS / 4;  // a group of four warps unpacks a stage, the groups take turns
 constexpr int X_WARPS = 2;
@@ -71,8 +74,8 @@ __global__ void __launch_bounds__(Cfg<NT>::THREADS, 1)
     uint64_t* empty = aready + NSTAGE;   // its products are done
     uint64_t* sfull = empty + NSTAGE;    // a group's scales landed in this block
     uint64_t* dfull = sfull + NS;        // a group's accumulator is complete
-    uint64_t* dfree = dfull + 2;         // it has been drained
-    uint32_t* tmem_slot = (uint32_t*)(dfree + 2);
+    uint64_t* dfree = dfull + ND;         // it has been drained
+    uint32_t* tmem_slot = (uint32_t*)(dfree + ND);
     int* flag = (int*)(tmem_slot + 1);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -83,12 +86,12 @@ __global__ void __launch_bounds__(Cfg<NT>::THREADS, 1)
 
     if (threadIdx.x == 0) {
         for (int i = 0; i < NSTAGE; i++) {
-            mbar_init(&full[i], gathered ? 1 + X_WARPS : 1);
+            mbar_init(&full[i], gathered ? 1 + X_WARPS : 2);
             mbar_init(&aready[i], 4);
             mbar_init(&empty[i], 1);
         }
         for (int i = 0; i < NS; i++) mbar_init(&sfull[i], 1);
-        for (int i = 0; i < 2; i++) { mbar_init(&dfull[i], 1); mbar_init(&dfree[i], DR_WARPS); }
+        for (int i = 0; i < ND; i++) { mbar_init(&dfull[i], 1); mbar_init(&dfree[i], DR_WARPS); }
         mbar_fence_init();
     }
     if (warp == MMA_WARP) {
@@ -99,16 +102,16 @@ __global__ void __launch_bounds__(Cfg<NT>::THREADS, 1)
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-    const uint32_t tmem = *tmem_slot, tmem_a = tmem + 256;  // accumulators at columns 0 and 128, weights from 256 on
+    const uint32_t tmem = *tmem_slot, tmem_a = tmem + 256;  // accumulators at columns 0, 64, 128 and 192, weights from 256 on
     pdl_launch_dependents();
 
     // every role walks the same segments (tile, groups [g0, g1)); st counts stages, gr groups, from the start
     if (warp == COPY_WARP) {
         if (lane == 0) {
             const uint64_t pol = policy_evict_first();
-            bool ok = true, waited = false;
+            bool ok = true;
             uint32_t st = 0;
-            while (ok && walk.next(tile, g0, g1)) {
+            while (ok && walk.next(tile, g0, g1)) {  // (the weights do not depend on the kernel before: no wait for it)
                 const int n0 = tile * BH;
                 for (int gi = g0; gi < g1; gi++, st++) {
                     // (the scales' slot: the group NS before this one was drained long ago: this stage waits for products
@@ -118,18 +121,12 @@ __global__ void __launch_bounds__(Cfg<NT>::THREADS, 1)
                         ok = mbar_wait(&empty[s], ((st / NSTAGE) - 1) & 1);
                         if (!ok) break;
                     }
-                    mbar_expect_tx(&full[s], W_BYTES + (gathered ? 0 : XB));
+                    mbar_expect_tx(&full[s], W_BYTES);
                     tma_load_2d(wsmem + s * W_BYTES, &wmap, n0, gi * (BK / 16), &full[s]);
                     mbar_expect_tx(&sfull[sl], BH * 2);
                     bulk_g2s(ssmem + sl * BH, a.S + (size_t)gi * a.N + n0, BH * 2, &sfull[sl], pol);
-                    if (!gathered) {
-                        if (!waited) { pdl_wait(); waited = true; }  // the weights above do not depend on the kernel before
-                        tma_load_2d(smem + s * XB, &xmap, gi * BK, 0, &full[s]);
-                        tma_load_2d(smem + s * XB + C::XH, &xmap, gi * BK + 64, 0, &full[s]);
-                    }
                 }
             }
-            if (!waited) pdl_wait();
             if (!ok) atomicExch(a.err, 9);
         }
         __syncwarp();
@@ -176,7 +173,25 @@ __global__ void __launch_bounds__(Cfg<NT>::THREADS, 1)
             asm volatile("cp.async.wait_group 0;\n" ::: "memory");
             if (st > 1) hand(st - 2);
             if (st > 0) hand(st - 1);
+        } else if (warp == X_WARP && lane == 0) {  // contiguous rows: the tensor map, from a thread of its own (70 cycles per copy)
+            pdl_wait();
+            bool ok = true;
+            uint32_t st = 0;
+            while (ok && walk.next(tile, g0, g1)) {
+                for (int gi = g0; gi < g1; gi++, st++) {
+                    const int s = (int)(st % NSTAGE);
+                    if (st >= NSTAGE) {
+                        ok = mbar_wait(&empty[s], ((st / NSTAGE) - 1) & 1);
+                        if (!ok) break;
+                    }
+                    mbar_expect_tx(&full[s], XB);
+                    tma_load_2d(smem + s * XB, &xmap, gi * BK, 0, &full[s]);
+                    tma_load_2d(smem + s * XB + C::XH, &xmap, gi * BK + 64, 0, &full[s]);
+                }
+            }
+            if (!ok) atomicExch(a.err, 9);
         }
+        __syncwarp();
     } else if (warp < DQ_WARPS) {
         // ---------------------------------------------------------------- q - 8 into tensor memory
         const int q = warp & 3, h = warp >> 2;
@@ -240,16 +255,16 @@ __global__ void __launch_bounds__(Cfg<NT>::THREADS, 1)
             for (int j = 0; j < 32; j++) acc[j] = 0.f;
 #pragma unroll 1
             for (int gi = g0; gi < g1; gi++, gr++) {
-                const int p = (int)(gr & 1), sl = (int)(gr % NS);
+                const int p = (int)(gr % ND), sl = (int)(gr % NS);
                 if (!dead) {
-                    dead = !mbar_wait(&sfull[sl], (gr / NS) & 1) || !mbar_wait(&dfull[p], (gr >> 1) & 1);
+                    dead = !mbar_wait(&sfull[sl], (gr / NS) & 1) || !mbar_wait(&dfull[p], (gr / ND) & 1);
                     if (dead && lane == 0) atomicExch(a.err, 11);
                 }
                 asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
                 // scale of output 16 b + 8 i + r of a c64 at 8 r + 2 b + i
                 const float sc = __half2float(ssmem[sl * BH + (lrow >> 6) * 64 + 8 * (lrow & 7) + ((lrow & 63) >> 3)]);
                 uint32_t v[32];
-                tmem_ld32(tq + p * 128, v);
+                tmem_ld32(tq + p * 64, v);
                 asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
                 asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
                 __syncwarp();
@@ -322,18 +337,19 @@ __global__ void __launch_bounds__(Cfg<NT>::THREADS, 1)
         }
         if (EPI == QB_EPI_ARGMAX && best && t0 + lane < a.m) atomicMax(a.keys + a.y0 + t0 + lane, best);
     } else {
-        // ---------------------------------------------------------------- the products: one lane per accumulator
+        // ---------------------------------------------------------------- the products: two lanes take turns
         if (lane == 0) {
-            const int p = warp - MMA_WARP;
+            const int turn = warp - MMA_WARP;
             bool ok = true;
             uint32_t st = 0;
-            const uint32_t xs = smem_u32(smem), d = tmem + p * 128;
+            const uint32_t xs = smem_u32(smem);
             while (ok && walk.next(tile, g0, g1)) {
                 for (int gi = g0; gi < g1; gi++, st++) {
-                    if ((int)(st & 1) != p) continue;
-                    const int s = (int)(st % NSTAGE);
+                    if ((int)(st & 1) != turn) continue;
+                    const int s = (int)(st % NSTAGE), p = (int)(st % ND);
+                    const uint32_t d = tmem + p * 64;
                     const uint32_t at = tmem_a + (int)(st % NA) * (BK / 2);
-                    if (st >= 2) ok = mbar_wait(&dfree[p], ((st >> 1) - 1) & 1);
+                    if (st >= ND) ok = mbar_wait(&dfree[p], ((st / ND) - 1) & 1);
                     ok = ok && mbar_wait(&aready[s], (st / NSTAGE) & 1);
                     if (!ok) break;
                     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
