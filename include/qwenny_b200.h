@@ -44,9 +44,10 @@ const char* qb_version(void);
 
 /* ---- W4A16 product over a Marlin-packed matrix. Replaces the launches of Gemm::marlin
  * (src/cuda/core.rs:569-612) of marlin_m1_n8_{plain,silu,argmax} (kernels/marlin.cuh:588-602) for m <= 16 rows and of
- * marlin_m{1..4}_n16_* (the prompt chunks' products, kernels/qwen.cu:48) beyond: more than 16 contiguous rows with the
- * plain or SwiGLU epilogue run on the tensor-core product (tcgen05), gathered rows and the argmax epilogue as 16-row
- * slabs of the first.
+ * marlin_m{1..4}_n16_* (the prompt chunks' products, kernels/qwen.cu:48) beyond: 17 to 64 rows run on a tensor-core
+ * product (tcgen05) with every epilogue, contiguous or gathered; more than 64 contiguous rows with the plain or SwiGLU
+ * epilogue on the prompt-sized one, the others as 64-row slabs. The first such product takes the context's scratch for
+ * them; where it cannot be had (no memory, a stream being captured) up to 64 rows run as 16-row slabs.
  *   X      f16 [.][k]; rows row0 .. row0+m-1 are read, or rows xrows[0..m) when xrows != NULL (this folds
  *          marlin_gather, kernels/marlin.cuh:605-608, into the product)
  *   B      Marlin words, k/16 x 2n u32 (src/cuda/core.rs:262-311 pack_marlin); S f16 [k/128][n] permuted scales
@@ -66,7 +67,8 @@ int qb_marlin_early(qb_ctx* ctx, int stages);
 
 /* The zero-point variants marlin_*_z (kernels/marlin.cuh:126-133,588-594): same arguments; S holds the scales followed
  * by the table (8 - z) * scale (qb_pack_marlin_z). w = (q - 8) * scale + (8 - z) * scale; the second term needs only
- * the group's sum of x, which the kernel has anyway. More than 16 rows run as 16-row slabs. */
+ * the group's sum of x, which the kernel has anyway. More than 16 contiguous rows with the plain or SwiGLU epilogue run on
+ * the prompt-sized tensor-core product, the others as 16-row slabs. */
 int qb_marlin_gemm_z(qb_ctx* ctx, void* stream, const void* X, const void* B, void* Y, const void* S, int m, int n,
                      int k, int row0, int epi, const int* xrows, unsigned long long* keys, int n_valid);
 

@@ -29,8 +29,8 @@ namespace qb {
 
 // grid (LQKV / 512 + 1, ceil(n / PREP_TOK)), block 128: a warp is one head, a lane four of its channels; the last column of
 // blocks makes the gates. Bound by the rows' way from memory and back (n x 80 KB): every row of the tile is requested
-// before anything is used, 16 bytes per lane, and the head's norm is a warp reduction (2048 tokens: 79 us with a channel
-// per thread, four bytes per request and the gates behind the first head's channels).
+// before anything is used, 16 bytes per lane, and the head's norm is a warp reduction (2048 tokens: 62 us; 79 us with
+// a channel per thread, four bytes per request and the gates behind the first head's channels).
 // PREP_TOK: the tokens a block slides along. 8 leave room for five blocks per SM, 16 read less history: the mixer of 40 rows takes
 // 48.0 and 51.2 us with them, of 150 138 and 129, of 333 179 and 174, of 700 245 and 256, of 1300 328 and 338.
 template <int PREP_TOK>

@@ -51,7 +51,7 @@ __global__ void __launch_bounds__(ROW_THREADS) embed_q8_kernel(const uint8_t* E,
 // threads (k16 < tables * groups, lane < 16) also write row lane's scale of group k16 to its permuted place.
 __global__ void __launch_bounds__(256) put_block_kernel(uint32_t* B, __half* S, const uint32_t* words, const __half* sc,
                                                         int n, int c64, int blk, int groups, int tables, int k16s) {
-    pdl_launch_dependents();
+    // (no early launch of the next kernel: the products request weights before they wait for the kernel before them)
     pdl_wait();
     const int k16 = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (k16 >= k16s) return;
