@@ -28,7 +28,7 @@ using namespace tc;
 
 constexpr int BH = 128;             // outputs per block
 constexpr int BK = 128;             // k per stage: a group of scales
-constexpr int NSTAGE = 8;           // stages in shared memory (words, X): a copy takes some 2000 cycles, a stage's products 400
+constexpr int NSTAGE = 8;           // stages in shared memory (words, X): a copy takes some 2000 cycles
 constexpr int NA = 4;               // stages in tensor memory (64 columns each)
 constexpr int ND = 4;               // accumulators in tensor memory (64 columns each)
 constexpr int NS = 16;              // groups in the ring of scales: those of the ring's stages and of the accumulators being drained
