@@ -4,8 +4,9 @@
 //
 // A block owns 128 outputs and the weights go from registers to tensor memory in the layout that a Marlin word already has
 // (w4a16_gemm_tc.cu). The floor is the weights' way from HBM (0.52 bytes each, read once): 380 cycles per block and 128 of
-// k. What bounds it is the products: with A in tensor memory a K = 16 step costs some 128 cycles of a block's time beside
-// the stores of the next weights, whatever N is up to 64 (a probe of such products alone: 47), so a stage takes some 1150 cycles.
+// k. It takes some 1150: the eight products of a stage take their issuing lane 700 (tensor pipe 15 % active, DRAM 20 %; a probe
+// of such products alone takes 47 each), so their way through tensor memory beside the stores of the next weights is
+// what the stages wait for.
 // 40 rows: 16384 x 5120 30.5 us, 5120 x 6144 23.0, 34816 x 5120 47.8 (62 as pairs of blocks), 5120 x 17408 34.5; padded to 256
 // tokens they took 69, 68, 70 and 89. What else differs from the prompt-sized product:
 //   - the weights are the exact integers q - 8; a group of 128 columns is one accumulation, and the drain warps multiply its
