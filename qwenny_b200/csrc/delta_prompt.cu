@@ -31,9 +31,11 @@ namespace qb {
 // blocks makes the gates. Bound by the rows' way from memory and back (n x 80 KB): every row of the tile is requested
 // before anything is used, 16 bytes per lane, and the head's norm is a warp reduction (2048 tokens: 62 us; 79 us with
 // a channel per thread, four bytes per request and the gates behind the first head's channels).
+// VEC: p and cv start on 16 bytes, as a device allocation does; elsewhere (any float address is allowed) a lane moves its four
+// channels one by one.
 // PREP_TOK: the tokens a block slides along. 8 leave room for five blocks per SM, 16 read less history: the mixer of 40 rows takes
 // 48.0 and 51.2 us with them, of 150 138 and 129, of 333 179 and 174, of 700 245 and 256, of 1300 328 and 338.
-template <int PREP_TOK>
+template <int PREP_TOK, bool VEC>
 __global__ void __launch_bounds__(128, PREP_TOK == 8 ? 5 : 4)
 delta_prep_kernel(const float* p, int splits, int n, const float* ba, int ba_splits, const float* cw,
                   const float* a_log, const float* dt_bias, const float* mem, long long sst, float* cv,
@@ -64,22 +66,23 @@ delta_prep_kernel(const float* p, int splits, int n, const float* ba, int ba_spl
     for (int c = 0; c < 4; c++) taps[c] = ld4(cw + (size_t)(ch + c) * CONV_K);
     pdl_wait();
     const size_t stride = (size_t)n * DELTA_IN;
+    auto row4 = [](const float* r) { return VEC ? ld4(r) : make_float4(r[0], r[1], r[2], r[3]); };
     // lane i < PREP_TOK: token tb + i's slot and position; the next three: the slots of the three tokens before the tile
     const int mt = min(lane < PREP_TOK ? tb + lane : max(tb - PREP_TOK - 3 + lane, 0), n - 1);
     const int my_slot = tok_slot[mt], my_pos = tok_pos[mt];
     float4 x[PREP_TOK], h[3];  // h: the conv inputs at the three positions before the current token
 #pragma unroll
-    for (int i = 0; i < 3; i++) h[i] = ld4(p + (size_t)max(tb - 3 + i, 0) * DELTA_IN + ch);
+    for (int i = 0; i < 3; i++) h[i] = row4(p + (size_t)max(tb - 3 + i, 0) * DELTA_IN + ch);
 #pragma unroll
-    for (int i = 0; i < PREP_TOK; i++) x[i] = ld4(p + (size_t)min(tb + i, n - 1) * DELTA_IN + ch);
+    for (int i = 0; i < PREP_TOK; i++) x[i] = row4(p + (size_t)min(tb + i, n - 1) * DELTA_IN + ch);
     // (the other partial sums in a loop of their own: one inside the row's load makes the loads wait for one another)
     for (int s = 1; s < splits; s++) {
         const float* ps = p + s * stride + ch;
         auto add = [](float4& v, float4 w) { v.x += w.x; v.y += w.y; v.z += w.z; v.w += w.w; };
 #pragma unroll
-        for (int i = 0; i < 3; i++) add(h[i], ld4(ps + (size_t)max(tb - 3 + i, 0) * DELTA_IN));
+        for (int i = 0; i < 3; i++) add(h[i], row4(ps + (size_t)max(tb - 3 + i, 0) * DELTA_IN));
 #pragma unroll
-        for (int i = 0; i < PREP_TOK; i++) add(x[i], ld4(ps + (size_t)min(tb + i, n - 1) * DELTA_IN));
+        for (int i = 0; i < PREP_TOK; i++) add(x[i], row4(ps + (size_t)min(tb + i, n - 1) * DELTA_IN));
     }
     int prev_slot = -1;
 #pragma unroll
@@ -123,7 +126,9 @@ delta_prep_kernel(const float* p, int splits, int n, const float* ba, int ba_spl
                 if (head < LK_HEADS) sc *= rsqrtf((float)LKD);
                 y.x *= sc; y.y *= sc; y.z *= sc; y.w *= sc;
             }
-            *(float4*)(cv + (size_t)t * CVW + ch) = y;
+            float* to = cv + (size_t)t * CVW + ch;
+            if (VEC) *(float4*)to = y;
+            else { to[0] = y.x; to[1] = y.y; to[2] = y.z; to[3] = y.w; }
         }
     }
 }
@@ -682,8 +687,11 @@ int qb_delta_conv(qb_ctx* ctx, void* stream, const float* p, int splits, int n, 
         return QB_ERR_ARG;
     const bool wide = n > 128 && n <= 512;
     const dim3 grid(LQKV / 512 + 1, wide ? (n + 15) / 16 : (n + 7) / 8);
-    return launch(ctx, wide ? delta_prep_kernel<16> : delta_prep_kernel<8>, grid, dim3(128), 0, (cudaStream_t)stream, p, splits, n, ba,
-                  ba_splits, cw, a_log, dt_bias, mem, sst, cv, tok_slot, tok_pos);
+    const bool vec = (((uintptr_t)p | (uintptr_t)cv) & 15) == 0;
+    auto kern = vec ? (wide ? delta_prep_kernel<16, true> : delta_prep_kernel<8, true>)
+                    : (wide ? delta_prep_kernel<16, false> : delta_prep_kernel<8, false>);
+    return launch(ctx, kern, grid, dim3(128), 0, (cudaStream_t)stream, p, splits, n, ba, ba_splits, cw, a_log, dt_bias, mem, sst, cv,
+                  tok_slot, tok_pos);
 }
 
 // The scratch of the chunked form (T, P and the log decays of every chunk and value head of a step of up to 2048

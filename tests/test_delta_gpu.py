@@ -382,3 +382,24 @@ def test_chunked_rule_against_the_oracle(ctx, lens):
     want = R.delta_rule(part.numpy(), cvh, omem, SST, meta, st["seg_start"], st["seg_len"], st["seg_slot"], st["seg_pos0"])
     assert close(out.cpu().numpy(), want).all()
     assert np.abs(dmem.cpu().numpy() - omem).max() < 1e-4
+
+
+@pytest.mark.parametrize("n", [5, 150])
+def test_conv_of_rows_at_any_float_address(ctx, n):
+    """p and cv may start at any float address (a slice of a larger buffer): the bits of the 16-byte aligned call, in both
+    tile sizes."""
+    g = synth.gen(191 + n)
+    conv_w, a_log, dt_bias, _ = (t.cuda() for t in weights(g))
+    mem, part = (fresh_mem(1, g) * 100).cuda(), torch.randn(2, n, R.DELTA_IN, generator=g).cuda()
+    ba = torch.randn(3, n, 2 * R.LV_HEADS, generator=g).cuda()
+    st = R.build_step([(0, 0, 7 + i) for i in range(n)], [])
+    dv = ref_cuda.upload_step(st)
+    want = torch.zeros(n, R.CVW, device="cuda")
+    ctx.delta_conv(part, 2, n, ba, 3, conv_w, a_log, dt_bias, mem, SST, want, dv)
+    for dp, dc in ((1, 0), (0, 1), (3, 2)):
+        p = torch.zeros(part.numel() + 4, device="cuda")[dp:dp + part.numel()].view_as(part)
+        p.copy_(part)
+        cv = torch.zeros(want.numel() + 4, device="cuda")[dc:dc + want.numel()].view_as(want)
+        assert p.data_ptr() % 16 == 4 * dp and cv.data_ptr() % 16 == 4 * dc
+        ctx.delta_conv(p, 2, n, ba, 3, conv_w, a_log, dt_bias, mem, SST, cv, dv)
+        assert torch.equal(cv, want)
