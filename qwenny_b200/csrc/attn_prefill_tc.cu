@@ -96,7 +96,8 @@ attn_prefill_tc_kernel(const float* q, const uint8_t* kc, const uint8_t* vc, con
     uint64_t* s_ready = v_free + NST;     // [2] S of a stage is complete in tensor memory
     uint64_t* p_ready = s_ready + 2;       // [2] (first block) P of a stage is written over its S in both blocks
     uint64_t* o_done = p_ready + 2;        // [2] O += P V of a stage is complete
-    uint32_t* tmem_slot = (uint32_t*)(o_done + 2);
+    uint64_t* sc_ready = o_done + 2;       // [NSC] a stage's scales are written in this block (for its softmax warps)
+    uint32_t* tmem_slot = (uint32_t*)(sc_ready + NSC);
 
     const int g = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, rank = (int)cluster_ctarank();
     if (threadIdx.x == 0) {
@@ -111,6 +112,7 @@ attn_prefill_tc_kernel(const float* q, const uint8_t* kc, const uint8_t* vc, con
             mbar_init(&p_ready[i], 2 * SM_WARPS);
             mbar_init(&o_done[i], 1);
         }
+        for (int i = 0; i < NSC; i++) mbar_init(&sc_ready[i], CVT_WARPS);
         mbar_fence_init();
     }
     if (warp == MMA_WARP) {
@@ -209,7 +211,9 @@ attn_prefill_tc_kernel(const float* q, const uint8_t* kc, const uint8_t* vc, con
             float m = -INFINITY, l = 0.f;
             for (int i = 0; i < nstg; i++) {
                 const int J = jbase + i, b2 = J & 1, kb0 = i * SK + 64 * half;
-                w_sm.wait(&s_ready[b2], (J >> 1) & 1, lane);
+                // the scales come from the convert warps by plain stores: a barrier of this block orders them (S itself goes by way of
+                // the first block's tensor core, which promises nothing about the second block's plain stores)
+                w_sm.wait_both(&s_ready[b2], (J >> 1) & 1, &sc_ready[J % NSC], (J / NSC) & 1, lane);
                 tc_fence_after();
                 const uint32_t ts = trow + S_COL + b2 * SK + 64 * half;
                 const float4* ksc4 = (const float4*)(scl + (J % NSC) * 2 * SK + 64 * half);
@@ -373,7 +377,10 @@ attn_prefill_tc_kernel(const float* q, const uint8_t* kc, const uint8_t* vc, con
                 scl[(J % NSC) * 2 * SK + ct] = sraw;
                 async_proxy_fence();
                 __syncwarp();
-                if (lane == 0) mbar_arrive_at(k_ready0 + 8 * rs);
+                if (lane == 0) {
+                    mbar_arrive(&sc_ready[J % NSC]);
+                    mbar_arrive_at(k_ready0 + 8 * rs);
+                }
                 if (i + 1 < nstg) fetch_k(i + 1);  // (after the fence, which would wait for it)
                 if (J >= NST) w_cv.wait(&v_free[rs], (J / NST - 1) & 1, lane);
                 uint8_t* vt = vf + rs * V_BYTES + (vt0 >> 2) * (V_BYTES / 2);

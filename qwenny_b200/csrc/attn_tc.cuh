@@ -84,6 +84,19 @@ struct Waiter {
             if (lane == 0) atomicExch(err, code);
         }
     }
+    // two barriers at once, a lane each: about as long as one wait (2048 rows of prompt attention at context 30720: 1917 us
+    // without the second wait, 2024 with one after the other, 1930 so)
+    __device__ __forceinline__ void wait_both(uint64_t* bar, uint32_t parity, uint64_t* bar1, uint32_t parity1, int lane) {
+        if (dead) return;
+        bool ok = true;
+        if (lane < 2) ok = mbar_wait_sleepy(lane ? bar1 : bar, lane ? parity1 : parity);
+        ok = __all_sync(0xffffffffu, ok);
+        if (!ok) {
+            dead = true;
+            if (lane == 0) atomicExch(err, code);
+        }
+        __syncwarp();  // (orders the other lanes' reads behind both)
+    }
 };
 
 }  // namespace tc

@@ -10,6 +10,7 @@ import torch
 from oracle import ref_cuda
 from oracle import ref_ops as R
 from qwenny_b200 import synth
+from qwenny_b200._lib import lib
 
 pytestmark = pytest.mark.gpu
 RTOL, ATOL = 1e-2, 2e-3
@@ -304,3 +305,32 @@ def test_attn_decode_of_a_ragged_batch(ctx, rows):
         assert torch.equal(one, full[a:e])
     want = R.attn_decode(q.numpy(), gate.numpy(), *[t.numpy() for t in cache], st["tok_slot"], st["tok_pos"], cap)
     assert close(full.cpu().numpy(), want).all()
+
+
+def test_attn_prefill_several_sequences_on_pairs(ctx):
+    """The form on pairs of blocks over runs of several sequences: pairs with one, two and three runs of one to four tiles, odd and
+    even stage counts, a cache whose length is an odd multiple of 64 and keys in its last half stage, against the oracle at
+    the ends of every sequence and tile."""
+    g = synth.gen(167)
+    lens, pos0, cap = (25, 33, 12, 47, 280), (2080, 1700, 1900, 40, 1663), 2112
+    cache = make_cache(len(lens), cap, g, 0)
+    toks = [(0, s, p + i) for s, (n, p) in enumerate(zip(lens, pos0)) for i in range(n)]
+    n = len(toks)
+    q = torch.randn(n, R.NH, R.HD, generator=g) * QSCALE
+    gate = torch.sigmoid(torch.randn(n, R.MIX, generator=g))
+    st = R.build_step(toks, list(range(n)))
+    keys = st["tile_max_pos"] + 1
+    assert st["ndec"] == 0 and st["ntile"] == 42 and 1664 < keys <= cap and cap % 128 == 64 and cap - keys < 64
+    assert lib().qb_attn_tile_splits(st["ntile"], keys) == 1  # one key split: the tcgen05 kernels
+    mine, mix = run_prefill(ctx, q.cuda(), gate.cuda(), [t.cuda() for t in cache], st, ref_cuda.upload_step(st), cap, n, mix=True)
+    torch.cuda.synchronize()
+    assert ctx.device_error() == 0
+    a = mine.cpu().numpy()
+    assert np.array_equal(mix.cpu().numpy(), a.astype(np.float16))
+    rows, at = [], 0
+    for m in lens:
+        rows += [at, at + min(9, m - 1), at + min(10, m - 1), at + m // 2, at + m - 1]
+        at += m
+    want = R.attn_decode(q.numpy()[rows], gate.numpy()[rows], *[t.numpy() for t in cache], st["tok_slot"][rows],
+                         st["tok_pos"][rows], cap)
+    assert close(a[rows], want).all()
