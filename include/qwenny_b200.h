@@ -32,7 +32,9 @@ typedef struct qb_ctx qb_ctx;
 enum { QB_EPI_PLAIN = 0, QB_EPI_SILU = 1, QB_EPI_ARGMAX = 2 };
 
 /* ---- context: what Gemm::load allocates once (src/cuda/core.rs:437-464: SM count, Marlin's `red` and `locks`).
- * Allocates the split-K scratch and tickets on `device`; everything after creation is allocation-free. Like the
+ * Allocates the scratch and tickets on `device`: 32 MiB for the skinny products and, where there is room, 91 MB for the
+ * prompt-sized kernels (without them 17 to 64 rows run as 16-row slabs, larger products as whole tiles and the delta rule
+ * token by token). Everything after creation is allocation-free. Like the
  * reference's single `red` / `locks` pair, a context serves one stream at a time: launches that share a context must
  * not overlap on the device (models that run concurrently take a context each). */
 int qb_create(int device, qb_ctx** out);
@@ -46,8 +48,7 @@ const char* qb_version(void);
  * (src/cuda/core.rs:569-612) of marlin_m1_n8_{plain,silu,argmax} (kernels/marlin.cuh:588-602) for m <= 16 rows and of
  * marlin_m{1..4}_n16_* (the prompt chunks' products, kernels/qwen.cu:48) beyond: 17 to 64 rows run on a tensor-core
  * product (tcgen05) with every epilogue, contiguous or gathered; more than 64 contiguous rows with the plain or SwiGLU
- * epilogue on the prompt-sized one, the others as 64-row slabs. The first such product takes the context's scratch for
- * them; where it cannot be had (no memory, a stream being captured) up to 64 rows run as 16-row slabs.
+ * epilogue on the prompt-sized one, the others as 64-row slabs.
  *   X      f16 [.][k]; rows row0 .. row0+m-1 are read, or rows xrows[0..m) when xrows != NULL (this folds
  *          marlin_gather, kernels/marlin.cuh:605-608, into the product)
  *   B      Marlin words, k/16 x 2n u32 (src/cuda/core.rs:262-311 pack_marlin); S f16 [k/128][n] permuted scales

@@ -74,31 +74,56 @@ const char* qb_version(void) { return "qwenny_b200 0.1 (sm_100a)"; }
 int qb_create(int device, qb_ctx** out) {
     if (!out) return QB_ERR_ARG;
     QB_CUDA(cudaSetDevice(device));
+    int sms = 0;
+    QB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
+    // One allocation: the words that must be zero (counters, error word, tickets), the split-K partials of the skinny products,
+    // then what only prompt-sized kernels use. Calls allocate nothing, so that they can be captured and a host may give all
+    // other memory away; where the last part does not fit, the context does without it.
+    // The split-K partials' largest user is a 16-row product, [n/64][nsplit][2][4][32] float4; 32 MiB covers
+    // n * nsplit up to 2^17 * 8 (the 27B shapes need under 6 MiB).
+    const size_t ncounters = 1 << 14, err_at = ncounters * sizeof(int), tickets_at = err_at + 256;
+    const size_t scratch_at = tickets_at + QB_TC_TICKETS * sizeof(int), scratch_bytes = 32u << 20, part_at = scratch_at + scratch_bytes;
+    const size_t tp_at = part_at + qb_tc_part_bytes(sms);
+    char* b = nullptr;
+    const bool all = cudaMalloc(&b, tp_at + qb_delta_tp_bytes()) == cudaSuccess;
+    if (!all) {
+        (void)cudaGetLastError();
+        QB_CUDA(cudaMalloc(&b, part_at));
+    }
+    cudaError_t e = cudaMemset(b, 0, scratch_at);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(0);  // (a context's stream need not wait for the default one)
+    if (e != cudaSuccess) {
+        cudaFree(b);
+        return (int)e;
+    }
     qb_ctx* c = new qb_ctx();
     c->device = device;
-    QB_CUDA(cudaDeviceGetAttribute(&c->sms, cudaDevAttrMultiProcessorCount, device));
-    // the largest user: split-K partials of a 16-row product, [n/64][nsplit][2][4][32] float4; 32 MiB covers
-    // n * nsplit up to 2^17 * 8 (the 27B shapes need under 6 MiB)
-    c->scratch_bytes = 32u << 20;
-    QB_CUDA(cudaMalloc(&c->scratch, c->scratch_bytes));
-    c->ncounters = 1 << 14;
-    QB_CUDA(cudaMalloc(&c->counters, c->ncounters * sizeof(int)));
-    QB_CUDA(cudaMemset(c->counters, 0, c->ncounters * sizeof(int)));
-    QB_CUDA(cudaMalloc(&c->err, 64));
-    QB_CUDA(cudaMemset(c->err, 0, 64));
+    c->sms = sms;
+    c->block = b;
+    c->counters = (int*)b;
+    c->ncounters = ncounters;
+    c->err = (int*)(b + err_at);
+    c->scratch = (float*)(b + scratch_at);
+    c->scratch_bytes = scratch_bytes;
+    if (all) {
+        c->tc_tickets = (int*)(b + tickets_at);
+        c->tc_part = (float*)(b + part_at);
+        c->delta_tp = (float*)(b + tp_at);
+    }
     *out = c;
     return QB_OK;
 }
 
 void qb_destroy(qb_ctx* c) {
     if (!c) return;
-    cudaFree(c->scratch);
-    cudaFree(c->counters);
-    cudaFree(c->err);
-    cudaFree(c->delta_tp);
-    cudaFree(c->tc_part);
-    cudaFree(c->tc_tickets);
+    cudaFree(c->block);
     delete c;
+}
+
+int qb_scratch_forget(qb_ctx* c) {
+    if (!c) return QB_ERR_ARG;
+    c->tc_part = nullptr; c->tc_tickets = nullptr; c->delta_tp = nullptr;
+    return QB_OK;
 }
 
 int qb_device_error(qb_ctx* c) {

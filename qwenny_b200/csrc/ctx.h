@@ -15,10 +15,12 @@ struct qb_ctx {
     int* counters = nullptr;
     size_t ncounters = 0;
     int* err = nullptr;  // device word
-    float* tc_part = nullptr;   // partial tiles of the tensor-core W4A16 product's stream-K shares (sms x 256 KB), taken with its first call
-    int* tc_tickets = nullptr;  // its tickets, two per tile (QB_TC_TICKETS, zero between launches)
-    float* delta_tp = nullptr;  // scratch of the chunked delta rule (T, P, log decays per chunk and value head), taken by
-                                // the first prompt-sized DeltaNet step
+    // The prompt-sized kernels' scratch. It is taken at creation like the rest, in one allocation with it (`block`); a device
+    // that has room for the rest alone gets a context without it, whose calls take the forms that need none.
+    void* block = nullptr;
+    float* tc_part = nullptr;   // partial tiles of the tensor-core W4A16 products' shares (sms x 256 KB)
+    int* tc_tickets = nullptr;  // their tickets, two per tile (QB_TC_TICKETS, zero between launches)
+    float* delta_tp = nullptr;  // the chunked delta rule's T, P and log decays per chunk and value head (52 MB)
     // measurement override of the GEMV plan (0: built-in choice)
     int tune_cg = 0, tune_kg = 0, tune_nstages = 0, tune_ctas = 0;
     bool no_cluster = false, no_tc = false;
@@ -74,8 +76,9 @@ int qb_attn_prefill_short_launch(qb_ctx* ctx, cudaStream_t st, const float* q, c
 // S carries the offsets' table after the scales) for more than 16 rows
 int qb_gemm_tc_launch(qb_ctx* ctx, cudaStream_t st, const void* X, const void* B, void* Y, const void* S, int m, int n,
                       int k, int row0, int epi, int zp);
-// the scratch of the two products on pairs of blocks (partial tiles, tickets), taken with the first one
-int qb_tc_scratch(qb_ctx* ctx);
+// bytes of the prompt-sized kernels' scratch: tc_part on a part with `sms` SMs, delta_tp
+size_t qb_tc_part_bytes(int sms);
+size_t qb_delta_tp_bytes();
 // the product for 17 .. 64 rows (w4a16_gemm_mid.cu), symmetric matrices; reached through qb_marlin_gemm
 int qb_gemm_mid_launch(qb_ctx* ctx, cudaStream_t st, const void* X, const void* B, void* Y, const void* S, int m, int n, int k,
                        int row0, int epi, const int* xrows, unsigned long long* keys, int n_valid);

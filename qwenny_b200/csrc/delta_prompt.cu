@@ -136,6 +136,7 @@ delta_prep_kernel(const float* p, int splits, int n, const float* ba, int ba_spl
 // ------------------------------------------------------------------------------------------------ the chunked form
 constexpr int CH = 64;                   // tokens per chunk
 constexpr int TP_FLOATS = 2 * CH * CH + CH;  // per (chunk, value head): T, P, the cumulative log decays
+constexpr int TP_TOK = 2048;             // tokens of a step at most
 constexpr int KLD = LKD + 4;             // row stride of the q / k / state tiles (floats): fragment loads hit 32 banks
 constexpr int TLD = CH + 4;              // ... of T and P
 
@@ -392,7 +393,7 @@ delta_scan_kernel(const float* p, int splits, int n, const float* cv, const floa
     }
     pdl_wait();
 
-    const int l0 = chunked_tokens(len);
+    const int l0 = tp ? chunked_tokens(len) : 0;
     if (l0 > 0) {
         // ================================================================ chunks
         st_rows<8>(&M.s[lc][0], S, sub);
@@ -677,6 +678,8 @@ delta_gate_norm_kernel(const float* p, int splits, int n, const float* nw, const
 
 using namespace qb;
 
+size_t qb_delta_tp_bytes() { return (size_t)(TP_TOK / CH + 1) * LV_HEADS * TP_FLOATS * sizeof(float); }
+
 extern "C" {
 
 int qb_delta_conv(qb_ctx* ctx, void* stream, const float* p, int splits, int n, const float* ba, int ba_splits,
@@ -694,23 +697,18 @@ int qb_delta_conv(qb_ctx* ctx, void* stream, const float* p, int splits, int n, 
                   tok_slot, tok_pos);
 }
 
-// The scratch of the chunked form (T, P and the log decays of every chunk and value head of a step of up to 2048
-// tokens, 52 MB) belongs to the context and is allocated by the first step that has a segment long enough to run in
-// chunks: a prompt-sized step, which is never captured into a graph.
+// The chunked form's scratch (T, P and the log decays of every chunk and value head of a step of up to 2048 tokens, 52 MB)
+// belongs to the context; one that was created without it runs every segment in the token form.
 int qb_delta_rule(qb_ctx* ctx, void* stream, const float* p, int splits, int n, const float* cv, float* mem,
                   long long sst, const int* meta, float* out, const int* seg_start, const int* seg_len,
                   const int* seg_slot, const int* seg_pos0, int segs) {
     if (!ctx || !p || !cv || !mem || !meta || !out || !seg_start || !seg_len || !seg_slot || !seg_pos0 || n <= 0 ||
         segs <= 0 || splits < 1)
         return QB_ERR_ARG;
-    constexpr int MAX_TOK = 2048;
     cudaStream_t st = (cudaStream_t)stream;
-    const int chunks = chunked_tokens(n) / CH;  // of the longest segment the step can hold
+    if (n > TP_TOK) return QB_ERR_TOO_LARGE;
+    const int chunks = ctx->delta_tp ? chunked_tokens(n) / CH : 0;  // of the longest segment the step can hold
     if (chunks > 0) {
-        if (n > MAX_TOK) return QB_ERR_TOO_LARGE;
-        if (!ctx->delta_tp) {
-            QB_CUDA(cudaMalloc(&ctx->delta_tp, (size_t)(MAX_TOK / CH + 1) * LV_HEADS * TP_FLOATS * sizeof(float)));
-        }
         int rc = launch(ctx, delta_chunk_prep_kernel, dim3(chunks, LK_HEADS, segs), dim3(CP_THREADS), CP_SMEM, st, cv,
                         ctx->delta_tp, seg_start, seg_len);
         if (rc) return rc;

@@ -254,17 +254,6 @@ static int gemm_rows(qb_ctx* ctx, cudaStream_t st, const void* X, const void* B,
 #undef QB_GO
 }
 
-// The product for 17 .. 64 rows needs the pair products' scratch, which the first one allocates. Where that cannot be had (no
-// memory left, a stream being captured) the rows run as 16-row slabs, which need nothing.
-static bool pair_scratch(qb_ctx* ctx, cudaStream_t st) {
-    if (ctx->tc_part) return true;
-    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(st, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) return false;
-    if (qb_tc_scratch(ctx) == QB_OK) return true;
-    (void)cudaGetLastError();
-    return false;
-}
-
 extern "C" int qb_marlin_gemm(qb_ctx* ctx, void* stream, const void* X, const void* B, void* Y, const void* S, int m,
                               int n, int k, int row0, int epi, const int* xrows, unsigned long long* keys,
                               int n_valid) {
@@ -284,7 +273,7 @@ extern "C" int qb_marlin_gemm(qb_ctx* ctx, void* stream, const void* X, const vo
     int mm;
     for (int r = 0; r < m; r += mm) {
         mm = m - r;
-        if (mm > 16 && !ctx->no_tc && pair_scratch(ctx, st)) {
+        if (mm > 16 && !ctx->no_tc && ctx->tc_part) {
             if (mm > 64) mm = 64;
             int rc = qb_gemm_mid_launch(ctx, st, X, B, Y, S, mm, n, k, xrows ? 0 : row0 + r, epi, xrows ? xrows + r : nullptr,
                                         keys ? keys + (xrows ? r : 0) : nullptr, n_valid);

@@ -23,6 +23,8 @@ int qb_model_fail_captures(struct qb_model* m, int n);
  * kernel-attribute bookkeeping; 0 when they hold. */
 int qb_graph_cache_selftest(void);
 int qb_attr_cache_selftest(void);
+/* Tests: the context goes on as one that was created where the prompt-sized kernels' scratch did not fit. */
+int qb_scratch_forget(qb_ctx* ctx);
 /* Tests: one block waits on an mbarrier that nothing arrives on, with the library's bounded wait cut to `limit` polls
  * (at most 2^20); the wait runs out and the context's error word reads 99 (qb_device_error). */
 int qb_wait_probe(qb_ctx* ctx, void* stream, unsigned limit);

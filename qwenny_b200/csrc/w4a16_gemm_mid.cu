@@ -390,7 +390,7 @@ using namespace qb;
 // 1 .. 64 rows of X (row0 .., or xrows[0 .. m)); results at rows y0 .. of Y; keys[y0 .. y0 + m) for the argmax epilogue
 int qb_gemm_mid_launch(qb_ctx* ctx, cudaStream_t st, const void* X, const void* B, void* Y, const void* S, int m, int n, int k,
                        int row0, int epi, const int* xrows, unsigned long long* keys, int n_valid) {
-    if (n % mid::BH || k % 128 || m < 1 || m > 64) return QB_ERR_ARG;
+    if (n % mid::BH || k % 128 || m < 1 || m > 64 || !ctx->tc_part) return QB_ERR_ARG;
     EncodeTiled enc = encode_tiled();
     if (!enc) return QB_ERR_UNSUPPORTED;
     const int nt = m <= 32 ? 32 : m <= 48 ? 48 : 64;
@@ -411,7 +411,6 @@ int qb_gemm_mid_launch(qb_ctx* ctx, cudaStream_t st, const void* X, const void* 
     if (enc(&wmap, CU_TENSOR_MAP_DATA_TYPE_UINT64, 2, (void*)B, wd, ws, wb, one, CU_TENSOR_MAP_INTERLEAVE_NONE,
             CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
         return QB_ERR_ARG;
-    if (int rc = qb_tc_scratch(ctx)) return rc;
     mid::Args a;
     a.X = (const __half*)X; a.xrows = xrows; a.S = (const __half*)S; a.Y = Y; a.keys = keys; a.m = m; a.N = n; a.K = k;
     a.row0 = row0; a.y0 = xrows ? 0 : row0; a.n_valid = n_valid; a.err = ctx->err; a.part = ctx->tc_part;

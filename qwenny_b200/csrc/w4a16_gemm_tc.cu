@@ -326,18 +326,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
 
 using namespace qb;
 
-int qb_tc_scratch(qb_ctx* ctx) {
-    if (ctx->tc_part) return QB_OK;
-    if (!ctx->tc_tickets) {
-        int* t = nullptr;
-        QB_CUDA(cudaMalloc(&t, QB_TC_TICKETS * sizeof(int)));
-        ctx->tc_tickets = t;
-    }
-    QB_CUDA(cudaMemset(ctx->tc_tickets, 0, QB_TC_TICKETS * sizeof(int)));
-    QB_CUDA(cudaStreamSynchronize(0));  // (the product's stream need not wait for the default one)
-    QB_CUDA(cudaMalloc(&ctx->tc_part, (size_t)(ctx->sms / 2) * 2 * tc::BT * tc::BO * sizeof(float)));  // two partial tiles per pair
-    return QB_OK;
-}
+size_t qb_tc_part_bytes(int sms) { return (size_t)(sms / 2) * 2 * tc::BT * tc::BO * sizeof(float); }  // two partial tiles per pair
 
 // Y = X . W^T for many rows: plain (f32 [m][n]) or SwiGLU (f16 [m][n/2]). X f16 [.][k], rows row0 .. row0 + m - 1.
 int qb_gemm_tc_launch(qb_ctx* ctx, cudaStream_t st, const void* X, const void* B, void* Y, const void* S, int m, int n,
@@ -365,7 +354,6 @@ int qb_gemm_tc_launch(qb_ctx* ctx, cudaStream_t st, const void* X, const void* B
             CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
         return QB_ERR_ARG;
     const int pairs = ctx->sms / 2;
-    if (int rc = qb_tc_scratch(ctx)) return rc;
     tc::Args a;
     a.B = (const uint32_t*)B; a.S = (const __half*)S; a.Y = Y; a.m = m; a.N = n; a.K = k; a.row0 = row0; a.err = ctx->err;
     a.zp = zp ? 1 : 0; a.part = ctx->tc_part; a.tickets = ctx->tc_tickets; a.iters = tiles * (k / tc::BK);
@@ -379,6 +367,7 @@ int qb_gemm_tc_launch(qb_ctx* ctx, cudaStream_t st, const void* X, const void* B
     bool whole = (long long)(waves + 0.999999) < 1.2 * waves;
     if (ctx->tune_ctas == 1000) whole = false;  // measurement: shares whatever the shape
     if (ctx->tune_ctas == 1001) whole = true;   //              tiles whatever the shape
+    if (!ctx->tc_part) whole = true;            // a context without the scratch
     const int G = whole ? (int)tiles : (int)(a.iters < pairs ? a.iters : pairs);
     dim3 grid((unsigned)(2 * G));
     if (epi == QB_EPI_SILU)

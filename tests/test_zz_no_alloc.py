@@ -169,3 +169,98 @@ def test_a_product_whose_stage_never_lands_gives_up_and_reports_it(ctx):
         finally:
             lib().qb_marlin_probe(ctx.h, 0)
             ctx.tune()
+
+
+def _prompt_calls(c, g):
+    """Calls of every kernel that uses the prompt-sized scratch, as closures that return their outputs: 40 gathered rows with
+    greedy keys, 600 rows in equal shares of the tile list, the delta rule over 150 tokens (chunks and a token tail)."""
+    from oracle import ref_cuda, ref_ops as R
+    dev = lambda a: torch.from_numpy(a).cuda()
+    codes, sc = synth.int4_matrix(1024, 2048, g)
+    words, s16 = host.pack_marlin(codes, sc)
+    wd, sd = dev(words.view(np.int32)), dev(s16.view(np.int16)).view(torch.float16)
+    x40, x600 = (dev(synth.activations(m, 2048, g)) for m in (40, 600))
+    order = torch.randperm(40, generator=g).to(torch.int32).cuda()
+    y40, y600, keys = torch.zeros(40, 1024, device="cuda"), torch.zeros(600, 1024, device="cuda"), torch.zeros(40, dtype=torch.int64, device="cuda")
+    n, sst = 150, (R.SLOT_FLOATS + 1023) // 1024 * 1024
+    dv = ref_cuda.upload_step(R.build_step([(0, 0, i) for i in range(n)], []))
+    part, out = torch.randn(1, n, R.DELTA_IN, generator=g).cuda(), torch.zeros(n, R.MIX, device="cuda")
+    cv = torch.randn(n, R.CVW, generator=g).cuda() * 0.1
+    cv[:, R.LQKV:] = torch.rand(n, 2 * R.LV_HEADS, generator=g).cuda() * 0.5 + 0.4
+    mem0 = (torch.randn(sst, generator=g) * 0.01).cuda()
+    mem, meta = mem0.clone(), torch.zeros(1, 4, dtype=torch.int32, device="cuda")
+
+    def product():
+        keys.zero_()
+        c.marlin_gemm(x40, wd, sd, epi="argmax", y=y40, xrows=order, keys=keys, n_valid=1000)
+        return y40, keys
+
+    def shares():
+        c.marlin_gemm(x600, wd, sd, y=y600)
+        return (y600,)
+
+    def rule():
+        mem.copy_(mem0)
+        c.delta_rule(part, 1, n, cv, mem, sst, meta, out, dv, 1)
+        return out, mem
+    return product, shares, rule
+
+
+def _outputs(calls):
+    r = [[t.clone() for t in f()] for f in calls]
+    torch.cuda.synchronize()
+    return r
+
+
+def test_calls_on_a_context_allocate_nothing(ctx):
+    """The header's contract: a context allocates at creation and nowhere else. Free device memory is the same before and after
+    the first prompt-sized calls on a new context, and such first calls may be captured: a replay gives the eager bits."""
+    from qwenny_b200.ops import Context
+    want = _outputs(_prompt_calls(ctx, synth.gen(901)))   # (loads the kernels)
+    c = Context(0)
+    calls = _prompt_calls(c, synth.gen(901))
+    torch.cuda.synchronize()
+    before = torch.cuda.mem_get_info()[0]
+    for f in calls:
+        f()
+    torch.cuda.synchronize()
+    assert torch.cuda.mem_get_info()[0] == before
+    c.close()
+    c = Context(0)
+    calls = _prompt_calls(c, synth.gen(901))
+    graph = torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph):
+        outs = [f() for f in calls]
+    graph.replay()
+    torch.cuda.synchronize()
+    for a, b in zip(outs, want):
+        assert all(torch.equal(x, y) for x, y in zip(a, b))
+    assert c.device_error() == 0
+    del graph
+    c.close()
+
+
+def test_a_context_without_the_prompt_sized_scratch(ctx):
+    """A context created where the prompt-sized scratch did not fit: the same calls run as 16-row slabs, as whole tiles and token by
+    token, with the bits of those forms, and allocate nothing."""
+    from qwenny_b200.ops import Context
+    calls = _prompt_calls(ctx, synth.gen(902))
+    want = _outputs(calls)
+    try:
+        ctx.tune(nstages=-1)
+        slabs = _outputs(calls[:1])[0]
+        ctx.tune(ctas=1001)
+        whole = _outputs(calls[1:2])[0]
+    finally:
+        ctx.tune()
+    c = Context(0)
+    assert lib().qb_scratch_forget(c.h) == 0 and lib().qb_scratch_forget(None) == 1000
+    got = _outputs(_prompt_calls(c, synth.gen(902)))
+    assert all(torch.equal(a, b) for a, b in zip(got[0], slabs))
+    assert torch.equal(got[1][0], whole[0])
+    # outputs of the two forms of the rule agree as closely as the chunked form with the recurrence: 1e-4 of the state's scale
+    for a, b in zip(got[2], want[2]):
+        assert (a - b).abs().max() < 1e-4 * max(1.0, b.abs().max().item())
+    assert c.device_error() == 0
+    c.close()
