@@ -180,17 +180,19 @@ __device__ __forceinline__ void mma3(float* c, const FragA& a, float b0, float b
 // grid (chunks of the longest possible segment, LK_HEADS, segs), block 256. tp: [chunk index][LV_HEADS][TP_FLOATS],
 // chunk index = first token of the chunk / 64 (distinct for disjoint 64-token ranges).
 constexpr int CP_THREADS = 256;
-constexpr int CP_SMEM = (2 * CH * KLD + 6 * CH) * 4;  // 69 KB: three blocks per SM
-static_assert(4 * CH * (CH + 1) <= 2 * CH * KLD, "the three A matrices and K K^T reuse the q / k tiles");
+// 102 KB: two blocks per SM. With K K^T and Q K^T over the tiles (69 KB, three blocks) the second exponential and barrier cost
+// more than the third block gives: 2048 tokens 120 -> 126 us, eight segments of 100 63 -> 85, three of 150 with the scan 135 -> 156.
+constexpr int CP_SMEM = (2 * CH * KLD + 2 * CH * (CH + 1) + 6 * CH) * 4;
+static_assert(3 * CH * (CH + 1) <= 2 * CH * KLD, "the three A matrices reuse the q / k tiles");
 
 __global__ void __launch_bounds__(CP_THREADS)
 delta_chunk_prep_kernel(const float* cv, float* tp, const int* seg_start, const int* seg_len) {
     extern __shared__ __align__(16) float cps[];
     float* Ks = cps;                         // [64][KLD]; later A of the three value heads [3][64][65]
     float* Qs = Ks + CH * KLD;
-    float* QK = Ks;                          // [64][65] over the q / k tiles, then A over it
-    float* KK = Ks + 3 * CH * (CH + 1);      // [64][65] behind the place of the three A; later scratch of the inverse
-    float* gs = Qs + CH * KLD;               // [3][64] cumulative log decay
+    float* KK = Qs + CH * KLD;               // [64][65]; later scratch of the inverse
+    float* QK = KK + CH * (CH + 1);
+    float* gs = QK + CH * (CH + 1);          // [3][64] cumulative log decay
     float* bs = gs + 3 * CH;                 // [3][64] beta
     pdl_launch_dependents();
     const int c = blockIdx.x, kh = blockIdx.y, sg = blockIdx.z, tid = threadIdx.x;
@@ -240,7 +242,6 @@ delta_chunk_prep_kernel(const float* cv, float* tp, const int* seg_start, const 
             for (int j = 0; j < 8; j++)
                 if (j < nts) mma3(acc[j], a, br[8 * j * KLD + k0], br[8 * j * KLD + k0 + 4]);
         }
-        __syncthreads();  // every warp is done with the tiles
 #pragma unroll
         for (int j = 0; j < 8; j++) {
             float* d0 = dst + (16 * m + g8) * (CH + 1) + 8 * j + 2 * t4;
@@ -249,20 +250,15 @@ delta_chunk_prep_kernel(const float* cv, float* tp, const int* seg_start, const 
         }
     }
     __syncthreads();
-    // P straight to global memory, then A of the three value heads (over Q K^T, which is done with)
-    for (int x = tid; x < 3 * CH * CH; x += CP_THREADS) {
-        const int hv = x / (CH * CH), i = (x / CH) % CH, j = x % CH;
-        const float dec = j <= i ? expf(gs[hv * CH + i] - gs[hv * CH + j]) : 0.f;
-        float* out = tp + ((size_t)(tok >> 6) * LV_HEADS + kh * G + hv) * TP_FLOATS;
-        out[CH * CH + i * CH + j] = j <= i ? QK[i * (CH + 1) + j] * dec : 0.f;
-        if (j == 0) out[2 * CH * CH + i] = gs[hv * CH + i];
-    }
-    __syncthreads();
+    // A of the three value heads over the q / k tiles (done with), and P straight to global memory
     float* As = Ks;
     for (int x = tid; x < 3 * CH * CH; x += CP_THREADS) {
         const int hv = x / (CH * CH), i = (x / CH) % CH, j = x % CH;
-        As[(hv * CH + i) * (CH + 1) + j] =
-            j < i ? bs[hv * CH + i] * KK[i * (CH + 1) + j] * expf(gs[hv * CH + i] - gs[hv * CH + j]) : 0.f;
+        const float dec = j <= i ? expf(gs[hv * CH + i] - gs[hv * CH + j]) : 0.f;
+        As[(hv * CH + i) * (CH + 1) + j] = j < i ? bs[hv * CH + i] * KK[i * (CH + 1) + j] * dec : 0.f;
+        float* out = tp + ((size_t)(tok >> 6) * LV_HEADS + kh * G + hv) * TP_FLOATS;
+        out[CH * CH + i * CH + j] = j <= i ? QK[i * (CH + 1) + j] * dec : 0.f;
+        if (j == 0) out[2 * CH * CH + i] = gs[hv * CH + i];
     }
     __syncthreads();
     // T = (I + A)^-1, unit lower triangular, IN PLACE over A. The four 16 x 16 diagonal blocks by forward substitution,
@@ -270,7 +266,7 @@ delta_chunk_prep_kernel(const float* cv, float* tp, const int* seg_start, const 
     // 16 -> 32 -> 64: for a block pair [[T11, 0], [T21, T22]] the lower left part is T21 = -T22 (A21 T11), two small
     // products spread over the block (X = A21 T11 goes through scratch, so T21 may overwrite A21).
     float* D0 = KK;                    // [3][4][16][17] the diagonal blocks' inverses
-    float* Xs = KK;                    // [3][32][33] scratch of the merges, once the diagonal blocks are back in place
+    float* Xs = KK + 3 * 4 * 16 * 17;  // [3][32][33] scratch of the merges (K K^T and Q K^T are done with)
     float* Ts = As;
     if (tid < 3 * CH) {
         const int hv = tid / CH, blk = (tid % CH) / 16, b0 = blk * 16, col = tid % 16;
@@ -364,7 +360,7 @@ delta_scan_kernel(const float* p, int splits, int n, const float* cv, const floa
     const int vs = blockIdx.x, h = blockIdx.y, sg = blockIdx.z, kh = h / (LV_HEADS / LK_HEADS);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g8 = lane >> 2, t4 = lane & 3;
     // this block's columns; EVEN: all blocks have SC_COLS, known to the compiler (as run-time values the tests on them cost
-    // the halves a tenth: three segments of 150 tokens 135 -> 158 us, one of 79 44 -> 48)
+    // the halves a tenth: 12 segments of 40 tokens 228 -> 253 us, one of 79 44 -> 48)
     constexpr bool EVEN = LVD % SC_COLS == 0;
     const int width = EVEN ? SC_COLS : min(SC_COLS, LVD - vs * SC_COLS);
     const int lc = tid >> 3, sub = tid & 7;   // token form: 8 lanes per value column
