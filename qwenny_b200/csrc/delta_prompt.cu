@@ -334,8 +334,10 @@ delta_chunk_prep_kernel(const float* cv, float* tp, const int* seg_start, const 
 
 // A scan block has COLS of a value head's 128 columns, 8 threads per column. Steps with chunks are bound by the tf32 mma.sync
 // rate of each SM, chunk after chunk: three blocks per head (48, 48 and 32 columns) put one sequence on 144 of 148 SMs where
-// two halves leave 52 idle (2048 tokens: 355 us in halves, 299 us in three parts); the launch takes whichever finishes its
-// waves of blocks first. Steps without chunks (the token form alone) take halves: fewer blocks stage the tokens.
+// two halves leave 52 idle (2048 tokens: 355 us in halves, 299 us in three parts, one wave of blocks each); the launch takes
+// whichever finishes its waves first, a wave of parts as 84 % of one of halves (not their 75 % of the columns: five
+// segments of 200 tokens are 5 waves against 4, 346 us against 322). Steps without chunks (the token form alone) take
+// halves: fewer blocks stage the tokens.
 constexpr int SC_TAIL = 16;                      // tokens staged per round of the token form
 template <int COLS>
 struct ScanSmem {
@@ -713,7 +715,7 @@ int qb_delta_rule(qb_ctx* ctx, void* stream, const float* p, int splits, int n, 
         if (rc) return rc;
     }
     auto waves = [&](long long parts) { return (parts * LV_HEADS * segs + ctx->sms - 1) / ctx->sms; };
-    if (chunks > 0 && waves(3) * 48 < waves(2) * 64)
+    if (chunks > 0 && waves(3) * 84 < waves(2) * 100)
         return launch(ctx, delta_scan_kernel<48>, dim3(3, LV_HEADS, segs), dim3(48 * 8), sizeof(ScanSmem<48>), st, p, splits, n, cv,
                       (const float*)ctx->delta_tp, mem, sst, meta, out, seg_start, seg_len, seg_slot, seg_pos0);
     return launch(ctx, delta_scan_kernel<64>, dim3(2, LV_HEADS, segs), dim3(64 * 8), sizeof(ScanSmem<64>), st, p, splits, n, cv,
