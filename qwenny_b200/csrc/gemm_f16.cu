@@ -5,6 +5,7 @@
 // A block is one (tile, k split, block of 8 NTT tokens); its 4 warps take alternate k16 steps and add up in shared memory in warp order.
 #include "common.cuh"
 #include "launch.h"
+#include "measure.h"
 
 namespace qb {
 
@@ -77,10 +78,8 @@ __global__ void __launch_bounds__(128) gemm_f16_plain_kernel(const uint4* __rest
     }
 }
 
-// The same for more than 32 tokens (prompt steps): a block multiplies its 32 tokens by TILES tiles, so that a fragment of X,
-// which is gathered in 4-byte pieces, is loaded once for all of them. One tile per block loaded X six times over for the
-// 96 x 5120 pair (the DeltaNet mixer of 2048 rows, this product included: 559 us so, 535 with six). Same order of additions
-// per output.
+// The same for prompt steps: a block multiplies its 32 tokens by TILES tiles, so that a fragment of X, which is gathered in
+// 4-byte pieces, is loaded once for all of them (qb_gemm_f16_block_tiles says where). Same order of additions per output.
 template <int TILES>
 __global__ void __launch_bounds__(128) gemm_f16_wide_kernel(const uint4* __restrict__ W, const __half* __restrict__ X,
                                                             const int* __restrict__ xrows, int K, int ntiles, int n,
@@ -154,6 +153,22 @@ __global__ void __launch_bounds__(128) gemm_f16_wide_kernel(const uint4* __restr
 
 using namespace qb;
 
+// Tiles per block. More than one from the row count on at which one per block fills the SMs (5/6 of a block each): below that, more
+// blocks in flight are worth more than X loaded once. 96 x 5120 in 5 splits, one tile per block against six: 33 rows 5.9 and
+// 7.8 us, 128 rows (120 blocks) 7.1 and 8.0, 160 rows (150) 8.5 and 8.0, 333 rows 11.3 and 8.7, 2048 rows 37.0 and 17.0.
+// Six tiles of a split of less than 256 columns leave a warp a few steps: there four blocks of one tile per SM are as good
+// (40 splits, 64 rows, 480 blocks: 3.1 and 3.3 us; 96 rows, 720 blocks: 4.8 and 3.5). Blocks of two save little work each
+// and lose where their second wave is partly filled (5 splits of 1024: 160 outputs, 200 rows, 175 blocks of two 11.4 and
+// 9.8; 333 rows, 275 blocks 11.7 and 15.2; 512 rows, 400 blocks 18.0 and 17.6; 1024 rows 31.8 and 19.6).
+extern "C" int qb_gemm_f16_block_tiles(int ntiles, int splits, int kper, int n, int sms) {
+    const int per = ntiles % 6 == 0 ? 6 : ntiles % 4 == 0 ? 4 : ntiles % 2 == 0 ? 2 : 1;
+    const long long blocks = (long long)ntiles * splits * ((n + 31) / 32);
+    if (n <= 32 || 6 * blocks <= 5ll * sms) return 1;
+    if (per == 6 && kper < 256 && blocks <= 4ll * sms) return 1;
+    if (per == 2 && 2 * blocks > 5ll * sms && 5 * blocks < 26ll * sms) return 1;
+    return per;
+}
+
 extern "C" int qb_gemm_f16_plain(qb_ctx* ctx, void* stream, const void* W, const void* X, const int* xrows, int K,
                                  int ntiles, int n, int kper, float* Y, int ldy) {
     if (!ctx || !W || !X || !Y || K <= 0 || K % 16 || ntiles <= 0 || n <= 0 || n > 65535 * 32 || kper <= 0 || kper % 16 ||
@@ -166,8 +181,8 @@ extern "C" int qb_gemm_f16_plain(qb_ctx* ctx, void* stream, const void* W, const
     const __half* x = (const __half*)X;
     if (n <= 8) return launch(ctx, gemm_f16_plain_kernel<1>, grid, dim3(128), 0, st, w, x, xrows, K, ntiles, n, kper, Y, ldy);
     if (n <= 16) return launch(ctx, gemm_f16_plain_kernel<2>, grid, dim3(128), 0, st, w, x, xrows, K, ntiles, n, kper, Y, ldy);
-    if (n > 32 && ntiles % 2 == 0) {  // the widest block that divides the tiles
-        const int per = ntiles % 6 == 0 ? 6 : ntiles % 4 == 0 ? 4 : 2;
+    const int per = qb_gemm_f16_block_tiles(ntiles, split, kper, n, ctx->sms);
+    if (per > 1) {
         grid.x = ntiles / per;
         if (per == 6) return launch(ctx, gemm_f16_wide_kernel<6>, grid, dim3(128), 0, st, w, x, xrows, K, ntiles, n, kper, Y, ldy);
         if (per == 4) return launch(ctx, gemm_f16_wide_kernel<4>, grid, dim3(128), 0, st, w, x, xrows, K, ntiles, n, kper, Y, ldy);

@@ -23,6 +23,8 @@ int qb_model_fail_captures(struct qb_model* m, int n);
  * kernel-attribute bookkeeping; 0 when they hold. */
 int qb_graph_cache_selftest(void);
 int qb_attr_cache_selftest(void);
+/* The 16-row tiles that a block of qb_gemm_f16_plain multiplies its 32 rows by, on a part with `sms` SMs. */
+int qb_gemm_f16_block_tiles(int ntiles, int splits, int kper, int n, int sms);
 /* Tests: the context goes on as one that was created where the prompt-sized kernels' scratch did not fit. */
 int qb_scratch_forget(qb_ctx* ctx);
 /* Tests: one block waits on an mbarrier that nothing arrives on, with the library's bounded wait cut to `limit` polls

@@ -6,6 +6,7 @@ import torch
 
 from oracle import ref_ops as R
 from qwenny_b200 import host, synth
+from qwenny_b200._lib import lib
 
 pytestmark = pytest.mark.gpu
 H = R.H
@@ -134,3 +135,20 @@ def test_gemm_f16_blocks_of_tiles(ctx, n, tiles, kper):
     want = x.double()[rows.long()] @ w.double().T
     got = y.double().cpu().sum(0)
     assert y.shape[0] == -(-K // kper) and (got - want).abs().max() < 1e-5 * want.abs().max()
+
+
+@pytest.mark.parametrize("n,tiles,kper,per", [(700, 6, 256, 6), (1633, 4, 128, 4), (261, 10, 256, 2), (530, 12, 144, 6),
+                                              (2111, 2, 384, 2), (97, 6, 256, 1)])
+def test_gemm_f16_blocks_of_tiles_have_the_bits_of_one_tile(ctx, n, tiles, kper, per):
+    """Where a block takes several tiles, and below: the bits of the same rows in calls of 32, which take one tile per block
+    and add in the same order."""
+    K = 384
+    assert lib().qb_gemm_f16_block_tiles(tiles, -(-K // kper), kper, n, ctx.sms) == per
+    g = synth.gen(390 + n)
+    w = (torch.randn(tiles * 16, K, generator=g) * 0.1).half()
+    x, rows = torch.randn(n + 3, K, generator=g).half().cuda(), torch.randint(0, n + 3, (n,), generator=g).to(torch.int32).cuda()
+    wp = torch.from_numpy(R.pack_f16(w.numpy())).cuda()
+    y = ctx.gemm_f16_plain(wp, x, n, K, tiles, kper, xrows=rows)
+    slabs = [ctx.gemm_f16_plain(wp, x, min(32, n - a), K, tiles, kper, xrows=rows[a:a + 32].contiguous()) for a in range(0, n, 32)]
+    torch.cuda.synchronize()
+    assert torch.equal(y, torch.cat(slabs, 1))

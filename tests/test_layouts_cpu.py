@@ -185,3 +185,17 @@ def test_decode_attention_grid_holds_every_split():
         for keys in range(1, 40000, 61):
             most = max(most, lib().qb_attn_dec_splits_sm(keys, sms))
             assert most <= grid(keys, sms) <= 64
+
+
+def test_tiles_per_block_of_the_16_bit_product():
+    """One tile per block while the blocks do not fill the SMs (the DeltaNet gates' 96 x 5120 product in 5 splits up to 128 rows, where
+    blocks of six tiles are a third slower), several beyond; never tiles that do not divide."""
+    from qwenny_b200._lib import lib
+    per = lambda n, tiles=6, splits=5, kper=1024, sms=148: lib().qb_gemm_f16_block_tiles(tiles, splits, kper, n, sms)
+    assert [per(n) for n in (1, 32, 33, 64, 128)] == [1] * 5 and [per(n) for n in (160, 333, 2048)] == [6] * 3
+    assert all(per(n, tiles=7) == 1 for n in (1, 64, 500, 5000)) and per(2048, tiles=4) == 4
+    assert [per(n, tiles=10) for n in (96, 200, 333, 1024)] == [2, 2, 1, 2]  # blocks of two: not where their second wave is partly filled
+    assert per(64, splits=40, kper=128) == 1 and per(96, splits=40, kper=128) == 6
+    for tiles in range(1, 40):
+        for n in (1, 33, 100, 400, 3000):
+            assert tiles % per(n, tiles=tiles) == 0
