@@ -13,8 +13,9 @@
 //               kernels/qwen.cu:136-138)
 // The size of a key split is a function of the key count alone (dec_chunk), so a token's sums are the same whether
 // it runs alone or with drafts.
-#include "attn_common.cuh"
+#include "attn_tc.cuh"
 #include "launch.h"
+#include "measure.h"
 
 namespace qb {
 
@@ -866,6 +867,16 @@ attn_combine_tiles_kernel(const float* part_ml, const float* part_acc, const int
     combine_row(part_ml, part_acc, ((size_t)t * NH + h) * z, (keys + chunk - 1) / chunk, out + o, mix ? mix + o : nullptr);
 }
 
+// one block: which form the two tcgen05 kernels behind it take. It does not let them start before it ends: the one that works holds
+// whole SMs and their tensor memory, and nothing should wait there for a step that is not its own.
+constexpr int FORM_THREADS = 512;
+__global__ void __launch_bounds__(FORM_THREADS)
+attn_form_kernel(const int* ptile, int ntile, const int* tok_slot, const int* tok_pos, int sms, int* on_pairs) {
+    pdl_wait();
+    const bool p = tc::tiles_on_pairs(ptile, ntile, tok_slot, tok_pos, sms);
+    if (threadIdx.x == 0) *on_pairs = p;
+}
+
 }  // namespace qb
 
 using namespace qb;
@@ -931,17 +942,68 @@ int qb_attn_tile_splits(int ntile, int max_keys) { return ntile > 0 && max_keys 
 int qb_attn_prefill(qb_ctx* ctx, void* stream, const float* q, const void* kc, const void* vc, const float* ks,
                     const float* vs, const int* ptile, const int* tok_slot, const int* tok_pos, int cap, int ntile,
                     int max_keys, float* part_ml, float* part_acc, float* out, void* mix_f16) {
+    return qb_attn_prefill_as(ctx, stream, q, kc, vc, ks, vs, ptile, tok_slot, tok_pos, cap, ntile, max_keys, part_ml, part_acc, out,
+                              mix_f16, -1);
+}
+
+// what attn_form_kernel says, from the arrays on the host
+int qb_attn_tiles_on_pairs(const int* h_ptile, int ntile, const int* h_tok_slot, const int* h_tok_pos, int sms) {
+    if (!h_ptile || !h_tok_slot || !h_tok_pos || ntile <= 0 || sms <= 0) return 0;
+    unsigned long long sum[2] = {0ull, 0ull};
+    unsigned top[2] = {0u, 0u}, unit[2] = {0u, 0u};
+    for (int t = 0; t < ntile; t++) {
+        const bool on = t + 1 < ntile && tc::tile_goes_on(h_ptile, h_tok_slot, h_tok_pos, t);
+        const int keys = h_tok_pos[h_ptile[2 * t] + h_ptile[2 * t + 1] - 1] + 1;
+        for (int f = 0; f < 2; f++) {
+            const int of = f ? 2 : 4;
+            if (t % of == 0) unit[f] = 0u;
+            if (!on || t % of == of - 1) {
+                const unsigned c = f ? tc::block_pass_cost(keys) : tc::pair_pass_cost(keys);
+                sum[f] += c;
+                unit[f] += c;
+            }
+            if (unit[f] > top[f]) top[f] = unit[f];
+        }
+    }
+    return tc::pairs_win(sum[0], sum[1], top[0], top[1], sms);
+}
+
+}  // extern "C"
+
+namespace {
+// One key split: two tiles per block or four per pair of blocks. Up to 1664 keys as blocks: a stage of 128 keys and the pair's
+// set-up cost more there than the faster stages give (100 rows at context 0 40.1 us as blocks, 43.7 as pairs; 1500 at 100
+// 200 and 210; 2048 at 0 289 and 277; 1024 at 2000 257 and 225). Beyond, the runs of the tiles decide (attn_tc.cuh): 0
+// blocks, 1 pairs. A caller that has the tiles on the host says which; for the others (2) a small kernel works it out and
+// both forms are launched, one of which returns (2 to 4 us: 400 rows at 4000 126 -> 128, 2048 at 30720 1922 -> 1926).
+int prefill_form(const qb_ctx* ctx, int max_keys, int as) {
+    if (ctx->tune_ctas == 1002 || ctx->tune_ctas == 1003) return ctx->tune_ctas - 1002;  // measurement
+    return max_keys <= 1664 ? 0 : as < 0 ? 2 : as;
+}
+}  // namespace
+
+int qb_attn_prefill_launches(const qb_ctx* ctx, int ntile, int max_keys, int as) {
+    if (tile_splits(ntile, max_keys) > 1) return 2;
+    return prefill_form(ctx, max_keys, as) == 2 ? 3 : 1;
+}
+
+int qb_attn_prefill_as(qb_ctx* ctx, void* stream, const float* q, const void* kc, const void* vc, const float* ks,
+                       const float* vs, const int* ptile, const int* tok_slot, const int* tok_pos, int cap, int ntile,
+                       int max_keys, float* part_ml, float* part_acc, float* out, void* mix_f16, int as) {
     if (!ctx || !q || !kc || !vc || !ks || !vs || !ptile || !tok_slot || !tok_pos || !out || ntile <= 0 || cap % 64 ||
         max_keys <= 0 || max_keys > cap)
         return QB_ERR_ARG;
     const int z = tile_splits(ntile, max_keys);
     if (z > 1 && (!part_ml || !part_acc)) return QB_ERR_ARG;
     if (z == 1) {
-        // many tiles, on tcgen05: four tiles per pair of blocks, or, up to 1664 keys, two per block: a stage of 128 keys and the
-        // pair's set-up cost more there than the faster stages give (100 rows at context 0 40.1 us as blocks, 43.7 as
-        // pairs; 1500 at 100 200 and 210; 2048 at 0 289 and 277; 1024 at 2000 257 and 225; 2048 at 30720 2786 and 2019)
-        return (max_keys <= 1664 ? qb_attn_prefill_short_launch : qb_attn_prefill_tc_launch)(ctx, (cudaStream_t)stream, q, kc, vc, ks, vs, ptile, ntile, tok_slot, tok_pos,
-                                         cap, out, mix_f16);
+        const int form = prefill_form(ctx, max_keys, as);
+        const int* word = form == 2 ? ctx->form : nullptr;
+        cudaStream_t st = (cudaStream_t)stream;
+        int rc = QB_OK;
+        if (word) rc = launch(ctx, attn_form_kernel, dim3(1), dim3(FORM_THREADS), 0, st, ptile, ntile, tok_slot, tok_pos, ctx->sms, ctx->form);
+        if (!rc && form != 0) rc = qb_attn_prefill_tc_launch(ctx, st, q, kc, vc, ks, vs, ptile, ntile, tok_slot, tok_pos, cap, out, mix_f16, word);
+        if (!rc && form != 1) rc = qb_attn_prefill_short_launch(ctx, st, q, kc, vc, ks, vs, ptile, ntile, tok_slot, tok_pos, cap, out, mix_f16, word);
+        return rc;
     }
     using C = DecCfg<4, 2, 5>;  // 10 tokens x 6 heads = 60 rows: 4 row tiles; 2 warps each; 5 stages of 32 keys
     static_assert(PTILE * GROUP <= 64, "a prompt tile fills at most 4 row tiles");
@@ -953,5 +1015,3 @@ int qb_attn_prefill(qb_ctx* ctx, void* stream, const float* q, const void* kc, c
     return launch(ctx, attn_combine_tiles_kernel, dim3(ntile * PTILE, NH), dim3(HD), 0, st, (const float*)part_ml,
                   (const float*)part_acc, ptile, tok_pos, z, out, (__half*)mix_f16);
 }
-
-}  // extern "C"

@@ -50,8 +50,12 @@ using namespace tc;
 __global__ void __launch_bounds__(THREADS, 1)
 attn_prefill_short_kernel(const float* q, const uint8_t* kc, const uint8_t* vc, const float* ks, const float* vs,
                        const int* ptile, int ntile, const int* tok_slot, const int* tok_pos, int cap, float* out,
-                       __half* mix, int* err) {
+                       __half* mix, int* err, const int* on_pairs) {
     extern __shared__ uint8_t smem_raw[];
+    if (on_pairs) {  // both forms are launched, and the step decides: the other one returns before it takes anything
+        pdl_wait();
+        if (*(const volatile int*)on_pairs) return;
+    }
     uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     uint8_t* kf = smem;                    // [NST][K_BYTES]
     uint8_t* vf = kf + NST * K_BYTES;      // [NST][V_BYTES]
@@ -343,12 +347,12 @@ attn_prefill_short_kernel(const float* q, const uint8_t* kc, const uint8_t* vc, 
 }  // namespace pfs
 }  // namespace qb
 
-// the many-tile form of qb_attn_prefill (one key split): see attn.cu
+// the many-tile form of qb_attn_prefill (one key split): see attn.cu, and attn_prefill_tc.cu for on_pairs
 int qb_attn_prefill_short_launch(qb_ctx* ctx, cudaStream_t st, const float* q, const void* kc, const void* vc, const float* ks,
                               const float* vs, const int* ptile, int ntile, const int* tok_slot, const int* tok_pos,
-                              int cap, float* out, void* mix_f16) {
+                              int cap, float* out, void* mix_f16, const int* on_pairs) {
     using namespace qb;
     return launch(ctx, pfs::attn_prefill_short_kernel, dim3((ntile + 1) / 2, NKV), dim3(pfs::THREADS), pfs::SMEM_BYTES, st, q,
                   (const uint8_t*)kc, (const uint8_t*)vc, ks, vs, ptile, ntile, tok_slot, tok_pos, cap, out,
-                  (__half*)mix_f16, ctx->err);
+                  (__half*)mix_f16, ctx->err, on_pairs);
 }

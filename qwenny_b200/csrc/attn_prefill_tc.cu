@@ -80,7 +80,11 @@ __device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
 attn_prefill_tc_kernel(const float* q, const uint8_t* kc, const uint8_t* vc, const float* ks, const float* vs,
                        const int* ptile, int ntile, const int* tok_slot, const int* tok_pos, int cap, float* out,
-                       __half* mix, int* err) {
+                       __half* mix, int* err, const int* on_pairs) {
+    if (on_pairs) {  // both forms are launched, and the step decides: the other one returns before it takes anything
+        pdl_wait();
+        if (!*(const volatile int*)on_pairs) return;
+    }
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     uint8_t* qf = smem;                    // [Q_BYTES]
@@ -415,12 +419,13 @@ attn_prefill_tc_kernel(const float* q, const uint8_t* kc, const uint8_t* vc, con
 }  // namespace pft
 }  // namespace qb
 
-// the many-tile form of qb_attn_prefill (one key split): see attn.cu
+// the many-tile form of qb_attn_prefill (one key split): see attn.cu. on_pairs: null, or a word on the device that says whether
+// this form (1) or the other (0) does the step
 int qb_attn_prefill_tc_launch(qb_ctx* ctx, cudaStream_t st, const float* q, const void* kc, const void* vc, const float* ks,
                               const float* vs, const int* ptile, int ntile, const int* tok_slot, const int* tok_pos,
-                              int cap, float* out, void* mix_f16) {
+                              int cap, float* out, void* mix_f16, const int* on_pairs) {
     using namespace qb;
     return launch(ctx, pft::attn_prefill_tc_kernel, dim3(2 * ((ntile + 3) / 4), NKV), dim3(pft::THREADS), pft::SMEM_BYTES, st, q,
                   (const uint8_t*)kc, (const uint8_t*)vc, ks, vs, ptile, ntile, tok_slot, tok_pos, cap, out,
-                  (__half*)mix_f16, ctx->err);
+                  (__half*)mix_f16, ctx->err, on_pairs);
 }

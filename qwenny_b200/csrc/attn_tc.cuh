@@ -99,5 +99,64 @@ struct Waiter {
     }
 };
 
+// ---- Prompt steps with one key split and more than 1664 keys: pairs of blocks (four tiles, attn_prefill_tc.cu) or one block per
+// two tiles (attn_prefill_short.cu). A pair passes over its tiles once per RUN of consecutive tiles of one sequence, on two
+// SMs, so it wins over long runs (2048 rows at context 30720: 2716 us as blocks, 1920 as pairs) and loses over short ones (40
+// sequences of 10 rows at 2000: 176 and 295 us; 30 of 20 at 8000: 290 and 402; 8 of 100 at 8000: 545 and 595).
+// The estimate, in units of 100 cycles: a pass costs its stages (5200 cycles per 128 keys over a pair, 3700 per 64 keys)
+// and its ends (some 30 us: Q and the gates are read a row per thread); a form takes its passes spread over the SMs, and up
+// to its longest unit of work more. Of 33 steps timed as either (single sequences, equal and unequal batches, 38 to 205 tiles)
+// it names the faster one for all.
+__host__ __device__ __forceinline__ unsigned pair_pass_cost(int keys) { return 52u * (unsigned)((keys + 127) / 128) + 600u; }
+__host__ __device__ __forceinline__ unsigned block_pass_cost(int keys) { return 37u * (unsigned)((keys + 63) / 64) + 520u; }
+// tile t + 1 continues tile t
+__host__ __device__ __forceinline__ bool tile_goes_on(const int* ptile, const int* tok_slot, const int* tok_pos, int t) {
+    const int fa = ptile[2 * t], na = ptile[2 * t + 1], fb = ptile[2 * t + 2];
+    return fb == fa + na && tok_slot[fb] == tok_slot[fa] && tok_pos[fb] == tok_pos[fa] + na;
+}
+__host__ __device__ __forceinline__ bool pairs_win(unsigned long long pair_sum, unsigned long long block_sum, unsigned pair_most,
+                                                   unsigned block_most, int sms) {
+    const unsigned long long pairs = sms > 1 ? sms / 2 : 1;
+    return NKV * pair_sum / pairs + pair_most <= NKV * block_sum / (unsigned long long)sms + block_most;
+}
+// the answer for a step, in every thread of the block (all threads call it, whole warps)
+__device__ __forceinline__ bool tiles_on_pairs(const int* ptile, int ntile, const int* tok_slot, const int* tok_pos, int sms) {
+    __shared__ unsigned long long part[2][32];
+    __shared__ unsigned most[2][32];
+    unsigned long long sum[2] = {0ull, 0ull};
+    unsigned top[2] = {0u, 0u};
+    for (int t0 = 0; t0 < ntile; t0 += blockDim.x) {  // (a unit's tiles are neighbouring lanes of a warp)
+        const int t = t0 + threadIdx.x;
+        unsigned cost[2] = {0u, 0u};
+        if (t < ntile) {
+            const bool on = t + 1 < ntile && tile_goes_on(ptile, tok_slot, tok_pos, t);
+            const int keys = tok_pos[ptile[2 * t] + ptile[2 * t + 1] - 1] + 1;
+            if (!on || (t & 3) == 3) cost[0] = pair_pass_cost(keys);
+            if (!on || (t & 1) == 1) cost[1] = block_pass_cost(keys);
+        }
+#pragma unroll
+        for (int f = 0; f < 2; f++) {
+            sum[f] += cost[f];
+            unsigned unit = cost[f] + __shfl_xor_sync(0xffffffffu, cost[f], 1);
+            if (f == 0) unit += __shfl_xor_sync(0xffffffffu, unit, 2);
+            top[f] = max(top[f], unit);
+        }
+    }
+#pragma unroll
+    for (int f = 0; f < 2; f++) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) sum[f] += __shfl_xor_sync(0xffffffffu, sum[f], o);
+        top[f] = __reduce_max_sync(0xffffffffu, top[f]);
+        if ((threadIdx.x & 31) == 0) { part[f][threadIdx.x >> 5] = sum[f]; most[f][threadIdx.x >> 5] = top[f]; }
+    }
+    __syncthreads();
+    sum[0] = sum[1] = 0ull;
+    top[0] = top[1] = 0u;
+    for (int w = 0; w < (int)(blockDim.x >> 5); w++)
+#pragma unroll
+        for (int f = 0; f < 2; f++) { sum[f] += part[f][w]; top[f] = max(top[f], most[f][w]); }
+    return pairs_win(sum[0], sum[1], top[0], top[1], sms);
+}
+
 }  // namespace tc
 }  // namespace qb

@@ -103,6 +103,7 @@ int qb_create(int device, qb_ctx** out) {
     c->counters = (int*)b;
     c->ncounters = ncounters;
     c->err = (int*)(b + err_at);
+    c->form = c->err + 16;
     c->scratch = (float*)(b + scratch_at);
     c->scratch_bytes = scratch_bytes;
     if (all) {

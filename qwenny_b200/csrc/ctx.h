@@ -15,6 +15,7 @@ struct qb_ctx {
     int* counters = nullptr;
     size_t ncounters = 0;
     int* err = nullptr;  // device word
+    int* form = nullptr; // device word: the form of the prompt attention that the step under way takes
     // The prompt-sized kernels' scratch. It is taken at creation like the rest, in one allocation with it (`block`); a device
     // that has room for the rest alone gets a context without it, whose calls take the forms that need none.
     void* block = nullptr;
@@ -68,10 +69,15 @@ int prepare_kernel(int device, const void* kern, int smem);
 // the many-tile prompt attention on tcgen05 (attn_prefill_tc.cu); reached through qb_attn_prefill
 int qb_attn_prefill_tc_launch(qb_ctx* ctx, cudaStream_t st, const float* q, const void* kc, const void* vc, const float* ks,
                               const float* vs, const int* ptile, int ntile, const int* tok_slot, const int* tok_pos,
-                              int cap, float* out, void* mix_f16);
+                              int cap, float* out, void* mix_f16, const int* on_pairs);
 int qb_attn_prefill_short_launch(qb_ctx* ctx, cudaStream_t st, const float* q, const void* kc, const void* vc, const float* ks,
                                  const float* vs, const int* ptile, int ntile, const int* tok_slot, const int* tok_pos,
-                              int cap, float* out, void* mix_f16);  // short contexts (attn_prefill_short.cu)
+                                 int cap, float* out, void* mix_f16, const int* on_pairs);  // short contexts, short runs (attn_prefill_short.cu)
+// qb_attn_prefill for a caller that knows qb_attn_tiles_on_pairs of its tiles (as: 0 or 1; -1: not known), and its launches
+int qb_attn_prefill_as(qb_ctx* ctx, void* stream, const float* q, const void* kc, const void* vc, const float* ks, const float* vs,
+                       const int* ptile, const int* tok_slot, const int* tok_pos, int cap, int ntile, int max_keys, float* part_ml,
+                       float* part_acc, float* out, void* mix_f16, int as);
+int qb_attn_prefill_launches(const qb_ctx* ctx, int ntile, int max_keys, int as);
 // the prompt-sized W4A16 product on tcgen05 (w4a16_gemm_tc.cu); reached through qb_marlin_gemm / qb_marlin_gemm_z (zp:
 // S carries the offsets' table after the scales) for more than 16 rows
 int qb_gemm_tc_launch(qb_ctx* ctx, cudaStream_t st, const void* X, const void* B, void* Y, const void* S, int m, int n,

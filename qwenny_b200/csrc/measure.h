@@ -25,6 +25,9 @@ int qb_graph_cache_selftest(void);
 int qb_attr_cache_selftest(void);
 /* The 16-row tiles that a block of qb_gemm_f16_plain multiplies its 32 rows by, on a part with `sms` SMs. */
 int qb_gemm_f16_block_tiles(int ntiles, int splits, int kper, int n, int sms);
+/* Host only (host pointers): whether a prompt attention of more than 1664 keys and one key split runs on pairs of blocks (1) or as a
+ * block per two tiles (0) on a part with `sms` SMs. qb_marlin_tune with ctas_per_sm 1002 / 1003 forces blocks / pairs. */
+int qb_attn_tiles_on_pairs(const int* h_ptile, int ntile, const int* h_tok_slot, const int* h_tok_pos, int sms);
 /* Tests: the context goes on as one that was created where the prompt-sized kernels' scratch did not fit. */
 int qb_scratch_forget(qb_ctx* ctx);
 /* Tests: one block waits on an mbarrier that nothing arrives on, with the library's bounded wait cut to `limit` polls

@@ -16,6 +16,7 @@
 #include "common.cuh"
 #include "ctx.h"
 #include "graphs.h"
+#include "measure.h"
 #include "session.h"
 #include "step_arrays.h"
 
@@ -77,7 +78,7 @@ struct qb_model {
     unsigned long long* h_keys = nullptr;  // pinned
     // host-side shape of the uploaded step
     int n = 0, n_out = 0, segs = 0, ndec = 0, ntile = 0, ndseg = 0, dmax = 0, max_seg = 0, dec_max_pos = 0,
-        tile_max_pos = 0;
+        tile_max_pos = 0, on_pairs = 0;
     // MTP draft layer (optional): stored as layers[nlayers]; fc's input, the rows of the residual stream its tokens take
     // their hidden states from, the drafts of the running chains
     bool has_mtp = false;
@@ -193,9 +194,9 @@ int launch_mixer(qb_model* m, cudaStream_t st, int layer, int& k) {
             k += 2;
         }
         if (m->ntile > 0) {
-            QB_TRY(qb_attn_prefill(c, s, m->q, L.kc, L.vc, L.ks, L.vs, m->ptile, m->tok_slot, m->tok_pos, L.cap, m->ntile,
-                                   m->tile_max_pos + 1, m->ml, m->acc, m->o, m->mix));
-            k += qb_attn_tile_splits(m->ntile, m->tile_max_pos + 1) > 1 ? 2 : 1;
+            QB_TRY(qb_attn_prefill_as(c, s, m->q, L.kc, L.vc, L.ks, L.vs, m->ptile, m->tok_slot, m->tok_pos, L.cap, m->ntile,
+                                      m->tile_max_pos + 1, m->ml, m->acc, m->o, m->mix, m->on_pairs));
+            k += qb_attn_prefill_launches(c, m->ntile, m->tile_max_pos + 1, m->on_pairs);
         }
     }
     return QB_OK;
@@ -564,6 +565,8 @@ static int upload_step(qb_model* m, void* stream, const qb_tok* toks, int n, con
         for (int i = 0; i < n && !m->lora_step; i++) m->lora_step = m->h_scale[toks[i].slot] != 0.f;
     m->n = sh.n; m->n_out = sh.n_out; m->segs = sh.segs; m->ndec = sh.ndec; m->ntile = sh.ntile; m->ndseg = sh.ndseg;
     m->dmax = sh.dmax; m->max_seg = sh.max_seg; m->dec_max_pos = sh.dec_max_pos; m->tile_max_pos = sh.tile_max_pos;
+    const StepLayout L;
+    m->on_pairs = sh.ntile ? qb_attn_tiles_on_pairs(h + L.ptile, sh.ntile, h + L.tok_slot, h + L.tok_pos, m->ctx->sms) : 0;
     return QB_OK;
 }
 

@@ -307,30 +307,44 @@ def test_attn_decode_of_a_ragged_batch(ctx, rows):
     assert close(full.cpu().numpy(), want).all()
 
 
-def test_attn_prefill_several_sequences_on_pairs(ctx):
-    """The form on pairs of blocks over runs of several sequences: pairs with one, two and three runs of one to four tiles, odd and
-    even stage counts, a cache whose length is an odd multiple of 64 and keys in its last half stage, against the oracle at
-    the ends of every sequence and tile."""
-    g = synth.gen(167)
-    lens, pos0, cap = (25, 33, 12, 47, 280), (2080, 1700, 1900, 40, 1663), 2112
+@pytest.mark.parametrize("lens,pos0,cap,pairs", [
+    ((25, 33, 12, 47, 280), (2080, 1700, 1900, 40, 1663), 2112, 1),
+    ((50,) * 8, (8000, 30, 7990, 8060, 4000, 64, 8127, 2000), 8192, 1),      # 5 tiles each: runs of 1 to 4 tiles in a pair
+    ((10,) * 40, (2000,) * 39 + (2102,), 2112, 0),
+    ((400,), (4003,), 4416, 1)])
+def test_attn_prefill_forms_over_several_sequences(ctx, lens, pos0, cap, pairs):
+    """Steps of more than 1664 keys as pairs of blocks and as a block per two tiles, against the oracle at the ends of every
+    sequence and tile: passes over runs of one to four tiles, odd and even stage counts, caches whose length is an odd
+    multiple of 64 with keys in the last half stage. Left to itself the call takes the form of qb_attn_tiles_on_pairs."""
+    g = synth.gen(167 + len(lens))
     cache = make_cache(len(lens), cap, g, 0)
     toks = [(0, s, p + i) for s, (n, p) in enumerate(zip(lens, pos0)) for i in range(n)]
     n = len(toks)
     q = torch.randn(n, R.NH, R.HD, generator=g) * QSCALE
     gate = torch.sigmoid(torch.randn(n, R.MIX, generator=g))
     st = R.build_step(toks, list(range(n)))
-    keys = st["tile_max_pos"] + 1
-    assert st["ndec"] == 0 and st["ntile"] == 42 and 1664 < keys <= cap and cap % 128 == 64 and cap - keys < 64
-    assert lib().qb_attn_tile_splits(st["ntile"], keys) == 1  # one key split: the tcgen05 kernels
-    mine, mix = run_prefill(ctx, q.cuda(), gate.cuda(), [t.cuda() for t in cache], st, ref_cuda.upload_step(st), cap, n, mix=True)
+    keys, dv, dc = st["tile_max_pos"] + 1, ref_cuda.upload_step(st), [t.cuda() for t in cache]
+    assert st["ndec"] == 0 and keys > 1664 and lib().qb_attn_tile_splits(st["ntile"], keys) == 1
+    h = [np.ascontiguousarray(st[k], dtype=np.int32) for k in ("ptile", "tok_slot", "tok_pos")]
+    assert lib().qb_attn_tiles_on_pairs(h[0].ctypes.data, st["ntile"], h[1].ctypes.data, h[2].ctypes.data, ctx.sms) == pairs
+    run = lambda: run_prefill(ctx, q.cuda(), gate.cuda(), dc, st, dv, cap, n, mix=True)
+    mine, mix = run()
+    try:
+        ctx.tune(ctas=1002)
+        forms = [run()]
+        ctx.tune(ctas=1003)
+        forms += [run()]
+    finally:
+        ctx.tune()
     torch.cuda.synchronize()
     assert ctx.device_error() == 0
-    a = mine.cpu().numpy()
-    assert np.array_equal(mix.cpu().numpy(), a.astype(np.float16))
+    assert torch.equal(mine, forms[pairs][0]) and torch.equal(mix, forms[pairs][1])
+    assert not torch.equal(forms[0][0], forms[1][0])   # (they round P against other running maxima)
     rows, at = [], 0
     for m in lens:
-        rows += [at, at + min(9, m - 1), at + min(10, m - 1), at + m // 2, at + m - 1]
+        rows += sorted({at, at + min(9, m - 1), at + min(10, m - 1), at + m // 2, at + m - 1})
         at += m
     want = R.attn_decode(q.numpy()[rows], gate.numpy()[rows], *[t.numpy() for t in cache], st["tok_slot"][rows],
                          st["tok_pos"][rows], cap)
-    assert close(a[rows], want).all()
+    for out, m16 in forms:
+        assert close(out.cpu().numpy()[rows], want).all() and torch.equal(m16, out.half())

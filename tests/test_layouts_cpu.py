@@ -199,3 +199,30 @@ def test_tiles_per_block_of_the_16_bit_product():
     for tiles in range(1, 40):
         for n in (1, 33, 100, 400, 3000):
             assert tiles % per(n, tiles=tiles) == 0
+
+
+def prompt_tiles(segs):
+    """ptile, tok_slot, tok_pos of a step with the segments (rows, first position), each a sequence of its own."""
+    slot = [i for i, (n, _) in enumerate(segs) for _ in range(n)]
+    pos = [p + j for n, p in segs for j in range(n)]
+    tiles, at = [], 0
+    for n, _ in segs:
+        tiles += [v for o in range(0, n, 10) for v in (at + o, min(10, n - o))]
+        at += n
+    return tuple(np.array(a, dtype=np.int32) for a in (tiles, slot, pos))
+
+
+def test_form_of_the_prompt_attention():
+    """The choice between pairs of blocks and a block per two tiles beyond 1664 keys follows the faster one as measured (us as
+    blocks, as pairs): it depends on the runs that the tiles form, not on the key count alone."""
+    from qwenny_b200._lib import lib
+    def pairs(segs, sms=148):
+        t, slot, pos = prompt_tiles(segs)
+        return lib().qb_attn_tiles_on_pairs(t.ctypes.data, len(t) // 2, slot.ctypes.data, pos.ctypes.data, sms)
+    for segs in ([(2048, 30720)], [(1024, 2000)], [(400, 4000)], [(380, 30000)], [(50, 8000)] * 8, [(250, 8000)] * 8,
+                 [(80, 2500)] * 25, [(30, 8000)] * 16, [(1024, 8000)] + [(10, 100)] * 30, [(30, 100)] * 60 + [(100, 30000)]):
+        assert pairs(segs) == 1, segs    # 2716/1920, 214/179, 160/127, 887/638, 531/401, 1053/804, 346/295, 535/401, 570/448, 970/759
+    for segs in ([(10, 2000)] * 40, [(10, 8000)] * 40, [(20, 4000)] * 20, [(20, 8000)] * 30, [(100, 8000)] * 8, [(10, 3000)] * 200,
+                 [(500, 4000)] * 4, [(30, 2500)] * 66, [(10, 16000)] * 40 + [(800, 0)]):
+        assert pairs(segs) == 0, segs    # 176/295, 540/770, 164/248, 288/401, 542/592, 706/1122, 493/517, 518/543, 1070/1434
+    assert pairs([(7, 5)], sms=1) in (0, 1) and lib().qb_attn_tiles_on_pairs(None, 3, None, None, 148) == 0
