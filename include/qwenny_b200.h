@@ -39,7 +39,13 @@ enum { QB_EPI_PLAIN = 0, QB_EPI_SILU = 1, QB_EPI_ARGMAX = 2 };
  * not overlap on the device (models that run concurrently take a context each). */
 int qb_create(int device, qb_ctx** out);
 void qb_destroy(qb_ctx* ctx);
-/* Non-zero once a kernel gave up a bounded wait (1 producer, 2 consumer, ...); reads and clears the word (syncs). */
+/* Non-zero once a kernel gave up a bounded wait; reads and clears the word (syncs). Which kernel:
+ *    1, 2    W4A16 product, up to 16 rows (copies, products)
+ *    3, 4    decode attention and the prompt attention of a few tiles (copies, products)
+ *    5 .. 8  W4A16 product of prompt rows (copies, dequantisation, products, epilogue)
+ *   11 .. 13 prompt attention on tcgen05 (products, softmax, conversion)
+ *   14 .. 17 W4A16 product, 17 to 64 rows (copies, unpacking, draining, products)
+ *   99       qb_wait_probe's test */
 int qb_device_error(qb_ctx* ctx);
 int qb_sm_count(const qb_ctx* ctx); /* 0 for a null context */
 const char* qb_version(void);

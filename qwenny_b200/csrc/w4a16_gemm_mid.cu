@@ -128,7 +128,7 @@ __global__ void __launch_bounds__(Cfg<NT>::THREADS, 1)
                     bulk_g2s(ssmem + sl * BH, a.S + (size_t)gi * a.N + n0, BH * 2, &sfull[sl], pol);
                 }
             }
-            if (!ok) atomicExch(a.err, 9);
+            if (!ok) atomicExch(a.err, 14);
         }
         __syncwarp();
     } else if (warp >= X_WARP) {
@@ -158,7 +158,7 @@ __global__ void __launch_bounds__(Cfg<NT>::THREADS, 1)
                     if (st >= NSTAGE && ok) {
                         if (lane == 0) ok = mbar_wait(&empty[s], ((st / NSTAGE) - 1) & 1);
                         ok = __shfl_sync(0xffffffffu, ok, 0);
-                        if (!ok && lane == 0) atomicExch(a.err, 9);
+                        if (!ok && lane == 0) atomicExch(a.err, 14);
                     }
                     if (ok) {
 #pragma unroll
@@ -190,7 +190,7 @@ __global__ void __launch_bounds__(Cfg<NT>::THREADS, 1)
                     tma_load_2d(smem + s * XB + C::XH, &xmap, gi * BK + 64, 0, &full[s]);
                 }
             }
-            if (!ok) atomicExch(a.err, 9);
+            if (!ok) atomicExch(a.err, 14);
         }
         __syncwarp();
     } else if (warp < DQ_WARPS) {
@@ -207,7 +207,7 @@ __global__ void __launch_bounds__(Cfg<NT>::THREADS, 1)
                     dead = !mbar_wait(&full[s], (st / NSTAGE) & 1);
                     // (the tensor-memory slot: the products of the stage NA before have read it)
                     if (!dead && st >= NA) dead = !mbar_wait(&empty[(st - NA) % NSTAGE], ((st - NA) / NSTAGE) & 1);
-                    if (dead && lane == 0) atomicExch(a.err, 10);
+                    if (dead && lane == 0) atomicExch(a.err, 15);
                 }
                 asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
                 const int sa = (int)(st % NA);
@@ -259,7 +259,7 @@ __global__ void __launch_bounds__(Cfg<NT>::THREADS, 1)
                 const int p = (int)(gr % ND), sl = (int)(gr % NS);
                 if (!dead) {
                     dead = !mbar_wait(&sfull[sl], (gr / NS) & 1) || !mbar_wait(&dfull[p], (gr / ND) & 1);
-                    if (dead && lane == 0) atomicExch(a.err, 11);
+                    if (dead && lane == 0) atomicExch(a.err, 16);
                 }
                 asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
                 // scale of output 16 b + 8 i + r of a c64 at 8 r + 2 b + i
@@ -360,7 +360,7 @@ __global__ void __launch_bounds__(Cfg<NT>::THREADS, 1)
                     umma_commit(&dfull[p]);
                 }
             }
-            if (!ok) atomicExch(a.err, 12);
+            if (!ok) atomicExch(a.err, 17);
         }
         __syncwarp();
     }

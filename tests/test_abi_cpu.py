@@ -88,3 +88,24 @@ def test_the_header_is_plain_c(tmp_path):
     r = subprocess.run(["gcc", "-std=c99", "-Wall", "-Wextra", "-pedantic", "-Werror", "-fsyntax-only",
                         "-I", os.path.join(ROOT, "include"), str(src)], capture_output=True, text=True)
     assert r.returncode == 0, r.stderr
+
+
+def test_error_words_name_one_kernel():
+    """No two kernels report a wait that ran out with the same word, and the header lists the words in use."""
+    csrc = os.path.join(os.path.dirname(_lib.LIB_PATH), "csrc")
+    used = {}
+    for f in sorted(os.listdir(csrc)):
+        if f.endswith((".cu", ".cuh")):
+            text = open(os.path.join(csrc, f)).read()
+            kernel = "prompt attention" if f.startswith("attn_prefill") else f   # (two forms of one call)
+            for w in re.findall(r"atomicExch\((?:a\.)?err, (\d+)\)|\{err, (\d+)\}", text):
+                used.setdefault(int(w[0] or w[1]), set()).add(kernel)
+    assert len(used) > 12 and all(len(k) == 1 for k in used.values()), used
+    header = open(os.path.join(csrc, "..", "..", "include", "qwenny_b200.h")).read()
+    listed = header[header.index("Which kernel:"):header.index("int qb_device_error(")]
+    words = set()
+    for line in listed.splitlines()[1:]:
+        m = re.match(r" \*\s+(\d+)(?:( \.\. |, )(\d+))?\s", line)
+        if m:
+            words |= set(range(int(m[1]), int(m[3] or m[1]) + 1))
+    assert words == set(used)
