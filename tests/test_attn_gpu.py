@@ -259,8 +259,9 @@ def test_attn_prefill_pairs_and_segment_boundaries(ctx, ref):
 
 @pytest.mark.parametrize("lens,pos0", [((25, 33, 12, 47), (300, 40, 0, 450)), ((400,), (4003,)), ((10, 30, 10), (5, 64, 127))])
 def test_attn_prefill_runs_of_tiles(ctx, lens, pos0):
-    """A pair of blocks takes four tiles of a step, in passes over runs of one sequence: runs of one to four tiles, ragged
-    last tiles, keys that end on and off a 64-key stage, against the oracle."""
+    """Several sequences of up to 512 keys (a block per two tiles), one of 4403 (pairs of blocks), and a few tiles (no tcgen05):
+    ragged last tiles, keys that end on and off a 64-key stage, against the oracle. The forms over runs of several longer
+    sequences are in test_attn_prefill_forms_over_several_sequences."""
     g = synth.gen(137 + len(lens))
     cap = 4480 if pos0[0] > 4000 else 512
     cache = make_cache(len(lens), cap, g, 0)

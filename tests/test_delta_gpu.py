@@ -338,12 +338,15 @@ def test_rollback_after_a_chunked_prompt(ctx):
         assert torch.equal(outsA[i], outsB[i]), f"position {i}"
 
 
+@pytest.mark.parametrize("lens,pos0", [((1, 2, 17, 31, 40, 3), (0, 5, 1, 100, 2, 40)),
+                                       ((5, 1, 2, 90, 3, 16, 33, 4), (7, 0, 1, 2, 3, 500, 0, 1)),
+                                       ((300, 7, 150, 1, 64), (1, 2, 0, 30, 3))])
 @pytest.mark.parametrize("splits", [1, 2])
-def test_conv_tiles(ctx, splits):
-    """Segments that start and end anywhere in the conv's tiles, shorter than its history of three, from
-    position 0, from the slot's ring and across tiles, against the oracle (2e-4: the fast exponential of SiLU, as in test_delta_conv)."""
+def test_conv_tiles(ctx, splits, lens, pos0):
+    """Segments that start and end anywhere in the conv's tiles (8 tokens; 16 for steps of 129 to 512), shorter than its history of
+    three, from position 0, from the slot's ring and across tiles, against the oracle (2e-4: the fast exponential of
+    SiLU, as in test_delta_conv)."""
     g = synth.gen(171 + splits)
-    lens, pos0 = [1, 2, 17, 31, 40, 3], [0, 5, 1, 100, 2, 40]
     toks = [(0, s, p + i) for s, (n, p) in enumerate(zip(lens, pos0)) for i in range(n)]
     n = len(toks)
     conv_w, a_log, dt_bias, _ = weights(g)

@@ -170,10 +170,17 @@ def test_stages_requested_ahead_of_the_kernel_before_do_not_change_the_result(ct
         ctx.set_pdl(False)
 
 
-def test_many_rows_fall_back_to_slabs(ctx):
+def test_40_rows_and_the_same_in_16_row_slabs(ctx):
     x, wdq, xd, wd, sd = make(512, 512, False, 21, 40)
+    want = R.marlin_gemm(x, wdq)
     y = ctx.marlin_gemm(xd, wd, sd).cpu().numpy()
-    assert close(y, R.marlin_gemm(x, wdq)).all()
+    assert close(y, want).all()
+    ctx.tune(nstages=-1)  # this kernel in 16-row slabs, as contexts without the larger products' scratch run them
+    try:
+        slabs = ctx.marlin_gemm(xd, wd, sd).cpu().numpy()
+    finally:
+        ctx.tune()
+    assert close(slabs, want).all()
 
 
 @pytest.mark.parametrize("m,epi", [(1, "plain"), (5, "plain"), (13, "plain"), (5, "silu"), (5, "argmax"), (40, "plain"),

@@ -118,6 +118,45 @@ def test_few_rows_gathered_argmax_vs_oracle(ctx, m, rows, cols):
     assert torch.equal(keys, again)
 
 
+@pytest.mark.parametrize("m,rows,cols", [(17, 16384, 5120), (40, 65536, 5120), (64, 34816, 5120), (70, 16384, 5120), (48, 5120, 17408)])
+def test_few_rows_over_long_shares(ctx, m, rows, cols):
+    """The layer's sizes and an output layer, where a block walks tens of stages (the rings and accumulators turn over many times)
+    through the tail of one tile, whole tiles and the head of another: sampled outputs against the exact product (the
+    bound of the test above), the greedy keys of all outputs, the same bits on repeat, and contiguous rows with the bits
+    of the same rows gathered, plain and SwiGLU."""
+    from qwenny_b200 import model as M
+    g = torch.Generator(device="cuda").manual_seed(800 + m)
+    w, x = M.Marlin.random(rows, cols, g), torch.randn(m + 5, cols, generator=g, device="cuda").half()
+    order = torch.randint(0, m + 5, (m,), generator=g, device="cuda").to(torch.int32)
+    valid, keys, again = rows - 100, *(torch.zeros(m, dtype=torch.int64, device="cuda") for _ in "ab")
+    y = ctx.marlin_gemm(x, w.words, w.scales, epi="argmax", xrows=order, keys=keys, n_valid=valid)
+    assert torch.equal(y, ctx.marlin_gemm(x, w.words, w.scales, epi="argmax", xrows=order, keys=again, n_valid=valid))
+    torch.cuda.synchronize()
+    assert torch.equal(keys, again) and ctx.device_error() == 0
+    a = y.cpu().numpy()
+    assert (keys.cpu().numpy().view(np.uint64) == R.argmax_keys(a, valid)).all()
+    x64, last = x[order.long()].double().cpu().numpy(), rows // 64 - 1
+    groups = sorted({0, 1, last, *np.random.default_rng(m).integers(0, last, 5).tolist()})
+    exact = {}
+    for c in groups:
+        q, s = R.unpack_marlin(w.words[:, 128 * c:128 * (c + 1)].cpu().numpy().view(np.uint32), w.scales[:, 64 * c:64 * (c + 1)].cpu().numpy())
+        exact[c] = x64 @ ((q.astype(np.float64) - 8) * np.repeat(s.astype(np.float64), 128, 1)).T
+    top = max(np.abs(e).max() for e in exact.values())
+    for c, e in exact.items():
+        assert np.abs(a[:, 64 * c:64 * (c + 1)] - e).max() < 1e-5 * top
+    if m > 64:
+        return
+    rows3 = torch.arange(3, 3 + m, dtype=torch.int32, device="cuda")
+    flat = ctx.marlin_gemm(x, w.words, w.scales, y=torch.zeros(m + 5, rows, device="cuda"), row0=3, m=m)
+    assert torch.equal(flat[3:3 + m], ctx.marlin_gemm(x, w.words, w.scales, xrows=rows3)) and not flat[:3].any() and not flat[3 + m:].any()
+    gl = ctx.marlin_gemm(x, w.words, w.scales, epi="silu", y=torch.zeros(m + 5, rows // 2, dtype=torch.float16, device="cuda"), row0=3, m=m)
+    assert torch.equal(gl[3:3 + m], ctx.marlin_gemm(x, w.words, w.scales, epi="silu", xrows=rows3))
+    gate, up = (t.double().reshape(m, -1) for t in flat[3:3 + m].view(m, rows // 16, 2, 8).unbind(2))
+    want = gate / (1 + torch.exp(-gate)) * up   # (of the f32 sums: the f16 result falls on it or a neighbour)
+    assert ((gl[3:3 + m].double() - want).abs() <= 2 ** -10 * want.abs() + 2 ** -23).all()
+    assert ctx.device_error() == 0
+
+
 @pytest.mark.parametrize("m,rows,cols", [(17, 256, 128), (40, 1024, 640), (64, 512, 1024)])
 def test_few_rows_contiguous_from_row0(ctx, m, rows, cols):
     x, wdq, xd, wd, sd = make(rows, cols, True, 600 + m, m + 20)
@@ -137,9 +176,10 @@ def test_few_rows_contiguous_from_row0(ctx, m, rows, cols):
     assert (got[7:7 + m] == R.argmax_keys(b[7:7 + m], rows)).all() and np.all(got[:7] == 0) and np.all(got[7 + m:] == 0)
 
 
-@pytest.mark.parametrize("m", [65, 97, 256, 257, 333])
+@pytest.mark.parametrize("m", [17, 32, 33, 64, 65, 97, 256, 257, 333])
 def test_token_tile_widths_and_zero_points(ctx, m):
-    """The tile's width follows the row count (96, 128, 256, 2 x 160, 2 x 192 tokens); zero-point matrices take the same path."""
+    """The tile's width follows the row count (32, 64, 96, 128, 256, 2 x 160, 2 x 192 tokens) of zero-point matrices, which take
+    the prompt-sized product from 17 rows on."""
     g = synth.gen(700 + m)
     x = synth.activations(m, 384, g)
     codes, sc = synth.int4_matrix(512, 384, g)
