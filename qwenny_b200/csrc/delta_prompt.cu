@@ -3,7 +3,7 @@
 // (kernels/qwen_deltanet.cuh: delta_conv :84-131, delta_rule :172-288, delta_norm :295-315), another algorithm:
 //
 //  delta_prep_kernel        the causal depthwise conv, SiLU, the L2 norms of the q and k heads and the two gates. A
-//                           lane owns FOUR channels and slides along 8 or 16 tokens with the conv's four inputs in
+//                           lane owns FOUR channels and slides along 8 tokens with the conv's four inputs in
 //                           registers (each input row is read once, not four times); the 128 channels of a warp are
 //                           one q, k or v head, so the head's norm is a warp reduction per token.
 //  delta_chunk_prep_kernel  the part of the CHUNKED delta rule that does not depend on the state (the WY form the
@@ -29,14 +29,15 @@ namespace qb {
 
 // grid (LQKV / 512 + 1, ceil(n / PREP_TOK)), block 128: a warp is one head, a lane four of its channels; the last column of
 // blocks makes the gates. Bound by the rows' way from memory and back (n x 80 KB): every row of the tile is requested
-// before anything is used, 16 bytes per lane, and the head's norm is a warp reduction (2048 tokens: 62 us; 79 us with
+// before anything is used, 16 bytes per lane, and the head's norm is a warp reduction (2048 tokens: 53 us; 76 us with
 // a channel per thread, four bytes per request and the gates behind the first head's channels).
 // VEC: p and cv start on 16 bytes, as a device allocation does; elsewhere (any float address is allowed) a lane moves its four
 // channels one by one.
-// PREP_TOK: the tokens a block slides along. 8 leave room for five blocks per SM, 16 read less history: the mixer of 40 rows takes
-// 48.0 and 51.2 us with them, of 150 138 and 129, of 333 179 and 174, of 700 245 and 256, of 1300 328 and 338.
-template <int PREP_TOK, bool VEC>
-__global__ void __launch_bounds__(128, PREP_TOK == 8 ? 5 : 4)
+// 8 tokens per block leave room for five blocks per SM; 16 read less history but take 9.4 us for 129 tokens (8: 5.8), 10.5 for
+// 333 (10.3), 17.5 for 512 (11.9), 61 for 2048 (53), and gain only around 420 (10.6, 11.0).
+constexpr int PREP_TOK = 8;  // tokens a block slides along
+template <bool VEC>
+__global__ void __launch_bounds__(128, 5)
 delta_prep_kernel(const float* p, int splits, int n, const float* ba, int ba_splits, const float* cw,
                   const float* a_log, const float* dt_bias, const float* mem, long long sst, float* cv,
                   const int* tok_slot, const int* tok_pos) {
@@ -689,11 +690,8 @@ int qb_delta_conv(qb_ctx* ctx, void* stream, const float* p, int splits, int n, 
     if (!ctx || !p || !ba || !cw || !a_log || !dt_bias || !mem || !cv || !tok_slot || !tok_pos || n <= 0 ||
         splits < 1 || ba_splits < 1)
         return QB_ERR_ARG;
-    const bool wide = n > 128 && n <= 512;
-    const dim3 grid(LQKV / 512 + 1, wide ? (n + 15) / 16 : (n + 7) / 8);
-    const bool vec = (((uintptr_t)p | (uintptr_t)cv) & 15) == 0;
-    auto kern = vec ? (wide ? delta_prep_kernel<16, true> : delta_prep_kernel<8, true>)
-                    : (wide ? delta_prep_kernel<16, false> : delta_prep_kernel<8, false>);
+    const dim3 grid(LQKV / 512 + 1, (n + PREP_TOK - 1) / PREP_TOK);
+    auto kern = (((uintptr_t)p | (uintptr_t)cv) & 15) == 0 ? delta_prep_kernel<true> : delta_prep_kernel<false>;
     return launch(ctx, kern, grid, dim3(128), 0, (cudaStream_t)stream, p, splits, n, ba, ba_splits, cw, a_log, dt_bias, mem, sst, cv,
                   tok_slot, tok_pos);
 }

@@ -343,9 +343,9 @@ def test_rollback_after_a_chunked_prompt(ctx):
                                        ((300, 7, 150, 1, 64), (1, 2, 0, 30, 3))])
 @pytest.mark.parametrize("splits", [1, 2])
 def test_conv_tiles(ctx, splits, lens, pos0):
-    """Segments that start and end anywhere in the conv's tiles (8 tokens; 16 for steps of 129 to 512), shorter than its history of
-    three, from position 0, from the slot's ring and across tiles, against the oracle (2e-4: the fast exponential of
-    SiLU, as in test_delta_conv)."""
+    """Segments that start and end anywhere in the conv's tiles of 8 tokens, shorter than its history of three, from
+    position 0, from the slot's ring and across tiles, against the oracle (2e-4: the fast exponential of SiLU, as in
+    test_delta_conv)."""
     g = synth.gen(171 + splits)
     toks = [(0, s, p + i) for s, (n, p) in enumerate(zip(lens, pos0)) for i in range(n)]
     n = len(toks)
@@ -389,8 +389,7 @@ def test_chunked_rule_against_the_oracle(ctx, lens):
 
 @pytest.mark.parametrize("n", [5, 150])
 def test_conv_of_rows_at_any_float_address(ctx, n):
-    """p and cv may start at any float address (a slice of a larger buffer): the bits of the 16-byte aligned call, in both
-    tile sizes."""
+    """p and cv may start at any float address (a slice of a larger buffer): the bits of the 16-byte aligned call."""
     g = synth.gen(191 + n)
     conv_w, a_log, dt_bias, _ = (t.cuda() for t in weights(g))
     mem, part = (fresh_mem(1, g) * 100).cuda(), torch.randn(2, n, R.DELTA_IN, generator=g).cuda()
