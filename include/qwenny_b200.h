@@ -32,8 +32,8 @@ typedef struct qb_ctx qb_ctx;
 enum { QB_EPI_PLAIN = 0, QB_EPI_SILU = 1, QB_EPI_ARGMAX = 2 };
 
 /* ---- context: what Gemm::load allocates once (src/cuda/core.rs:437-464: SM count, Marlin's `red` and `locks`).
- * Allocates the scratch and tickets on `device`: 32 MiB for the skinny products and, where there is room, 91 MB for the
- * prompt-sized kernels (without them 17 to 64 rows run as 16-row slabs, larger products as whole tiles and the delta rule
+ * Allocates the scratch and tickets on `device`: 52 MB that all calls use in turn, or, where there is no room, the 32 MiB of
+ * the skinny products (17 to 64 rows then run as 16-row slabs, larger products as whole tiles and the delta rule
  * token by token). Everything after creation is allocation-free. Like the
  * reference's single `red` / `locks` pair, a context serves one stream at a time: launches that share a context must
  * not overlap on the device (models that run concurrently take a context each). */

@@ -1,6 +1,7 @@
 // Context creation and the error word.
 #include "ctx.h"
 #include "common.cuh"
+#include <algorithm>
 #include <array>
 #include <map>
 #include <mutex>
@@ -76,21 +77,24 @@ int qb_create(int device, qb_ctx** out) {
     QB_CUDA(cudaSetDevice(device));
     int sms = 0;
     QB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
-    // One allocation: the words that must be zero (counters, error word, tickets), the split-K partials of the skinny products,
-    // then what only prompt-sized kernels use. Calls allocate nothing, so that they can be captured and a host may give all
-    // other memory away; where the last part does not fit, the context does without it.
+    // One allocation: the words that must be zero (counters, error word, tickets) and one area that the skinny products, the
+    // prompt-sized ones and the delta rule use in turn (none leaves anything there for a later call, and every kernel waits
+    // for the one before it before it writes there). Calls allocate nothing, so that they can be captured and a host may give all
+    // other memory away; where only the skinny products' part fits, the context does without the rest.
     // The split-K partials' largest user is a 16-row product, [n/64][nsplit][2][4][32] float4; 32 MiB covers
     // n * nsplit up to 2^17 * 8 (the 27B shapes need under 6 MiB).
     const size_t ncounters = 1 << 14, err_at = ncounters * sizeof(int), tickets_at = err_at + 256;
-    const size_t scratch_at = tickets_at + QB_TC_TICKETS * sizeof(int), scratch_bytes = 32u << 20, part_at = scratch_at + scratch_bytes;
-    const size_t tp_at = part_at + qb_tc_part_bytes(sms);
+    // The area starts on a 2 MiB page of its own (behind the tickets on the same page the 17 to 64-row products took 1 to 3 %
+    // longer: 5120 x 17408, 40 rows 33.0 and 33.7 us).
+    const size_t zeroed = tickets_at + QB_TC_TICKETS * sizeof(int), scratch_at = 2u << 20, scratch_bytes = 32u << 20;
+    static_assert((1 << 14) * sizeof(int) + 256 + QB_TC_TICKETS * sizeof(int) <= (2u << 20), "the words come before the area");
     char* b = nullptr;
-    const bool all = cudaMalloc(&b, tp_at + qb_delta_tp_bytes()) == cudaSuccess;
+    const bool all = cudaMalloc(&b, scratch_at + std::max({scratch_bytes, qb_tc_part_bytes(sms), qb_delta_tp_bytes()})) == cudaSuccess;
     if (!all) {
         (void)cudaGetLastError();
-        QB_CUDA(cudaMalloc(&b, part_at));
+        QB_CUDA(cudaMalloc(&b, scratch_at + scratch_bytes));
     }
-    cudaError_t e = cudaMemset(b, 0, scratch_at);
+    cudaError_t e = cudaMemset(b, 0, zeroed);
     if (e == cudaSuccess) e = cudaStreamSynchronize(0);  // (a context's stream need not wait for the default one)
     if (e != cudaSuccess) {
         cudaFree(b);
@@ -108,8 +112,7 @@ int qb_create(int device, qb_ctx** out) {
     c->scratch_bytes = scratch_bytes;
     if (all) {
         c->tc_tickets = (int*)(b + tickets_at);
-        c->tc_part = (float*)(b + part_at);
-        c->delta_tp = (float*)(b + tp_at);
+        c->tc_part = c->delta_tp = c->scratch;
     }
     *out = c;
     return QB_OK;

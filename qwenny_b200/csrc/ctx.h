@@ -16,8 +16,9 @@ struct qb_ctx {
     size_t ncounters = 0;
     int* err = nullptr;  // device word
     int* form = nullptr; // device word: the form of the prompt attention that the step under way takes
-    // The prompt-sized kernels' scratch. It is taken at creation like the rest, in one allocation with it (`block`); a device
-    // that has room for the rest alone gets a context without it, whose calls take the forms that need none.
+    // The prompt-sized kernels' scratch, in one area with `scratch` (calls use it in turn) and one allocation with the rest
+    // (`block`). A device that has room for the skinny products' part alone gets a context without it, whose calls take the
+    // forms that need none.
     void* block = nullptr;
     float* tc_part = nullptr;   // partial tiles of the tensor-core W4A16 products' shares (sms x 256 KB)
     int* tc_tickets = nullptr;  // their tickets, two per tile (QB_TC_TICKETS, zero between launches)
@@ -78,8 +79,8 @@ int qb_attn_prefill_as(qb_ctx* ctx, void* stream, const float* q, const void* kc
                        const int* ptile, const int* tok_slot, const int* tok_pos, int cap, int ntile, int max_keys, float* part_ml,
                        float* part_acc, float* out, void* mix_f16, int as);
 int qb_attn_prefill_launches(const qb_ctx* ctx, int ntile, int max_keys, int as);
-// the prompt-sized W4A16 product on tcgen05 (w4a16_gemm_tc.cu); reached through qb_marlin_gemm / qb_marlin_gemm_z (zp:
-// S carries the offsets' table after the scales) for more than 16 rows
+// the prompt-sized W4A16 product on tcgen05 (w4a16_gemm_tc.cu); reached through qb_marlin_gemm for more than 64 rows and
+// qb_marlin_gemm_z (zp: S carries the offsets' table after the scales) for more than 16
 int qb_gemm_tc_launch(qb_ctx* ctx, cudaStream_t st, const void* X, const void* B, void* Y, const void* S, int m, int n,
                       int k, int row0, int epi, int zp);
 // bytes of the prompt-sized kernels' scratch: tc_part on a part with `sms` SMs, delta_tp
