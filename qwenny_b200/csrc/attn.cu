@@ -415,13 +415,6 @@ attn_decode_kernel(const float* q, const uint8_t* kc, const uint8_t* vc, const f
 }
 
 // ------------------------------------------------------------------------------------------------ decode attention
-// 2^x, results below 2^-126 as 0 (exp2f spends three more instructions on those; P is rounded to f16 next)
-__device__ __forceinline__ float exp2_ftz(float x) {
-    float y;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
-
 // Block (short segment, kv head, key split) of the decode / verify attention: 2 to 4 QUADS of four compute warps and a
 // copy warp. The keys and values of the split arrive in 64-key stages through a ring fed by bulk copies; the quads
 // take the stages in turn. Inside a quad the work of a stage is dealt so that no byte is converted twice:
@@ -659,7 +652,7 @@ attn_dec4_kernel(const float* q, const uint8_t* kc, const uint8_t* vc, const flo
 #pragma unroll
                     for (int e = 0; e < 2; e++) {
                         const float sv = v[rt][nn][2 * h2 + e];
-                        const float pp = sv == -INFINITY ? 0.f : exp2_ftz(sv - m[rt][h2]);
+                        const float pp = sv == -INFINITY ? 0.f : tc::ex2(sv - m[rt][h2]);
                         sum[h2] += pp;
                         pv[nn][2 * h2 + e] = pp * vsc[nn][e];
                     }

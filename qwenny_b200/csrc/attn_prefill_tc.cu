@@ -11,7 +11,7 @@
 // the int8 -> f16 conversion and the shared memory per block are half of what one block per tile pair needs.
 // Over a pair an instruction takes some 128 cycles whatever its N, so the stage is 128 keys: 2048 rows at context 30720 take 2.79
 // ms with one block per two tiles and 64-key stages, 2.66 as pairs with 64-key stages (S then takes 2000 of 3100 cycles
-// per stage), 2.02 as pairs with 128.
+// per stage), 2.02 as pairs with 128. The pair passes over its tiles once per run of consecutive tiles of one sequence.
 //   warps 8-15  read the block's share of a stage's int8 keys and values from the cache (128-bit loads, one stage ahead in
 //               registers) and write it as f16 where the tensor core wants it: K as four [64 keys][64 dims] K-major
 //               tiles, V transposed as two [128 dims][64 keys] tiles, with the 128-byte swizzle; the codes are
@@ -24,8 +24,8 @@
 //               row, 64 keys each, and exchange their maxima through shared memory. Scores are scaled by the keys'
 //               scales, masked causally where the stage reaches the diagonal, and P = 2^(s - m) times the values'
 //               scales goes back as f16 (tcgen05.st), m the row's running maximum: the same rounding points as the
-//               reference's kernel; the arithmetic runs on pairs of f32, and half of the scores is read twice to keep the
-//               registers of a thread. A stage in which some row's maximum grows rescales that warp's accumulator rows
+//               reference's kernel; the arithmetic runs on pairs of f32, and half of the scores is read twice: 17 warps leave a
+//               thread 96 registers (40 bytes spill even so). A stage in which some row's maximum grows rescales that warp's accumulator rows
 //               (tcgen05.ld / st, half of the dims per thread); a lazier rule (rescale only past a threshold) was
 //               measured 1 % faster and decorrelates the f16 rounding of P from the reference's, so it is not used
 // At the end the softmax threads read their rows of O, divide by the row sum, multiply by the gate and write f32
@@ -158,7 +158,7 @@ attn_prefill_tc_kernel(const float* q, const uint8_t* kc, const uint8_t* vc, con
         const int tokn = mt < run && tok < ptile[2 * (ta + mt) + 1] ? ptile[2 * (ta + mt)] + tok : -1;
         const uint32_t trow = tmem + ((uint32_t)(qd * 32) << 16);
 
-        // ---- Q of the 128 rows into tensor memory: every softmax thread converts and stores half of its row
+        // ---- Q of the 128 rows into shared memory: every softmax thread converts and stores half of its row
         if (warp < SM_WARPS) {
             const float* qp = q + ((size_t)max(tokn, 0) * NH + head) * HD;
 #pragma unroll 8  // (16 loads in flight: a thread reads a row of its own)
@@ -210,7 +210,7 @@ attn_prefill_tc_kernel(const float* q, const uint8_t* kc, const uint8_t* vc, con
             }
           }
         } else if (warp < SM_WARPS) {
-            // ------------------------------------------------------------ softmax: two threads per row, 32 keys each
+            // ------------------------------------------------------------ softmax: two threads per row, 64 keys each
             const int lim = tokn >= 0 ? tok_pos[tokn] + 1 : 1 << 30;  // (rows without a token: Q = 0, nothing masked)
             float m = -INFINITY, l = 0.f;
             for (int i = 0; i < nstg; i++) {

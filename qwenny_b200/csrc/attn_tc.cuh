@@ -1,6 +1,6 @@
 // What the attention on the 5th-generation tensor cores needs beside pair_tc.cuh: wide tensor-memory loads and stores, the
-// exact int8 -> f16 conversion of cache bytes, the 128-byte swizzle of a K-major tile, and bounded waits that sleep
-// instead of polling.
+// exact int8 -> f16 conversion of cache bytes, the 128-byte swizzle of a K-major tile, bounded waits that sleep instead of
+// polling, and the choice between its two forms.
 #pragma once
 #include "attn_common.cuh"
 #include "pair_tc.cuh"
@@ -63,6 +63,7 @@ __device__ __forceinline__ bool mbar_wait_sleepy(uint64_t* bar, uint32_t parity)
         if (mbar_try_wait_hint(bar, parity, 2000)) return true;
     return false;
 }
+// 2^x, results below 2^-126 as 0 (exp2f spends three more instructions on those; P is rounded to f16 next)
 __device__ __forceinline__ float ex2(float x) {
     float y;
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));

@@ -1,5 +1,5 @@
-// What the W4A16 products on pairs of blocks (tcgen05 cta_group::2) share: descriptors, the product / commit / tensor-memory
-// wrappers, barriers across the pair, the exact unpacking of a Marlin word, and the dealing of (tile, k block) lists.
+// What the tcgen05 kernels share (the W4A16 products and the prompt attention; one block or a pair of blocks per tile):
+// descriptors, the product / commit / tensor-memory wrappers, arrivals across a pair, and the dealing of (tile, k block) lists.
 #pragma once
 #include <cuda.h>
 #include "common.cuh"

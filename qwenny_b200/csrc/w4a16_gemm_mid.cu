@@ -6,7 +6,8 @@
 // (w4a16_gemm_tc.cu). The floor is the weights' way from HBM (0.52 bytes each, read once): 380 cycles per block and 128 of
 // k. It takes some 1150: the eight products of a stage take their issuing lane 700 (tensor pipe 15 % active, DRAM 20 %; a probe
 // of such products alone takes 47 each), so their way through tensor memory beside the stores of the next weights is
-// what the stages wait for.
+// what the stages wait for. Besides, a drain thread holds 32 sums and 32 loaded values: with 48 and 64 tokens its 80 registers
+// spill 20 to 60 bytes, read back with every group.
 // 40 rows: 16384 x 5120 30.5 us, 5120 x 6144 23.0, 34816 x 5120 47.8 (62 as pairs of blocks), 5120 x 17408 34.5; padded to 256
 // tokens they took 69, 68, 70 and 89. What else differs from the prompt-sized product:
 //   - the weights are the exact integers q - 8; a group of 128 columns is one accumulation, and the drain warps multiply its

@@ -1,5 +1,5 @@
-// W4A16 product for prompt-sized steps (more than 16 token rows) on the 5th-generation tensor cores: Y = X . W^T with
-// W int4 in the reference's Marlin layout. Replaces marlin::mul<{1..4},16,4,*> (kernels/marlin.cuh:171-582,
+// W4A16 product for prompt-sized steps (more than 64 token rows; zero-point matrices: more than 16) on the 5th-generation
+// tensor cores: Y = X . W^T with W int4 in the reference's Marlin layout. Replaces marlin::mul<{1..4},16,4,*> (kernels/marlin.cuh:171-582,
 // launched by Gemm::marlin, src/cuda/core.rs:569-612, for n > 16).
 //
 // A pair of blocks (a cluster of two, one block per SM) computes a tile of 256 outputs x up to 256 tokens with
@@ -19,7 +19,7 @@
 // tile's last arriver adds the parts in pair order and runs the epilogue, nobody waits. Otherwise a pair is a tile.
 // Per (tile, k block):
 //   warps 0-7   dequantise: lop3 / hsub2 to q - 8, one hfma2 by the f16 group scale (the reference's rounding:
-//               w = f16((q - 8) s), kernels/marlin.cuh:100-124), tcgen05.st into the stage's 32 columns; then they run
+//               w = f16((q - 8) s), kernels/marlin.cuh:100-124), tcgen05.st into the stage's 64 columns; then they run
 //               the epilogue: tcgen05.ld of the accumulators, Y [token][output] f32, or silu(gate) * up as f16 for
 //               the interleaved SwiGLU matrices (or the partial tile)
 //   warp 8      copies, one lane: the X half tile (tensor map, 128-byte swizzle), the 8 KB of words (tensor map), the
@@ -50,7 +50,6 @@ constexpr int TMEM_COLS = 512;
 constexpr int A_COLS = BK / 2;              // tensor-memory columns of a stage's weights
 
 struct Args {
-    const uint32_t* B;   // Marlin words [K/16][2N]
     const __half* S;     // scales [K/128][N]
     void* Y;             // plain: f32 [.][N]; silu: f16 [.][N/2]; rows row0 ..
     int m, N, K, row0;
@@ -355,7 +354,7 @@ int qb_gemm_tc_launch(qb_ctx* ctx, cudaStream_t st, const void* X, const void* B
         return QB_ERR_ARG;
     const int pairs = ctx->sms / 2;
     tc::Args a;
-    a.B = (const uint32_t*)B; a.S = (const __half*)S; a.Y = Y; a.m = m; a.N = n; a.K = k; a.row0 = row0; a.err = ctx->err;
+    a.S = (const __half*)S; a.Y = Y; a.m = m; a.N = n; a.K = k; a.row0 = row0; a.err = ctx->err;
     a.zp = zp ? 1 : 0; a.part = ctx->tc_part; a.tickets = ctx->tc_tickets; a.iters = tiles * (k / tc::BK);
     a.bt = bt; a.tiles = (int)tiles;
     // One pair per tile (the hardware hands a freed pair of SMs the next tile) when the partly filled last wave wastes
