@@ -94,8 +94,15 @@ int qb_create(int device, qb_ctx** out) {
         (void)cudaGetLastError();
         QB_CUDA(cudaMalloc(&b, scratch_at + scratch_bytes));
     }
-    cudaError_t e = cudaMemset(b, 0, zeroed);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(0);  // (a context's stream need not wait for the default one)
+    // zeroed on a stream of its own: the context's stream need not wait for the default one, and creation need not wait for
+    // what runs there
+    cudaStream_t st = nullptr;
+    cudaError_t e = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking);
+    if (e == cudaSuccess) {
+        e = cudaMemsetAsync(b, 0, zeroed, st);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+        cudaStreamDestroy(st);
+    }
     if (e != cudaSuccess) {
         cudaFree(b);
         return (int)e;
