@@ -860,14 +860,17 @@ attn_combine_tiles_kernel(const float* part_ml, const float* part_acc, const int
     combine_row(part_ml, part_acc, ((size_t)t * NH + h) * z, (keys + chunk - 1) / chunk, out + o, mix ? mix + o : nullptr);
 }
 
-// one block: which form the two tcgen05 kernels behind it take. It does not let them start before it ends: the one that works holds
-// whole SMs and their tensor memory, and nothing should wait there for a step that is not its own.
+// one block: which form the two tcgen05 kernels behind it take
 constexpr int FORM_THREADS = 512;
 __global__ void __launch_bounds__(FORM_THREADS)
 attn_form_kernel(const int* ptile, int ntile, const int* tok_slot, const int* tok_pos, int sms, int* on_pairs) {
+    pdl_launch_dependents();
     pdl_wait();
     const bool p = tc::tiles_on_pairs(ptile, ntile, tok_slot, tok_pos, sms);
-    if (threadIdx.x == 0) *on_pairs = p;
+    if (threadIdx.x == 0) {
+        on_pairs[0] = p;
+        on_pairs[1] = 0;
+    }
 }
 
 }  // namespace qb
@@ -968,7 +971,9 @@ namespace {
 // set-up cost more there than the faster stages give (100 rows at context 0 40.1 us as blocks, 43.7 as pairs; 1500 at 100
 // 200 and 210; 2048 at 0 289 and 277; 1024 at 2000 257 and 225). Beyond, the runs of the tiles decide (attn_tc.cuh): 0
 // blocks, 1 pairs. A caller that has the tiles on the host says which; for the others (2) a small kernel works it out and
-// both forms are launched, one of which returns (2 to 4 us: 400 rows at 4000 126 -> 128, 2048 at 30720 1922 -> 1926).
+// both forms are launched, one of which returns before it takes anything (with attn_prep, in a graph: 600 rows at 2000
+// 106 -> 112 us, 400 at 4000 136.6 -> 138.6, 2048 at 1700 370 -> 376, 2048 at 8000 734 -> 734; each of the blocks working it
+// out for itself: 4 to 6 % throughout).
 int prefill_form(const qb_ctx* ctx, int max_keys, int as) {
     if (ctx->tune_ctas == 1002 || ctx->tune_ctas == 1003) return ctx->tune_ctas - 1002;  // measurement
     return max_keys <= 1664 ? 0 : as < 0 ? 2 : as;
@@ -990,7 +995,7 @@ int qb_attn_prefill_as(qb_ctx* ctx, void* stream, const float* q, const void* kc
     if (z > 1 && (!part_ml || !part_acc)) return QB_ERR_ARG;
     if (z == 1) {
         const int form = prefill_form(ctx, max_keys, as);
-        const int* word = form == 2 ? ctx->form : nullptr;
+        int* word = form == 2 ? ctx->form : nullptr;
         cudaStream_t st = (cudaStream_t)stream;
         int rc = QB_OK;
         if (word) rc = launch(ctx, attn_form_kernel, dim3(1), dim3(FORM_THREADS), 0, st, ptile, ntile, tok_slot, tok_pos, ctx->sms, ctx->form);

@@ -47,12 +47,16 @@ constexpr int TMEM_COLS = 512, O_COL = 0, S_COL = 256, Q_COL = 384;
 
 using namespace tc;
 
+// CHOOSE: the form behind attn_form_kernel, which says whether this one does the step (on_pairs[0] == 0). A block per SM at most,
+// which take the units (pair of tiles, kv head) in turn from the counter on_pairs[1], so that few blocks start for nothing.
+template <bool CHOOSE>
 __global__ void __launch_bounds__(THREADS, 1)
 attn_prefill_short_kernel(const float* q, const uint8_t* kc, const uint8_t* vc, const float* ks, const float* vs,
                        const int* ptile, int ntile, const int* tok_slot, const int* tok_pos, int cap, float* out,
-                       __half* mix, int* err, const int* on_pairs) {
+                       __half* mix, int* err, int* on_pairs) {
     extern __shared__ uint8_t smem_raw[];
-    if (on_pairs) {  // both forms are launched, and the step decides: the other one returns before it takes anything
+    if (CHOOSE) {
+        pdl_launch_dependents();
         pdl_wait();
         if (*(const volatile int*)on_pairs) return;
     }
@@ -68,8 +72,9 @@ attn_prefill_short_kernel(const float* q, const uint8_t* kc, const uint8_t* vc, 
     uint64_t* p_ready = s_ready + 2;       // [2] P of a stage is written over its S (8 warps)
     uint64_t* o_done = p_ready + 2;        // [2] O += P V of a stage is complete
     uint32_t* tmem_slot = (uint32_t*)(o_done + 2);
+    int* next = (int*)(tmem_slot + 1);
 
-    const int g = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
         for (int i = 0; i < NST; i++) {
             mbar_init(&kv_ready[i], CVT_WARPS);
@@ -91,11 +96,23 @@ attn_prefill_short_kernel(const float* q, const uint8_t* kc, const uint8_t* vc, 
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
-    pdl_launch_dependents();
-    pdl_wait();
+    if (!CHOOSE) {
+        pdl_launch_dependents();
+        pdl_wait();
+    }
 
-    // the block's tiles: 2 pair, 2 pair + 1 (the last pairs, with the longest contexts, first)
-    const int pair = gridDim.x - 1 - blockIdx.x, ta = 2 * pair, tb = ta + 1;
+    int jbase = 0;  // stages of earlier passes: ring slots and barrier phases run on
+    Waiter w_mma{err, 11}, w_sm{err, 12}, w_cv{err, 13};
+    const int npair = (ntile + 1) / 2;
+    for (int unit = blockIdx.x;;) {
+    if (CHOOSE) {
+        if (threadIdx.x == 0) *next = atomicAdd(on_pairs + 1, 1);
+        __syncthreads();
+        unit = *next;
+        if (unit >= npair * NKV) break;
+    }
+    // the unit's tiles: 2 pair, 2 pair + 1 (the last pairs, with the longest contexts, first)
+    const int g = unit / npair, pair = npair - 1 - unit % npair, ta = 2 * pair, tb = ta + 1;
     const int firstA = ptile[2 * ta], ntA = ptile[2 * ta + 1];
     int firstB = 0, ntB = 0;
     bool paired = false;
@@ -104,9 +121,6 @@ attn_prefill_short_kernel(const float* q, const uint8_t* kc, const uint8_t* vc, 
         paired = firstB == firstA + ntA && tok_slot[firstB] == tok_slot[firstA] && tok_pos[firstB] == tok_pos[firstA] + ntA;
     }
     const int npass = tb < ntile && !paired ? 2 : 1;
-    int jbase = 0;  // stages of earlier passes: ring slots and barrier phases run on
-    Waiter w_mma{err, 11}, w_sm{err, 12}, w_cv{err, 13};
-
     for (int pass = 0; pass < npass; pass++) {
         // rows 0..63: tile 0 of the pass; rows 64..127: its partner (present only in a pair of consecutive tiles)
         const int first0 = pass == 0 ? firstA : firstB, nt0 = pass == 0 ? ntA : ntB;
@@ -337,6 +351,8 @@ attn_prefill_short_kernel(const float* q, const uint8_t* kc, const uint8_t* vc, 
         __syncthreads();  // the pass is complete: Q may be rewritten
         tc_fence_after();
     }
+    if (!CHOOSE) break;
+    }
     tc_fence_before();
     __syncthreads();
     if (warp == MMA_WARP) {
@@ -350,9 +366,11 @@ attn_prefill_short_kernel(const float* q, const uint8_t* kc, const uint8_t* vc, 
 // the many-tile form of qb_attn_prefill (one key split): see attn.cu, and attn_prefill_tc.cu for on_pairs
 int qb_attn_prefill_short_launch(qb_ctx* ctx, cudaStream_t st, const float* q, const void* kc, const void* vc, const float* ks,
                               const float* vs, const int* ptile, int ntile, const int* tok_slot, const int* tok_pos,
-                              int cap, float* out, void* mix_f16, const int* on_pairs) {
+                              int cap, float* out, void* mix_f16, int* on_pairs) {
     using namespace qb;
-    return launch(ctx, pfs::attn_prefill_short_kernel, dim3((ntile + 1) / 2, NKV), dim3(pfs::THREADS), pfs::SMEM_BYTES, st, q,
+    const int units = (ntile + 1) / 2 * NKV;
+    return launch(ctx, on_pairs ? pfs::attn_prefill_short_kernel<true> : pfs::attn_prefill_short_kernel<false>,
+                  dim3(on_pairs && units > ctx->sms ? ctx->sms : units), dim3(pfs::THREADS), pfs::SMEM_BYTES, st, q,
                   (const uint8_t*)kc, (const uint8_t*)vc, ks, vs, ptile, ntile, tok_slot, tok_pos, cap, out,
                   (__half*)mix_f16, ctx->err, on_pairs);
 }

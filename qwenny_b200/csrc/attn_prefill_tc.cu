@@ -81,7 +81,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
 attn_prefill_tc_kernel(const float* q, const uint8_t* kc, const uint8_t* vc, const float* ks, const float* vs,
                        const int* ptile, int ntile, const int* tok_slot, const int* tok_pos, int cap, float* out,
                        __half* mix, int* err, const int* on_pairs) {
-    if (on_pairs) {  // both forms are launched, and the step decides: the other one returns before it takes anything
+    if (on_pairs) {  // the form behind attn_form_kernel: where the other one does the step, return before anything is taken
         pdl_wait();
         if (!*(const volatile int*)on_pairs) return;
     }

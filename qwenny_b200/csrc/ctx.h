@@ -15,7 +15,7 @@ struct qb_ctx {
     int* counters = nullptr;
     size_t ncounters = 0;
     int* err = nullptr;  // device word
-    int* form = nullptr; // device word: the form of the prompt attention that the step under way takes
+    int* form = nullptr; // two device words: the form of the prompt attention that the step under way takes, a counter of its work
     // The prompt-sized kernels' scratch, in one area with `scratch` (calls use it in turn) and one allocation with the rest
     // (`block`). A device that has room for the skinny products' part alone gets a context without it, whose calls take the
     // forms that need none.
@@ -73,7 +73,7 @@ int qb_attn_prefill_tc_launch(qb_ctx* ctx, cudaStream_t st, const float* q, cons
                               int cap, float* out, void* mix_f16, const int* on_pairs);
 int qb_attn_prefill_short_launch(qb_ctx* ctx, cudaStream_t st, const float* q, const void* kc, const void* vc, const float* ks,
                                  const float* vs, const int* ptile, int ntile, const int* tok_slot, const int* tok_pos,
-                                 int cap, float* out, void* mix_f16, const int* on_pairs);  // short contexts, short runs (attn_prefill_short.cu)
+                                 int cap, float* out, void* mix_f16, int* on_pairs);  // short contexts, short runs (attn_prefill_short.cu)
 // qb_attn_prefill for a caller that knows qb_attn_tiles_on_pairs of its tiles (as: 0 or 1; -1: not known), and its launches
 int qb_attn_prefill_as(qb_ctx* ctx, void* stream, const float* q, const void* kc, const void* vc, const float* ks, const float* vs,
                        const int* ptile, const int* tok_slot, const int* tok_pos, int cap, int ntile, int max_keys, float* part_ml,
