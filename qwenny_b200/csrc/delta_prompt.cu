@@ -181,19 +181,23 @@ __device__ __forceinline__ void mma3(float* c, const FragA& a, float b0, float b
 // grid (chunks of the longest possible segment, LK_HEADS, segs), block 256. tp: [chunk index][LV_HEADS][TP_FLOATS],
 // chunk index = first token of the chunk / 64 (distinct for disjoint 64-token ranges).
 constexpr int CP_THREADS = 256;
-// 102 KB: two blocks per SM. With K K^T and Q K^T over the tiles (69 KB, three blocks) the second exponential and barrier cost
-// more than the third block gives: 2048 tokens 120 -> 126 us, eight segments of 100 63 -> 85, three of 150 with the scan 135 -> 156.
-constexpr int CP_SMEM = (2 * CH * KLD + 2 * CH * (CH + 1) + 6 * CH) * 4;
-static_assert(3 * CH * (CH + 1) <= 2 * CH * KLD, "the three A matrices reuse the q / k tiles");
+// Two blocks per SM (102 KB), or, TIGHT, three (69 KB: K K^T and Q K^T over the tiles, which costs a second exponential and a
+// barrier). Three are slower wherever two do as well (2048 tokens 126 us against 120, eight segments of 100 85 against 63,
+// where active blocks crowd onto few SMs), and win where they make one wave of two: one sequence with more chunks x key
+// heads than two per SM and no more than three (1232 to 1807 tokens: the rule of 1300 260 us with three, 277 with two).
+template <bool TIGHT>
+constexpr int CP_SMEM = (2 * CH * KLD + (TIGHT ? 0 : 2 * CH * (CH + 1)) + 6 * CH) * 4;
+static_assert(4 * CH * (CH + 1) <= 2 * CH * KLD, "the three A matrices (and K K^T) reuse the q / k tiles");
 
+template <bool TIGHT>
 __global__ void __launch_bounds__(CP_THREADS)
 delta_chunk_prep_kernel(const float* cv, float* tp, const int* seg_start, const int* seg_len) {
     extern __shared__ __align__(16) float cps[];
     float* Ks = cps;                         // [64][KLD]; later A of the three value heads [3][64][65]
     float* Qs = Ks + CH * KLD;
-    float* KK = Qs + CH * KLD;               // [64][65]; later scratch of the inverse
-    float* QK = KK + CH * (CH + 1);
-    float* gs = QK + CH * (CH + 1);          // [3][64] cumulative log decay
+    float* KK = TIGHT ? Ks + 3 * CH * (CH + 1) : Qs + CH * KLD;  // [64][65]; later scratch of the inverse
+    float* QK = TIGHT ? Ks : KK + CH * (CH + 1);
+    float* gs = TIGHT ? Qs + CH * KLD : QK + CH * (CH + 1);      // [3][64] cumulative log decay
     float* bs = gs + 3 * CH;                 // [3][64] beta
     pdl_launch_dependents();
     const int c = blockIdx.x, kh = blockIdx.y, sg = blockIdx.z, tid = threadIdx.x;
@@ -243,6 +247,7 @@ delta_chunk_prep_kernel(const float* cv, float* tp, const int* seg_start, const 
             for (int j = 0; j < 8; j++)
                 if (j < nts) mma3(acc[j], a, br[8 * j * KLD + k0], br[8 * j * KLD + k0 + 4]);
         }
+        if (TIGHT) __syncthreads();  // every warp is done with the tiles
 #pragma unroll
         for (int j = 0; j < 8; j++) {
             float* d0 = dst + (16 * m + g8) * (CH + 1) + 8 * j + 2 * t4;
@@ -251,23 +256,32 @@ delta_chunk_prep_kernel(const float* cv, float* tp, const int* seg_start, const 
         }
     }
     __syncthreads();
-    // A of the three value heads over the q / k tiles (done with), and P straight to global memory
+    // A of the three value heads over the q / k tiles (done with), and P straight to global memory (TIGHT: A over Q K^T after it)
     float* As = Ks;
     for (int x = tid; x < 3 * CH * CH; x += CP_THREADS) {
         const int hv = x / (CH * CH), i = (x / CH) % CH, j = x % CH;
         const float dec = j <= i ? expf(gs[hv * CH + i] - gs[hv * CH + j]) : 0.f;
-        As[(hv * CH + i) * (CH + 1) + j] = j < i ? bs[hv * CH + i] * KK[i * (CH + 1) + j] * dec : 0.f;
+        if (!TIGHT) As[(hv * CH + i) * (CH + 1) + j] = j < i ? bs[hv * CH + i] * KK[i * (CH + 1) + j] * dec : 0.f;
         float* out = tp + ((size_t)(tok >> 6) * LV_HEADS + kh * G + hv) * TP_FLOATS;
         out[CH * CH + i * CH + j] = j <= i ? QK[i * (CH + 1) + j] * dec : 0.f;
         if (j == 0) out[2 * CH * CH + i] = gs[hv * CH + i];
     }
     __syncthreads();
+    if (TIGHT) {
+        for (int x = tid; x < 3 * CH * CH; x += CP_THREADS) {
+            const int hv = x / (CH * CH), i = (x / CH) % CH, j = x % CH;
+            As[(hv * CH + i) * (CH + 1) + j] =
+                j < i ? bs[hv * CH + i] * KK[i * (CH + 1) + j] * expf(gs[hv * CH + i] - gs[hv * CH + j]) : 0.f;
+        }
+        __syncthreads();
+    }
     // T = (I + A)^-1, unit lower triangular, IN PLACE over A. The four 16 x 16 diagonal blocks by forward substitution,
     // a thread per column (T_ic = -sum_{c <= j < i} A_ij T_jc), into scratch and back; then blocks merge pairwise,
     // 16 -> 32 -> 64: for a block pair [[T11, 0], [T21, T22]] the lower left part is T21 = -T22 (A21 T11), two small
     // products spread over the block (X = A21 T11 goes through scratch, so T21 may overwrite A21).
     float* D0 = KK;                    // [3][4][16][17] the diagonal blocks' inverses
-    float* Xs = KK + 3 * 4 * 16 * 17;  // [3][32][33] scratch of the merges (K K^T and Q K^T are done with)
+    // [3][32][33] scratch of the merges (K K^T and Q K^T are done with; TIGHT: once the diagonal blocks are back in place)
+    float* Xs = TIGHT ? KK : KK + 3 * 4 * 16 * 17;
     float* Ts = As;
     if (tid < 3 * CH) {
         const int hv = tid / CH, blk = (tid % CH) / 16, b0 = blk * 16, col = tid % 16;
@@ -708,8 +722,10 @@ int qb_delta_rule(qb_ctx* ctx, void* stream, const float* p, int splits, int n, 
     if (n > TP_TOK) return QB_ERR_TOO_LARGE;
     const int chunks = ctx->delta_tp ? chunked_tokens(n) / CH : 0;  // of the longest segment the step can hold
     if (chunks > 0) {
-        int rc = launch(ctx, delta_chunk_prep_kernel, dim3(chunks, LK_HEADS, segs), dim3(CP_THREADS), CP_SMEM, st, cv,
-                        ctx->delta_tp, seg_start, seg_len);
+        const int blocks = chunks * LK_HEADS;
+        const bool tight = segs == 1 && blocks > 2 * ctx->sms && blocks <= 3 * ctx->sms;
+        int rc = launch(ctx, tight ? delta_chunk_prep_kernel<true> : delta_chunk_prep_kernel<false>, dim3(chunks, LK_HEADS, segs),
+                        dim3(CP_THREADS), tight ? CP_SMEM<true> : CP_SMEM<false>, st, cv, ctx->delta_tp, seg_start, seg_len);
         if (rc) return rc;
     }
     auto waves = [&](long long parts) { return (parts * LV_HEADS * segs + ctx->sms - 1) / ctx->sms; };

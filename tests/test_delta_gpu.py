@@ -363,10 +363,11 @@ def test_conv_tiles(ctx, splits, lens, pos0):
     assert np.allclose(cv.cpu().numpy(), want, rtol=2e-4, atol=1e-5)
 
 
-@pytest.mark.parametrize("lens", [(80,), (79, 150), (300,), (80, 150, 81)])
+@pytest.mark.parametrize("lens", [(80,), (79, 150), (300,), (80, 150, 81), (1300,)])
 def test_chunked_rule_against_the_oracle(ctx, lens):
-    """The scan in parts of 48, 48 and 32 value columns and (three segments) in halves, chunks and the token form after them:
-    outputs and state of one to three segments, from zeros and from a stored state, against the oracle's f64 recurrence."""
+    """The scan in parts of 48, 48 and 32 value columns and (three segments) in halves, chunks and the token form after them, the
+    chunks prepared by two and (1300 tokens) by three blocks per SM: outputs and state of one to three segments, from
+    zeros and from a stored state, against the oracle's f64 recurrence."""
     g = synth.gen(181 + len(lens))
     toks = [(0, s, 7 * s + i) for s, n in enumerate(lens) for i in range(n)]
     n = len(toks)
