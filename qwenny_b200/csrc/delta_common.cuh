@@ -31,6 +31,15 @@ __device__ __forceinline__ Plan make_plan(const int* meta, int slot, int p0, int
     return p;
 }
 
+// Ahead of the kernel before, which may still write them: the slot's state (COLS columns of a head from `row` on) is asked into L2 by a
+// block of THREADS. The metadata read here only says which buffer; a stale value costs the hint.
+template <int COLS, int THREADS>
+__device__ __forceinline__ void hint_state(const int* meta, int slot, int p0, const float* sm0, int row) {
+    const int end = __ldcg(meta + slot * META), eb = __ldcg(meta + slot * META + 2);
+    const float* s = sm0 + (size_t)((p0 == end ? eb : 1 - eb) & 1) * SLOT_STATE + (size_t)row * LKD;
+    for (int x = threadIdx.x; x < COLS * LKD / 32; x += THREADS) asm volatile("prefetch.global.L2 [%0];\n" ::"l"(s + 32 * x));
+}
+
 __device__ __forceinline__ float4 ld4(const float* p) { return *(const float4*)p; }
 
 // The state rows of a thread, LPC lanes per value column. LPC = 4, sub = rg: rows 4 (rg + 4 j) + i as x[4 j + i],

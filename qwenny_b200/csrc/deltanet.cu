@@ -41,7 +41,7 @@ __global__ void __launch_bounds__(FNT)
 delta_fused_kernel(const float* p, int splits, int n, const float* ba, int ba_splits, const float* cw,
                    const float* a_log, const float* dt_bias, const float* nw, float* mem, long long sst, int* meta,
                    float* out, __half* y, const int* seg_start, const int* seg_len, const int* seg_slot,
-                   const int* seg_pos0, int segs, int* ticket, long long* trace) {
+                   const int* seg_pos0, int segs, int* ticket, long long* trace, int ahead) {
     extern __shared__ __align__(16) uint8_t fsm[];
     FusedRound& R = *(FusedRound*)fsm;
     pdl_launch_dependents();
@@ -60,11 +60,16 @@ delta_fused_kernel(const float* p, int splits, int n, const float* ba, int ba_sp
         return ch < LKD ? kh * LKD + ch : ch < 2 * LKD ? LK_HEADS * LKD + kh * LKD + (ch - LKD)
                                                        : 2 * LK_HEADS * LKD + h * LVD + hf * FCOLS + (ch - 2 * LKD);
     };
-    // ---- everything that does not depend on this step's earlier kernels: the taps, the norm weight, the state
+    // ---- everything that does not depend on this step's earlier kernels: the taps, the norm weight and, where the caller vouches
+    // for it (`ahead`), the state
     for (int c = tid; c < FCH; c += FNT) *(float4*)R.w[c] = ld4(cw + gchan(c) * CONV_K);
     const float nwv = nw[hf * FCOLS + tid % FCOLS], alog = a_log[h], dtb = dt_bias[h];
-    const Plan pl = make_plan(meta, slot, p0, len);
     float* sm0 = mem + slot * sst;
+    if (!ahead) {
+        hint_state<FCOLS, FNT>(meta, slot, p0, sm0, h * LVD + hf * FCOLS);
+        pdl_wait();
+    }
+    const Plan pl = make_plan(meta, slot, p0, len);
     auto sbuf = [&](int b) { return sm0 + (size_t)b * SLOT_STATE + ((size_t)h * LVD + col) * LKD; };
     auto entry = [&](int b, int pos) { return sm0 + 2 * SLOT_STATE + (size_t)b * SLOT_BANK + (size_t)(pos % KEEP) * REP; };
     float S[RPT];
@@ -333,13 +338,10 @@ delta_fused_kernel(const float* p, int splits, int n, const float* ba, int ba_sp
 
 }  // namespace qb
 
-// conv + rule + norm in one launch (same arguments as the three together); `out` (the raw output before the gated
-// norm, f32 [n][MIX]) may be NULL
-extern "C" int qb_delta_mixer(qb_ctx* ctx, void* stream, const float* p, int splits, int n, const float* ba,
-                              int ba_splits, const float* cw, const float* a_log, const float* dt_bias,
-                              const float* nw, float* mem, long long sst, int* meta, float* out, void* y,
-                              const int* seg_start, const int* seg_len, const int* seg_slot, const int* seg_pos0,
-                              int segs) {
+// qb_delta_mixer, for a caller that says whether the kernels may read the slots ahead of the kernel before (ctx.h)
+int qb_delta_mixer_as(qb_ctx* ctx, void* stream, const float* p, int splits, int n, const float* ba, int ba_splits, const float* cw,
+                      const float* a_log, const float* dt_bias, const float* nw, float* mem, long long sst, int* meta, float* out, void* y,
+                      const int* seg_start, const int* seg_len, const int* seg_slot, const int* seg_pos0, int segs, int ahead) {
     if (!ctx || !p || !ba || !cw || !a_log || !dt_bias || !nw || !mem || !meta || !y || !seg_start || !seg_len ||
         !seg_slot || !seg_pos0 || n <= 0 || segs <= 0 || splits < 1 || ba_splits < 1)
         return QB_ERR_ARG;
@@ -363,6 +365,17 @@ extern "C" int qb_delta_mixer(qb_ctx* ctx, void* stream, const float* p, int spl
     lc.numAttrs = ctx->pdl ? 2 : 1;
     cudaError_t e = cudaLaunchKernelEx(&lc, qb::delta_fused_kernel, p, splits, n, ba, ba_splits, cw, a_log, dt_bias, nw, mem,
                                        sst, meta, out, (__half*)y, seg_start, seg_len, seg_slot, seg_pos0, segs, ticket,
-                                       ctx->trace);
+                                       ctx->trace, ahead);
     return e == cudaSuccess ? QB_OK : (int)e;
+}
+
+// conv + rule + norm in one launch (same arguments as the three together); `out` (the raw output before the gated
+// norm, f32 [n][MIX]) may be NULL
+extern "C" int qb_delta_mixer(qb_ctx* ctx, void* stream, const float* p, int splits, int n, const float* ba,
+                              int ba_splits, const float* cw, const float* a_log, const float* dt_bias,
+                              const float* nw, float* mem, long long sst, int* meta, float* out, void* y,
+                              const int* seg_start, const int* seg_len, const int* seg_slot, const int* seg_pos0,
+                              int segs) {
+    return qb_delta_mixer_as(ctx, stream, p, splits, n, ba, ba_splits, cw, a_log, dt_bias, nw, mem, sst, meta, out, y, seg_start, seg_len,
+                             seg_slot, seg_pos0, segs, 0);
 }

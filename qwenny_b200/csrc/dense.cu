@@ -14,8 +14,8 @@ static_assert(H % 8 == 0 && H / 8 == ROW_THREADS, "a row of H is one vector of 8
 // out[t] = E[ids[t]] (bf16 -> f32); the first nkeys blocks clear the step's argmax keys
 __global__ void __launch_bounds__(ROW_THREADS) embed_kernel(const __nv_bfloat16* E, const int* ids, float* out,
                                                             unsigned long long* keys, int nkeys) {
+    pdl_wait();  // first: see launch.h
     pdl_launch_dependents();
-    pdl_wait();
     int t = blockIdx.x;
     if (threadIdx.x == 0 && t < nkeys) keys[t] = 0;
     const uint4* row = (const uint4*)(E + (size_t)ids[t] * H);
@@ -142,8 +142,8 @@ __global__ void __launch_bounds__(256) sum_parts_kernel(const float* x, int spli
 // One block per segment: a segment at position 0 clears its slot's set, then its marked tokens are set
 __global__ void __launch_bounds__(256) mark_seen_kernel(unsigned* seen, const int* mark, const int* mark_at,
                                                         const int* seg_slot, const int* seg_pos0, int seen_words) {
+    pdl_wait();  // first: see launch.h
     pdl_launch_dependents();
-    pdl_wait();
     int sg = blockIdx.x;
     unsigned* sb = seen + (size_t)seg_slot[sg] * seen_words;
     if (seg_pos0[sg] == 0) {

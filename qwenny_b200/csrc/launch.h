@@ -1,6 +1,12 @@
 // One launch helper for every kernel: cudaLaunchKernelEx with the programmatic-dependent-launch attribute when the
-// context asks for it. Every kernel of the library calls pdl_wait() before it touches anything an earlier kernel of
-// the stream wrote, so the chain of dependencies stays transitive whichever launches carry the attribute.
+// context asks for it. Every grid of the library calls pdl_wait() before it ends and before it touches anything that an earlier kernel
+// of the stream may still write, so a grid's end means the end of all before it, whichever launches carry the attribute.
+//
+// What a kernel reads BEFORE its wait is therefore weights, and the step's token lists, which no kernel writes. A kernel that lets
+// its dependents start at its first line says nothing about the kernels before it: several small ones in a row can all be resident
+// at once, so "written by an earlier step" is not enough for an early read. It is enough behind a kernel that waits first and lets
+// its dependents start only then (mark_seen and embed, the first of a step): whatever starts after that one starts after the
+// end of everything before it. The model runner reads the DeltaNet slots early on that ground (qb_delta_mixer_as, qb_delta_rule_as: ahead = 1).
 #pragma once
 #include "ctx.h"
 

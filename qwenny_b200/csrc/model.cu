@@ -163,7 +163,8 @@ int launch_in_proj(qb_model* m, cudaStream_t st, int layer, int& k) {
     return QB_OK;
 }
 
-// A layer's mixer: m->part (+ m->ba) -> m->mix (f16)
+// A layer's mixer: m->part (+ m->ba) -> m->mix (f16). The slots are read ahead (1): every step starts with a kernel that waits for all
+// before it before it lets the next one start (mark_seen, embed).
 int launch_mixer(qb_model* m, cudaStream_t st, int layer, int& k) {
     qb_ctx* c = m->ctx;
     const qb_layer& L = m->layers[layer].w;
@@ -173,14 +174,14 @@ int launch_mixer(qb_model* m, cudaStream_t st, int layer, int& k) {
         const int ba_splits = H / m->ba_kper;
         if (m->fork) QB_CUDA(cudaStreamWaitEvent(st, m->ev[2 * layer + 1], 0));  // the 16-bit in-projection joins
         if (m->fused && n <= CR - CONV_K + 1) {
-            QB_TRY(qb_delta_mixer(c, s, m->part, 1, n, m->ba, ba_splits, L.conv_w, L.a_log, L.dt_bias, L.norm_w, L.mem,
+            QB_TRY(qb_delta_mixer_as(c, s, m->part, 1, n, m->ba, ba_splits, L.conv_w, L.a_log, L.dt_bias, L.norm_w, L.mem,
                                   L.sst, L.meta, nullptr, m->mix, m->seg_start, m->seg_len, m->seg_slot, m->seg_pos0,
-                                  m->segs)); k++;
+                                  m->segs, 1)); k++;
         } else {
             QB_TRY(qb_delta_conv(c, s, m->part, 1, n, m->ba, ba_splits, L.conv_w, L.a_log, L.dt_bias, L.mem, L.sst,
                                  m->cv, m->tok_slot, m->tok_pos)); k++;
-            QB_TRY(qb_delta_rule(c, s, m->part, 1, n, m->cv, L.mem, L.sst, L.meta, m->o, m->seg_start, m->seg_len,
-                                 m->seg_slot, m->seg_pos0, m->segs)); k++;
+            QB_TRY(qb_delta_rule_as(c, s, m->part, 1, n, m->cv, L.mem, L.sst, L.meta, m->o, m->seg_start, m->seg_len,
+                                    m->seg_slot, m->seg_pos0, m->segs, 1)); k++;
             QB_TRY(qb_delta_norm(c, s, m->part, 1, n, L.norm_w, m->o, m->mix, L.meta, m->seg_len, m->seg_slot,
                                  m->seg_pos0, m->segs)); k++;
         }
