@@ -79,14 +79,12 @@ int qb_attn_prefill_as(qb_ctx* ctx, void* stream, const float* q, const void* kc
                        const int* ptile, const int* tok_slot, const int* tok_pos, int cap, int ntile, int max_keys, float* part_ml,
                        float* part_acc, float* out, void* mix_f16, int as);
 int qb_attn_prefill_launches(const qb_ctx* ctx, int ntile, int max_keys, int as);
-// qb_delta_mixer and qb_delta_rule for a caller that vouches (ahead = 1) for the slots: between this call and the last kernel that wrote
+// qb_delta_mixer for a caller that vouches (ahead = 1) for the slots: between this call and the last kernel that wrote
 // them lies one whose blocks all wait for the kernels before it before they let the next one start. The slots' metadata, state
-// and bank are then read ahead of the kernel before; the public entry points (ahead = 0) read them behind it.
+// and bank are then read ahead of the kernel before; the public entry point (ahead = 0) reads them behind it.
 int qb_delta_mixer_as(qb_ctx* ctx, void* stream, const float* p, int splits, int n, const float* ba, int ba_splits, const float* cw,
                       const float* a_log, const float* dt_bias, const float* nw, float* mem, long long sst, int* meta, float* out, void* y,
                       const int* seg_start, const int* seg_len, const int* seg_slot, const int* seg_pos0, int segs, int ahead);
-int qb_delta_rule_as(qb_ctx* ctx, void* stream, const float* p, int splits, int n, const float* cv, float* mem, long long sst, const int* meta,
-                     float* out, const int* seg_start, const int* seg_len, const int* seg_slot, const int* seg_pos0, int segs, int ahead);
 // the prompt-sized W4A16 product on tcgen05 (w4a16_gemm_tc.cu); reached through qb_marlin_gemm for more than 64 rows and
 // qb_marlin_gemm_z (zp: S carries the offsets' table after the scales) for more than 16
 int qb_gemm_tc_launch(qb_ctx* ctx, cudaStream_t st, const void* X, const void* B, void* Y, const void* S, int m, int n,

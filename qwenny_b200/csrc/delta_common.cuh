@@ -35,6 +35,7 @@ __device__ __forceinline__ Plan make_plan(const int* meta, int slot, int p0, int
 // block of THREADS. The metadata read here only says which buffer; a stale value costs the hint.
 template <int COLS, int THREADS>
 __device__ __forceinline__ void hint_state(const int* meta, int slot, int p0, const float* sm0, int row) {
+    if (p0 == 0) return;
     const int end = __ldcg(meta + slot * META), eb = __ldcg(meta + slot * META + 2);
     const float* s = sm0 + (size_t)((p0 == end ? eb : 1 - eb) & 1) * SLOT_STATE + (size_t)row * LKD;
     for (int x = threadIdx.x; x < COLS * LKD / 32; x += THREADS) asm volatile("prefetch.global.L2 [%0];\n" ::"l"(s + 32 * x));

@@ -543,7 +543,7 @@ __device__ __forceinline__ uint64_t mn_desc(uint32_t addr, uint32_t stride) {
 template <bool CHUNKS>
 __global__ void __launch_bounds__(CHUNKS ? SC_THREADS + 64 : SC_THREADS, CHUNKS ? 1 : 2)
 delta_scan_kernel(const float* p, int splits, int n, const float* cv, uint8_t* tp, float* mem, long long sst, const int* meta, float* out,
-                  const int* seg_start, const int* seg_len, const int* seg_slot, const int* seg_pos0, int segs, int all, int* err, int ahead) {
+                  const int* seg_start, const int* seg_len, const int* seg_slot, const int* seg_pos0, int segs, int all, int* err) {
     extern __shared__ __align__(16) uint8_t scan_raw[];
     ScanSmem& M = *(ScanSmem*)(((uintptr_t)scan_raw + 1023) & ~(uintptr_t)1023);
     const int vs = blockIdx.x, h = blockIdx.y, sg = CHUNKS && segs > 1 ? long_segment(seg_len, segs, blockIdx.z) : blockIdx.z, kh = h / (LV_HEADS / LK_HEADS);
@@ -660,16 +660,14 @@ delta_scan_kernel(const float* p, int splits, int n, const float* cv, uint8_t* t
         const int lc = tid >> 3, sub = tid & 7, col = vs * SC_COLS + lc;  // token form: 8 lanes per value column
         int slot = seg_slot[sg], p0 = seg_pos0[sg];
         float* sm0 = mem + slot * sst;
-        if (!ahead) {
-            hint_state<SC_COLS, SC_THREADS>(meta, slot, p0, sm0, h * LVD + vs * SC_COLS);
-            pdl_wait();
-        }
+        if (!CHUNKS) hint_state<SC_COLS, SC_THREADS>(meta, slot, p0, sm0, h * LVD + vs * SC_COLS);  // (beside the chunks its registers spill)
+        pdl_wait();
         Plan pl = make_plan(meta, slot, p0, len);
         auto sbuf = [&](int b) { return sm0 + (size_t)b * SLOT_STATE + ((size_t)h * LVD + col) * LKD; };
         auto entry = [&](int b, int pos) { return sm0 + 2 * SLOT_STATE + (size_t)b * SLOT_BANK + (size_t)(pos % KEEP) * REP; };
         auto sync = [] { named_bar_sync(1, SC_THREADS); };
         constexpr int RPT = LKD / 8;
-        // ---- the state, and the replay of accepted tokens from the bank: nothing of it is written by this step's kernels before
+        // ---- the state, and the replay of accepted tokens from the bank
         float S[RPT];
         if (pl.zero) {
 #pragma unroll
@@ -687,7 +685,6 @@ delta_scan_kernel(const float* p, int splits, int n, const float* cv, uint8_t* t
 #pragma unroll
             for (int j = 0; j < RPT; j++) S[j] = ex * S[j] + k[j] * delta;
         }
-        pdl_wait();
 
         if (nc > 0) {
             // ============================================================ chunks: thread = key, 16 columns
@@ -908,13 +905,6 @@ extern "C" {
 int qb_delta_rule(qb_ctx* ctx, void* stream, const float* p, int splits, int n, const float* cv, float* mem,
                   long long sst, const int* meta, float* out, const int* seg_start, const int* seg_len,
                   const int* seg_slot, const int* seg_pos0, int segs) {
-    return qb_delta_rule_as(ctx, stream, p, splits, n, cv, mem, sst, meta, out, seg_start, seg_len, seg_slot, seg_pos0, segs, 0);
-}
-
-}  // extern "C"
-
-int qb_delta_rule_as(qb_ctx* ctx, void* stream, const float* p, int splits, int n, const float* cv, float* mem, long long sst, const int* meta,
-                     float* out, const int* seg_start, const int* seg_len, const int* seg_slot, const int* seg_pos0, int segs, int ahead) {
     if (!ctx || !p || !cv || !mem || !meta || !out || !seg_start || !seg_len || !seg_slot || !seg_pos0 || n <= 0 ||
         segs <= 0 || splits < 1)
         return QB_ERR_ARG;
@@ -930,9 +920,11 @@ int qb_delta_rule_as(qb_ctx* ctx, void* stream, const float* p, int splits, int 
     // the segments in the token form, unless the step's only one may run in chunks
     if (l0 == 0 || segs > 1) {
         int rc = launch(ctx, delta_scan_kernel<false>, dim3(LVD / SC_COLS, LV_HEADS, segs), dim3(SC_THREADS), sizeof(TokenSmem), st, p, splits, n, cv,
-                        (uint8_t*)nullptr, mem, sst, meta, out, seg_start, seg_len, seg_slot, seg_pos0, segs, l0 == 0, ctx->err, ahead);
+                        (uint8_t*)nullptr, mem, sst, meta, out, seg_start, seg_len, seg_slot, seg_pos0, segs, l0 == 0, ctx->err);
         if (rc || l0 == 0) return rc;
     }
     return launch(ctx, delta_scan_kernel<true>, dim3(LVD / SC_COLS, LV_HEADS, most), dim3(SC_THREADS + 64), SCAN_SMEM, st, p, splits, n, cv,
-                  (uint8_t*)ctx->delta_tp, mem, sst, meta, out, seg_start, seg_len, seg_slot, seg_pos0, segs, 0, ctx->err, ahead);
+                  (uint8_t*)ctx->delta_tp, mem, sst, meta, out, seg_start, seg_len, seg_slot, seg_pos0, segs, 0, ctx->err);
 }
+
+}  // extern "C"
