@@ -467,8 +467,9 @@ attn_dec4_kernel(const float* q, const uint8_t* kc, const uint8_t* vc, const flo
     __syncthreads();
     pdl_launch_dependents();
     // The step's token lists are uploaded before its first kernel, so they are read ahead of the kernel before (this
-    // step's attn_prep), and so are the stages of keys and values that earlier steps wrote: whatever ends `old_margin`
-    // positions or more before the segment's last key (0: nothing is read ahead).
+    // step's attn_prep), and so, where the caller vouches for them, are the stages of keys and values that earlier steps wrote: whatever
+    // ends `old_margin` positions or more before the segment's last key (0: nothing is read ahead, the first stages are only
+    // asked into L2).
     const int first = dseg[2 * seg], nt = dseg[2 * seg + 1];
     const int tlast = dtok[first + nt - 1], keys = tok_pos[tlast] + 1;
     const int chunk = dec_chunk(keys, dsplits), ns = (keys + chunk - 1) / chunk;
@@ -484,6 +485,11 @@ attn_dec4_kernel(const float* q, const uint8_t* kc, const uint8_t* vc, const flo
         const float* ksh = ks + scale_head(slot, g, cap);
         const float* vsh = vs + scale_head(slot, g, cap);
         bool waited = false;
+        if (old_margin <= 0 && lane < min(nstg, NSTG)) {
+            const size_t at = (size_t)(kbeg + lane * SK) * HD;
+            bulk_prefetch(kh + at, SK * HD);
+            bulk_prefetch(vh + at, SK * HD);
+        }
         for (int j = 0; j < nstg; j++) {
             const int sl = j % NSTG;
             if (!waited && (old_margin <= 0 || kbeg + (j + 1) * SK > keys - old_margin)) {
@@ -900,6 +906,15 @@ int qb_attn_decode(qb_ctx* ctx, void* stream, const float* q, const void* kc, co
                    const float* vs, const int* dseg, const int* dtok, const int* dkeys, const int* tok_slot,
                    const int* tok_pos, int cap, int ndseg, int ndec, int dmax, int max_keys, float* part_ml,
                    float* part_acc, float* out, void* mix_f16) {
+    return qb_attn_decode_as(ctx, stream, q, kc, vc, ks, vs, dseg, dtok, dkeys, tok_slot, tok_pos, cap, ndseg, ndec, dmax, max_keys,
+                             part_ml, part_acc, out, mix_f16, 0);
+}
+
+}  // extern "C"
+
+int qb_attn_decode_as(qb_ctx* ctx, void* stream, const float* q, const void* kc, const void* vc, const float* ks, const float* vs,
+                      const int* dseg, const int* dtok, const int* dkeys, const int* tok_slot, const int* tok_pos, int cap, int ndseg,
+                      int ndec, int dmax, int max_keys, float* part_ml, float* part_acc, float* out, void* mix_f16, int ahead) {
     if (!ctx || !q || !kc || !vc || !ks || !vs || !dseg || !dtok || !dkeys || !tok_slot || !tok_pos || !part_ml ||
         !part_acc || !out || ndseg <= 0 || ndec <= 0 || dmax <= 0 || dmax > 8 || max_keys <= 0 || cap % 64 ||
         max_keys > cap)
@@ -908,9 +923,9 @@ int qb_attn_decode(qb_ctx* ctx, void* stream, const float* q, const void* kc, co
     const int z = dec_splits_upto(max_keys, dsplits), rt = (dmax * GROUP + 15) / 16;
     cudaStream_t st = (cudaStream_t)stream;
     dim3 grid(ndseg, NKV, z);
-    // a step has at most 64 decode tokens: whatever lies 64 positions or more before a segment's last key is from
-    // earlier steps
-    const int old_margin = ndec <= 64 ? 64 : 0;
+    // (the model's steps have at most 64 decode tokens: whatever lies 64 positions or more before a segment's last key is from
+    // earlier steps)
+    const int old_margin = ahead && ndec <= 64 ? 64 : 0;
     int rc;
 #define QB_DEC(RT, NQ)                                                                                          \
     {                                                                                                           \
@@ -927,6 +942,8 @@ int qb_attn_decode(qb_ctx* ctx, void* stream, const float* q, const void* kc, co
     return launch(ctx, attn_combine_kernel, dim3(ndec, NH), dim3(HD), 0, st, (const float*)part_ml,
                   (const float*)part_acc, dtok, dkeys, z, dsplits, out, (__half*)mix_f16);
 }
+
+extern "C" {
 
 int qb_attn_tile_splits(int ntile, int max_keys) { return ntile > 0 && max_keys > 0 ? tile_splits(ntile, max_keys) : 0; }
 

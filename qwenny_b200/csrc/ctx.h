@@ -85,6 +85,10 @@ int qb_attn_prefill_launches(const qb_ctx* ctx, int ntile, int max_keys, int as)
 int qb_delta_mixer_as(qb_ctx* ctx, void* stream, const float* p, int splits, int n, const float* ba, int ba_splits, const float* cw,
                       const float* a_log, const float* dt_bias, const float* nw, float* mem, long long sst, int* meta, float* out, void* y,
                       const int* seg_start, const int* seg_len, const int* seg_slot, const int* seg_pos0, int segs, int ahead);
+// qb_attn_decode for a caller that vouches in the same way (ahead = 1) for the cache entries of earlier steps
+int qb_attn_decode_as(qb_ctx* ctx, void* stream, const float* q, const void* kc, const void* vc, const float* ks, const float* vs,
+                      const int* dseg, const int* dtok, const int* dkeys, const int* tok_slot, const int* tok_pos, int cap, int ndseg,
+                      int ndec, int dmax, int max_keys, float* part_ml, float* part_acc, float* out, void* mix_f16, int ahead);
 // the prompt-sized W4A16 product on tcgen05 (w4a16_gemm_tc.cu); reached through qb_marlin_gemm for more than 64 rows and
 // qb_marlin_gemm_z (zp: S carries the offsets' table after the scales) for more than 16
 int qb_gemm_tc_launch(qb_ctx* ctx, cudaStream_t st, const void* X, const void* B, void* Y, const void* S, int m, int n,

@@ -6,8 +6,8 @@
 // its dependents start at its first line says nothing about the kernels before it: several small ones in a row can all be resident
 // at once, so "written by an earlier step" is not enough for an early read. It is enough behind a kernel that waits first and lets
 // its dependents start only then (mark_seen and embed, the first of a step): whatever starts after that one starts after the
-// end of everything before it. The model runner reads the slots of its one-launch mixers early on that ground (qb_delta_mixer_as:
-// ahead = 1).
+// end of everything before it. The model runner reads the slots of its one-launch mixers and the older cache entries early on that
+// ground (qb_delta_mixer_as, qb_attn_decode_as: ahead = 1).
 #pragma once
 #include "ctx.h"
 

@@ -163,7 +163,7 @@ int launch_in_proj(qb_model* m, cudaStream_t st, int layer, int& k) {
     return QB_OK;
 }
 
-// A layer's mixer: m->part (+ m->ba) -> m->mix (f16). The slots are read ahead (1): every step starts with a kernel that waits for all
+// A layer's mixer: m->part (+ m->ba) -> m->mix (f16). The slots and the caches of earlier steps are read ahead (1): every step starts with a kernel that waits for all
 // before it before it lets the next one start (mark_seen, embed).
 int launch_mixer(qb_model* m, cudaStream_t st, int layer, int& k) {
     qb_ctx* c = m->ctx;
@@ -190,8 +190,8 @@ int launch_mixer(qb_model* m, cudaStream_t st, int layer, int& k) {
         QB_TRY(qb_attn_prep(c, s, m->part, 1, n, L.q_norm, L.k_norm, L.inv_freq, qscale, m->q, m->o, L.kc, L.vc, L.ks,
                             L.vs, m->tok_slot, m->tok_pos, L.cap)); k++;
         if (m->ndec > 0) {
-            QB_TRY(qb_attn_decode(c, s, m->q, L.kc, L.vc, L.ks, L.vs, m->dseg, m->dtok, m->dkeys, m->tok_slot, m->tok_pos,
-                                  L.cap, m->ndseg, m->ndec, m->dmax, m->dec_max_pos + 1, m->ml, m->acc, m->o, m->mix));
+            QB_TRY(qb_attn_decode_as(c, s, m->q, L.kc, L.vc, L.ks, L.vs, m->dseg, m->dtok, m->dkeys, m->tok_slot, m->tok_pos,
+                                  L.cap, m->ndseg, m->ndec, m->dmax, m->dec_max_pos + 1, m->ml, m->acc, m->o, m->mix, 1));
             k += 2;
         }
         if (m->ntile > 0) {

@@ -132,8 +132,8 @@ def test_attn_decode_row_invariance_and_two_slots(ctx):
 
 
 def test_attn_decode_more_than_64_decode_tokens(ctx):
-    """Up to 64 decode tokens in a call, the kernel requests the cache entries that lie 64 positions or more before a
-    segment's last key ahead of the kernel enqueued before it; with more it waits first. 13 slots x 5 tokens = 65
+    """A call of the entry point waits for the kernel before it ahead of the first cache entry (only the model runner, with up to 64
+    decode tokens in a step, asks for entries of earlier steps before that). 13 slots x 5 tokens = 65
     tokens (the host's planner stops at 64; the C entry point does not), with programmatic dependent launch on, against
     the CPU oracle on three of the rows, and bit for bit against the same rows run as 13 calls of 5 tokens."""
     g = synth.gen(88)
@@ -349,3 +349,59 @@ def test_attn_prefill_forms_over_several_sequences(ctx, lens, pos0, cap, pairs):
                          st["tok_pos"][rows], cap)
     for out, m16 in forms:
         assert close(out.cpu().numpy()[rows], want).all() and torch.equal(m16, out.half())
+
+
+@pytest.mark.parametrize("prompt,rows,steps", [(96, 1, 6), (200, 5, 4), (70, 8, 5)])
+def test_calls_back_to_back_on_one_cache(ctx, prompt, rows, steps):
+    """A prompt's cache entries and the decode steps that read them right behind it (one graph, programmatic dependent launch on): the
+    bits of the same calls one at a time without early launches."""
+    g = synth.gen(140 + prompt)
+    cap, n = 512, prompt + rows * steps
+    part = torch.randn(1, n, R.ATTN_IN, generator=g).cuda()
+    qn, kn = (1 + torch.randn(R.HD, generator=g) * 0.02).cuda(), (1 + torch.randn(R.HD, generator=g) * 0.02).cuda()
+    inv = torch.from_numpy(R.rope_inv_freq()).cuda()
+    cuts = [(0, prompt)] + [(prompt + i * rows, prompt + (i + 1) * rows) for i in range(steps)]
+    sts = [R.build_step([(0, 0, p) for p in range(a, e)], [0]) for a, e in cuts]
+    last = R.build_step([(0, 0, prompt - 1)], [0])  # the prompt's last token alone, behind the prompt's cache entries
+    dvs, dlast = [ref_cuda.upload_step(s) for s in sts], ref_cuda.upload_step(last)
+    parts = [part[:, a:e].contiguous() for a, e in cuts]
+    ml, acc = torch.zeros(4096 * R.NH * 2, device="cuda"), torch.zeros(4096 * R.NH * R.HD, device="cuda")
+
+    def run(graph):
+        kc, vc = (torch.zeros(R.NKV * cap * R.HD, dtype=torch.uint8, device="cuda") for _ in "kv")
+        ks, vs = (torch.zeros(R.NKV * cap, device="cuda") for _ in "kv")
+        qs = [torch.zeros(e - a, R.NH, R.HD, device="cuda") for a, e in cuts]
+        os = [torch.zeros(e - a, R.MIX, device="cuda") for a, e in cuts]
+        o1 = torch.ones(1, R.MIX, device="cuda")
+        q1 = torch.randn(1, R.NH, R.HD, generator=synth.gen(7)).cuda() * QSCALE
+
+        def all_steps():
+            for i, (a, e) in enumerate(cuts):
+                ctx.attn_prep(parts[i], 1, e - a, qn, kn, inv, QSCALE, qs[i], os[i], kc, vc, ks, vs, dvs[i]["tok_slot"], dvs[i]["tok_pos"], cap)
+                if i == 0:
+                    ctx.attn_decode(q1, kc, vc, ks, vs, dlast, last, cap, ml, acc, o1)
+                    ctx.attn_prefill(qs[i], kc, vc, ks, vs, dvs[i], sts[i], cap, ml, acc, os[i])
+                else:
+                    ctx.attn_decode(qs[i], kc, vc, ks, vs, dvs[i], sts[i], cap, ml, acc, os[i])
+        if graph:
+            cg = torch.cuda.CUDAGraph()
+            torch.cuda.synchronize()
+            with torch.cuda.graph(cg):
+                all_steps()
+            for t in (kc, vc, ks, vs):
+                t.zero_()
+            o1.fill_(1)
+            cg.replay()
+        else:
+            all_steps()
+        torch.cuda.synchronize()
+        return os + [o1, kc, vc, ks, vs]
+
+    want = run(False)
+    ctx.set_pdl(True)
+    try:
+        for _ in range(3):
+            assert all(torch.equal(a, b) for a, b in zip(run(True), want))
+    finally:
+        ctx.set_pdl(False)
+    assert ctx.device_error() == 0
