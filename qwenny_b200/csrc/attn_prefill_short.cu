@@ -55,8 +55,7 @@ attn_prefill_short_kernel(const float* q, const uint8_t* kc, const uint8_t* vc, 
                        const int* ptile, int ntile, const int* tok_slot, const int* tok_pos, int cap, float* out,
                        __half* mix, int* err, int* on_pairs) {
     extern __shared__ uint8_t smem_raw[];
-    if (CHOOSE) {
-        pdl_launch_dependents();
+    if (CHOOSE) {  // where the other form does the step, return before anything is taken
         pdl_wait();
         if (*(const volatile int*)on_pairs) return;
     }
@@ -96,10 +95,10 @@ attn_prefill_short_kernel(const float* q, const uint8_t* kc, const uint8_t* vc, 
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
-    if (!CHOOSE) {
-        pdl_launch_dependents();
-        pdl_wait();
-    }
+    // (not before the tensor memory is taken: tcgen05.alloc waits without a limit, and a dependent's block that came first would wait
+    // for this grid)
+    pdl_launch_dependents();
+    pdl_wait();
 
     int jbase = 0;  // stages of earlier passes: ring slots and barrier phases run on
     Waiter w_mma{err, 11}, w_sm{err, 12}, w_cv{err, 13};
