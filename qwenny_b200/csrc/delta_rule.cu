@@ -522,6 +522,8 @@ struct ScanSmem {
     uint32_t tmem;
 };
 constexpr int SCAN_SMEM = sizeof(ScanSmem) + 1024;
+constexpr int APART_SMEM = 116 * 1024;  // of a block that shares its SM with no other of its kind
+static_assert(2 * (APART_SMEM + 1024) > 228 * 1024 && APART_SMEM >= sizeof(TokenSmem), "an SM holds 228 KB, 1 KB of them per block its own");
 static_assert(SCAN_SMEM <= 227 * 1024, "shared memory of a block");
 
 // instruction descriptor of tcgen05.mma kind::f16, M = 128, N = n, A / B in MN-major order where asked
@@ -535,10 +537,13 @@ __device__ __forceinline__ uint64_t mn_desc(uint32_t addr, uint32_t stride) {
 }
 
 // CHUNKS: segment blockIdx.z of those that run in chunks; 16 warps carry the state, one copies, one issues the products. Otherwise
-// the segments without chunks (all of them where no chunks were prepared, `all`), two blocks per SM: 12 segments of 8 tokens
-// in the kernel for chunks, one block per SM, took the mixer 109 us.
-template <bool CHUNKS>
-__global__ void __launch_bounds__(CHUNKS ? SC_THREADS + 64 : SC_THREADS, CHUNKS ? 1 : 2)
+// the segments without chunks (all of them where no chunks were prepared, `all`), PER_SM blocks per SM: two, or one where the SMs hold
+// every block so, which then asks for more than half of an SM's shared memory. A token's loop is bound by issue, and early-launched
+// blocks of one segment (96 on 148 SMs) pair up on SMs that the kernels before have left while others idle. The mixer, two / one:
+// one segment of 30 tokens 47.6 / 36.4 us, 46 62 / 46.5, 64 79 / 59, 79 90 / 66.6; 5 segments of 8 39.4 / 44, 12 of 8 74 / 90, 12 of 40
+// 219 / 261.
+template <bool CHUNKS, int PER_SM>
+__global__ void __launch_bounds__(CHUNKS ? SC_THREADS + 64 : SC_THREADS, PER_SM)
 delta_scan_kernel(const float* p, int splits, int n, const float* cv, uint8_t* tp, float* mem, long long sst, const int* meta, float* out,
                   const int* seg_start, const int* seg_len, const int* seg_slot, const int* seg_pos0, int segs, int all, int* err) {
     extern __shared__ __align__(16) uint8_t scan_raw[];
@@ -916,11 +921,13 @@ int qb_delta_rule(qb_ctx* ctx, void* stream, const float* p, int splits, int n, 
     }
     // the segments in the token form, unless the step's only one may run in chunks
     if (l0 == 0 || segs > 1) {
-        int rc = launch(ctx, delta_scan_kernel<false>, dim3(LVD / SC_COLS, LV_HEADS, segs), dim3(SC_THREADS), sizeof(TokenSmem), st, p, splits, n, cv,
-                        (uint8_t*)nullptr, mem, sst, meta, out, seg_start, seg_len, seg_slot, seg_pos0, segs, l0 == 0, ctx->err);
+        const bool apart = (LVD / SC_COLS) * LV_HEADS * segs <= ctx->sms;
+        int rc = launch(ctx, apart ? delta_scan_kernel<false, 1> : delta_scan_kernel<false, 2>, dim3(LVD / SC_COLS, LV_HEADS, segs), dim3(SC_THREADS),
+                        apart ? APART_SMEM : sizeof(TokenSmem), st, p, splits, n, cv, (uint8_t*)nullptr, mem, sst, meta, out, seg_start, seg_len,
+                        seg_slot, seg_pos0, segs, l0 == 0, ctx->err);
         if (rc || l0 == 0) return rc;
     }
-    return launch(ctx, delta_scan_kernel<true>, dim3(LVD / SC_COLS, LV_HEADS, most), dim3(SC_THREADS + 64), SCAN_SMEM, st, p, splits, n, cv,
+    return launch(ctx, delta_scan_kernel<true, 1>, dim3(LVD / SC_COLS, LV_HEADS, most), dim3(SC_THREADS + 64), SCAN_SMEM, st, p, splits, n, cv,
                   (uint8_t*)ctx->delta_tp, mem, sst, meta, out, seg_start, seg_len, seg_slot, seg_pos0, segs, 0, ctx->err);
 }
 
