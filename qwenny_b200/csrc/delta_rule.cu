@@ -11,11 +11,13 @@
 //                           in registers from chunk to chunk: D = U - W S, O = gam Q S + P D,
 //                           S' = gam_C S + K^T diag(exp(G_C - G_j)) D: three products on tcgen05, two of them in sequence.
 //
-// Precision. The tensor cores take every f32 operand x as TWO f16 values of s x, hi = the upper 11 bits of s x and lo = f16(s x - hi): 22 bits,
-// with s a power of two that brings the largest finite entry of the tile into [2^14, 2^15), so that what is lost at the
-// small end lies 2^-39 below it. a . b ~ hi_a hi_b + hi_a lo_b + lo_a hi_b, summed in f32 (3 x TF32 keeps 21 bits for twice
-// the instructions). Q, P and the D that P meets only feed the step's outputs: one f16 (11 bits, as TF32 has). The scales of the
-// state and of D belong to 16 columns each and leave infinities and NaN out, so that those stay in their column.
+// Precision. The tensor cores take every f32 operand x as TWO f16 values of s x, hi = f16(s x) to nearest and lo = f16(s x - hi): 23 bits,
+// with s a power of two that brings the largest finite entry of the tile (K, V, W: 64 x 128; the state and D: 16 columns) into
+// [2^14, 2^15). f16 ends at 2^-24: what is lost lies 2^-39 below that entry, so values down to 2^-16 of it keep 22 bits, values
+// below that fewer (3 x TF32 kept 21 bits of each for twice the instructions). a . b ~ hi_a hi_b + hi_a lo_b + lo_a hi_b,
+// summed in f32. Q, P and the D that P meets only feed the step's outputs: one f16 to nearest (11 bits, as TF32 has; P and D down to
+// 2^-28 of their tile's largest, D's a bound of it). The scales of the state and of D leave infinities and NaN out, so that those
+// stay in their column.
 #include "attn_tc.cuh"
 #include "delta_common.cuh"
 #include "launch.h"
@@ -82,9 +84,10 @@ __device__ __forceinline__ float scale_of(float m) {
 }
 __device__ __forceinline__ float inverse_of(float s) { return __uint_as_float((254u << 23) - __float_as_uint(s)); }
 __device__ __forceinline__ void split2(float a, float b, uint32_t& hi, uint32_t& lo) {
-    const float ah = __uint_as_float(__float_as_uint(a) & 0xffffe000u), bh = __uint_as_float(__float_as_uint(b) & 0xffffe000u);
-    hi = pack_half2(ah, bh);
-    lo = pack_half2(a - ah, b - bh);
+    const __half2 h = __floats2half2_rn(a, b);
+    const float2 f = __half22float2(h);
+    hi = *(const uint32_t*)&h;
+    lo = pack_half2(a - f.x, b - f.y);
 }
 __device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(smem_u32(dst)), "l"(src),
