@@ -120,7 +120,7 @@ struct PrepSmem {
     uint8_t p[TILE];
     float t[CH][TST];         // A, inverted in place
     float s[32][36];          // a merge's intermediate product
-    float g[CH], b[CH], bg[CH];  // G in base 2, b, b gam
+    float g[CH], b[CH], bg[CH];  // G - G_C in base 2, b, b gam
     float rows[4][CH];        // row sums of |W| by quarters of the columns
     uint32_t kmax[8], qmax[8], vmax[8], pmax[4], wmax[8], tmax[8], umax[2][GROUPS];
     float bmax, bgmax;        // largest b, largest b gam
@@ -187,15 +187,19 @@ delta_chunk_prep_kernel(const float* cv, uint8_t* tp, const int* seg_start, cons
             const float b0 = in0 ? e0[LV_HEADS] : 0.f, b1 = in1 ? e0[CVW + LV_HEADS] : 0.f;
             l0 = l0 < -160.f ? -160.f : l0;
             l1 = l1 < -160.f ? -160.f : l1;
-            float run = l0 + l1;  // inclusive scan of the pair sums over the lanes
+            // sums of the log decays from the chunk's start (for gam) and to its end. What else is taken, the difference of two tokens' G,
+            // comes from the sums to the end: those are small, and exact, at the tokens that the state behind the chunk still
+            // sees (taken from the start's, that state was 2.1e-6 off)
+            float run = l0 + l1, back = run;
 #pragma unroll
             for (int o = 1; o < 32; o <<= 1) {
-                const float up = __shfl_up_sync(0xffffffffu, run, o);
+                const float up = __shfl_up_sync(0xffffffffu, run, o), down = __shfl_down_sync(0xffffffffu, back, o);
                 if (lane >= o) run += up;
+                if (lane + o < 32) back += down;
             }
-            const float end = __shfl_sync(0xffffffffu, run, 31), g0 = run - l1, m0 = exp2f(g0), m1 = exp2f(run);
-            const float d0 = exp2f(end - g0), d1 = exp2f(end - run);
-            *(float2*)&M.g[2 * lane] = make_float2(g0, run);
+            back = __shfl_down_sync(0xffffffffu, back, 1);
+            const float to1 = lane < 31 ? back : 0.f, to0 = to1 + l1, m0 = exp2f(run - l1), m1 = exp2f(run), d0 = exp2f(to0), d1 = exp2f(to1);
+            *(float2*)&M.g[2 * lane] = make_float2(-to0, -to1);
             *(float2*)&M.b[2 * lane] = make_float2(b0, b1);
             *(float2*)&M.bg[2 * lane] = make_float2(b0 * m0, b1 * m1);
             const float bm = warp_max(fmaxf(fabsf(b0), fabsf(b1))), gm = warp_max(fmaxf(fabsf(b0 * m0), fabsf(b1 * m1)));
