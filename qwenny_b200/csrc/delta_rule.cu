@@ -12,7 +12,7 @@
 //                           S' = gam_C S + K^T diag(exp(G_C - G_j)) D: three products on tcgen05, two of them in sequence.
 //
 // Precision. The tensor cores take every f32 operand x as TWO f16 values of s x, hi = f16(s x) to nearest and lo = f16(s x - hi): 23 bits,
-// with s a power of two that brings the largest finite entry of the tile (K, V, W: 64 x 128; the state and D: 16 columns) into
+// with s a power of two that brings the largest finite entry of the tile (K, W: 64 x 128; V, the state and D: 16 columns) into
 // [2^14, 2^15). f16 ends at 2^-24: what is lost lies 2^-39 below that entry, so values down to 2^-16 of it keep 22 bits, values
 // below that fewer (3 x TF32 kept 21 bits of each for twice the instructions). a . b ~ hi_a hi_b + hi_a lo_b + lo_a hi_b,
 // summed in f32. Q, P and the D that P meets only feed the step's outputs: one f16 to nearest (11 bits, as TF32 has; P and D down to
@@ -122,7 +122,7 @@ struct PrepSmem {
     float s[32][36];          // a merge's intermediate product
     float g[CH], b[CH], bg[CH];  // G - G_C in base 2, b, b gam
     float rows[4][CH];        // row sums of |W| by quarters of the columns
-    uint32_t kmax[8], qmax[8], vmax[8], pmax[4], wmax[8], tmax[8], umax[2][GROUPS];
+    uint32_t kmax[8], qmax[8], vmax[8][GROUPS], pmax[4], wmax[8], tmax[8], umax[2][GROUPS];
     float bmax, bgmax;        // largest b, largest b gam
 };
 
@@ -162,6 +162,19 @@ delta_chunk_prep_kernel(const float* cv, uint8_t* tp, const int* seg_start, cons
 #pragma unroll
         for (int i = 0; i < 8; i++) m = finite_max(finite_max(finite_max(finite_max(m, v[i].x), v[i].y), v[i].z), v[i].w);
         return warp_most(m);
+    };
+    auto group_most = [&](const float4* v) {  // of the lane's group of 16 columns: lanes 4 j .. 4 j + 3
+        uint32_t m = 0;
+#pragma unroll
+        for (int i = 0; i < 8; i++) m = finite_max(finite_max(finite_max(finite_max(m, v[i].x), v[i].y), v[i].z), v[i].w);
+        m = max(m, __shfl_xor_sync(0xffffffffu, m, 1));
+        return max(m, __shfl_xor_sync(0xffffffffu, m, 2));
+    };
+    auto vscale = [&](int group) {
+        uint32_t m = M.vmax[0][group];
+#pragma unroll
+        for (int i = 1; i < 8; i++) m = max(m, M.vmax[i][group]);
+        return scale_of(finite_value(m));
     };
     auto tile_store = [&](uint8_t (*to)[TILE], const float4* v, float s) {  // hi into tiles 0 and 1, lo into 2 and 3
 #pragma unroll
@@ -282,18 +295,15 @@ delta_chunk_prep_kernel(const float* cv, uint8_t* tp, const int* seg_start, cons
                 }
             }
         }
-        const uint32_t vm = tile_most(v);
+        const uint32_t vm = group_most(v);
         pm = warp_most(pm);
-        if (lane == 0) {
-            M.vmax[warp] = vm;
-            if (warp >= 4) M.pmax[m] = pm;
-        }
+        if ((lane & 3) == 0) M.vmax[warp][lane >> 2] = vm;
+        if (lane == 0 && warp >= 4) M.pmax[m] = pm;
     }
     if (first && tid == 0) asm volatile("cp.async.bulk.wait_group.read 0;\n" ::: "memory");  // V goes where Q was
     __syncthreads();
     // ---- T = (I + A)^-1 in place: the four 16 x 16 diagonal blocks by forward substitution, a thread per column (warps 0, 1);
     // then blocks merge pairwise, 16 -> 32 -> 64: T21 = -T22 (A21 T11)
-    const float vscale = scale_of(most8(M.vmax));
     uint32_t tm = 0;
     if (warp < 2) {
         const int b0 = (tid >> 4) * 16, col = tid & 15;
@@ -328,7 +338,7 @@ delta_chunk_prep_kernel(const float* cv, uint8_t* tp, const int* seg_start, cons
                 }
         if (tid == 128) ((Gates*)(vh + GATES_AT))->pinv = inverse_of(ps);
     }
-    tile_store(M.x, v, vscale);
+    tile_store(M.x, v, vscale(lane >> 2));
     __syncthreads();
     {
         const int pr = tid >> 7, i = (tid >> 3) & 15, j = 2 * (tid & 7), base = 32 * pr;
@@ -381,7 +391,8 @@ delta_chunk_prep_kernel(const float* cv, uint8_t* tp, const int* seg_start, cons
 #pragma unroll 1
     for (int pass = 0; pass < 2; pass++) {
         const float* f = pass ? M.bg : M.b;
-        const float s = scale_of(tmost * (pass ? M.bgmax : M.bmax)), inv = inverse_of(s) * (pass ? kinv : inverse_of(vscale));
+        const float s = scale_of(tmost * (pass ? M.bgmax : M.bmax)), sinv = inverse_of(s);
+        const float inv[2] = {sinv * (pass ? kinv : inverse_of(vscale(2 * nq))), sinv * (pass ? kinv : inverse_of(vscale(2 * nq + 1)))};
         const uint32_t xb = smem_u32(pass ? M.k : M.x);
 #pragma unroll
         for (int e = 0; e < 32; e++) w[e >> 4][(e >> 2) & 3][e & 3] = 0.f;
@@ -418,7 +429,7 @@ delta_chunk_prep_kernel(const float* cv, uint8_t* tp, const int* seg_start, cons
             }
         }
 #pragma unroll
-        for (int e = 0; e < 32; e++) w[e >> 4][(e >> 2) & 3][e & 3] *= inv;
+        for (int e = 0; e < 32; e++) w[e >> 4][(e >> 2) & 3][e & 3] *= inv[(e >> 3) & 1];
         if (pass) break;
         uint32_t um[2] = {0u, 0u};
 #pragma unroll
