@@ -32,9 +32,10 @@ typedef struct qb_ctx qb_ctx;
 enum { QB_EPI_PLAIN = 0, QB_EPI_SILU = 1, QB_EPI_ARGMAX = 2 };
 
 /* ---- context: what Gemm::load allocates once (src/cuda/core.rs:437-464: SM count, Marlin's `red` and `locks`).
- * Allocates the scratch and tickets on `device`: 141 MB that all calls use in turn; where there is no room, 39 MB (the delta
- * rule then runs token by token), or the 32 MiB of the skinny products (17 to 64 rows then run as 16-row slabs, larger
- * products as whole tiles). Everything after creation is allocation-free. Like the
+ * Allocates the scratch and tickets on `device`: 221 MB that all calls use in turn. Where there is no room: 142 MB (the delta rule of a
+ * step that may have more than 32 chunks of 64 tokens, 2048 tokens of several sequences, then runs token by token), 55 MB (more
+ * than 12 chunks, 784 tokens of one), 41 MB (token by token throughout) or 36 MB, the skinny products' part (17 to 64 rows then
+ * run as 16-row slabs, larger products as whole tiles). Everything after creation is allocation-free. Like the
  * reference's single `red` / `locks` pair, a context serves one stream at a time: launches that share a context must
  * not overlap on the device (models that run concurrently take a context each). */
 int qb_create(int device, qb_ctx** out);

@@ -143,6 +143,7 @@ MEASURE_SIGNATURES = {
     "qb_model_fail_captures": [P, I],
     "qb_wait_probe": [P, P, C.c_uint],
     "qb_scratch_forget": [P],
+    "qb_scratch_chunks": [P, I],
     "qb_attn_tiles_on_pairs": [P, I, P, P, I],
     "qb_gemm_f16_block_tiles": [I, I, I, I, I],
 }

@@ -108,12 +108,15 @@ int qb_create(int device, qb_ctx** out) {
     const size_t zeroed = tickets_at + QB_TC_TICKETS * sizeof(int), scratch_at = 2u << 20, scratch_bytes = 32u << 20;
     static_assert((1 << 14) * sizeof(int) + 256 + QB_TC_TICKETS * sizeof(int) <= (2u << 20), "the words come before the area");
     char* b = nullptr;
-    // everything; without the delta rule's tiles; without the prompt-sized products' part as well
-    const size_t areas[3] = {std::max({scratch_bytes, qb_tc_part_bytes(sms), qb_delta_tp_bytes()}), std::max(scratch_bytes, qb_tc_part_bytes(sms)),
-                             scratch_bytes};
+    // The delta rule's chunks: those of any step (219 MB), those of 2048 tokens of one sequence (140 MB), of 784 (52 MB); no chunks (39 MB); without
+    // the prompt-sized products' part as well.
+    const int chunks[4] = {QB_DELTA_CHUNKS, 32, 12, 0};
     int got = 0;
-    for (; got < 2 && cudaMalloc(&b, scratch_at + areas[got]) != cudaSuccess; got++) (void)cudaGetLastError();
-    if (got == 2) QB_CUDA(cudaMalloc(&b, scratch_at + areas[2]));
+    auto bytes = [&](int i) {
+        return scratch_at + (i == 4 ? scratch_bytes : std::max({scratch_bytes, qb_tc_part_bytes(sms), qb_delta_tp_bytes(chunks[i])}));
+    };
+    for (; got < 4 && cudaMalloc(&b, bytes(got)) != cudaSuccess; got++) (void)cudaGetLastError();
+    if (got == 4) QB_CUDA(cudaMalloc(&b, bytes(4)));
     const cudaError_t e = qb::zero_now(device, b, zeroed);
     if (e != cudaSuccess) {
         cudaFree(b);
@@ -129,11 +132,12 @@ int qb_create(int device, qb_ctx** out) {
     c->form = c->err + 16;
     c->scratch = (float*)(b + scratch_at);
     c->scratch_bytes = scratch_bytes;
-    if (got < 2) {
+    if (got < 4) {
         c->tc_tickets = (int*)(b + tickets_at);
         c->tc_part = c->scratch;
+        c->delta_tp = c->scratch;
+        c->delta_chunks = chunks[got];
     }
-    if (got == 0) c->delta_tp = c->scratch;
     *out = c;
     return QB_OK;
 }
@@ -147,6 +151,13 @@ void qb_destroy(qb_ctx* c) {
 int qb_scratch_forget(qb_ctx* c) {
     if (!c) return QB_ERR_ARG;
     c->tc_part = nullptr; c->tc_tickets = nullptr; c->delta_tp = nullptr;
+    c->delta_chunks = 0;
+    return QB_OK;
+}
+
+int qb_scratch_chunks(qb_ctx* c, int chunks) {
+    if (!c || chunks < 0 || chunks > c->delta_chunks) return QB_ERR_ARG;
+    c->delta_chunks = chunks;
     return QB_OK;
 }
 

@@ -17,12 +17,13 @@ struct qb_ctx {
     int* err = nullptr;  // device word
     int* form = nullptr; // two device words: the form of the prompt attention that the step under way takes, a counter of its work
     // The prompt-sized kernels' scratch, in one area with `scratch` (calls use it in turn) and one allocation with the rest
-    // (`block`). A device that has room for the skinny products' part alone gets a context without it, whose calls take the
+    // (`block`). A device with less room gets a context with fewer chunks, or without either part, whose calls take the
     // forms that need none.
     void* block = nullptr;
     float* tc_part = nullptr;   // partial tiles of the tensor-core W4A16 products' shares (sms x 256 KB)
     int* tc_tickets = nullptr;  // their tickets, two per tile (QB_TC_TICKETS, zero between launches)
-    void* delta_tp = nullptr;   // the chunked delta rule's tiles per chunk, key head and value head (141 MB)
+    void* delta_tp = nullptr;   // the chunked delta rule's tiles per chunk, key head and value head (4.4 MB a chunk)
+    int delta_chunks = 0;       // .. of so many chunks
     // measurement override of the GEMV plan (0: built-in choice)
     int tune_cg = 0, tune_kg = 0, tune_nstages = 0, tune_ctas = 0;
     bool no_cluster = false, no_tc = false;
@@ -34,6 +35,7 @@ struct qb_ctx {
     long long* trace = nullptr;  // measurement: per-block timestamps of the next products
 };
 
+constexpr int QB_DELTA_CHUNKS = 50;     // the most chunks of a step of 2048 tokens (25 segments of 81)
 constexpr int QB_TC_TICKETS = 1 << 17;  // two per tile of a tensor-core W4A16 product (256 outputs x 256 tokens each)
 #define QB_CUDA(x)                         \
     do {                                   \
@@ -95,7 +97,7 @@ int qb_gemm_tc_launch(qb_ctx* ctx, cudaStream_t st, const void* X, const void* B
                       int k, int row0, int epi, int zp);
 // bytes of the prompt-sized kernels' scratch: tc_part on a part with `sms` SMs, delta_tp
 size_t qb_tc_part_bytes(int sms);
-size_t qb_delta_tp_bytes();
+size_t qb_delta_tp_bytes(int chunks);
 // the product for 17 .. 64 rows (w4a16_gemm_mid.cu), symmetric matrices; reached through qb_marlin_gemm
 int qb_gemm_mid_launch(qb_ctx* ctx, cudaStream_t st, const void* X, const void* B, void* Y, const void* S, int m, int n, int k,
                        int row0, int epi, const int* xrows, unsigned long long* keys, int n_valid);

@@ -1,8 +1,9 @@
 // The gated delta rule of a step's segments (qb_delta_rule), the reference's kernel delta_rule (kernels/qwen_deltanet.cuh:172-288)
 // by another algorithm. Segments of 80 tokens and more run in CHUNKS of 64 tokens (the WY form the reference states for its
-// MLX backend, src/mlx/delta.rs:6-15,85-137); the last 16..79 tokens of a segment (the last 16 of a step's only one), any
+// MLX backend, src/mlx/delta.rs:6-15,85-137), the last one shorter where need be; the last 16 tokens of a segment, any
 // replayed tokens and short segments run in the token form with the operation order of the decode mixer, so the checkpoint, the
-// replay bank and a later rollback see the bits a decode step would make.
+// replay bank and a later rollback see the bits a decode step would make. What a segment's tokens run in depends on its length
+// alone (given the scratch), so its bits do not depend on what else is in the step.
 //
 //  delta_chunk_prep_kernel  everything of a chunk that does not depend on the state, all chunks of all segments in parallel: with
 //                           G the running sum of the log decays, gam_i = exp(G_i), A_ij = b_i (k_i . k_j) exp(G_i - G_j) (j < i),
@@ -30,20 +31,31 @@ constexpr int CH = 64;                   // tokens per chunk
 constexpr int TP_TOK = 2048;             // tokens of a step at most
 constexpr int GROUPS = 8, GCOLS = 16;    // a value head's columns in groups of 16: a group shares its scales
 
-// Tokens of a segment that run in chunks: they end at least KEEP tokens before the segment's end (the checkpoint and the bank of
-// the rollback plan are made in the token form). Whole chunks; where the step has one segment (`one`), a last shorter one too.
-__host__ __device__ __forceinline__ int chunked_tokens(int len, bool one) {
-    return len < CH + KEEP ? 0 : one ? len - KEEP : (len - KEEP) / CH * CH;
+// Tokens of a segment that run in chunks: all but the last KEEP (the checkpoint and the bank of the rollback plan are made in the token
+// form); the last chunk may be a short one.
+__host__ __device__ __forceinline__ int chunked_tokens(int len) { return len < CH + KEEP ? 0 : len - KEEP; }
+__host__ __device__ __forceinline__ int chunks_of(int len) { return (chunked_tokens(len) + CH - 1) / CH; }
+// the most chunks that `segs` segments of n tokens in all can have: (len + CH - KEEP - 1) / CH of one, for those of CH + KEEP and more
+static int chunks_most(int n, int segs) {
+    const int k = segs < n / (CH + KEEP) ? segs : n / (CH + KEEP);
+    return (n + k * (CH - KEEP - 1)) / CH;
 }
 
-// the z-th of a step's segments that run in chunks, or -1
-__device__ __forceinline__ int long_segment(const int* seg_len, int segs, int z) {
+// the z-th of a step's segments that run in chunks, or -1; `place`: the chunks of those before it
+__device__ __forceinline__ int long_segment(const int* seg_len, int segs, int z, int& place) {
+    place = 0;
+    const int lane = threadIdx.x & 31;
     for (int s0 = 0; s0 < segs; s0 += 32) {
-        const int s = s0 + (threadIdx.x & 31);
-        unsigned any = __ballot_sync(0xffffffffu, s < segs && chunked_tokens(seg_len[s], segs == 1) > 0);
-        if (z >= __popc(any)) { z -= __popc(any); continue; }
-        for (; z > 0; z--) any &= any - 1;
-        return s0 + __ffs(any) - 1;
+        const int nc = s0 + lane < segs ? chunks_of(seg_len[s0 + lane]) : 0;
+        unsigned any = __ballot_sync(0xffffffffu, nc > 0);
+        const bool here = z < __popc(any);
+        if (here)
+            for (; z > 0; z--) any &= any - 1;
+        else
+            z -= __popc(any);
+        const int at = here ? __ffs(any) - 1 : 32;
+        place += __reduce_add_sync(0xffffffffu, lane < at ? nc : 0);
+        if (here) return s0 + at;
     }
     return -1;
 }
@@ -64,10 +76,11 @@ static_assert(sizeof(Gates) % 16 == 0, "bulk copies");
 constexpr int KQ_BYTES = 6 * TILE, VH_BYTES = 9 * TILE + 1024, U_AT = 5 * TILE, GATES_AT = 9 * TILE;
 constexpr size_t CHUNK_BYTES = (size_t)LK_HEADS * KQ_BYTES + (size_t)LV_HEADS * VH_BYTES;
 static_assert(sizeof(Gates) <= 1024, "the gates' place");
-// chunk index = first token / 64: distinct for disjoint ranges of 64 tokens, and for the chunks of one segment
-__device__ __forceinline__ uint8_t* kq_at(uint8_t* tp, int tok, int kh) { return tp + (size_t)(tok >> 6) * CHUNK_BYTES + (size_t)kh * KQ_BYTES; }
-__device__ __forceinline__ uint8_t* vh_at(uint8_t* tp, int tok, int h) {
-    return tp + (size_t)(tok >> 6) * CHUNK_BYTES + (size_t)LK_HEADS * KQ_BYTES + (size_t)h * VH_BYTES;
+static_assert(CHUNK_BYTES == 4374528, "what the documents say of a context's scratch");
+// place: the step's chunks in a row, segment after segment
+__device__ __forceinline__ uint8_t* kq_at(uint8_t* tp, int place, int kh) { return tp + (size_t)place * CHUNK_BYTES + (size_t)kh * KQ_BYTES; }
+__device__ __forceinline__ uint8_t* vh_at(uint8_t* tp, int place, int h) {
+    return tp + (size_t)place * CHUNK_BYTES + (size_t)LK_HEADS * KQ_BYTES + (size_t)h * VH_BYTES;
 }
 __device__ __forceinline__ uint32_t u_at(int group, int token, int piece) {  // byte offset
     return (uint32_t)(group * (CH * 64) + token * 64 + ((piece ^ ((token >> 1) & 3)) << 4));
@@ -131,17 +144,18 @@ delta_chunk_prep_kernel(const float* cv, uint8_t* tp, const int* seg_start, cons
     extern __shared__ uint8_t cp_raw[];
     PrepSmem& M = *(PrepSmem*)(((uintptr_t)cp_raw + 1023) & ~(uintptr_t)1023);
     pdl_launch_dependents();
-    const int c = blockIdx.x, h = blockIdx.y, sg = long_segment(seg_len, segs, blockIdx.z), kh = h / (LV_HEADS / LK_HEADS);
+    int place;
+    const int c = blockIdx.x, h = blockIdx.y, sg = long_segment(seg_len, segs, blockIdx.z, place), kh = h / (LV_HEADS / LK_HEADS);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g8 = lane >> 2, t4 = lane & 3;
-    const int t0 = sg < 0 ? 0 : seg_start[sg], cnt = sg < 0 ? 0 : min(CH, chunked_tokens(seg_len[sg], segs == 1) - c * CH);  // the chunk's tokens
+    const int t0 = sg < 0 ? 0 : seg_start[sg], cnt = sg < 0 ? 0 : min(CH, chunked_tokens(seg_len[sg]) - c * CH);  // the chunk's tokens
     if (cnt <= 0) {
         pdl_wait();  // (the kernel after this one relies on it for the kernels before)
         return;
     }
     const int tok = t0 + c * CH;
     const bool first = h % (LV_HEADS / LK_HEADS) == 0;  // this block stores the key head's tiles
-    uint8_t* const kq = kq_at(tp, tok, kh);
-    uint8_t* const vh = vh_at(tp, tok, h);
+    uint8_t* const kq = kq_at(tp, place + c, kh);
+    uint8_t* const vh = vh_at(tp, place + c, h);
     pdl_wait();
     const float* const row0 = cv + (size_t)tok * CVW;
     auto warp_most = [](uint32_t m) { return __reduce_max_sync(0xffffffffu, m); };
@@ -566,11 +580,12 @@ delta_scan_kernel(const float* p, int splits, int n, const float* cv, uint8_t* t
                   const int* seg_start, const int* seg_len, const int* seg_slot, const int* seg_pos0, int segs, int all, int* err) {
     extern __shared__ __align__(16) uint8_t scan_raw[];
     ScanSmem& M = *(ScanSmem*)(((uintptr_t)scan_raw + 1023) & ~(uintptr_t)1023);
-    const int vs = blockIdx.x, h = blockIdx.y, sg = CHUNKS && segs > 1 ? long_segment(seg_len, segs, blockIdx.z) : blockIdx.z, kh = h / (LV_HEADS / LK_HEADS);
+    int place = 0;
+    const int vs = blockIdx.x, h = blockIdx.y, sg = CHUNKS && segs > 1 ? long_segment(seg_len, segs, blockIdx.z, place) : blockIdx.z, kh = h / (LV_HEADS / LK_HEADS);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     int t0 = sg < 0 ? 0 : seg_start[sg], len = sg < 0 ? 0 : seg_len[sg];
-    const int l0 = CHUNKS ? chunked_tokens(len, segs == 1) : 0, nc = (l0 + CH - 1) / CH;
-    if (CHUNKS ? sg < 0 : !all && chunked_tokens(len, segs == 1) > 0) {  // another kernel's, or nobody's
+    const int l0 = CHUNKS ? chunked_tokens(len) : 0, nc = (l0 + CH - 1) / CH;
+    if (CHUNKS ? sg < 0 : !all && chunked_tokens(len) > 0) {  // another kernel's, or nobody's
         pdl_launch_dependents();
         pdl_wait();
         return;
@@ -603,8 +618,7 @@ delta_scan_kernel(const float* p, int splits, int n, const float* cv, uint8_t* t
             // one of the blocks that read them
             auto ahead = [&](int c) {
                 if (c >= nc) return;
-                const int tok = t0 + c * CH;
-                const uint8_t *kq = kq_at(tp, tok, kh), *vh = vh_at(tp, tok, h);
+                const uint8_t *kq = kq_at(tp, place + c, kh), *vh = vh_at(tp, place + c, h);
                 if (vs == 0) bulk_prefetch(vh, 5 * TILE);
                 bulk_prefetch(vh + U_AT + vs * 2 * TILE, 2 * TILE);
                 if (vs == 0 && h % (LV_HEADS / LK_HEADS) == 0) bulk_prefetch(kq, KQ_BYTES);
@@ -614,8 +628,7 @@ delta_scan_kernel(const float* p, int splits, int n, const float* cv, uint8_t* t
             bool ok = true;
             for (int c = 0; c < nc && ok; c++) {
                 ahead(c + 2);
-                const int tok = t0 + c * CH;
-                const uint8_t *kq = kq_at(tp, tok, kh), *vh = vh_at(tp, tok, h);
+                const uint8_t *kq = kq_at(tp, place + c, kh), *vh = vh_at(tp, place + c, h);
                 if (c > 0) ok = mbar_wait(&M.g1done, (c - 1) & 1);  // (all state warps are past chunk c - 2 as well)
                 if (!ok) break;
                 uint64_t* uf = &M.ufull[c & 1];
@@ -916,12 +929,13 @@ delta_scan_kernel(const float* p, int splits, int n, const float* cv, uint8_t* t
 
 using namespace qb;
 
-size_t qb_delta_tp_bytes() { return (size_t)(TP_TOK / CH + 1) * CHUNK_BYTES; }
+size_t qb_delta_tp_bytes(int chunks) { return (size_t)chunks * CHUNK_BYTES; }
+static_assert(TP_TOK / (CH + KEEP) * (CH - KEEP - 1) + TP_TOK < (QB_DELTA_CHUNKS + 1) * CH, "room for the chunks of any step");
 
 extern "C" {
 
-// The chunked form's scratch (the chunks' tiles of a step of up to 2048 tokens, 141 MB) belongs to the context; one that was
-// created without it runs every segment in the token form.
+// The chunked form's scratch (the chunks' tiles) belongs to the context; a step that may have more chunks than its context has room
+// for runs every segment in the token form.
 int qb_delta_rule(qb_ctx* ctx, void* stream, const float* p, int splits, int n, const float* cv, float* mem,
                   long long sst, const int* meta, float* out, const int* seg_start, const int* seg_len,
                   const int* seg_slot, const int* seg_pos0, int segs) {
@@ -930,7 +944,7 @@ int qb_delta_rule(qb_ctx* ctx, void* stream, const float* p, int splits, int n, 
         return QB_ERR_ARG;
     cudaStream_t st = (cudaStream_t)stream;
     if (n > TP_TOK) return QB_ERR_TOO_LARGE;
-    const int l0 = ctx->delta_tp ? chunked_tokens(n, segs == 1) : 0;  // of the longest segment the step can hold
+    const int l0 = chunks_most(n, segs) <= ctx->delta_chunks ? chunked_tokens(n) : 0;  // of the longest segment the step can hold
     const int most = segs < n / (CH + KEEP) ? segs : n / (CH + KEEP);  // segments that can run in chunks
     if (l0 > 0) {
         int rc = launch(ctx, delta_chunk_prep_kernel, dim3((l0 + CH - 1) / CH, LV_HEADS, most), dim3(CP_THREADS), sizeof(PrepSmem) + 1024, st, cv,

@@ -30,6 +30,8 @@ int qb_gemm_f16_block_tiles(int ntiles, int splits, int kper, int n, int sms);
 int qb_attn_tiles_on_pairs(const int* h_ptile, int ntile, const int* h_tok_slot, const int* h_tok_pos, int sms);
 /* Tests: the context goes on as one that was created where the prompt-sized kernels' scratch did not fit. */
 int qb_scratch_forget(qb_ctx* ctx);
+/* .. as one where the delta rule's tiles of only so many chunks fit (0: none). */
+int qb_scratch_chunks(qb_ctx* ctx, int chunks);
 /* Tests: one block waits on an mbarrier that nothing arrives on, with the library's bounded wait cut to `limit` polls
  * (at most 2^20); the wait runs out and the context's error word reads 99 (qb_device_error). */
 int qb_wait_probe(qb_ctx* ctx, void* stream, unsigned limit);

@@ -264,3 +264,18 @@ def test_a_context_without_the_prompt_sized_scratch(ctx):
         assert (a - b).abs().max() < 1e-4 * max(1.0, b.abs().max().item())
     assert c.device_error() == 0
     c.close()
+
+
+def test_a_context_without_room_for_chunks(ctx):
+    """A context created where the delta rule's tiles did not fit but the prompt-sized products' part did: the products' bits are those of a
+    full context, the rule runs token by token."""
+    from qwenny_b200.ops import Context
+    want = _outputs(_prompt_calls(ctx, synth.gen(903)))
+    c = Context(0)
+    assert lib().qb_scratch_chunks(c.h, 0) == 0
+    got = _outputs(_prompt_calls(c, synth.gen(903)))
+    assert all(torch.equal(a, b) for i in (0, 1) for a, b in zip(got[i], want[i]))
+    for a, b in zip(got[2], want[2]):
+        assert not torch.equal(a, b) and (a - b).abs().max() < 1e-4 * max(1.0, b.abs().max().item())
+    assert c.device_error() == 0
+    c.close()
