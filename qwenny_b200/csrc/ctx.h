@@ -87,6 +87,8 @@ int qb_attn_prefill_launches(const qb_ctx* ctx, int ntile, int max_keys, int as)
 int qb_delta_mixer_as(qb_ctx* ctx, void* stream, const float* p, int splits, int n, const float* ba, int ba_splits, const float* cw,
                       const float* a_log, const float* dt_bias, const float* nw, float* mem, long long sst, int* meta, float* out, void* y,
                       const int* seg_start, const int* seg_len, const int* seg_slot, const int* seg_pos0, int segs, int ahead);
+// the kernels that qb_delta_rule launches for a step of n tokens
+int qb_delta_rule_launches(const qb_ctx* ctx, int n, int segs);
 // qb_attn_decode for a caller that vouches in the same way (ahead = 1) for the cache entries of earlier steps
 int qb_attn_decode_as(qb_ctx* ctx, void* stream, const float* q, const void* kc, const void* vc, const float* ks, const float* vs,
                       const int* dseg, const int* dtok, const int* dkeys, const int* tok_slot, const int* tok_pos, int cap, int ndseg,

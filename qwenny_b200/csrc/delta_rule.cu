@@ -932,6 +932,11 @@ using namespace qb;
 size_t qb_delta_tp_bytes(int chunks) { return (size_t)chunks * CHUNK_BYTES; }
 static_assert(TP_TOK / (CH + KEEP) * (CH - KEEP - 1) + TP_TOK < (QB_DELTA_CHUNKS + 1) * CH, "room for the chunks of any step");
 
+// of the longest segment that the step can hold
+static int chunked_of(const qb_ctx* ctx, int n, int segs) { return chunks_most(n, segs) <= ctx->delta_chunks ? chunked_tokens(n) : 0; }
+
+int qb_delta_rule_launches(const qb_ctx* ctx, int n, int segs) { return chunked_of(ctx, n, segs) == 0 ? 1 : segs > 1 ? 3 : 2; }
+
 extern "C" {
 
 // The chunked form's scratch (the chunks' tiles) belongs to the context; a step that may have more chunks than its context has room
@@ -944,7 +949,7 @@ int qb_delta_rule(qb_ctx* ctx, void* stream, const float* p, int splits, int n, 
         return QB_ERR_ARG;
     cudaStream_t st = (cudaStream_t)stream;
     if (n > TP_TOK) return QB_ERR_TOO_LARGE;
-    const int l0 = chunks_most(n, segs) <= ctx->delta_chunks ? chunked_tokens(n) : 0;  // of the longest segment the step can hold
+    const int l0 = chunked_of(ctx, n, segs);
     const int most = segs < n / (CH + KEEP) ? segs : n / (CH + KEEP);  // segments that can run in chunks
     if (l0 > 0) {
         int rc = launch(ctx, delta_chunk_prep_kernel, dim3((l0 + CH - 1) / CH, LV_HEADS, most), dim3(CP_THREADS), sizeof(PrepSmem) + 1024, st, cv,

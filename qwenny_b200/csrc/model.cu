@@ -181,7 +181,7 @@ int launch_mixer(qb_model* m, cudaStream_t st, int layer, int& k) {
             QB_TRY(qb_delta_conv(c, s, m->part, 1, n, m->ba, ba_splits, L.conv_w, L.a_log, L.dt_bias, L.mem, L.sst,
                                  m->cv, m->tok_slot, m->tok_pos)); k++;
             QB_TRY(qb_delta_rule(c, s, m->part, 1, n, m->cv, L.mem, L.sst, L.meta, m->o, m->seg_start, m->seg_len,
-                                 m->seg_slot, m->seg_pos0, m->segs)); k++;
+                                 m->seg_slot, m->seg_pos0, m->segs)); k += qb_delta_rule_launches(c, n, m->segs);
             QB_TRY(qb_delta_norm(c, s, m->part, 1, n, L.norm_w, m->o, m->mix, L.meta, m->seg_len, m->seg_slot,
                                  m->seg_pos0, m->segs)); k++;
         }

@@ -223,3 +223,31 @@ def test_launching_ahead_of_the_kernel_before_does_not_change_a_bit():
     assert on.device_error() == 0 and off.device_error() == 0
     a.close()
     b.close()
+
+
+def test_a_prompt_step_counts_the_kernels_of_the_delta_rule(ctx):
+    """qb_model_step_kernels counts one kernel of the rule for a step without chunks, two for one long segment and three beside another:
+    as many as a capture of qb_delta_rule itself holds."""
+    from cuda.bindings import runtime
+    from oracle import ref_cuda, ref_ops as R
+    m = M.synthetic(ctx, nlayers=1, slots=2, max_ctx=512, vocab=2000, seed=12, pattern=("delta",))
+    sst = (R.SLOT_FLOATS + 1023) // 1024 * 1024
+    steps, held = [], []
+    for lens in ((79,), (130,), (130, 40)):
+        toks = [(i, s, i) for s, n in enumerate(lens) for i in range(n)]
+        m.step(toks, [0])
+        steps.append(m.step_kernels)
+        n, dv = len(toks), ref_cuda.upload_step(R.build_step(toks, []))
+        z = lambda *shape: torch.zeros(*shape, device="cuda")
+        args = z(1, n, R.DELTA_IN), 1, n, z(n, R.CVW), z(2 * sst), sst, torch.zeros(2, 4, dtype=torch.int32, device="cuda"), z(n, R.MIX), dv, len(lens)
+        ctx.delta_rule(*args)
+        torch.cuda.synchronize()
+        g = torch.cuda.CUDAGraph(keep_graph=True)
+        with torch.cuda.graph(g):
+            ctx.delta_rule(*args)
+        err, _, count = runtime.cudaGraphGetNodes(g.raw_cuda_graph())
+        assert int(err) == 0
+        held.append(count)
+    assert held == [1, 2, 3]
+    assert [k - steps[0] for k in steps] == [h - held[0] for h in held]
+    m.close()
