@@ -28,8 +28,8 @@ constexpr int SLOT_BANK = KEEP * REP;
 constexpr int SLOT_RING = 2 * SLOT_STATE + 2 * SLOT_BANK;
 constexpr int CVW = LQKV + 2 * LV_HEADS;  // 10336
 
-// Every bounded wait gives up after this many polls (each may itself sleep for WAIT_NS: half a second in all), sets the error word
-// and lets the kernel drain: nothing here can spin forever.
+// Every bounded wait gives up after this many polls, sets the error word and lets the kernel drain: nothing here can spin forever. A
+// poll that nothing ends takes 2.05 us (WAIT_NS is an upper limit to the hardware; timed): 0.54 s in all.
 constexpr uint32_t WAIT_LIMIT = 1u << 18;
 // A waiting thread sleeps in the barrier unit until the phase completes or this many ns are over. Without the hint it polls, and
 // beside 16 polling warps a check of a completed barrier takes 250 cycles instead of 125 and an arrival 110 instead of 10

@@ -137,6 +137,21 @@ def test_a_wait_that_runs_out_is_reported_and_the_context_lives_on(ctx):
 
 
 @pytest.mark.gpu
+def test_how_long_a_wait_lasts_that_runs_out(ctx):
+    """A poll of the bounded waits sleeps for up to 2 us, which the 2^18 polls of a wait count on: half a second in all. The hint is an upper
+    limit, so what a poll that nothing ends takes is timed: 1 to 4 us (2.05 measured), 2^18 of them 0.26 to 1.05 s."""
+    st = torch.cuda.current_stream().cuda_stream
+    ctx.wait_probe(1 << 4, st)
+    a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+    a.record()
+    ctx.wait_probe(1 << 14, st)
+    b.record()
+    torch.cuda.synchronize()
+    assert ctx.device_error() == 99
+    assert 1e-3 < a.elapsed_time(b) / (1 << 14) < 4e-3   # ms
+
+
+@pytest.mark.gpu
 def test_a_product_whose_stage_never_lands_gives_up_and_reports_it(ctx):
     """The skinny product's own way out: the copy warp leaves out the second stage of every block (a measurement switch),
     the consumers' wait for it runs out after 1024 polls, each warp records error 2, walks the rest of its schedule
