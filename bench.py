@@ -243,7 +243,7 @@ def reference_kernels(ctx, torch):
     theirs = _time_us(torch, lambda: ref.delta(part_l, 1, T, None, 0, None, None, None, None, mems[1], sst, meta0, cv_l,
                                                 o_l, None, st3, dv3, which=("rule",)), reps=5)
     res["deltanet_rule_2048rows"] = {"ours_us": ours, "reference_us": theirs, "reference": "delta_rule (sequential)",
-                                     "ours": "chunked scan, chunk 64, 3 x TF32 (two launches)"}
+                                     "ours": "chunked scan, chunk 64, pairs of f16 per operand (two launches)"}
     # ---- the 16-bit in-projection of a DeltaNet layer (in_proj_b / in_proj_a, 96 x 5120)
     K, rows = 5120, 96
     wp = (torch.randn(rows // 16, K // 16, 32, 8, generator=g, device="cuda") * 0.02).half()

@@ -12,7 +12,7 @@
 //               write them as f16 where the tensor core wants them: K as four [64 keys][64 dims] K-major tiles, V
 //               transposed as one [256 dims][64 keys] tile, both with the 128-byte swizzle; the codes are converted
 //               EXACTLY (1024 + byte via prmt, minus 1152), so no offset has to be folded out afterwards
-//   warp 16     one elected lane issues S = Q K^T (M 128 rows, N 64 keys, K 256 dims: 16 tcgen05.mma, A from tensor
+//   warp 16     issues, as a whole warp, S = Q K^T (M 128 rows, N 64 keys, K 256 dims: 16 tcgen05.mma, A from tensor
 //               memory) and O += P V (M 128, N 256 dims, K 64 keys: 4 tcgen05.mma, A = P from tensor memory);
 //               tcgen05.commit tells the others when a product is complete. S of stage i + 1 is issued before P V of
 //               stage i, so the tensor core has work while the softmax of stage i runs

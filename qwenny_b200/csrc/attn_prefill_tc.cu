@@ -16,7 +16,7 @@
 //               registers) and write it as f16 where the tensor core wants it: K as four [64 keys][64 dims] K-major
 //               tiles, V transposed as two [128 dims][64 keys] tiles, with the 128-byte swizzle; the codes are
 //               converted EXACTLY (1024 + byte via prmt, minus 1152), so no offset has to be folded out afterwards
-//   warp 16     of the first block: one lane issues S = Q K^T (M 256 rows, N 128 keys, K 256 dims: 16 tcgen05.mma) and
+//   warp 16     of the first block: issues, as a whole warp, S = Q K^T (M 256 rows, N 128 keys, K 256 dims: 16 tcgen05.mma) and
 //               O += P V (N 256 dims, K 128 keys: 8 tcgen05.mma, A = P from tensor memory); tcgen05.commit tells both
 //               blocks when a product is complete. S of stage i + 1 is issued before P V of stage i, so the tensor core has
 //               work while the softmax of stage i runs

@@ -55,7 +55,7 @@ struct Waiter {
     int code;
     bool dead = false;
     // (the compiler's loop: beside 16 softmax and conversion warps the written-out one of mbar_wait costs 1 %, 2048 rows at context
-    // 30720 1993 and 2014 us)
+    // 30720 1997 and 2019 us, 600 at 2000 114.0 and 114.9, in turn)
     __device__ __forceinline__ static bool sleep(uint64_t* bar, uint32_t parity) {
         for (uint32_t i = 0; i < WAIT_LIMIT; i++)
             if (mbar_try_wait(bar, parity)) return true;

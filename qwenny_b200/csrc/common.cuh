@@ -33,7 +33,8 @@ constexpr int CVW = LQKV + 2 * LV_HEADS;  // 10336
 constexpr uint32_t WAIT_LIMIT = 1u << 18;
 // A waiting thread sleeps in the barrier unit until the phase completes or this many ns are over. Without the hint it polls, and
 // beside 16 polling warps a check of a completed barrier takes 250 cycles instead of 125 and an arrival 110 instead of 10
-// (40-row MLP 78.9 -> 77.7 us, 16-row MLP 53.0 -> 52.1, decode attention of 5 rows at 32000 keys 34.7 -> 34.4).
+// (without / with, in turn from a graph: 16-row MLP 53.3 / 52.1 us, 40-row MLP 79.8 / 78.1, 40-row output layer 310.6 / 299.0, prompt
+// attention of 2048 rows at context 30720 2029 / 1997; decode attention and the delta rule the same).
 constexpr uint32_t WAIT_NS = 2000;
 
 // ---------------------------------------------------------------- small math
@@ -129,8 +130,9 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
         : "memory");
     return ok != 0;
 }
-// Bounded wait: false when the limit ran out (the caller records it and drains). The loop is written out: five instructions a poll
-// where the compiler made eight (5-row MLP 33.6 -> 33.2 us, 40-row output layer 321 -> 317).
+// Bounded wait: false when the limit ran out (the caller records it and drains). The loop is written out: as a C++ loop the 5-row MLP
+// takes 34.4 us instead of 33.9 and the 40-row output layer 300.4 instead of 299.2 (in turn from a graph; 17 to 64 rows of the MLP
+// and decode attention the same).
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, uint32_t limit = WAIT_LIMIT) {
     uint32_t ok;
     asm volatile(

@@ -1,4 +1,4 @@
-// Gated DeltaNet pieces shared by the one-launch decode mixer (deltanet.cu) and the prompt path (delta_prompt.cu): the
+// Gated DeltaNet pieces shared by the one-launch decode mixer (deltanet.cu) and the prompt path (delta_rule.cu): the
 // rollback plan of a segment's step, and the token form of the delta rule on a thread's slice of the f32 state.
 // Slot memory, plan and metadata are the reference's (kernels/qwen_deltanet.cuh:12-82; they are what its host saves,
 // loads and rolls back): state [2][48][128 v][128 k] f32, banks [2][16][REP], ring [32][LQKV]; meta {end, ck, ebuf, _}.

@@ -123,8 +123,8 @@ __device__ __forceinline__ void ldsm_x4(uint32_t* r, uint32_t addr) { ldsm_x4(r[
 
 // ------------------------------------------------------------------------------------------------ chunk preparation
 // grid (chunks of the longest possible segment, LV_HEADS, segments that may be long enough), block 256, two blocks per SM. The products run on mma.sync (two f16
-// per operand). 120 us for 2048 tokens, bound by the issue of 34,000 warp instructions a block (43 % of the slots) and the latency of its
-// short phases; the tensor pipe is busy for a quarter of it. W and U are made here, where all chunks run in parallel, so that the
+// per operand). 120 us for 2048 tokens (126 alone and cold), bound by the issue of 34,500 warp instructions a block (43 % of the slots) and
+// the latency of its short phases at 3.7 warps per scheduler; the tensor pipe is busy for a fifth of it. W and U are made here, where all chunks run in parallel, so that the
 // scan has two products in sequence per chunk instead of three.
 constexpr int CP_THREADS = 256, TST = 72;  // TST: row stride of T (a fragment's pairs hit 32 banks)
 struct PrepSmem {
@@ -524,9 +524,11 @@ delta_chunk_prep_kernel(const float* cv, uint8_t* tp, const int* seg_start, cons
 
 // ------------------------------------------------------------------------------------------------ the scan
 // 2048 tokens: some 145 us, 190 with polling waits, spilled registers and tiles from memory, 299 with 3 x TF32 on mma.sync. Bound by a chain per
-// chunk: the barrier to the product warp, 16 products (830 cycles), D (1250), 8 products (600), S (1300). 64 columns a block: a product with
-// N = 128 (hi and lo) takes 66 cycles, with N = 64 50, so narrower blocks would hardly be faster, and two blocks per head load each
-// tile twice instead of three times.
+// chunk, 7900 cycles (clock64 of a state warp that converts D): 2550 until W S is there (the product warp's checks and 16 products, which take
+// the tensor core 930), 2750 to convert D beside the other half's outputs of the chunk before, 950 until K^T D is there (8 products), 1150 to
+// update the state and hand it on, 400 for U; some 12 us for the last 16 tokens. Issue slots 30 % active, tensor pipe 16 %. 64
+// columns a block: a product with N = 128 (hi and lo) takes 66 cycles, with N = 64 50, so narrower blocks would hardly be faster, and two
+// blocks per head load each tile twice instead of three times.
 constexpr int SC_COLS = 64, SC_THREADS = SC_COLS * 8;  // the state's threads: one per key and 16 columns; token form: 8 per column
 constexpr int SC_TAIL = 16;                            // tokens staged per round of the token form
 constexpr int KLD = LKD + 4;                           // row stride of the f32 state tile
@@ -614,7 +616,7 @@ delta_scan_kernel(const float* p, int splits, int n, const float* cv, uint8_t* t
     if (CHUNKS && warp == COPY_WARP) {
         pdl_wait();
         if (lane == 0) {
-            // a chunk's tiles are asked into L2 two chunks ahead (from memory a copy took up to 3900 cycles, half a chunk's time), by
+            // a chunk's tiles are asked into L2 two chunks ahead (from memory a copy took up to 3900 cycles, half of a chunk's time), by
             // one of the blocks that read them
             auto ahead = [&](int c) {
                 if (c >= nc) return;

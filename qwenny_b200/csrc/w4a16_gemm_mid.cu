@@ -4,12 +4,12 @@
 //
 // A block owns 128 outputs and the weights go from registers to tensor memory in the layout that a Marlin word already has
 // (w4a16_gemm_tc.cu). The floor is the weights' way from HBM (0.52 bytes each, read once): 380 cycles per block and 128 of
-// k. It takes some 1000: a stage's way from barrier to barrier (copied, unpacked, multiplied, drained: each check some 125 to 250
-// cycles) and the waiting warps' polls, which take a third of the issue slots (59 % active, tensor pipe 17 %, DRAM 25 %).
+// k. It takes some 1200 (40 rows of gate_up: 91,500 cycles for 73.5 stages a block): a stage's way from barrier to barrier (copied,
+// unpacked, multiplied, drained: each check some 125 cycles) and the issue of 2770 warp instructions a stage (issue slots 64 %
+// active there and 60 % in down, 6 warps per scheduler; tensor pipe 17 %, DRAM 23 %).
 // A drain warp takes 16 tokens: with 32 its threads held 64 values and spilled (40 rows of the MLP 84.7 -> 78.9 us).
-// The MLP of 17, 40 and 64 rows 71, 77.7 and 85 us (75, 86 and 89 with 32-token drains and polling waits), the output layer over
-// 40 rows 299 (310); padded to 256 tokens
-// 40 rows took 168. What else differs from the prompt-sized product:
+// From a graph the MLP of 17, 40 and 64 rows takes 72, 78 and 86 us, the output layer over 40 rows 299 (316 with other weights in every
+// pass); padded to 256 tokens 40 rows of the MLP took 168. What else differs from the prompt-sized product:
 //   - the weights are the exact integers q - 8; a group of 128 columns is one accumulation, and the drain warps multiply its
 //     f32 sums by the f32 value of the group's scale and add them up in registers (one thread per output, a register
 //     per token): one rounding per group, the arithmetic of the product for up to 16 rows (w4a16_gemv.cuh), where

@@ -10,7 +10,7 @@
 // dequantised halves go from registers to tensor memory without touching shared memory. What that buys: the form that
 // wrote them to shared memory (one block per tile, two M = 128 halves re-reading the X tile) moved 169 KB through an SM's
 // shared memory per 1024 cycles of products and was bound by it (tensor pipe 65 % active); this one moves 80 KB per
-// 1024. A stage is 128 of k because the issuing threads are the next limit: a wait, a commit and their like cost 180 cycles per
+// 1024. A stage is 128 of k because the issuing warps are the next limit: a wait, a commit and their like cost 180 cycles per
 // stage beside 65 per product, and the copying lane 70 per copy (64 of k per stage: 600 cycles of the 512 at N = 256).
 //
 // The work is the list of (tile, k block of 128) pairs, tile after tile. Where whole tiles would leave the last wave
@@ -24,7 +24,7 @@
 //               the interleaved SwiGLU matrices (or the partial tile)
 //   warp 8      copies, one lane: the X half tile (tensor map, 128-byte swizzle), the 8 KB of words (tensor map), the
 //               group's scales; full/empty mbarriers, a ring of 4 stages
-//   warp 9      of the pair's first block: one lane issues the products (K = 16 each), tcgen05.commit hands the stage
+//   warp 9      of the pair's first block: issues the products (K = 16 each) as a whole warp, tcgen05.commit hands the stage
 //               back in both blocks when they have read it
 #include "launch.h"
 #include "pair_tc.cuh"
