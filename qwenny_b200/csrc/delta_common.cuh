@@ -32,7 +32,8 @@ __device__ __forceinline__ Plan make_plan(const int* meta, int slot, int p0, int
 }
 
 // Ahead of the kernel before, which may still write them: the slot's state (COLS columns of a head from `row` on) is asked into L2 by a
-// block of THREADS. The metadata read here only says which buffer; a stale value costs the hint.
+// block of THREADS. The metadata read here only says which buffer; a stale value costs the hint. (Mixers of many layers in turn, their
+// states not in L2, without / with it: 1 row 18.3 / 17.4 us, 12 segments of 2 79.2 / 76.9; on a state in L2 5 segments of 5 44.1 / 44.6.)
 template <int COLS, int THREADS>
 __device__ __forceinline__ void hint_state(const int* meta, int slot, int p0, const float* sm0, int row) {
     if (p0 == 0) return;

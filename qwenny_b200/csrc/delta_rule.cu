@@ -628,6 +628,7 @@ delta_scan_kernel(const float* p, int splits, int n, const float* cv, uint8_t* t
             ahead(0);
             ahead(1);
             bool ok = true;
+            int na = 0, nk = 0, np = 0;  // chunks whose W, Q and U, whose K and whose P are asked for
             for (int c = 0; c < nc && ok; c++) {
                 ahead(c + 2);
                 const uint8_t *kq = kq_at(tp, place + c, kh), *vh = vh_at(tp, place + c, h);
@@ -644,15 +645,23 @@ delta_scan_kernel(const float* p, int splits, int n, const float* cv, uint8_t* t
                     bulk_load(M.a[0][i][1], kq + (4 + i) * TILE, TILE, &M.afull);
                     bulk_load(M.a[1][i][0], vh + (2 + i) * TILE, TILE, &M.afull);
                 }
+                na++;
                 if (c > 0) ok = mbar_wait(&M.g3done, (c - 1) & 1);
                 if (!ok) break;
                 mbar_expect_tx(&M.kfull, 4 * TILE);
                 bulk_load(M.k, kq, 4 * TILE, &M.kfull);
+                nk++;
                 if (c > 0) ok = mbar_wait(&M.pdone, (c - 1) & 1);
                 if (!ok) break;
                 mbar_expect_tx(&M.pfull, TILE);
                 bulk_load(M.p, vh + 4 * TILE, TILE, &M.pfull);
+                np++;
             }
+            // the block does not end before its copies have landed, also where the warps that use them have given up
+            for (int u = max(na - 2, 0); u < na; u++) mbar_wait(&M.ufull[u & 1], (u >> 1) & 1);
+            if (na) mbar_wait(&M.afull, (na - 1) & 1);
+            if (nk) mbar_wait(&M.kfull, (nk - 1) & 1);
+            if (np) mbar_wait(&M.pfull, (np - 1) & 1);
             if (!ok) atomicExch(err, 20);
         }
         __syncwarp();
@@ -663,6 +672,7 @@ delta_scan_kernel(const float* p, int splits, int n, const float* cv, uint8_t* t
                            K64 = idesc_mn(64, true, true);
         const uint32_t tm = uniform(tmem);
         bool ok = true;
+        int n1 = 0, n3 = 0, np = 0;  // products committed
         for (int c = 0; c < nc; c++) {
             ok = warp_wait(&M.afull, c & 1) && warp_wait(&M.sready, c & 1);
             if (!ok) break;
@@ -675,6 +685,7 @@ delta_scan_kernel(const float* p, int splits, int n, const float* cv, uint8_t* t
             for (int i = 0; i < 8; i++)
                 umma_ss<1>(tm + (c & 1) * 128, smem_desc(a + 4 * TILE + (i >> 2) * 2 * TILE + (i & 3) * 32), mn_desc(s + i * 2048, 2 * TILE), W64, 1);
             umma_commit(&M.g1done);
+            n1++;
             ok = warp_wait(&M.kfull, c & 1) && warp_wait(&M.dready, c & 1);
             if (!ok) break;
             tc_fence_after();
@@ -683,12 +694,18 @@ delta_scan_kernel(const float* p, int splits, int n, const float* cv, uint8_t* t
 #pragma unroll
             for (int i = 0; i < 4; i++) umma_ss<1>(tm + ACC_S, mn_desc(k + 2 * TILE + i * 2048, TILE), mn_desc(dd + i * 2048, TILE), K64, 1);
             umma_commit(&M.g3done);
+            n3++;
             ok = warp_wait(&M.pfull, c & 1);
             if (!ok) break;
 #pragma unroll
             for (int i = 0; i < 4; i++) umma_ss<1>(tm + ACC_P + (c & 1) * 64, smem_desc(pt + i * 32), mn_desc(d + i * 2048, TILE), W64, i > 0);
             umma_commit(&M.pdone);
+            np++;
         }
+        // (nor before its products are done: this warp gives the tensor memory back)
+        if (n1) warp_wait(&M.g1done, (n1 - 1) & 1);
+        if (n3) warp_wait(&M.g3done, (n3 - 1) & 1);
+        if (np) warp_wait(&M.pdone, (np - 1) & 1);
         if (!ok && lane == 0) atomicExch(err, 21);
         __syncwarp();
     } else {
