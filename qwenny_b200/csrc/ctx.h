@@ -103,3 +103,6 @@ size_t qb_delta_tp_bytes(int chunks);
 // the product for 17 .. 64 rows (w4a16_gemm_mid.cu), symmetric matrices; reached through qb_marlin_gemm
 int qb_gemm_mid_launch(qb_ctx* ctx, cudaStream_t st, const void* X, const void* B, void* Y, const void* S, int m, int n, int k,
                        int row0, int epi, const int* xrows, unsigned long long* keys, int n_valid);
+int qb_gemm_mid_gathers(const qb_ctx* ctx, int m, int k);  // whether it can take gathered rows: they are copied together first
+// the kernels that qb_marlin_gemm launches for m gathered rows
+int qb_marlin_gathered_launches(const qb_ctx* ctx, int m, int k);

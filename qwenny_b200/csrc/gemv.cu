@@ -254,6 +254,16 @@ static int gemm_rows(qb_ctx* ctx, cudaStream_t st, const void* X, const void* B,
 #undef QB_GO
 }
 
+int qb_marlin_gathered_launches(const qb_ctx* ctx, int m, int k) {
+    int launches = 0;
+    for (int mm; m > 0; m -= mm, launches++) {
+        mm = m < 64 ? m : 64;
+        if (mm > 16 && !ctx->no_tc && ctx->tc_part && qb_gemm_mid_gathers(ctx, mm, k)) launches++;
+        else if (mm > 16) mm = 16;
+    }
+    return launches;
+}
+
 extern "C" int qb_marlin_gemm(qb_ctx* ctx, void* stream, const void* X, const void* B, void* Y, const void* S, int m,
                               int n, int k, int row0, int epi, const int* xrows, unsigned long long* keys,
                               int n_valid) {
@@ -266,17 +276,17 @@ extern "C" int qb_marlin_gemm(qb_ctx* ctx, void* stream, const void* X, const vo
     if (m > 64 && epi != QB_EPI_ARGMAX && !xrows && !ctx->no_tc)
         return qb_gemm_tc_launch(ctx, st, X, B, Y, S, m, n, k, row0, epi, 0);
     // slabs: 17 .. 64 rows through the tensor-core product for a few rows, up to 16 through the skinny kernel. At 16 rows the
-    // skinny kernel takes 22, 11, 31 and 24 us over the layer's four shapes, at 17 the other 28, 20, 46 and 32 (two skinny
-    // slabs 43, 22, 62 and 48); 40 gathered rows of a 248,320-row output layer take 577 us as three 16-row slabs, 320 so.
+    // skinny kernel takes 22, 11, 31 and 24 us over the layer's four shapes, at 17 the other 20, 12, 33 and 20 (two skinny
+    // slabs 43, 22, 62 and 48); 40 gathered rows of a 248,320-row output layer take 577 us as three 16-row slabs, 218 so.
     // The upper bound is that of its tiles, not where times cross: the prompt-sized product has no gathered and no argmax
     // form, and it rounds each weight to f16, which is exact for bf16 scales only (error against 64 bits 5e-5; with the
-    // group's scale applied to the f32 sum 8e-7, as up to 16 rows). Where it could run it would be the faster one, by
-    // most at the first shape: 17 rows 23, 18, 45 and 31 us, 64 rows 24, 22, 47 and 34 against 32, 24, 52 and 36.
+    // group's scale applied to the f32 sum 8e-7, as up to 16 rows). At 17 rows it takes 23, 18, 45 and 31 us, at 64 24, 22, 47 and 34
+    // against 24, 15, 40 and 25.
     int mm;
     for (int r = 0; r < m; r += mm) {
         mm = m - r;
-        if (mm > 16 && !ctx->no_tc && ctx->tc_part) {
-            if (mm > 64) mm = 64;
+        if (mm > 64) mm = 64;
+        if (mm > 16 && !ctx->no_tc && ctx->tc_part && (!xrows || qb_gemm_mid_gathers(ctx, mm, k))) {
             int rc = qb_gemm_mid_launch(ctx, st, X, B, Y, S, mm, n, k, xrows ? 0 : row0 + r, epi, xrows ? xrows + r : nullptr,
                                         keys ? keys + (xrows ? r : 0) : nullptr, n_valid);
             if (rc) return rc;

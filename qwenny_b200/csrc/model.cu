@@ -328,7 +328,8 @@ int launch_mtp(qb_model* m, cudaStream_t st, bool own) {
         auto product = head && M.head_zero_points ? qb_marlin_gemm_z : qb_marlin_gemm;
         QB_TRY(product(c, s, m->xn, head ? M.head_w : m->lm_w, m->logits, head ? M.head_s : m->lm_s, m->n_out,
                        head ? M.head_rows : m->vocab_rows, H, 0, QB_EPI_ARGMAX, m->out_rows, m->keys,
-                       head ? M.head_valid : m->vocab_valid)); k++;
+                       head ? M.head_valid : m->vocab_valid));
+        k += head && M.head_zero_points ? (m->n_out + 15) / 16 : qb_marlin_gathered_launches(c, m->n_out, H);
     }
     m->step_kernels = k;
     return QB_OK;
@@ -359,7 +360,8 @@ int launch_step(qb_model* m, cudaStream_t st) {
     }
     if (m->n_out > 0) {
         QB_TRY(qb_marlin_gemm(c, s, m->xn, m->lm_w, m->logits, m->lm_s, m->n_out, m->vocab_rows, H, 0, QB_EPI_ARGMAX,
-                              m->out_rows, m->keys, m->vocab_valid)); k++;
+                              m->out_rows, m->keys, m->vocab_valid));
+        k += qb_marlin_gathered_launches(c, m->n_out, H);
     }
     m->step_kernels = k;
     return QB_OK;

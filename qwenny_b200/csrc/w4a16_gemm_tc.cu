@@ -57,7 +57,7 @@ struct Args {
     int bt, tiles;       // tokens per tile (a multiple of 32, at most BT), tiles
     float* part;         // [pair][2][block][BT][BH] partial tiles: [.][0] a share's first tile begun by an earlier pair, [.][1] its last, unfinished one
     int* tickets;        // two per tile (one per block of the pair), zero between launches
-    long long iters;     // tiles x k blocks
+    int iters;           // tiles x k blocks
     int zp;              // S holds a second table [K/128][N] after the scales: the offsets (8 - z) * scale of zero-point matrices
 };
 
@@ -354,7 +354,7 @@ int qb_gemm_tc_launch(qb_ctx* ctx, cudaStream_t st, const void* X, const void* B
     const int pairs = ctx->sms / 2;
     tc::Args a;
     a.S = (const __half*)S; a.Y = Y; a.m = m; a.N = n; a.K = k; a.row0 = row0; a.err = ctx->err;
-    a.zp = zp ? 1 : 0; a.part = ctx->tc_part; a.tickets = ctx->tc_tickets; a.iters = tiles * (k / tc::BK);
+    a.zp = zp ? 1 : 0; a.part = ctx->tc_part; a.tickets = ctx->tc_tickets; a.iters = (int)tiles * (k / tc::BK);
     a.bt = bt; a.tiles = (int)tiles;
     // One pair per tile (the hardware hands a freed pair of SMs the next tile) when the partly filled last wave wastes
     // less than a fifth of the time; otherwise one pair per two SMs and equal shares of the whole list, where a tile has
