@@ -455,13 +455,14 @@ attn_dec4_kernel(const float* q, const uint8_t* kc, const uint8_t* vc, const flo
     extern __shared__ __align__(128) uint8_t smem[];
     uint64_t* full = (uint64_t*)smem;
     uint64_t* empty = full + NSTG;
+    volatile int* issued = (volatile int*)(empty + NSTG);  // per slot: the stage whose copies were asked for last
     __half* qsh = (__half*)(smem + C::BAR_BYTES);
     uint8_t* xch = smem + C::BAR_BYTES + C::Q_BYTES;
     uint8_t* ring = xch + C::QUADS * C::X_BYTES;
 
     const int seg = blockIdx.x, g = blockIdx.y, s = blockIdx.z, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
-        for (int i = 0; i < NSTG; i++) { mbar_init(&full[i], 1); mbar_init(&empty[i], 4); }
+        for (int i = 0; i < NSTG; i++) { mbar_init(&full[i], 1); mbar_init(&empty[i], 4); issued[i] = 0; }
         mbar_fence_init();
     }
     __syncthreads();
@@ -507,7 +508,7 @@ attn_dec4_kernel(const float* q, const uint8_t* kc, const uint8_t* vc, const flo
             }
             uint8_t* base = ring + sl * STG_BYTES;
             const int kb = kbeg + j * SK;
-            if (lane == 0) mbar_expect_tx(&full[sl], STG_BYTES);
+            if (lane == 0) { mbar_expect_tx(&full[sl], STG_BYTES); issued[sl] = j; }
             __syncwarp();
             if (lane == 0) bulk_g2s(base, kh + (size_t)kb * HD, SK * HD, &full[sl], pol);
             if (lane == 1) bulk_g2s(base + SK * HD, vh + (size_t)kb * HD, SK * HD, &full[sl], pol);
@@ -569,7 +570,12 @@ attn_dec4_kernel(const float* q, const uint8_t* kc, const uint8_t* vc, const flo
         const int sl = j % NSTG;
         const uint32_t par = (j / NSTG) & 1;
         if (!dead) {
-            dead = !mbar_wait(&full[sl], par);
+            // A slot's stages go to different quads, and a parity says nothing to a waiter that is two phases behind: one whose slot still
+            // waits for its last stage's copies would be let through. A stage is asked for only when that one was consumed.
+            uint32_t polls = 0;
+            if (j >= NSTG)
+                while (issued[sl] != j && polls < WAIT_LIMIT) polls++;
+            dead = polls == WAIT_LIMIT || !mbar_wait(&full[sl], par);
             if (dead && lane == 0) atomicExch(err, 4);
         } else {
             for (int k = 0; k < 1024 && !mbar_try_wait(&full[sl], par); k++) {}

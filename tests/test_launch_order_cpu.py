@@ -36,3 +36,15 @@ def test_the_first_kernels_of_a_step_wait_before_they_let_others_start():
     assert len(first) == 2
     for name, body in first.items():
         assert 0 <= body.find("pdl_wait();") < body.find("pdl_launch_dependents();"), name
+
+
+def test_decode_attention_knows_its_stage_was_asked_for():
+    """The quads of a block share the ring's slots, so a quad may come to a slot whose last stage, another quad's, has not landed: the
+    parity of the stage it wants is then the parity of the phase before that one, and a wait on it ends at once. It looks first
+    whether its stage's copies were asked for (that is done once the slot's last stage has been consumed)."""
+    body = {name: body for _, name, body in kernels()}["attn_dec4_kernel"]
+    wait = body.index("mbar_wait(&full[sl]")
+    looks = body.rfind("while (issued[sl] != j", 0, wait)
+    assert looks > 0 and "if (j >= NSTG)" in body[looks - 60:looks]
+    asks = body.index("mbar_expect_tx(")
+    assert re.match(r"mbar_expect_tx\([^;]*\);\s*issued\[[^;]*= j;", body[asks:])
