@@ -415,29 +415,35 @@ attn_decode_kernel(const float* q, const uint8_t* kc, const uint8_t* vc, const f
 }
 
 // ------------------------------------------------------------------------------------------------ decode attention
-// Block (short segment, kv head, key split) of the decode / verify attention: 2 to 4 QUADS of four compute warps and a
-// copy warp. The keys and values of the split arrive in 64-key stages through a ring fed by bulk copies; the quads
-// take the stages in turn. Inside a quad the work of a stage is dealt so that no byte is converted twice:
+// Block (short segment, kv head, key split) of the decode / verify attention: 2 or 4 QUADS of four warps. The keys and values of the
+// split arrive in 64-key stages through a ring fed by bulk copies; the quads take the stages in turn. Inside a quad the work
+// of a stage is dealt so that no byte is converted twice:
 //   scores   warp w multiplies all the rows (RT tiles of 16 (token, head) rows) by the keys 16 w .. 16 w + 15 of the
 //            stage over the whole head dimension: one conversion of a key serves every row tile;
-//   softmax  the four warps agree on the rows' running maxima through shared memory, so that all of them scale by the
-//            same power of two, and exchange their 16-key slices of P (as f16 mma fragments); a lane keeps the sums of its
-//            own keys to the end;
+//   softmax  P = 2^(score - m) for a reference m per row that the quad shares. It moves, to the largest score so far, only when P times
+//            a value's scale comes near the end of f16: the warps tell one another with the barrier that hands over their 16-key slices of P (as f16
+//            mma fragments), so that most stages have one barrier and rescale nothing (maxima exchanged in every stage: two barriers, and
+//            30 rows' accumulators rescaled in nearly all of them). A lane keeps the sums of its own keys to the end;
 //   values   warp w accumulates the output dims 64 w .. 64 w + 63 over all 64 keys of the stage (for every row tile),
 //            so the output accumulators of a row are spread over four warps (RT x 32 registers each).
 // The int8 codes go to the tensor cores as 1152 + q halves (one prmt per pair) and the offset is folded out through the
-// row sums, as in the reference (kernels/attn.cuh:38-40,198-234). The four quads' partial results meet in shared memory
+// row sums, as in the reference (kernels/attn.cuh:38-40,198-234). The quads' partial results meet in shared memory
 // at the end; the block writes one (m, l, acc) partial per row, or the finished rows when the segment has one split.
+// Bound by latency: at 5 rows a quad's stage takes 4400 cycles (scores 1400, softmax and barrier 1050, values 1100, waits and copies 700) with
+// two warps per scheduler, and a block 3000 before its first stage behind the kernel before, 3000 after its last. From a graph with
+// attn_prep and the combine, us, before (a copy warp, maxima in every stage, Q row by row) / now: 5 rows at 100 keys 13.5 / 11.2, at 4000
+// 18.4 / 15.1, at 32000 35.0 / 30.5; 1 row at 32000 26.2 / 24.1; 8 rows 50.6 / 40.2 (registers spilled before); 8 sequences of 4 rows at 972
+// to 7777 66.5 / 59.7, at 4000 to 32000 140 / 128.5.
 template <int RT, int NQ>
 struct Dec4Cfg {
-    static constexpr int QUADS = NQ, CW = 4 * QUADS;   // compute warps
-    static constexpr int THREADS = (CW + 1) * 32;       // + the copy warp
-    static constexpr int SK = 64, NSTG = 5;             // keys per stage, ring depth
+    static constexpr int QUADS = NQ, CW = 4 * QUADS, THREADS = CW * 32;
+    static constexpr int SK = 64, NSTG = NQ > 2 ? 6 : 5;  // keys per stage, ring depth
     static constexpr int STG_BYTES = SK * HD * 2 + SK * 8;
     static constexpr int Q_BYTES = RT * 16 * SROW * 2;
-    // per quad: the warps' row maxima [4][RT][16], their P fragments [4][RT][32 lanes] x 16 B, their (sum, ps) [4][RT][16][2]
-    static constexpr int X_MAX = 4 * RT * 16 * 4, X_P = 4 * RT * 32 * 16, X_SUM = 4 * RT * 16 * 8;
-    static constexpr int X_BYTES = X_MAX + X_P + X_SUM;
+    // per quad: the warps' row maxima (and whether a row has left its reference) [4][RT][16], their P fragments, of two stages in turn, [2][4][RT][32 lanes] x 16 B, their (sum,
+    // ps) [4][RT][16][2]
+    static constexpr int X_MAX = 4 * RT * 16 * 8, X_P = 4 * RT * 32 * 16, X_SUM = 4 * RT * 16 * 8;
+    static constexpr int X_BYTES = X_MAX + 2 * X_P + X_SUM;
     static constexpr int BAR_BYTES = 128;
     static constexpr int SMEM = BAR_BYTES + Q_BYTES + QUADS * X_BYTES + NSTG * STG_BYTES;
     static constexpr int MERGE_BYTES = 8 * 32 * (RT * 8 * 4 + RT * 6) * 4;   // two quads' registers at a time
@@ -454,15 +460,14 @@ attn_dec4_kernel(const float* q, const uint8_t* kc, const uint8_t* vc, const flo
     constexpr int NSTG = C::NSTG, SK = C::SK, STG_BYTES = C::STG_BYTES;
     extern __shared__ __align__(128) uint8_t smem[];
     uint64_t* full = (uint64_t*)smem;
-    uint64_t* empty = full + NSTG;
-    volatile int* issued = (volatile int*)(empty + NSTG);  // per slot: the stage whose copies were asked for last
+    volatile int* issued = (volatile int*)(full + NSTG);  // per slot: the stage whose copies were asked for last
     __half* qsh = (__half*)(smem + C::BAR_BYTES);
     uint8_t* xch = smem + C::BAR_BYTES + C::Q_BYTES;
     uint8_t* ring = xch + C::QUADS * C::X_BYTES;
 
     const int seg = blockIdx.x, g = blockIdx.y, s = blockIdx.z, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
-        for (int i = 0; i < NSTG; i++) { mbar_init(&full[i], 1); mbar_init(&empty[i], 4); issued[i] = 0; }
+        for (int i = 0; i < NSTG; i++) { mbar_init(&full[i], 1); issued[i] = 0; }
         mbar_fence_init();
     }
     __syncthreads();
@@ -472,84 +477,87 @@ attn_dec4_kernel(const float* q, const uint8_t* kc, const uint8_t* vc, const flo
     // ends `old_margin` positions or more before the segment's last key (0: nothing is read ahead, the first stages are only
     // asked into L2).
     const int first = dseg[2 * seg], nt = dseg[2 * seg + 1];
-    const int tlast = dtok[first + nt - 1], keys = tok_pos[tlast] + 1;
+    const int my_tok = dtok[first + min(lane, nt - 1)], my_pos = tok_pos[my_tok];  // lane i: the segment's token i
+    const int tlast = __shfl_sync(0xffffffffu, my_tok, nt - 1), keys = __shfl_sync(0xffffffffu, my_pos, nt - 1) + 1;
     const int chunk = dec_chunk(keys, dsplits), ns = (keys + chunk - 1) / chunk;
     if (s >= ns) return;
     const int kbeg = s * chunk, ke = min(keys, kbeg + chunk), nstg = (ke - kbeg + SK - 1) / SK;
-    const int slot = tok_slot[tlast];
 
-    if (warp == C::CW) {
-        // ------------------------------------------------------------ the copy warp
-        const uint64_t pol = policy_evict_first();
-        const uint8_t* kh = kc + cache_head(slot, g, cap);
-        const uint8_t* vh = vc + cache_head(slot, g, cap);
-        const float* ksh = ks + scale_head(slot, g, cap);
-        const float* vsh = vs + scale_head(slot, g, cap);
-        bool waited = false;
-        if (old_margin <= 0 && lane < min(nstg, NSTG)) {
-            const size_t at = (size_t)(kbeg + lane * SK) * HD;
-            bulk_prefetch(kh + at, SK * HD);
-            bulk_prefetch(vh + at, SK * HD);
-        }
-        for (int j = 0; j < nstg; j++) {
-            const int sl = j % NSTG;
-            if (!waited && (old_margin <= 0 || kbeg + (j + 1) * SK > keys - old_margin)) {
-                pdl_wait();
-                waited = true;
-            }
-            if (j >= NSTG) {
-                bool ok = true;
-                if (lane == 0) ok = mbar_wait(&empty[sl], ((j / NSTG) - 1) & 1);
-                ok = __shfl_sync(0xffffffffu, ok, 0);
-                if (!ok) {
-                    if (lane == 0) atomicExch(err, 3);
-                    return;
-                }
-            }
-            uint8_t* base = ring + sl * STG_BYTES;
-            const int kb = kbeg + j * SK;
-            if (lane == 0) { mbar_expect_tx(&full[sl], STG_BYTES); issued[sl] = j; }
-            __syncwarp();
-            if (lane == 0) bulk_g2s(base, kh + (size_t)kb * HD, SK * HD, &full[sl], pol);
-            if (lane == 1) bulk_g2s(base + SK * HD, vh + (size_t)kb * HD, SK * HD, &full[sl], pol);
-            if (lane == 2) bulk_g2s(base + 2 * SK * HD, ksh + kb, SK * 4, &full[sl], pol);
-            if (lane == 3) bulk_g2s(base + 2 * SK * HD + SK * 4, vsh + kb, SK * 4, &full[sl], pol);
-        }
-        return;
-    }
-
-    // ---------------------------------------------------------------- compute warps
+    // ---- the copies of a stage, its keys, values and scales, are shared out among the warps, at the start among all and later among a
+    // quad's (by one warp they take 690 cycles, which the others would wait for), behind a barrier of the warps before which the stage's
+    // own is armed. (A copy warp would be a third warp of one scheduler, and leave the others 168 registers instead of 255.)
     const int quad = warp >> 2, w = warp & 3, r = lane >> 2, t4 = lane & 3;
-    constexpr int NCW = C::CW * 32;
-    pdl_wait();  // q and the gates come from this step's attn_prep
-    // Q of the segment's rows (row = token * GROUP + head) as f16
-    for (int x = threadIdx.x; x < RT * 16 * HD / 4; x += NCW) {
-        const int row = x / (HD / 4), d = (x % (HD / 4)) * 4, tok = row / GROUP;
-        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (tok < nt) v = *(const float4*)(q + ((size_t)dtok[first + tok] * NH + g * GROUP + row % GROUP) * HD + d);
-        *(uint2*)&qsh[row * SROW + d] = make_uint2(pack_half2(v.x, v.y), pack_half2(v.z, v.w));
+    constexpr int NCW = C::THREADS;
+    const int slot = tok_slot[tlast];
+    const uint64_t pol = policy_evict_first();
+    auto copy = [&](int j, int part) {
+        const uint8_t* from = part == 0 ? kc + cache_head(slot, g, cap) + (size_t)kbeg * HD : part == 1 ? vc + cache_head(slot, g, cap) + (size_t)kbeg * HD
+                              : (const uint8_t*)((part == 2 ? ks : vs) + scale_head(slot, g, cap) + kbeg);
+        const uint32_t bytes = part < 2 ? SK * HD : SK * 4, at = part < 2 ? part * SK * HD : 2 * SK * HD + (part - 2) * SK * 4;
+        bulk_g2s(ring + (j % NSTG) * STG_BYTES + at, from + (size_t)j * bytes, bytes, &full[j % NSTG], pol);
+    };
+    auto arm = [&](int j) {
+        mbar_expect_tx(&full[j % NSTG], STG_BYTES);
+        issued[j % NSTG] = j;
+    };
+    const int begin = min(nstg, NSTG);
+    if (warp < begin && lane == 0) arm(warp);
+    named_bar_sync(1, NCW);
+    auto ask = [&](bool ahead) {  // the first stages
+        for (int x = warp; x < 4 * begin; x += C::CW) {
+            const bool old = old_margin > 0 && kbeg + ((x >> 2) + 1) * SK <= keys - old_margin;
+            if (old == ahead && lane == 0) copy(x >> 2, x & 3);
+        }
+        __syncwarp();
+    };
+    if (old_margin > 0)
+        ask(true);
+    else if (warp < begin && lane < 2)
+        bulk_prefetch((lane ? vc : kc) + cache_head(slot, g, cap) + (size_t)(kbeg + warp * SK) * HD, SK * HD);
+    pdl_wait();  // q, the gates and the step's own keys and values come from its attn_prep
+    // Q of the segment's rows (row = token * GROUP + head) as f16, and KV_OFF times each row's sum of those (a row's 64 threads: two
+    // warps). All of a thread's loads are under way together: one after the other, behind the token's own load, they took 4 us.
+    float2* xmax = (float2*)(xch + quad * C::X_BYTES);               // [4][RT][16]
+    uint8_t* xp_at = xch + quad * C::X_BYTES + C::X_MAX;             // [2][4][RT][32] x 16 B
+    float2* xsum = (float2*)(xch + quad * C::X_BYTES + C::X_MAX + 2 * C::X_P);  // [4][RT][16]
+    float* qsum = (float*)(xch + C::X_MAX);  // [RT * 16][2]: where the first quad's P goes later
+    {
+        constexpr int PER = RT * 16 * HD / 4 / NCW, RSTEP = NCW / (HD / 4);  // float4 per thread, rows at a time
+        const int r0 = threadIdx.x / (HD / 4), d = (threadIdx.x % (HD / 4)) * 4;
+        float4 v[PER];
+#pragma unroll
+        for (int i = 0; i < PER; i++) {
+            const int row = r0 + i * RSTEP, tok = row / GROUP;
+            const int t = __shfl_sync(0xffffffffu, my_tok, min(tok, nt - 1));
+            v[i] = tok < nt ? *(const float4*)(q + ((size_t)t * NH + g * GROUP + row % GROUP) * HD + d) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+        ask(false);
+#pragma unroll
+        for (int i = 0; i < PER; i++) {
+            const int row = r0 + i * RSTEP;
+            const uint2 h = make_uint2(pack_half2(v[i].x, v[i].y), pack_half2(v[i].z, v[i].w));
+            *(uint2*)&qsh[row * SROW + d] = h;
+            const float2 f0 = __half22float2(*(const __half2*)&h.x), f1 = __half22float2(*(const __half2*)&h.y);
+            const float sum = warp_sum((f0.x + f0.y) + (f1.x + f1.y));
+            if (lane == 0) qsum[row * 2 + (warp & 1)] = sum;
+        }
     }
     named_bar_sync(1, NCW);
     // this lane's rows 16 rt + r and + 8: the keys they may see end at lim; KV_OFF times the sums of their Q
-    int lim[RT][2];
+    int lim[RT][2], all_see = ke;  // (keys below all_see are seen by every row of the segment)
     float qoff[RT][2];
 #pragma unroll
-    for (int rt = 0; rt < RT; rt++) {
-        float qs = 0.f;
-        const __half* qr = qsh + (rt * 16 + (lane & 15)) * SROW + (lane >> 4) * (HD / 2);
-        for (int d = 0; d < HD / 2; d += 2) {
-            const float2 f = __half22float2(*(const __half2*)(qr + d));
-            qs += f.x + f.y;
-        }
-        qs += __shfl_xor_sync(0xffffffffu, qs, 16);
-        qoff[rt][0] = KV_OFF * __shfl_sync(0xffffffffu, qs, r);
-        qoff[rt][1] = KV_OFF * __shfl_sync(0xffffffffu, qs, r + 8);
+    for (int rt = 0; rt < RT; rt++)
 #pragma unroll
         for (int h2 = 0; h2 < 2; h2++) {
-            const int tok = (rt * 16 + r + 8 * h2) / GROUP;
-            lim[rt][h2] = tok < nt ? min(ke, tok_pos[dtok[first + tok]] + 1) : 0;
+            const int row = rt * 16 + r + 8 * h2, tok = row / GROUP;
+            const float2 x = *(const float2*)&qsum[row * 2];
+            qoff[rt][h2] = KV_OFF * (x.x + x.y);
+            const int p = __shfl_sync(0xffffffffu, my_pos, min(tok, nt - 1));
+            lim[rt][h2] = tok < nt ? min(ke, p + 1) : 0;
         }
-    }
+    all_see = min(all_see, __reduce_min_sync(0xffffffffu, my_pos) + 1);
+    // m: the rows' reference, a power of two that scores are taken from; -inf until a key was seen
     float m[RT][2], l[RT][2], ps[RT][2], o[RT][8][4];
 #pragma unroll
     for (int rt = 0; rt < RT; rt++) {
@@ -561,9 +569,7 @@ attn_dec4_kernel(const float* q, const uint8_t* kc, const uint8_t* vc, const flo
     uint32_t qa[RT];
 #pragma unroll
     for (int rt = 0; rt < RT; rt++) qa[rt] = smem_u32(qsh + (rt * 16 + (lane & 15)) * SROW + (lane >> 4) * 8);
-    float* xmax = (float*)(xch + quad * C::X_BYTES);                 // [4][RT][16]
-    uint4* xp = (uint4*)(xch + quad * C::X_BYTES + C::X_MAX);        // [4][RT][32]
-    float2* xsum = (float2*)(xch + quad * C::X_BYTES + C::X_MAX + C::X_P);  // [4][RT][16]
+    named_bar_sync(1, NCW);  // (the sums of Q have been read)
 
     bool dead = false;
     for (int j = quad; j < nstg; j += C::QUADS) {
@@ -580,11 +586,15 @@ attn_dec4_kernel(const float* q, const uint8_t* kc, const uint8_t* vc, const flo
         } else {
             for (int k = 0; k < 1024 && !mbar_try_wait(&full[sl], par); k++) {}
         }
+        // two quads: the slot of the quad's stage before this one is filled again in the middle of this one
+        const bool refill = C::QUADS == 2 && j >= 2 && j - 2 + NSTG < nstg;
+        if (refill && w == 0 && lane == 0) arm(j - 2 + NSTG);
         const uint8_t* base = ring + sl * STG_BYTES;
         const int kb = kbeg + j * SK + 16 * w;  // this warp's 16 keys of the stage
         const uint8_t* kp = base + (16 * w + r) * HD + 16 * t4;
         const float* ksc_s = (const float*)(base + 2 * SK * HD) + 16 * w;
         const float* vsc_s = ksc_s + SK;
+        const bool whole = kbeg + (j + 1) * SK <= all_see;  // every row sees every key of the stage
         float ksc[2][2], vsc[2][2];
 #pragma unroll
         for (int nn = 0; nn < 2; nn++)
@@ -596,11 +606,11 @@ attn_dec4_kernel(const float* q, const uint8_t* kc, const uint8_t* vc, const flo
                 vsc[nn][e] = in ? vsc_s[kk] : 0.f;
             }
         // ---- scores: S = Q K^T for every row tile, this warp's 16 keys
-        float sacc[RT][2][4];
+        float v[RT][2][4];
 #pragma unroll
         for (int rt = 0; rt < RT; rt++)
 #pragma unroll
-            for (int nn = 0; nn < 2; nn++) sacc[rt][nn][0] = sacc[rt][nn][1] = sacc[rt][nn][2] = sacc[rt][nn][3] = 0.f;
+            for (int nn = 0; nn < 2; nn++) v[rt][nn][0] = v[rt][nn][1] = v[rt][nn][2] = v[rt][nn][3] = 0.f;
 #pragma unroll
         for (int b = 0; b < HD / 64; b++) {
             const uint4 kf0 = *(const uint4*)(kp + 64 * b), kf1 = *(const uint4*)(kp + 8 * HD + 64 * b);
@@ -613,88 +623,109 @@ attn_dec4_kernel(const float* q, const uint8_t* kc, const uint8_t* vc, const flo
                 for (int rt = 0; rt < RT; rt++) {
                     uint32_t a[4];
                     ldsm_x4(a[0], a[1], a[2], a[3], qa[rt] + (b * 64 + st * 16) * 2);
-                    mma16816(sacc[rt][0], a, b00, b01);
-                    mma16816(sacc[rt][1], a, b10, b11);
+                    mma16816(v[rt][0], a, b00, b01);
+                    mma16816(v[rt][1], a, b10, b11);
                 }
             }
         }
-        // ---- the rows' maxima over this warp's keys, then over the quad's
-        float v[RT][2][4];
+        // ---- the scores proper
 #pragma unroll
         for (int rt = 0; rt < RT; rt++)
 #pragma unroll
-            for (int h2 = 0; h2 < 2; h2++) {
-                float mx = -INFINITY;
+            for (int nn = 0; nn < 2; nn++)
 #pragma unroll
-                for (int nn = 0; nn < 2; nn++)
+                for (int x = 0; x < 4; x++) {
+                    float& sv = v[rt][nn][x];
+                    sv = (sv - qoff[rt][x >> 1]) * ksc[nn][x & 1];
+                    if (!whole && kb + 8 * nn + 2 * t4 + (x & 1) >= lim[rt][x >> 1]) sv = -INFINITY;
+                }
+        // ---- P of this warp's keys (times the value scales, rounded to f16 as the products see it) and its row sums. The first time
+        // with the references as they are; where a row has left its own (P times a value scale near the end of f16, or P past 2^24), and
+        // in the quad's first stage, once more with new ones.
+        uint4* xp = (uint4*)(xp_at + (j / C::QUADS & 1) * C::X_P);  // (a warp may still be reading the stage before's)
+        float sum[RT][2], pr[RT][2];
+#pragma unroll 1
+        for (bool again = false;; again = true) {
+            bool left[RT][2], any_left = j == quad;
 #pragma unroll
-                    for (int e = 0; e < 2; e++) {
-                        const int k = kb + 8 * nn + 2 * t4 + e;
-                        const float sv = k < lim[rt][h2] ? (sacc[rt][nn][2 * h2 + e] - qoff[rt][h2]) * ksc[nn][e] : -INFINITY;
-                        v[rt][nn][2 * h2 + e] = sv;
-                        mx = fmaxf(mx, sv);
-                    }
-                mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
-                mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
-                if (t4 == 0) xmax[(w * RT + rt) * 16 + r + 8 * h2] = mx;
+            for (int rt = 0; rt < RT; rt++) {
+                float pv[2][4];
+#pragma unroll
+                for (int h2 = 0; h2 < 2; h2++) {
+                    const float mm = m[rt][h2] == -INFINITY ? 0.f : m[rt][h2];
+                    sum[rt][h2] = 0.f;
+#pragma unroll
+                    for (int nn = 0; nn < 2; nn++)
+#pragma unroll
+                        for (int e = 0; e < 2; e++) {
+                            const float pp = tc::ex2(v[rt][nn][2 * h2 + e] - mm);
+                            sum[rt][h2] += pp;
+                            pv[nn][2 * h2 + e] = pp * vsc[nn][e];
+                        }
+                    left[rt][h2] = fmaxf(fmaxf(pv[0][2 * h2], pv[0][2 * h2 + 1]), fmaxf(pv[1][2 * h2], pv[1][2 * h2 + 1])) > 32768.f || sum[rt][h2] > 0x1p24f;
+                    any_left |= left[rt][h2];
+                }
+                uint4 pa;
+                pa.x = pack_half2(pv[0][0], pv[0][1]); pa.y = pack_half2(pv[0][2], pv[0][3]);
+                pa.z = pack_half2(pv[1][0], pv[1][1]); pa.w = pack_half2(pv[1][2], pv[1][3]);
+                xp[(w * RT + rt) * 32 + lane] = pa;
+                const float2 f0 = __half22float2(*(const __half2*)&pa.x), f1 = __half22float2(*(const __half2*)&pa.y);
+                const float2 f2 = __half22float2(*(const __half2*)&pa.z), f3 = __half22float2(*(const __half2*)&pa.w);
+                pr[rt][0] = f0.x + f0.y + f2.x + f2.y;
+                pr[rt][1] = f1.x + f1.y + f3.x + f3.y;
             }
-        named_bar_sync(2 + quad, 128);
-        float corr[RT][2];
-        bool grew = false;
-#pragma unroll
-        for (int rt = 0; rt < RT; rt++)
-#pragma unroll
-            for (int h2 = 0; h2 < 2; h2++) {
-                float mn = m[rt][h2];
-#pragma unroll
-                for (int ww = 0; ww < 4; ww++) mn = fmaxf(mn, xmax[(ww * RT + rt) * 16 + r + 8 * h2]);
-                corr[rt][h2] = mn == -INFINITY ? 1.f : exp2f(m[rt][h2] - mn);
-                m[rt][h2] = mn;
-                grew |= corr[rt][h2] != 1.f;
+            if (again) {
+                named_bar_sync(2 + quad, 128);
+                break;
             }
-        // ---- P of this warp's keys (times the value scales, rounded to f16 as the products see it) and its row sums
-#pragma unroll
-        for (int rt = 0; rt < RT; rt++) {
-            float pv[2][4], sum[2];
-#pragma unroll
-            for (int h2 = 0; h2 < 2; h2++) {
-                sum[h2] = 0.f;
-#pragma unroll
-                for (int nn = 0; nn < 2; nn++)
-#pragma unroll
-                    for (int e = 0; e < 2; e++) {
-                        const float sv = v[rt][nn][2 * h2 + e];
-                        const float pp = sv == -INFINITY ? 0.f : tc::ex2(sv - m[rt][h2]);
-                        sum[h2] += pp;
-                        pv[nn][2 * h2 + e] = pp * vsc[nn][e];
-                    }
-            }
-            uint4 pa;
-            pa.x = pack_half2(pv[0][0], pv[0][1]); pa.y = pack_half2(pv[0][2], pv[0][3]);
-            pa.z = pack_half2(pv[1][0], pv[1][1]); pa.w = pack_half2(pv[1][2], pv[1][3]);
-            xp[(w * RT + rt) * 32 + lane] = pa;
-            __half2 h0, h1, h2v, h3;
-            *(uint32_t*)&h0 = pa.x; *(uint32_t*)&h1 = pa.y; *(uint32_t*)&h2v = pa.z; *(uint32_t*)&h3 = pa.w;
-            const float2 f0 = __half22float2(h0), f1 = __half22float2(h1), f2 = __half22float2(h2v), f3 = __half22float2(h3);
-            const float pr[2] = {f0.x + f0.y + f2.x + f2.y, f1.x + f1.y + f3.x + f3.y};
-            // a lane sums its own keys; lanes and warps are added up once, after the last stage (added up in every stage the
-            // shuffles and the exchange were some 700 of a stage's 6100 cycles)
-#pragma unroll
-            for (int h2 = 0; h2 < 2; h2++) {
-                l[rt][h2] = l[rt][h2] * corr[rt][h2] + sum[h2];
-                ps[rt][h2] = ps[rt][h2] * corr[rt][h2] + pr[h2];
-            }
-        }
-        named_bar_sync(2 + quad, 128);
-        if (__any_sync(0xffffffffu, grew)) {
+            if (!named_bar_or(2 + quad, 128, any_left)) break;
 #pragma unroll
             for (int rt = 0; rt < RT; rt++)
 #pragma unroll
-                for (int jd = 0; jd < 8; jd++) {
-                    o[rt][jd][0] *= corr[rt][0]; o[rt][jd][1] *= corr[rt][0];
-                    o[rt][jd][2] *= corr[rt][1]; o[rt][jd][3] *= corr[rt][1];
+                for (int h2 = 0; h2 < 2; h2++) {
+                    float x = fmaxf(fmaxf(v[rt][0][2 * h2], v[rt][0][2 * h2 + 1]), fmaxf(v[rt][1][2 * h2], v[rt][1][2 * h2 + 1]));
+                    x = fmaxf(x, __shfl_xor_sync(0xffffffffu, x, 1));
+                    x = fmaxf(x, __shfl_xor_sync(0xffffffffu, x, 2));
+                    const bool lf = (__ballot_sync(0xffffffffu, left[rt][h2]) >> (4 * r) & 15) != 0;
+                    if (t4 == 0) xmax[(w * RT + rt) * 16 + r + 8 * h2] = make_float2(x, lf ? 1.f : 0.f);
                 }
+            named_bar_sync(2 + quad, 128);
+#pragma unroll
+            for (int rt = 0; rt < RT; rt++) {
+                float corr[2];
+#pragma unroll
+                for (int h2 = 0; h2 < 2; h2++) {
+                    float mn = m[rt][h2];
+                    bool moves = j == quad;
+#pragma unroll
+                    for (int ww = 0; ww < 4; ww++) {
+                        const float2 x = xmax[(ww * RT + rt) * 16 + r + 8 * h2];
+                        mn = fmaxf(mn, x.x);
+                        moves |= x.y != 0.f;
+                    }
+                    moves &= mn > m[rt][h2];  // (it depends on the row's own scores alone, not on what else is in the step)
+                    corr[h2] = moves ? exp2f(m[rt][h2] - mn) : 1.f;
+                    if (moves) m[rt][h2] = mn;
+                    l[rt][h2] *= corr[h2];
+                    ps[rt][h2] *= corr[h2];
+                }
+#pragma unroll
+                for (int jd = 0; jd < 8; jd++) {
+                    o[rt][jd][0] *= corr[0]; o[rt][jd][1] *= corr[0];
+                    o[rt][jd][2] *= corr[1]; o[rt][jd][3] *= corr[1];
+                }
+            }
         }
+        // (a lane sums its own keys; lanes and warps are added up once, after the last stage)
+#pragma unroll
+        for (int rt = 0; rt < RT; rt++)
+#pragma unroll
+            for (int h2 = 0; h2 < 2; h2++) {
+                l[rt][h2] += sum[rt][h2];
+                ps[rt][h2] += pr[rt][h2];
+            }
+        // (the barrier above: all of the quad is done with its stage before this one, and the slot's barrier is armed)
+        if (refill && lane == 0) copy(j - 2 + NSTG, w);
         // ---- values: O += P V over the stage's 64 keys, this warp's 64 output dims
 #pragma unroll
         for (int kbk = 0; kbk < 4; kbk++) {
@@ -713,8 +744,11 @@ attn_dec4_kernel(const float* q, const uint8_t* kc, const uint8_t* vc, const flo
                 for (int rt = 0; rt < RT; rt++) mma16816(o[rt][jd], pa[rt], b0, b1);
             }
         }
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&empty[sl]);
+        if (C::QUADS > 2 && j + NSTG < nstg) {  // (few stages more than quads: the next stage's barrier would be late)
+            if (w == 0 && lane == 0) arm(j + NSTG);
+            named_bar_sync(2 + quad, 128);
+            if (lane == 0) copy(j + NSTG, w);
+        }
     }
 
     // ---- the quads merge pairwise through the ring, which is free (every stage was consumed): 1 -> 0 and 3 -> 2, then
@@ -941,7 +975,7 @@ int qb_attn_decode_as(qb_ctx* ctx, void* stream, const float* q, const void* kc,
                     part_acc, out, ctx->err);                                                                             \
     }
     // quads per block: as many as leave every warp its registers (a warp holds RT x 32 output accumulators per lane);
-    // measured at 5 rows: 2 quads 33.4 us, 3 quads (spills) 36.6 us, 4 quads 43.2 us
+    // measured at 5 rows with a copy warp beside them: 2 quads 33.4 us, 3 quads (spills) 36.6 us, 4 quads 43.2 us
     if (rt == 1) QB_DEC(1, 4) else if (rt == 2) QB_DEC(2, 2) else QB_DEC(3, 2)
 #undef QB_DEC
     if (rc) return rc;

@@ -221,6 +221,14 @@ __device__ __forceinline__ void named_bar_sync(int id, int threads) {
     asm volatile("bar.sync %0, %1;\n" ::"r"(id), "r"(threads) : "memory");
 }
 
+// the same barrier, and whether p holds in any of its threads
+__device__ __forceinline__ bool named_bar_or(int id, int threads, bool p) {
+    uint32_t any;
+    asm volatile("{\n.reg .pred p, q;\nsetp.ne.u32 p, %3, 0;\nbar.red.or.pred q, %1, %2, p;\nselp.u32 %0, 1, 0, q;\n}\n"
+                 : "=r"(any) : "r"(id), "r"(threads), "r"((uint32_t)p) : "memory");
+    return any != 0;
+}
+
 // ---------------------------------------------------------------- global loads that bypass L1 (data another CTA
 // wrote during this kernel)
 __device__ __forceinline__ float4 ld_cg4(const float4* p) { return __ldcg(p); }

@@ -282,6 +282,36 @@ def test_attn_prefill_runs_of_tiles(ctx, lens, pos0):
     assert close(a[rows], want).all()
 
 
+@pytest.mark.parametrize("rows,vmax", [(2, 0.05), (5, 0.05), (5, 6.0), (8, 0.05)])
+def test_attn_decode_references_that_move(ctx, rows, vmax):
+    """Splits of several stages whose scores rise from stage to stage for some rows and fall for others (past what a row's reference
+    allows, f16's 2^15 over the value's scale), with value scales of 0 among them and up to 6: the oracle's values, and a
+    row's bits do not depend on the other rows' references (as many row tiles, other rows). P is f16 relative to any reference, so the
+    tolerance is the one of the other cases; its absolute part is for values of scale 0.05 and grows with theirs."""
+    g = synth.gen(161 + rows)
+    cap, pos0 = 16384, 15990
+    kc, vc, ks, vs = make_cache(1, cap, g, 0)
+    at = torch.arange(cap).repeat(R.NKV)
+    ks = 0.01 + 0.2 * (at % 640) / 640.0  # (a split of 448 keys sees it rise, or rise and start again)
+    vs = torch.rand(R.NKV * cap, generator=g) * vmax
+    vs[at % 640 > 600] = 0.0
+    cache = [t.cuda() for t in (kc, vc, ks.float(), vs.float())]
+    q = torch.randn(rows, R.NH, R.HD, generator=g) * QSCALE * torch.linspace(0.1, 2.0, R.NH)[None, :, None]
+    gate = torch.sigmoid(torch.randn(rows, R.MIX, generator=g))
+    toks = [(0, 0, pos0 + i) for i in range(rows)]
+    st = R.build_step(toks, list(range(rows)))
+    dv = ref_cuda.upload_step(st)
+    got = run_decode(ctx, q.cuda(), gate.cuda(), cache, st, dv, cap, rows)
+    want = R.attn_decode(q.numpy(), gate.numpy(), *[t.cpu().numpy() for t in cache], st["tok_slot"], st["tok_pos"], cap)
+    a, b = got.cpu().numpy(), want
+    assert (np.abs(a - b) <= ATOL * max(1.0, vmax / 0.05) + RTOL * np.abs(b)).all()
+    other = q.clone()
+    other[1:] = other[1:] * 3 + 1
+    again = run_decode(ctx, other.cuda(), gate.cuda(), cache, st, dv, cap, rows)
+    assert torch.equal(again[0], got[0])
+    assert ctx.device_error() == 0
+
+
 @pytest.mark.parametrize("rows", [1, 4, 8])
 def test_attn_decode_of_a_ragged_batch(ctx, rows):
     """A batch of ragged sequences gives each token the bits that its sequence alone gives, and the oracle's values: also where
