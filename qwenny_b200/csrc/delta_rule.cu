@@ -718,20 +718,19 @@ delta_scan_kernel(const float* p, int splits, int n, const float* cv, uint8_t* t
         auto sbuf = [&](int b) { return sm0 + (size_t)b * SLOT_STATE + ((size_t)h * LVD + col) * LKD; };
         auto entry = [&](int b, int pos) { return sm0 + 2 * SLOT_STATE + (size_t)b * SLOT_BANK + (size_t)(pos % KEEP) * REP; };
         auto sync = [] { named_bar_sync(1, SC_THREADS); };
-        constexpr int RPT = LKD / 8;
         // ---- the state, and the replay of accepted tokens from the bank
         float S[RPT];
         if (pl.zero) {
 #pragma unroll
             for (int i = 0; i < RPT; i++) S[i] = 0.f;
         } else {
-            ld_rows<8>(S, sbuf(pl.in), sub);
+            ld_rows(S, sbuf(pl.in), sub);
         }
         for (int i = 0; i < pl.r; i++) {
             const float* e = entry(pl.in, pl.from + i);
             float k[RPT];
-            ld_rows<8>(k, e + kh * LKD, sub);
-            const float dk = dot_rows<8>(S, k);
+            ld_rows(k, e + kh * LKD, sub);
+            const float dk = dot_rows(S, k);
             const float ex = e[LK_HEADS * LKD + LV_HEADS * LVD + h], be = e[LK_HEADS * LKD + LV_HEADS * LVD + LV_HEADS + h];
             const float delta = (e[LK_HEADS * LKD + h * LVD + col] - ex * dk) * be;
 #pragma unroll
@@ -797,7 +796,7 @@ delta_scan_kernel(const float* p, int splits, int n, const float* cv, uint8_t* t
                 for (int ch = 0; ch < 2; ch++) put(M.o.s[0], M.o.s[1], key, ch, st + 8 * ch, s);
                 arrive(&M.sready);
             };
-            st_rows<8>(&M.state[lc][0], S, sub);
+            st_rows(&M.state[lc][0], S, sub);
             for (int x = tid; x < 2 * TILE / 16; x += SC_THREADS)  // the rows of Q's lo tiles
                 *(uint4*)(M.a[1][x / (TILE / 16)][1] + (x % (TILE / 16)) * 16) = make_uint4(0u, 0u, 0u, 0u);
             sync();
@@ -865,7 +864,7 @@ delta_scan_kernel(const float* p, int splits, int n, const float* cv, uint8_t* t
 #pragma unroll
             for (int j = 0; j < 16; j++) M.state[c16 + j][key] = st[j];
             sync();
-            ld_rows<8>(S, &M.state[lc][0], sub);
+            ld_rows(S, &M.state[lc][0], sub);
             // (read anew: kept across the chunks they would spill)
             t0 = __ldcg(seg_start + sg);
             len = __ldcg(seg_len + sg);
@@ -913,18 +912,18 @@ delta_scan_kernel(const float* p, int splits, int n, const float* cv, uint8_t* t
             }
             sync();
             for (int r = 0; r < m; r++) {
-                if (pl.wck && p0 + c0 + r == pl.ck) st_rows<8>(sbuf(pl.cbuf), S, sub);
+                if (pl.wck && p0 + c0 + r == pl.ck) st_rows(sbuf(pl.cbuf), S, sub);
                 float k[RPT], qv[RPT];
-                ld_rows<8>(k, T.k[r], sub);
-                ld_rows<8>(qv, T.q[r], sub);
-                const float dk = dot_rows<8>(S, k), dq = dot_rows<8>(S, qv);
+                ld_rows(k, T.k[r], sub);
+                ld_rows(qv, T.q[r], sub);
+                const float dk = dot_rows(S, k), dq = dot_rows(S, qv);
                 const float ex = T.te[r], delta = (T.v[r][lc] - ex * dk) * T.tb[r];
                 if (sub == 0) out[(size_t)(t0 + c0 + r) * MIX + h * LVD + col] = ex * dq + delta * T.tkq[r];
 #pragma unroll
                 for (int j = 0; j < RPT; j++) S[j] = ex * S[j] + k[j] * delta;
             }
         }
-        st_rows<8>(sbuf(pl.ebuf), S, sub);
+        st_rows(sbuf(pl.ebuf), S, sub);
         // ---- the conv ring: the conv inputs of the segment's last CR tokens, this block's share of the channels (after
         // delta_prep, which read the ring, has finished: it is an earlier kernel of the stream)
         const int nb = gridDim.x * gridDim.y, share = (LQKV + nb - 1) / nb;

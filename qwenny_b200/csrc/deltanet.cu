@@ -7,25 +7,27 @@
 
 namespace qb {
 constexpr int TCH = 8;                    // tokens per round
-constexpr int LPC = 4, RPT = LKD / LPC;   // lanes per value column, state rows per thread
 }  // namespace qb
 
 // delta_conv + delta_rule + delta_norm of a decode / verify step in ONE launch: a cluster of two blocks per (value
-// head h, segment), each with half of the head's 128 value columns (256 threads: column tid / 4, rows
-// 4 (tid % 4 + 4 j) + i: the operation order of dot_rows, so the token form of the prompt path gives the same bits). A
+// head h, segment), each with half of the head's 128 value columns (512 threads: column tid / 8, rows as ld_rows deals them to 8 lanes: the
+// operation order of dot_rows, so the token form of the prompt path gives the same bits). A
 // block's slice of the f32 state lives in its registers; it recomputes the conv of the 320 channels it needs (its key
 // head's q and k, its own v columns) from the in-projection rows or the ring, runs the recurrence, and the two blocks
-// finish the gated RMSNorm over the head's 128 columns together: they exchange their per-lane partial sums of
-// squares through distributed shared memory and add them in the order one warp over the whole row would. Every
+// finish the gated RMSNorm over the head's 128 columns together: each writes its per-lane partial sums of
+// squares into both blocks' shared memory, and both add them in the order one warp over the whole row would. Every
 // phase's global loads are issued together (one round trip per phase). The conv ring is written by the blocks in
-// shares; the slot metadata by the LAST block of the launch to finish (an atomic ticket), because every block reads
-// the old metadata when it starts.
+// shares; the slot metadata by the LAST block of the launch to have read it (an atomic ticket, taken early and looked at at the end).
+// Bound by its chain of phases, ns for one segment of 5 rows: the inputs 2000, conv 500, norms and k . q 800, 5 tokens of the rule and the
+// state's way out 2500, gated norm 1300; the code of each is fetched cold (with the next token's q and k loaded ahead, in a second
+// copy of the loop, 14.6 us instead of 14.0). From a graph with its 16-bit product, us, with 256 threads, a ticket behind a fence at the end
+// and partial sums read from the partner / now: 1 row 12.1 / 11.2, 5 15.4 / 14.0, 8 17.5 / 15.7, 25 39.9 / 36.6, 4 segments of 5 35.7 / 30.5,
+// 12 of 2 74.6 / 59.5; the 64-layer step 4655 / 4573.
 namespace qb {
 
-constexpr int FNT = 256;             // threads of a block
+constexpr int FNT = 512;             // threads of a block
 constexpr int FCOLS = LVD / 2;       // value columns of a block
 constexpr int FCH = 2 * LKD + FCOLS; // q, k, v channels of a block
-constexpr int FLD = 8;               // loads in flight per thread in the staging loops
 
 struct FusedRound {
     float x[TCH + CONV_K - 1][FCH];  // conv inputs of the round's tokens and the 3 positions before them
@@ -34,10 +36,11 @@ struct FusedRound {
     float o[TCH][FCOLS];             // raw outputs of the round
     float w[FCH][CONV_K];            // conv taps of the block's channels
     float lp[TCH][32];               // per token: the 32 lane partials of the row's sum of squares (16 per block)
-    float e[TCH], b[TCH], kq[TCH], rn[TCH];
+    float e[TCH], b[TCH], kq[TCH];
 };
 
-__global__ void __launch_bounds__(FNT)
+template <int PER_SM>
+__global__ void __launch_bounds__(FNT, PER_SM)
 delta_fused_kernel(const float* p, int splits, int n, const float* ba, int ba_splits, const float* cw,
                    const float* a_log, const float* dt_bias, const float* nw, float* mem, long long sst, int* meta,
                    float* out, __half* y, const int* seg_start, const int* seg_len, const int* seg_slot,
@@ -45,6 +48,7 @@ delta_fused_kernel(const float* p, int splits, int n, const float* ba, int ba_sp
     extern __shared__ __align__(16) uint8_t fsm[];
     FusedRound& R = *(FusedRound*)fsm;
     pdl_launch_dependents();
+    cluster_arrive();
     // measurement only: thread 0 stamps the phases of the (first) round into trace[block][10]
     long long* tr = trace && threadIdx.x == 0 ? trace + (size_t)(blockIdx.y * gridDim.x + blockIdx.x) * 10 : nullptr;
     auto stamp = [&](int i) {
@@ -52,7 +56,7 @@ delta_fused_kernel(const float* p, int splits, int n, const float* ba, int ba_sp
     };
     stamp(0);
     const int h = blockIdx.x >> 1, hf = blockIdx.x & 1, sg = blockIdx.y, kh = h / (LV_HEADS / LK_HEADS);
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, rg = tid % LPC, lc = tid / LPC;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, sub = tid % LPC, lc = tid / LPC;
     const int col = hf * FCOLS + lc;  // the thread's value column of the head
     const int t0 = seg_start[sg], len = seg_len[sg], slot = seg_slot[sg], p0 = seg_pos0[sg];
     // global conv channel of the block's channel ch
@@ -63,7 +67,7 @@ delta_fused_kernel(const float* p, int splits, int n, const float* ba, int ba_sp
     // ---- everything that does not depend on this step's earlier kernels: the taps, the norm weight and, where the caller vouches
     // for it (`ahead`), the state
     for (int c = tid; c < FCH; c += FNT) *(float4*)R.w[c] = ld4(cw + gchan(c) * CONV_K);
-    const float nwv = nw[hf * FCOLS + tid % FCOLS], alog = a_log[h], dtb = dt_bias[h];
+    const float alog = a_log[h], dtb = dt_bias[h];
     float* sm0 = mem + slot * sst;
     if (!ahead) {
         hint_state<FCOLS, FNT>(meta, slot, p0, sm0, h * LVD + hf * FCOLS);
@@ -77,13 +81,13 @@ delta_fused_kernel(const float* p, int splits, int n, const float* ba, int ba_sp
 #pragma unroll
         for (int i = 0; i < RPT; i++) S[i] = 0.f;
     } else {
-        ld_rows<4>(S, sbuf(pl.in), rg);
+        ld_rows(S, sbuf(pl.in), sub);
     }
     for (int i = 0; i < pl.r; i++) {
         const float* e = entry(pl.in, pl.from + i);
         float k[RPT];
-        ld_rows<4>(k, e + kh * LKD, rg);
-        float dk = dot_rows<4>(S, k);
+        ld_rows(k, e + kh * LKD, sub);
+        float dk = dot_rows(S, k);
         float ex = e[LK_HEADS * LKD + LV_HEADS * LVD + h], be = e[LK_HEADS * LKD + LV_HEADS * LVD + LV_HEADS + h];
         float delta = (e[LK_HEADS * LKD + h * LVD + col] - ex * dk) * be;
 #pragma unroll
@@ -95,9 +99,10 @@ delta_fused_kernel(const float* p, int splits, int n, const float* ba, int ba_sp
     // the block's share of the conv ring: channels cb .. cb + ch of the segment's last CR tokens
     constexpr int NB = 2 * LV_HEADS, CH = (LQKV + NB - 1) / NB;  // channels per block (the last block has fewer)
     const int cb = blockIdx.x * CH, mm = min(len, CR);
-    static_assert(TCH * ((LQKV + 2 * LV_HEADS - 1) / (2 * LV_HEADS)) <= 4 * FNT, "a round's ring share fits 4 values per thread");
+    static_assert(TCH * ((LQKV + 2 * LV_HEADS - 1) / (2 * LV_HEADS)) <= 2 * FNT, "a round's ring share fits 2 values per thread");
 
-    bool lp_pending = false;  // a cluster barrier phase this block has arrived at and not yet waited for
+    int tkt = 0;
+    bool lp_pending = true;  // a cluster barrier phase this block has arrived at and not yet waited for (the first: it has started)
     for (int c0 = 0; c0 < len; c0 += TCH) {
         const int m = min(TCH, len - c0);
         // ---- ONE round trip of independent loads: conv inputs (step rows or ring), z, gates, the ring share.
@@ -107,7 +112,7 @@ delta_fused_kernel(const float* p, int splits, int n, const float* ba, int ba_sp
         // same staging took 2 us just to ISSUE: the kernel runs once per launch, so every instruction of it is also
         // an instruction fetched cold.
         constexpr int NROW = TCH + CONV_K - 1, NZV = (TCH * FCOLS + FNT - 1) / FNT;
-        float ringv[4], gate = 0.f;
+        float ringv[2], gate = 0.f;
         const bool direct = splits == 1;
         if (direct) {
             const int nrow = m + CONV_K - 1;
@@ -128,31 +133,23 @@ delta_fused_kernel(const float* p, int splits, int n, const float* ba, int ba_sp
             }
             cp_async_commit();
         }
-        // several splits: thread tid takes channel tid of every row, and threads below FCH - FNT also channel FNT + tid
-        float xv[NROW][2], zv[NZV];
-        const int gc0 = gchan(tid), gc1 = gchan(min(FNT + tid, FCH - 1));
-        const bool two = FNT + tid < FCH;
+        // several splits: thread tid takes channel tid of every row
+        float xv[NROW], zv[NZV];
+        const int gc = gchan(min(tid, FCH - 1));
         if (!direct) {
 #pragma unroll
             for (int row = 0; row < NROW; row++) {
-                xv[row][0] = xv[row][1] = 0.f;
+                xv[row] = 0.f;
                 const int si = c0 + row - (CONV_K - 1), qp = p0 + si;
-                if (row < m + CONV_K - 1 && qp >= 0) {
+                if (tid < FCH && row < m + CONV_K - 1 && qp >= 0) {
                     if (si >= 0) {
                         // (the first split's value is a plain load, so that every row's first loads are in flight
                         // together: a warp issues in order, and a sum inside a loop waits for each load before the next)
-                        const float* pr = p + (size_t)(t0 + si) * DELTA_IN;
-                        xv[row][0] = __ldcg(pr + gc0);
-                        if (two) xv[row][1] = __ldcg(pr + gc1);
-                        for (int s = 1; s < splits; s++) {
-                            pr += (size_t)n * DELTA_IN;
-                            xv[row][0] += __ldcg(pr + gc0);
-                            if (two) xv[row][1] += __ldcg(pr + gc1);
-                        }
+                        const float* pr = p + (size_t)(t0 + si) * DELTA_IN + gc;
+                        xv[row] = __ldcg(pr);
+                        for (int s = 1; s < splits; s++) xv[row] += __ldcg(pr += (size_t)n * DELTA_IN);
                     } else {
-                        const float* rr = sm0 + SLOT_RING + (size_t)(qp & (CR - 1)) * LQKV;
-                        xv[row][0] = __ldcg(rr + gc0);
-                        if (two) xv[row][1] = __ldcg(rr + gc1);
+                        xv[row] = __ldcg(sm0 + SLOT_RING + (size_t)(qp & (CR - 1)) * LQKV + gc);
                     }
                 }
             }
@@ -169,7 +166,7 @@ delta_fused_kernel(const float* p, int splits, int n, const float* ba, int ba_sp
             }
         }
 #pragma unroll
-        for (int u = 0; u < 4; u++) {
+        for (int u = 0; u < 2; u++) {
             const int i = u * FNT + tid, tk = c0 + i / CH, c = cb + i % CH;
             ringv[u] = 0.f;
             if (i < m * CH && c < LQKV && tk >= len - mm) {
@@ -191,10 +188,7 @@ delta_fused_kernel(const float* p, int splits, int n, const float* ba, int ba_sp
         if (!direct) {
 #pragma unroll
             for (int row = 0; row < NROW; row++) {
-                if (row < m + CONV_K - 1) {
-                    R.x[row][tid] = xv[row][0];
-                    if (two) R.x[row][FNT + tid] = xv[row][1];
-                }
+                if (tid < FCH && row < m + CONV_K - 1) R.x[row][tid] = xv[row];
             }
 #pragma unroll
             for (int u = 0; u < NZV; u++) {
@@ -214,6 +208,15 @@ delta_fused_kernel(const float* p, int splits, int n, const float* ba, int ba_sp
         }
         if (direct) cp_async_wait_all();
         __syncthreads();
+        // (every thread of the block has read the slots' metadata: the launch's last block to get here records the step in them. The
+        // answer is not waited for.)
+        if (c0 == 0 && tid == 0) tkt = atomicAdd(ticket, 1);
+        // this round's rows of the conv ring (the block's channel share)
+#pragma unroll
+        for (int u = 0; u < 2; u++) {
+            const int i = u * FNT + tid, tk = c0 + i / CH, c = cb + i % CH;
+            if (i < m * CH && c < LQKV && tk >= len - mm) sm0[SLOT_RING + (size_t)((p0 + tk) & (CR - 1)) * LQKV + c] = ringv[u];
+        }
         stamp(2);
         // ---- conv + SiLU
         for (int x = tid; x < m * FCH; x += FNT) {
@@ -257,72 +260,52 @@ delta_fused_kernel(const float* p, int splits, int n, const float* ba, int ba_sp
         stamp(5);
         // ---- the recurrence
         for (int tk = 0; tk < m; tk++) {
-            if (pl.wck && p0 + c0 + tk == pl.ck) st_rows<4>(sbuf(pl.cbuf), S, rg);
+            if (pl.wck && p0 + c0 + tk == pl.ck) st_rows(sbuf(pl.cbuf), S, sub);
             float k[RPT], q[RPT];
-            ld_rows<4>(k, &R.c[tk][LKD], rg);
-            ld_rows<4>(q, &R.c[tk][0], rg);
-            float dk = dot_rows<4>(S, k), dq = dot_rows<4>(S, q);
+            ld_rows(k, &R.c[tk][LKD], sub);
+            ld_rows(q, &R.c[tk][0], sub);
+            float dk = dot_rows(S, k), dq = dot_rows(S, q);
             float ex = R.e[tk], delta = (R.c[tk][2 * LKD + lc] - ex * dk) * R.b[tk];
-            if (rg == 0) R.o[tk][lc] = ex * dq + delta * R.kq[tk];
+            if (sub == 0) R.o[tk][lc] = ex * dq + delta * R.kq[tk];
 #pragma unroll
             for (int j = 0; j < RPT; j++) S[j] = ex * S[j] + k[j] * delta;
         }
+        const bool more = c0 + TCH < len;
+        if (!more) st_rows(sbuf(pl.ebuf), S, sub);  // (on its way while the norm is made)
         __syncthreads();
         stamp(6);
         // ---- gated RMSNorm over the head's 128 value columns. One warp over the whole row would give lane L the
         // columns 4 L .. 4 L + 3 and add the 32 lane partials as a butterfly; this block has the columns of lanes
-        // 16 hf .. 16 hf + 15: it computes those partials, hands them to its partner through distributed shared
+        // 16 hf .. 16 hf + 15: it computes those partials, writes them into its own and into its partner's shared
         // memory, and both run the same butterfly over the 32.
         if (lp_pending) { cluster_wait(); lp_pending = false; }  // the partner is done with the last round's partials
-        for (int x = tid; x < m * 16; x += FNT) {
-            int tk = x >> 4, l16 = x & 15;
+        if (tid < m * 16) {
+            const int tk = tid >> 4, l16 = tid & 15;
             float4 v = ld4(&R.o[tk][l16 * 4]);
-            float part = v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
-            R.lp[tk][hf * 16 + l16] = part;
+            float* to = &R.lp[tk][hf * 16 + l16];
+            *to = v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
+            asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(cluster_map(to, hf ^ 1)), "f"(*to) : "memory");
         }
         cluster_sync();
-        {
-            const uint32_t rem = cluster_map(&R.lp[0][0], hf ^ 1);
-            for (int x = tid; x < m * 16; x += FNT) {
-                int tk = x >> 4, l16 = x & 15, idx = tk * 32 + (hf ^ 1) * 16 + l16;
-                float v;
-                asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(rem + idx * 4));
-                R.lp[tk][(hf ^ 1) * 16 + l16] = v;
-            }
+        static_assert(FNT / 32 == 2 * TCH && FCOLS == 64, "two warps per token, a column per lane");
+        if (warp < 2 * m) {
+            const int tk = warp >> 1, c = (warp & 1) * 32 + lane;
+            const float rn = rsqrtf(warp_sum(R.lp[tk][lane]) / LVD + EPS), o = R.o[tk][c];
+            const size_t at = (size_t)(t0 + c0 + tk) * MIX + h * LVD + hf * FCOLS + c;
+            if (out) out[at] = o;
+            y[at] = __float2half_rn(nw[hf * FCOLS + c] * (o * rn) * silu(R.z[tk][c]));
         }
-        cluster_arrive();  // this block has read its partner's partials (the matching wait: before they are rewritten)
-        __syncthreads();   // this block's copy of them is complete
-        lp_pending = true;
-        for (int tk = warp; tk < m; tk += FNT / 32) {
-            float ss = warp_sum(R.lp[tk][lane]);
-            if (lane == 0) R.rn[tk] = rsqrtf(ss / LVD + EPS);
-        }
-        __syncthreads();
-        for (int x = tid; x < m * FCOLS; x += FNT) {
-            int tk = x / FCOLS, c = x - tk * FCOLS, t = t0 + c0 + tk;
-            float o = R.o[tk][c];
-            if (out) out[(size_t)t * MIX + h * LVD + hf * FCOLS + c] = o;
-            y[(size_t)t * MIX + h * LVD + hf * FCOLS + c] = __float2half_rn(nwv * (o * R.rn[tk]) * silu(R.z[tk][c]));
-        }
-        // ---- this round's rows of the conv ring (the block's channel share), loaded with the round's inputs
-#pragma unroll
-        for (int u = 0; u < 4; u++) {
-            const int i = u * FNT + tid, tk = c0 + i / CH, c = cb + i % CH;
-            if (i < m * CH && c < LQKV && tk >= len - mm) sm0[SLOT_RING + (size_t)((p0 + tk) & (CR - 1)) * LQKV + c] = ringv[u];
+        if (more) {  // this block has read its partials (the matching wait: before the partner rewrites them)
+            cluster_arrive();
+            lp_pending = true;
         }
         __syncthreads();
         stamp(7);
     }
-    st_rows<4>(sbuf(pl.ebuf), S, rg);
     stamp(8);
-    if (lp_pending) cluster_wait();  // the partner may read this block's shared memory until here
     // ---- the last block of the launch records the segments' steps in the slot metadata
     __shared__ int last;
-    if (tid == 0) {
-        __threadfence();
-        int tkt = atomicAdd(ticket, 1);
-        last = tkt == (int)(gridDim.x * gridDim.y) - 1;
-    }
+    if (tid == 0) last = tkt == (int)(gridDim.x * gridDim.y) - 1;
     __syncthreads();
     if (last) {
         for (int s = tid; s < segs; s += FNT) {
@@ -350,7 +333,10 @@ int qb_delta_mixer_as(qb_ctx* ctx, void* stream, const float* p, int splits, int
     if (n > qb::CR - qb::CONV_K + 1) return QB_ERR_UNSUPPORTED;
     // the launch's ticket: the last int of the context's ticket array (the products use the first n / 64)
     int* ticket = ctx->counters + ctx->ncounters - 1;
-    if (int rc = qb::prepare_kernel(ctx->device, (const void*)qb::delta_fused_kernel, (int)sizeof(qb::FusedRound))) return rc;
+    // Two blocks per SM (64 registers, some spilled) where the SMs do not hold every block alone: one segment of 1 / 5 / 8 rows 11.2 /
+    // 14.0 / 15.7 us alone and 14.0 / 18.4 / 21.5 in twos, 4 segments of 5 rows 32.9 and 30.5, 12 of 2 70 and 60.
+    auto kern = 2 * qb::LV_HEADS * segs <= ctx->sms ? qb::delta_fused_kernel<1> : qb::delta_fused_kernel<2>;
+    if (int rc = qb::prepare_kernel(ctx->device, (const void*)kern, (int)sizeof(qb::FusedRound))) return rc;
     cudaLaunchConfig_t lc = {};
     lc.gridDim = dim3(2 * qb::LV_HEADS, segs);
     lc.blockDim = dim3(qb::FNT);
@@ -363,7 +349,7 @@ int qb_delta_mixer_as(qb_ctx* ctx, void* stream, const float* p, int splits, int
     at[1].val.programmaticStreamSerializationAllowed = 1;
     lc.attrs = at;
     lc.numAttrs = ctx->pdl ? 2 : 1;
-    cudaError_t e = cudaLaunchKernelEx(&lc, qb::delta_fused_kernel, p, splits, n, ba, ba_splits, cw, a_log, dt_bias, nw, mem,
+    cudaError_t e = cudaLaunchKernelEx(&lc, kern, p, splits, n, ba, ba_splits, cw, a_log, dt_bias, nw, mem,
                                        sst, meta, out, (__half*)y, seg_start, seg_len, seg_slot, seg_pos0, segs, ticket,
                                        ctx->trace, ahead);
     return e == cudaSuccess ? QB_OK : (int)e;
