@@ -30,6 +30,10 @@ __device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, i
             "r"(smem_u32(dst)), "l"(map), "r"(x), "r"(y), "r"(z), "r"(smem_u32(bar))
         : "memory");
 }
+__device__ __forceinline__ void tma_store_2d(const CUtensorMap* map, const void* src, int x, int y) {
+    asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.tile.bulk_group [%0, {%1, %2}], [%3];\n" ::"l"(map), "r"(x), "r"(y), "r"(smem_u32(src))
+                 : "memory");
+}
 // ---- The products and their commits are issued by WHOLE WARPS: every lane walks the loop and elect.sync picks the one that issues.
 // A tcgen05.mma takes its addresses and descriptors from uniform registers; in a branch that one lane takes the compiler moves
 // them there one by one, and the issue, 70 to 270 cycles a product, hid what the tensor core takes: a product of M = 128 takes 34

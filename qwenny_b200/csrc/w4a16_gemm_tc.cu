@@ -13,19 +13,23 @@
 // 1024. A stage is 128 of k because the issuing warps are the next limit: a wait, a commit and their like cost 180 cycles per
 // stage beside 65 per product, and the copying lane 70 per copy (64 of k per stage: 600 cycles of the 512 at N = 256).
 //
-// The work is the list of (tile, k block of 128) pairs, tile after tile. Where whole tiles would leave the last wave
-// mostly empty, a persistent grid of one pair per two SMs deals the list out in equal contiguous shares (stream-K): a
+// The work is the list of (tile, k block of 128) pairs, tile after tile, on a persistent grid of at most one pair per two SMs. Where whole tiles
+// leave pairs idle the list is dealt out in equal contiguous shares (stream-K; with few tiles each tile is cut into as many equal parts): a
 // pair that ends or starts inside a tile writes that tile's partial accumulators to scratch and takes a ticket; the
-// tile's last arriver adds the parts in pair order and runs the epilogue, nobody waits. Otherwise a pair is a tile.
+// tile's last arriver adds the parts in pair order and runs the epilogue, nobody waits.
 // Per (tile, k block):
 //   warps 0-7   dequantise: lop3 / hsub2 to q - 8, one hfma2 by the f16 group scale (the reference's rounding:
-//               w = f16((q - 8) s), kernels/marlin.cuh:100-124), tcgen05.st into the stage's 64 columns; then they run
-//               the epilogue: tcgen05.ld of the accumulators, Y [token][output] f32, or silu(gate) * up as f16 for
-//               the interleaved SwiGLU matrices (or the partial tile)
-//   warp 8      copies, one lane: the X half tile (tensor map, 128-byte swizzle), the 8 KB of words (tensor map), the
+//               w = f16((q - 8) s), kernels/marlin.cuh:100-124), tcgen05.st into the stage's 64 columns
+//   warps 8-15  the accumulators of a finished tile (or part): tcgen05.ld, Y [token][output] f32, or silu(gate) * up as f16 for
+//               the interleaved SwiGLU matrices, by way of shared memory and one bulk copy per 16 tokens x 32 outputs; the next tile's
+//               weights are unpacked meanwhile
+//   warp 16     copies, one lane: the X half tile (tensor map, 128-byte swizzle), the 8 KB of words (tensor map), the
 //               group's scales; full/empty mbarriers, a ring of 4 stages
-//   warp 9      of the pair's first block: issues the products (K = 16 each) as a whole warp, tcgen05.commit hands the stage
+//   warp 17     of the pair's first block: issues the products (K = 16 each) as a whole warp, tcgen05.commit hands the stage
 //               back in both blocks when they have read it
+// Bound by the tensor pipe and, where it runs for long, by the power it takes. With the epilogue in the unpacking warps, one block per
+// tile, 4-byte stores and a fence per thread / as it is, us from a graph: 2048 rows of 16384 x 5120 252 / 224, of 34816 x 5120 545 / 500,
+// 333 rows of 5120 x 6144 with zero points 36.3 / 29.3, 100 rows 25.3 / 17.5, 500 rows of 2048 x 2048 35 / 17, 70 of 1024 x 1024 15.8 / 8.1.
 #include "launch.h"
 #include "pair_tc.cuh"
 
@@ -43,9 +47,11 @@ constexpr int XH_BYTES = BT / 2 * 64 * 2;   // 16 KB: this block's half of the t
 constexpr int X_BYTES = 2 * XH_BYTES;
 constexpr int W_BYTES = BH * BK / 2;        // 8 KB of Marlin words
 constexpr int S_BYTES = 512;                // 128 f16 scales, then (zero-point matrices) their offsets (8 - z) * scale
-constexpr int SMEM_BYTES = NSTAGE * (X_BYTES + W_BYTES + S_BYTES) + 1024 /* barriers, tmem address */ + 1024 /* alignment slack */;
 constexpr int DQ_WARPS = 8, DQ_GROUPS = DQ_WARPS / 4;  // a group of four warps dequantises a stage; the groups take turns
-constexpr int THREADS = (DQ_WARPS + 2) * 32;
+constexpr int EP_WARPS = 8, COPY_WARP = DQ_WARPS + EP_WARPS, MMA_WARP = COPY_WARP + 1;
+constexpr int THREADS = (MMA_WARP + 1) * 32;
+constexpr int OUT_BYTES = 16 * 32 * 4;      // 16 tokens x 32 outputs of an epilogue warp on their way to Y (two of them in turn)
+constexpr int SMEM_BYTES = NSTAGE * (X_BYTES + W_BYTES + S_BYTES) + EP_WARPS * 2 * OUT_BYTES + 1024 /* barriers, tmem address */ + 1024 /* alignment slack */;
 constexpr int TMEM_COLS = 512;
 constexpr int A_COLS = BK / 2;              // tensor-memory columns of a stage's weights
 
@@ -55,26 +61,28 @@ struct Args {
     int m, N, K, row0;
     int* err;
     int bt, tiles;       // tokens per tile (a multiple of 32, at most BT), tiles
-    float* part;         // [pair][2][block][BT][BH] partial tiles: [.][0] a share's first tile begun by an earlier pair, [.][1] its last, unfinished one
+    float* part;         // [pair][2][block][BT / 4][BH][4] partial tiles: [.][0] a share's first tile begun by an earlier pair, [.][1] its last, unfinished one
     int* tickets;        // two per tile (one per block of the pair), zero between launches
     int iters;           // tiles x k blocks
+    int direct;          // Y does not start on 16 bytes: plain stores
     int zp;              // S holds a second table [K/128][N] after the scales: the offsets (8 - z) * scale of zero-point matrices
 };
 
 template <int EPI, bool SHARES>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
-    w4a16_gemm_tc_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap wmap, const Args a) {
+    w4a16_gemm_tc_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap wmap, const __grid_constant__ CUtensorMap ymap, const Args a) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);  // swizzled tiles want 1 KB
     uint8_t* wsmem = smem + NSTAGE * X_BYTES;
     uint8_t* ssmem = wsmem + NSTAGE * W_BYTES;
-    uint64_t* full = (uint64_t*)(ssmem + NSTAGE * S_BYTES);  // copies landed in this block
+    uint8_t* osmem = ssmem + NSTAGE * S_BYTES;
+    uint64_t* full = (uint64_t*)(osmem + EP_WARPS * 2 * OUT_BYTES);  // copies landed in this block
     uint64_t* aready = full + NSTAGE;           // (first block) the weights are in both blocks' tensor memory, X in both's shared memory
     uint64_t* empty = aready + NSTAGE;          // the stage's products are done
     uint64_t* done = empty + NSTAGE;            // all products of a segment are done
     uint64_t* accfree = done + 1;               // (first block) both blocks have read the segment's accumulators
     uint32_t* tmem_slot = (uint32_t*)(accfree + 1);
-    int* flag = (int*)(tmem_slot + 1);          // this block finishes its half of the tile (the ticket's answer, for warps 0-7)
+    int* flag = (int*)(tmem_slot + 1);          // this block finishes its half of the tile (the ticket's answer, for the epilogue warps); the first of the pairs that hold it, how many
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int rank = (int)cluster_ctarank(), pair = blockIdx.x >> 1, G = gridDim.x >> 1;
@@ -89,10 +97,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
             mbar_init(&empty[i], 1);
         }
         mbar_init(done, 1);
-        mbar_init(accfree, 2 * DQ_WARPS);
+        mbar_init(accfree, 2 * EP_WARPS);
         mbar_fence_init();
     }
-    if (warp == DQ_WARPS + 1) {  // the product warps own the tensor memory, one in each block
+    if (warp == MMA_WARP) {  // the product warps own the tensor memory, one in each block
         asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(tmem_slot)),
                      "r"(TMEM_COLS));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;\n");
@@ -107,7 +115,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
 
     // Every role walks the pair's share as the same list of segments (tile, k blocks [kb0, kb1)); `ring` counts the
     // stages of the whole share, so the ring's slots and phases run on from one segment to the next.
-    if (warp == DQ_WARPS) {
+    if (warp == COPY_WARP) {
         // ---------------------------------------------------------------- copies
         if (lane == 0) {
             const uint64_t pol = policy_evict_last();
@@ -139,12 +147,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
         // a warp writes the 32 tensor-memory lanes of its quarter q (warp % 4): two 16-row blocks of the whole stage
         const int q = warp & 3, h = warp >> 2, g = lane >> 2;
         const uint32_t quarter = (uint32_t)(q * 32) << 16;
-        const uint32_t aready0 = cluster_map(aready, 0), accfree_at = cluster_map(accfree, 0);
+        const uint32_t aready0 = cluster_map(aready, 0);
         bool dead = false;
         uint32_t ring = 0;
-        int seg = 0;
-        for (; walk.next(tile, kb0, kb1); seg++) {
-            const int n0 = (tile % ntn) * BO + rank * BH, tok0 = (tile / ntn) * a.bt;
+        while (walk.next(tile, kb0, kb1)) {
             for (int kb = kb0; kb < kb1; kb++, ring++) {
                 if ((int)(ring % DQ_GROUPS) != h) continue;
                 const int s = (int)(ring % NSTAGE);
@@ -195,21 +201,32 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
                 if (lane == 0) mbar_arrive_at(aready0 + 8 * s);
             }
 
-            // ------------------------------------------------------------ the segment's accumulators
+        }
+    } else if (warp < COPY_WARP) {
+        // ---------------------------------------------------------------- the segments' accumulators, then the epilogue
+        // (the two warps of a quarter share the tokens)
+        const int e = warp - DQ_WARPS, q = warp & 3, h = e >> 2, lrow = q * 32 + lane;
+        const uint32_t tbase = tmem + ((uint32_t)(q * 32) << 16), accfree_at = cluster_map(accfree, 0);
+        const int c_lo = h * (a.bt / 2), c_hi = c_lo + a.bt / 2;
+        uint8_t* const stage = osmem + e * 2 * OUT_BYTES;
+        constexpr int PS = BH * 4;  // of a part: [4 tokens][output][4], a thread's sums in 16-byte pieces
+        constexpr int FIRST_EP = DQ_WARPS * 32;
+        bool dead = false;
+        uint32_t puts = 0;
+        for (int seg = 0; walk.next(tile, kb0, kb1); seg++) {
+            const int n0 = (tile % ntn) * BO + rank * BH, tok0 = (tile / ntn) * a.bt, orow = n0 + lrow;
+            const bool cut = SHARES && (kb0 > 0 || kb1 < nkb);
+            if (cut && threadIdx.x == FIRST_EP) walk.parts_of(tile, flag[1], flag[2]);  // (read behind the barriers at the tile's end)
             if (!dead) {
                 dead = !mbar_wait(done, (uint32_t)seg & 1);
                 if (dead && lane == 0) atomicExch(a.err, 8);
             }
             asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-            const int lrow = q * 32 + lane, orow = n0 + lrow;  // this lane's output; the two warps of a quarter share the tokens
-            const uint32_t tbase = tmem + quarter;
-            const int c_lo = h * (a.bt / 2), c_hi = c_lo + a.bt / 2;
             int parts = 1, first = 0;
             bool finish = !dead;
-            if (SHARES && (kb0 > 0 || kb1 < nkb)) {
+            if (cut) {
                 // a part of the tile: store it, take the tile's ticket; the last arriver finishes the tile
-                walk.parts_of(tile, first, parts);
-                float* slot = a.part + ((size_t)(pair * 2 + (kb0 == 0 ? 1 : 0)) * 2 + rank) * (BT * BH);
+                float* slot = a.part + ((size_t)(pair * 2 + (kb0 == 0 ? 1 : 0)) * 2 + rank) * (BT * BH) + lrow * 4;
                 if (!dead) {
 #pragma unroll 1
                     for (int c = c_lo; c < c_hi; c += 16) {
@@ -217,44 +234,75 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
                         tmem_ld16(tbase + c, v);
                         asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
 #pragma unroll
-                        for (int j = 0; j < 16; j++) slot[(size_t)(c + j) * BH + lrow] = __uint_as_float(v[j]);
+                        for (int j = 0; j < 16; j += 4) *(uint4*)(slot + (size_t)((c + j) / 4) * PS) = make_uint4(v[j], v[j + 1], v[j + 2], v[j + 3]);
                     }
                 }
-                __threadfence();
-                named_bar_sync(1, DQ_WARPS * 32);
-                if (threadIdx.x == 0) {
-                    const int tk = atomicAdd(&a.tickets[2 * tile + rank], 1);
-                    *flag = tk == parts - 1;
-                    if (tk == parts - 1) a.tickets[2 * tile + rank] = 0;
+                named_bar_sync(1, EP_WARPS * 32);
+                if (threadIdx.x == FIRST_EP) {
+                    __threadfence();  // (for all warps' sums: the barrier orders them before it)
+                    const bool last = atomicAdd(&a.tickets[2 * tile + rank], 1) == flag[2] - 1;
+                    *flag = last;
+                    if (last) {
+                        a.tickets[2 * tile + rank] = 0;
+                        __threadfence();
+                    }
                 }
-                named_bar_sync(1, DQ_WARPS * 32);
+                named_bar_sync(1, EP_WARPS * 32);
                 finish = *flag != 0 && !dead;
-                named_bar_sync(1, DQ_WARPS * 32);  // (the flag may be rewritten by the next segment)
-                if (finish) __threadfence();
+                first = flag[1]; parts = flag[2];
+                named_bar_sync(1, EP_WARPS * 32);  // (the flag may be rewritten by the next segment)
             }
+            // where pair first + p keeps its part: its last tile's for the first of them, its first one's for the others
+            auto part_of = [&](int p) {
+                return (const float4*)(a.part + ((size_t)((first + p) * 2 + (p == 0 ? 1 : 0)) * 2 + rank) * (BT * BH) + lrow * 4);
+            };
             if (finish) {
                 const int mine = pair - first;
+                constexpr int UP = 3;  // parts on their way at a time
+                float4 x[UP][4];
+                auto ask = [&](int u, int p, int c) {
+#pragma unroll
+                    for (int j = 0; j < 4; j++) x[u][j] = __ldcg(part_of(p) + (c / 4 + j) * (PS / 4));
+                };
+                if (SHARES && parts == 2) ask(0, 1 - mine, c_lo);
 #pragma unroll 1
                 for (int c = c_lo; c < c_hi; c += 16) {
                     uint32_t v[16];
+                    auto add = [&](int u) {
+#pragma unroll
+                        for (int j = 0; j < 4; j++) {
+                            v[4 * j] = __float_as_uint(__uint_as_float(v[4 * j]) + x[u][j].x);
+                            v[4 * j + 1] = __float_as_uint(__uint_as_float(v[4 * j + 1]) + x[u][j].y);
+                            v[4 * j + 2] = __float_as_uint(__uint_as_float(v[4 * j + 2]) + x[u][j].z);
+                            v[4 * j + 3] = __float_as_uint(__uint_as_float(v[4 * j + 3]) + x[u][j].w);
+                        }
+                    };
                     if (!SHARES || parts <= 2) {
                         tmem_ld16(tbase + c, v);
                         asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
                         if (SHARES && parts == 2) {  // own + other = other + own: no order to keep
-                            const float* o = a.part + ((size_t)((first + 1 - mine) * 2 + (mine == 1 ? 1 : 0)) * 2 + rank) * (BT * BH);
-#pragma unroll
-                            for (int j = 0; j < 16; j++)
-                                v[j] = __float_as_uint(__uint_as_float(v[j]) + __ldcg(o + (size_t)(c + j) * BH + lrow));
+                            add(0);
+                            if (c + 16 < c_hi) ask(0, 1 - mine, c + 16);  // the next ones are on their way meanwhile
                         }
                     } else {  // more parts: all of them from scratch, in pair order
 #pragma unroll
                         for (int j = 0; j < 16; j++) v[j] = 0;
-                        for (int p = 0; p < parts; p++) {
-                            const float* o = a.part + ((size_t)((first + p) * 2 + (p == 0 ? 1 : 0)) * 2 + rank) * (BT * BH);
+#pragma unroll 1
+                        for (int p = 0; p < parts; p += UP) {
 #pragma unroll
-                            for (int j = 0; j < 16; j++)
-                                v[j] = __float_as_uint(__uint_as_float(v[j]) + __ldcg(o + (size_t)(c + j) * BH + lrow));
+                            for (int u = 0; u < UP; u++)
+                                if (p + u < parts) ask(u, p + u, c);
+#pragma unroll
+                            for (int u = 0; u < UP; u++)
+                                if (p + u < parts) add(u);
                         }
+                    }
+                    if (tok0 + c >= a.m) continue;
+                    // the 16 tokens go through shared memory to one copy of a 32-output box (what lies past the last row is left out)
+                    uint8_t* const ob = stage + (puts & 1) * OUT_BYTES;
+                    if (!a.direct) {
+                        if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 1;\n" ::: "memory");
+                        __syncwarp();
                     }
                     if (EPI == EPI_SILU_TC) {
                         // packed rows 16 p + i are gate rows, 16 p + 8 + i their up rows, 8 lanes on: the gate lanes take
@@ -264,17 +312,30 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
                         for (int j = 0; j < 16; j += 2) {
                             const uint32_t other = __shfl_xor_sync(0xffffffffu, up_lane ? v[j] : v[j + 1], 8);
                             const float gate = __uint_as_float(up_lane ? other : v[j]), up = __uint_as_float(up_lane ? v[j + 1] : other);
-                            const int tok = tok0 + c + j + (up_lane ? 1 : 0);
-                            if (tok < a.m)
-                                ((__half*)a.Y)[(size_t)(a.row0 + tok) * (a.N / 2) + (orow >> 4) * 8 + (orow & 7)] =
-                                    __float2half_rn(silu(gate) * up);
+                            const int t = j + (up_lane ? 1 : 0);
+                            const __half y = __float2half_rn(silu(gate) * up);
+                            if (!a.direct)
+                                ((__half*)ob)[t * 16 + (lane >> 4) * 8 + (lane & 7)] = y;
+                            else if (tok0 + c + t < a.m)
+                                ((__half*)a.Y)[(size_t)(a.row0 + tok0 + c + t) * (a.N / 2) + (orow >> 4) * 8 + (orow & 7)] = y;
                         }
                     } else {
 #pragma unroll
                         for (int j = 0; j < 16; j++) {
-                            const int tok = tok0 + c + j;
-                            if (tok < a.m) ((float*)a.Y)[(size_t)(a.row0 + tok) * a.N + orow] = __uint_as_float(v[j]);
+                            if (!a.direct)
+                                ((uint32_t*)ob)[j * 32 + lane] = v[j];
+                            else if (tok0 + c + j < a.m)
+                                ((uint32_t*)a.Y)[(size_t)(a.row0 + tok0 + c + j) * a.N + orow] = v[j];
                         }
+                    }
+                    if (!a.direct) {
+                        asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+                        __syncwarp();
+                        if (lane == 0) {
+                            tma_store_2d(&ymap, ob, EPI == EPI_SILU_TC ? (n0 + q * 32) / 2 : n0 + q * 32, a.row0 + tok0 + c);
+                            asm volatile("cp.async.bulk.commit_group;\n" ::: "memory");
+                        }
+                        puts++;
                     }
                 }
             }
@@ -283,6 +344,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
             __syncwarp();
             if (lane == 0) mbar_arrive_at(accfree_at);
         }
+        if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;\n" ::: "memory");  // (the writes themselves end with the grid)
     } else if (rank == 0) {
         // ---------------------------------------------------------------- the pair's products (one whole warp)
         bool ok = true;
@@ -313,7 +375,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
     __syncthreads();
     cluster_sync();  // the other block's products read this block's shared and tensor memory until here
-    if (warp == DQ_WARPS + 1) {
+    if (warp == MMA_WARP) {
         asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(TMEM_COLS));
     }
 }
@@ -337,7 +399,7 @@ int qb_gemm_tc_launch(qb_ctx* ctx, cudaStream_t st, const void* X, const void* B
     const int tt = (m + tc::BT - 1) / tc::BT, bt = ((m + tt - 1) / tt + 31) / 32 * 32;
     const long long tiles = (long long)(n / tc::BO) * tt;
     if (tiles > QB_TC_TICKETS / 2) return QB_ERR_ARG;
-    CUtensorMap xmap, wmap;
+    CUtensorMap xmap, wmap, ymap = {};
     const cuuint32_t one[2] = {1, 1};
     const cuuint64_t xd[2] = {(cuuint64_t)k, (cuuint64_t)m}, xs[1] = {(cuuint64_t)k * 2};
     const cuuint32_t xb[2] = {64, (cuuint32_t)(bt / 2)};
@@ -351,26 +413,51 @@ int qb_gemm_tc_launch(qb_ctx* ctx, cudaStream_t st, const void* X, const void* B
     if (enc(&wmap, CU_TENSOR_MAP_DATA_TYPE_UINT64, 2, (void*)B, wd, ws, wb, one, CU_TENSOR_MAP_INTERLEAVE_NONE,
             CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
         return QB_ERR_ARG;
+    // Y up to the last row of the call; boxes of 16 rows x 32 outputs (16 after SwiGLU)
+    const bool silu = epi == QB_EPI_SILU, direct = ((uintptr_t)Y & 15) != 0;
+    const cuuint64_t yd[2] = {(cuuint64_t)(silu ? n / 2 : n), (cuuint64_t)(row0 + m)}, ys[1] = {yd[0] * (silu ? 2 : 4)};
+    const cuuint32_t yb[2] = {silu ? 16u : 32u, 16};
+    if (!direct && enc(&ymap, silu ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, Y, yd, ys, yb, one,
+                       CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE,
+                       CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+        return QB_ERR_ARG;
     const int pairs = ctx->sms / 2;
     tc::Args a;
     a.S = (const __half*)S; a.Y = Y; a.m = m; a.N = n; a.K = k; a.row0 = row0; a.err = ctx->err;
     a.zp = zp ? 1 : 0; a.part = ctx->tc_part; a.tickets = ctx->tc_tickets; a.iters = (int)tiles * (k / tc::BK);
-    a.bt = bt; a.tiles = (int)tiles;
-    // One pair per tile (the hardware hands a freed pair of SMs the next tile) when the partly filled last wave wastes
-    // less than a fifth of the time; otherwise one pair per two SMs and equal shares of the whole list, where a tile has
-    // two parts, seldom three. Against one block per 256 x 256 tile with the weights through shared memory, at 2048 rows:
-    // 16384 x 5120 298 -> 260 us (1320 TFLOP/s), 34816 x 5120 624 -> 574, 5120 x 6144 144 -> 115, 5120 x 17408 327 -> 303;
-    // at 256 rows 77 -> 36, 79 -> 74, 73 -> 43 and 95 -> 60 us.
-    const double waves = (double)tiles / pairs;
-    bool whole = (long long)(waves + 0.999999) < 1.2 * waves;
-    if (ctx->tune_ctas == 1000) whole = false;  // measurement: shares whatever the shape
-    if (ctx->tune_ctas == 1001) whole = true;   //              tiles whatever the shape
-    if (!ctx->tc_part) whole = true;            // a context without the scratch
-    const int G = whole ? (int)tiles : (int)(a.iters < pairs ? a.iters : pairs);
+    a.bt = bt; a.tiles = (int)tiles; a.direct = direct;
+    // How the list is dealt. More tiles than pairs: whole tiles, pair by pair in turn, where they fill four fifths of the rounds, else equal
+    // shares of the list over all pairs (5120 x 6144, 2048 rows, 2.2 rounds: 97 us as shares, 100 as tiles; 1500 rows, 1.6: 74 and 69).
+    // Fewer tiles than pairs: whole ones, or each cut into `cuts` equal parts for as many pairs, or shares, by an estimate in ns of the
+    // stages of the longest part (the products, but no less than unpacking takes) and of what joining the parts costs, more with every part of
+    // a tile (shares: parts of two tiles a pair). Measured at 70 / 256 rows, us: 5120 x 6144 whole 23.1 / 35.9, two parts 17.0 / 28.5,
+    // three 16.1 / 27.2, shares 18.4 / 33.0; 5120 x 17408 56 / 85, 35 / 56, 28.4 / 46, 28.6 / 48; 2048 x 2048 10.8 / 16.9, 10.7 / 17.1, 11.7 /
+    // 19.5, 16.2 / 33; 1024 x 1024 8.1 / 12.3, 8.9 / 14.5, 10.6 / 17.9, 13 / 25; 5120 x 10240 at 333 rows 45 whole, 40.5 as shares.
+    bool whole;
+    int cuts = 1;
+    if (tiles > pairs) {
+        const long long rounds = (tiles + pairs - 1) / pairs;
+        whole = 5 * tiles >= 4 * rounds * pairs;
+    } else {
+        const int nkb = k / tc::BK;
+        const long long stage = 380 + (bt > 128 ? (bt - 128) * 7 / 5 : 0);
+        long long best = a.iters * stage / pairs + 70 * bt;
+        cuts = 0;
+        for (int c = 1; c * tiles <= pairs && c <= nkb; c++) {
+            const long long cost = (nkb + c - 1) / c * stage + (c > 1 ? bt * (10 + 25 * (c - 1) / 2) : 0);
+            if (cost < best) { best = cost; cuts = c; }
+        }
+        whole = cuts == 1;
+    }
+    if (ctx->tune_ctas == 1000) { whole = false; cuts = 0; }  // measurement: shares whatever the shape
+    if (ctx->tune_ctas == 1001) whole = true;                 //              tiles whatever the shape
+    if (!ctx->tc_part) whole = true;                          // a context without the scratch
+    const long long units = whole ? tiles : cuts > 1 ? tiles * cuts : a.iters;
+    const int G = (int)(units < pairs ? units : pairs);
     dim3 grid((unsigned)(2 * G));
     if (epi == QB_EPI_SILU)
-        return whole ? launch(ctx, tc::w4a16_gemm_tc_kernel<tc::EPI_SILU_TC, false>, grid, dim3(tc::THREADS), tc::SMEM_BYTES, st, xmap, wmap, a)
-                     : launch(ctx, tc::w4a16_gemm_tc_kernel<tc::EPI_SILU_TC, true>, grid, dim3(tc::THREADS), tc::SMEM_BYTES, st, xmap, wmap, a);
-    return whole ? launch(ctx, tc::w4a16_gemm_tc_kernel<tc::EPI_PLAIN_TC, false>, grid, dim3(tc::THREADS), tc::SMEM_BYTES, st, xmap, wmap, a)
-                 : launch(ctx, tc::w4a16_gemm_tc_kernel<tc::EPI_PLAIN_TC, true>, grid, dim3(tc::THREADS), tc::SMEM_BYTES, st, xmap, wmap, a);
+        return whole ? launch(ctx, tc::w4a16_gemm_tc_kernel<tc::EPI_SILU_TC, false>, grid, dim3(tc::THREADS), tc::SMEM_BYTES, st, xmap, wmap, ymap, a)
+                     : launch(ctx, tc::w4a16_gemm_tc_kernel<tc::EPI_SILU_TC, true>, grid, dim3(tc::THREADS), tc::SMEM_BYTES, st, xmap, wmap, ymap, a);
+    return whole ? launch(ctx, tc::w4a16_gemm_tc_kernel<tc::EPI_PLAIN_TC, false>, grid, dim3(tc::THREADS), tc::SMEM_BYTES, st, xmap, wmap, ymap, a)
+                 : launch(ctx, tc::w4a16_gemm_tc_kernel<tc::EPI_PLAIN_TC, true>, grid, dim3(tc::THREADS), tc::SMEM_BYTES, st, xmap, wmap, ymap, a);
 }

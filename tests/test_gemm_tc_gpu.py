@@ -96,6 +96,34 @@ def test_shares_of_the_tile_list_repeat_and_agree_with_whole_tiles(ctx, m, rows,
     assert np.abs(an - cn).max() <= (2e-3 if silu else 2e-4) * max(1.0, np.abs(want).max())
 
 
+@pytest.mark.parametrize("m,rows,cols,silu", [(65, 256, 4096, False), (70, 512, 6144, True), (100, 5120, 2048, False), (256, 1280, 5248, False),
+                                               (300, 9728, 256, True)])
+def test_tiles_cut_into_equal_parts_and_unaligned_results(ctx, m, rows, cols, silu):
+    """Few tiles with a long k are cut into equal parts (up to one per pair of blocks; 5248 columns are 41 groups, which no number of parts
+    divides), many more tiles than pairs are dealt in rounds: the oracle's values and the same bits in a repeated launch. A result that starts off a
+    16-byte boundary takes plain stores: the same bits, and nothing beside it is written. Only the order of the f32 sums over k may differ
+    from whole tiles: 2e-4 of the largest value (2e-3 where the result is f16), as above."""
+    x, wdq, xd, wd, sd = make(rows, cols, silu, 500 + m, m)
+    epi, n, dt = ("silu", rows // 2, torch.float16) if silu else ("plain", rows, torch.float32)
+    a = ctx.marlin_gemm(xd, wd, sd, epi=epi)
+    b = ctx.marlin_gemm(xd, wd, sd, epi=epi)
+    room = torch.full((m * n + 9,), 7.0, dtype=dt, device="cuda")
+    ctx.marlin_gemm(xd, wd, sd, epi=epi, y=room[1:])
+    try:
+        ctx.tune(ctas=1001)
+        c = ctx.marlin_gemm(xd, wd, sd, epi=epi)
+    finally:
+        ctx.tune()
+    torch.cuda.synchronize()
+    assert ctx.device_error() == 0
+    assert torch.equal(a, b) and torch.equal(room[1:1 + m * n].view(m, n), a)
+    assert room[0] == 7 and (room[1 + m * n:] == 7).all()
+    want = R.marlin_gemm(x, wdq, epi)
+    an, cn = a.float().cpu().numpy(), c.float().cpu().numpy()
+    assert close(an, want.astype(np.float32)).all()
+    assert np.abs(an - cn).max() <= (2e-3 if silu else 2e-4) * max(1.0, np.abs(want).max())
+
+
 @pytest.mark.parametrize("m,rows,cols", [(17, 256, 128), (32, 512, 384), (33, 256, 640), (40, 1024, 2048), (63, 768, 256),
                                          (64, 2048, 1152), (70, 512, 512), (130, 256, 256)])
 def test_few_rows_gathered_argmax_vs_oracle(ctx, m, rows, cols):
