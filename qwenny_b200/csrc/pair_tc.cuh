@@ -141,15 +141,16 @@ struct Shares {
 };
 
 // A pair's work as a list of segments (tile, k blocks [kb0, kb1)); every role of both blocks walks the same list.
-// SHARES: equal contiguous shares of the (tile, k block) list; otherwise pair b takes the whole tiles b, b + grid, ...
+// SHARES: equal contiguous shares of the (tile, k block) list, cut between units of `unit` k blocks (1, or nkb: whole tiles); otherwise
+// pair b takes the whole tiles b, b + grid, ...
 template <bool SHARES>
 struct Walk {
     int tiles, nkb, G, b, j = 0;
     int it, it1;
-    __device__ Walk(int iters, int tiles_, int nkb_, int G_, int b_) : tiles(tiles_), nkb(nkb_), G(G_), b(b_) {
-        const Shares s(iters, G);
-        it = SHARES ? s.start(b) : 0;
-        it1 = SHARES ? s.start(b + 1) : 0;
+    __device__ Walk(int iters, int tiles_, int nkb_, int G_, int b_, int unit = 1) : tiles(tiles_), nkb(nkb_), G(G_), b(b_) {
+        const Shares s(iters / unit, G);
+        it = SHARES ? s.start(b) * unit : 0;
+        it1 = SHARES ? s.start(b + 1) * unit : 0;
     }
     __device__ bool next(int& tile, int& kb0, int& kb1) {
         if (!SHARES) {

@@ -8,9 +8,9 @@
 // "free" to "multiplied" (unpacking 680, the issue of 16 products 800, 130 to 150 per check of a barrier, two slots in turn), and 40 KB through
 // shared memory a stage, 24 of them the rows again. What a launch spends beside its stages: 3 us from its first instruction to the
 // first unpacked stage, 3 us from a cut tile's last sum to its result (partial sums 0.2, fence and ticket 1.1, parts 0.6, epilogue 0.7).
-// From a graph, 40 rows: the MLP 62.8 us (one group per stage, a fence per thread and 64-bit divisions before the ticket, one round
-// trip per part: 78.7), 5120 x 6144 13.7 (19.6), the output layer of 248,320 rows 218 (298); 17 and 64 rows of the MLP 56.9 (72) and 68.5
-// (86.5). What differs from the prompt-sized product:
+// From a graph, 40 rows: the MLP 60.0 us (one group per stage, a fence per thread and 64-bit divisions before the ticket, one round
+// trip per part, shares whatever the shape: 78.7), 5120 x 6144 12.5 (19.6), the output layer of 248,320 rows 218 (298); 17 and 64 rows of
+// the MLP 55.0 (72) and 64.2 (86.5). What differs from the prompt-sized product:
 //   - the weights are the exact integers q - 8; a group of 128 columns is one accumulation, and the drain warps multiply its
 //     f32 sums by the f32 value of the group's scale and add them up in registers (one thread per output, a register
 //     per token): one rounding per group, the arithmetic of the product for up to 16 rows (w4a16_gemv.cuh), where
@@ -21,7 +21,7 @@
 //   - a drain warp takes 16 tokens: with 32 its threads held 64 values and spilled
 //   - gathered rows (the output layer) are copied together first, by a launch of their own: gathered by cp.async in every block they slowed
 //     the unpacking from 680 to 1070 cycles a stage (40 rows of 248,320 outputs 269 us against 218, launch included)
-// The (tile, group) list is dealt to one block per SM in equal shares; parts of a cut tile are added by its last arriver in
+// The (tile, group) list is dealt to at most one block per SM: whole tiles, tiles cut into equal parts, or equal shares; parts of a cut tile are added by its last arriver in
 // block order (the bits repeat). Its ticket is taken behind a barrier by one thread with one fence (a fence per thread: 2 us; a ticket
 // per warp instead of the barriers: the output layer 241 us against 232).
 #include "launch.h"
@@ -65,6 +65,7 @@ struct Args {
     int* tickets;
     int iters;           // tiles x groups
     int tiles;
+    int unit;            // groups that stay together in a share: 1, or a tile's
 };
 
 // a += s x, two values at a time (each rounded as fmaf rounds it)
@@ -92,7 +93,7 @@ __global__ void __launch_bounds__(Cfg<NT>::THREADS, 1)
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int ngr = a.K / 128;
-    Walk<true> walk(a.iters, a.tiles, ngr, gridDim.x, blockIdx.x);
+    Walk<true> walk(a.iters, a.tiles, ngr, gridDim.x, blockIdx.x, a.unit);
     int tile = 0, g0 = 0, g1 = 0;
 
     // the weights and scales of a stage from group gi of the tile (one lane)
@@ -441,7 +442,23 @@ int qb_gemm_mid_launch(qb_ctx* ctx, cudaStream_t st, const void* X, const void* 
     a.S = (const __half*)S; a.Y = Y; a.keys = keys; a.m = m; a.N = n; a.K = k;
     a.y0 = y0; a.n_valid = n_valid; a.err = ctx->err; a.part = ctx->tc_part;
     a.tickets = ctx->tc_tickets; a.iters = tiles * (k / 128); a.tiles = tiles;
-    const int G = (int)(a.iters < ctx->sms ? a.iters : ctx->sms);
+    // How the list is dealt: whole tiles in rounds, each tile cut into `cuts` equal parts for as many blocks (few tiles), or equal shares of
+    // the list (parts of two tiles a block), by an estimate in ns of the longest block's groups and of joining the parts. Measured
+    // at 40 rows, us: 16384 x 5120 whole 19.2, shares 21.4; 5120 x 6144 in two 14.9, in three 12.5, shares 13.7; 5120 x 17408 in three 23.5,
+    // shares 22.7; 2048 x 2048 whole 9.6, in four 8.1, shares 10.1; 1024 x 1024 whole 6.5, in two 7.3, shares 7.9.
+    const long long ngr = k / 128, sms = ctx->sms, group = 300 + nt * 6 / 5, rounds = (tiles + sms - 1) / sms;
+    long long best = a.iters * group / sms + 2000 + 67 * nt, units = a.iters;
+    a.unit = 1;
+    if (rounds * ngr * group + (rounds - 1) * 700 < best) {
+        best = rounds * ngr * group + (rounds - 1) * 700;
+        a.unit = (int)ngr;
+        units = tiles;
+    }
+    for (int c = 2; c * tiles <= sms && c <= ngr; c++) {
+        const long long cost = (ngr + c - 1) / c * group + 500 + nt * (31 + 5 * c);
+        if (cost < best) { best = cost; a.unit = 1; units = (long long)tiles * c; }
+    }
+    const int G = (int)(units < sms ? units : sms);
     if (nt == 32) return mid::go<32>(ctx, st, epi, G, xmap, wmap, a);
     if (nt == 48) return mid::go<48>(ctx, st, epi, G, xmap, wmap, a);
     return mid::go<64>(ctx, st, epi, G, xmap, wmap, a);
