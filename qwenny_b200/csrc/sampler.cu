@@ -5,11 +5,17 @@
 // The reference gives a logit row to ONE block of 1024 threads, which reads the 248,320 logits (and their penalty
 // bits) up to four times through a 4096-bin shared histogram. Here a row belongs to a CLUSTER of 8 blocks: each block
 // reads an eighth of the row ONCE, applies the penalties and keeps the order-preserving keys in its shared memory
-// (124 KB); the k-th largest key is then found by an 8-bit radix select whose histograms have one copy per lane (no
+// (124 KB, which a bulk copy brings while the row's parameters are read). The largest keys of each block's 256 groups of four threads
+// give a bound that at least k keys of the row reach and few more (some 90 for k = 50): the keys that reach it go to a
+// list per block, and the leading block fetches the lists, sorts them and draws. Two cluster barriers and one pass over the
+// keys. Where the bound lets through more than the list holds (ties), and for whole-vocabulary rows, the k-th
+// largest key is found by an 8-bit radix select whose histograms have one copy per lane (no
 // two lanes of a warp ever add to the same word) and are merged over the cluster through distributed shared memory:
-// one cluster barrier per level. The blocks append their candidates to the leading block's list with remote atomics;
-// that block sorts them and draws. The arithmetic of the draw (exp of (v - vmax) / temperature, the shape of the
+// one cluster barrier per level. The arithmetic of the draw (exp of (v - vmax) / temperature, the shape of the
 // prefix sums, every comparison) is the reference kernel's, so the tokens are identical draw for draw.
+// Bound by its chain of phases, cycles for five rows of 248,320 at top_k 50 with penalties: parameters 3400, keys 6600, bound 2500, lists 4700,
+// fetching them 2200, sorting 2800, cut and draw 2900; a row is eight blocks, 40 of 148 SMs. From a graph, us, radix select and a
+// network of shared-memory steps for every row / now: 5 rows at top_k 50 20.9 / 14.5, at 1024 34.3 / 20.9, 40 rows at 5 38.9 / 38.5, at 50 52.3 / 39.7.
 //
 // Rows over the whole vocabulary (top_k 0) with a top-p cut, the common serving setting, are the host's in the reference
 // (a full sort of 248,320 values per row and step). Here the blocks also sum the mass of all tokens, the cut is made
@@ -26,6 +32,9 @@ namespace {
 constexpr int SCL = 8;       // blocks of a row's cluster
 constexpr int STH = 1024;    // threads per block
 constexpr int SCAP = 2048;   // candidates the leading block sorts at most
+constexpr int SGROUPS = STH / 4;  // groups of four threads, whose largest keys bound the k-th
+constexpr int PIECE = 8192;  // logits of a copy to shared memory
+constexpr int SRANK = 384;   // candidates that are ranked by counting; more are sorted in a network
 constexpr int QD = QB_QD, QCAP = QB_QCAP;
 
 struct SamplerArgs {
@@ -41,10 +50,19 @@ struct SamplerArgs {
     float* qp;
     int *out_tok, *out_acc;
     int slice;       // logits per block (a multiple of 32)
+    int* err;
 };
 
-struct SamplerSmem {
-    unsigned hist[256 * 32];          // [bin][lane]
+struct __align__(16) SamplerSmem {
+    union {
+        unsigned hist[256 * 32];      // [bin][lane]
+        struct {
+            unsigned group[SGROUPS];  // the largest key of each four threads
+            unsigned bound[2];        // the block's: its ceil(k / 8)-th and its k-th largest of those
+            unsigned pad[2];
+            unsigned long long mine[SCAP];  // the block's keys at or above the bound
+        };
+    };
     unsigned long long cand[SCAP];    // leading block: (key << 32 | ~column), later (token << 32 | probability)
     unsigned tot[2][256];             // this block's histogram of a level, read by the whole cluster
     unsigned ctot[256];               // the cluster's
@@ -104,19 +122,60 @@ __device__ __forceinline__ float scan1024(float v, float* sh) {
     return r;
 }
 
-// Bitonic network over c[0 .. np), np a power of two: one compare-exchange per thread and step
+// c[0 .. n) in order, descending or ascending; no two keys are equal. SCAP entries of c are written.
 template <bool ASC>
-__device__ __forceinline__ void bitonic_sort(unsigned long long* c, int np, int tid) {
-    for (int size = 2; size <= np; size <<= 1)
-        for (int stride = size >> 1; stride > 0; stride >>= 1) {
-            for (int t = tid; t < (np >> 1); t += STH) {
-                const int i = ((t & ~(stride - 1)) << 1) | (t & (stride - 1)), o = i | stride;
-                const bool up = (i & size) == 0;
+__device__ __forceinline__ void sort_keys(unsigned long long* c, int n, int tid) {
+    int np = 1;
+    while (np < n) np <<= 1;
+    if (n <= SRANK) {
+        // a key's place is the number of those before it: `per` threads count for each
+        __syncthreads();
+        const int per = min(32, STH / np), x = tid / per, part = tid % per;
+        const unsigned long long mine = x < n ? c[x] : 0ull;
+        int place = 0;
+        if (x < n)
+            for (int y = part; y < n; y += per) place += ASC ? c[y] < mine : c[y] > mine;
+        for (int o = 1; o < per; o <<= 1) place += __shfl_xor_sync(0xffffffffu, place, o);
+        __syncthreads();
+        if (x < n && part == 0) c[place] = mine;
+        __syncthreads();
+        return;
+    }
+    // A bitonic network. A thread has keys 2 tid and 2 tid + 1, so that a warp's 64 keys are compared in registers; wider steps
+    // go through shared memory, behind a barrier each (all 66 steps of 2048 keys so: 33,000 cycles, 24 us of 34 for top_k 1024)
+    for (int i = n + tid; i < np; i += STH) c[i] = ASC ? ~0ull : 0ull;
+    __syncthreads();
+    const int i0 = 2 * tid;
+    const bool in = i0 < np;
+    unsigned long long e0 = 0, e1 = 0;
+    auto step = [&](int size, int stride) {  // stride <= 32
+        const bool up = (i0 & size) == 0;
+        if (stride == 1) {
+            if ((ASC ? e0 > e1 : e0 < e1) == up) { const unsigned long long x = e0; e0 = e1; e1 = x; }
+            return;
+        }
+        const bool first = ((i0 & stride) == 0) == (up != ASC);  // this side keeps the larger one
+        const unsigned long long p0 = __shfl_xor_sync(0xffffffffu, e0, stride >> 1), p1 = __shfl_xor_sync(0xffffffffu, e1, stride >> 1);
+        e0 = (p0 > e0) == first ? p0 : e0;
+        e1 = (p1 > e1) == first ? p1 : e1;
+    };
+    for (int size = 64; size <= np; size <<= 1) {
+        for (int stride = size >> 1; stride > 32; stride >>= 1) {
+            if (in) {
+                const int i = ((tid & ~(stride - 1)) << 1) | (tid & (stride - 1)), o = i | stride;
                 const unsigned long long a = c[i], b = c[o];
-                if ((ASC ? a > b : a < b) == up) { c[i] = b; c[o] = a; }
+                if ((ASC ? a > b : a < b) == ((i & size) == 0)) { c[i] = b; c[o] = a; }
             }
             __syncthreads();
         }
+        if (in) { e0 = c[i0]; e1 = c[i0 + 1]; }
+        if (size == 64)
+            for (int sz = 2; sz < 64; sz <<= 1)
+                for (int stride = sz >> 1; stride > 0; stride >>= 1) step(sz, stride);
+        for (int stride = 32; stride > 0; stride >>= 1) step(size, stride);
+        if (in) { c[i0] = e0; c[i0 + 1] = e1; }
+        __syncthreads();
+    }
 }
 
 __device__ __forceinline__ float q_lookup(const int* qid, const float* qp, int n, int id) {
@@ -133,11 +192,27 @@ template <bool DRAFT>
 __global__ void __launch_bounds__(STH, 1) sampler_kernel(const SamplerArgs a) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     SamplerSmem& S = *reinterpret_cast<SamplerSmem*>(smem_raw);
-    unsigned* stepbits = reinterpret_cast<unsigned*>(smem_raw + sizeof(SamplerSmem));
-    unsigned* vals = stepbits + a.slice / 32;
+    unsigned* vals = reinterpret_cast<unsigned*>(smem_raw + sizeof(SamplerSmem));
+    unsigned* stepbits = vals + a.slice;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int rank = blockIdx.x, j = blockIdx.y;
     pdl_wait();
+
+    // ---- this block's slice of the row is on its way to shared memory while the row's parameters are read
+    const int lo_i = rank * a.slice, n_loc = max(0, min(a.W, lo_i + a.slice) - lo_i), n4 = n_loc & ~3;
+    const float* L = a.logits + (size_t)j * a.ld;
+    uint64_t* bar = reinterpret_cast<uint64_t*>(S.cand);  // (the list's place, until the slice has landed) one per piece
+    const int pieces = (n4 + PIECE - 1) / PIECE;
+    const bool bulk = (reinterpret_cast<uintptr_t>(L + lo_i) & 15) == 0 && n4 > 0;
+    if (bulk && tid == 0) {
+        for (int i = 0; i < pieces; i++) mbar_init(&bar[i], 1);
+        mbar_fence_init();
+        for (int i = 0; i < pieces; i++) {
+            const int n = min(PIECE, n4 - i * PIECE) * 4;
+            mbar_expect_tx(&bar[i], n);
+            bulk_load(vals + i * PIECE, L + lo_i + i * PIECE, n, &bar[i]);
+        }
+    }
 
     const float* pr = a.params + j * 8;
     const float temp = pr[0], top_p = pr[2], rep = pr[3], u01 = pr[4], u2 = pr[5], pres = pr[7];
@@ -162,97 +237,107 @@ __global__ void __launch_bounds__(STH, 1) sampler_kernel(const SamplerArgs a) {
         wide = !greedy && top_k == 0 && top_p < 1.f;
         if (!greedy && !wide && (top_k == 0 || top_k > QCAP)) {  // more candidates than a block sorts: the host's row
             if (rank == 0 && tid == 0) a.out_acc[j] = -1;
+            if (bulk && tid == 0)  // (its copies do not outlive the block)
+                for (int i = 0; i < pieces; i++)
+                    if (!mbar_wait(&bar[i], 0)) atomicExch(a.err, 22);
             return;
         }
         k = greedy ? 1 : wide ? min(QCAP, a.W) : min(top_k, a.W);
     }
 
-    // ---- this block's slice: penalised logits as order-preserving keys, read once
-    const int lo_i = rank * a.slice, n_loc = max(0, min(a.W, lo_i + a.slice) - lo_i);
-    const float* L = a.logits + (size_t)j * a.ld;
     const bool penal = rep != 1.f || pres != 0.f;
     const unsigned* sb = a.seen + (size_t)slot * a.set_words;
     const unsigned* ob = a.outs + (size_t)slot * a.set_words;
+    unsigned* const repbits = stepbits;                                 // the slice's words of the penalty sets
+    unsigned* const presbits = reinterpret_cast<unsigned*>(S.cand) + 128;  // (behind the pieces' barriers)
     if (penal) {
         if (DRAFT) {
             if (tid < QD) S.chain[tid] = tid < t ? a.qtok[slot * QD + tid] : -1;
         } else {
-            // the step's tokens of the row's sequence after its first, up to the row's own (drafts fed so far)
-            for (int w = tid; w < a.slice / 32; w += STH) stepbits[w] = 0;
+            // the sets, and the step's tokens of the row's sequence after its first, up to the row's own (drafts fed so far)
+            for (int w = tid; w < a.slice / 32; w += STH) {
+                const int at = lo_i / 32 + w;
+                const bool in = at < a.set_words;
+                repbits[w] = in && rep != 1.f ? sb[at] : 0u;
+                presbits[w] = in && pres != 0.f ? ob[at] : 0u;
+            }
             __syncthreads();
             for (int q = first + 1 + tid; q <= row_tok; q += STH) {
                 const int x = a.ids[q] - lo_i;
-                if (x >= 0 && x < n_loc) atomicOr(&stepbits[x >> 5], 1u << (x & 31));
+                if (x >= 0 && x < n_loc) {
+                    if (rep != 1.f) atomicOr(&repbits[x >> 5], 1u << (x & 31));
+                    if (pres != 0.f) atomicOr(&presbits[x >> 5], 1u << (x & 31));
+                }
             }
         }
     }
-    if (!greedy)
+    // A lower bound of the k-th largest without counting anything (below); where it lets too many through, or the mass of all tokens
+    // is wanted, the histograms find the k-th itself.
+    const bool quick = !greedy && !wide;
+    const bool count = !greedy && !quick;
+    if (count)
         for (int w = tid; w < 256 * 32; w += STH) S.hist[w] = 0;
     __syncthreads();
-    {
-        const bool vec = (reinterpret_cast<uintptr_t>(L + lo_i) & 15) == 0;
-        // Four requests of 16 bytes per thread (and their words of the penalty sets) are in flight before the first is used:
-        // a row is 8 requests per thread, and one at a time each pays a round trip to memory. The first radix level is
-        // counted on the way. Five rows of 248,320 at top_k 50: 23.7 us one request at a time, 20.5 us so.
-        constexpr int UN = 4;
-        for (int i0 = tid * 4; i0 < n_loc; i0 += UN * 4 * STH) {
-            float4 f[UN];
-            unsigned rw[UN], pw[UN];
+    // ---- penalised logits as order-preserving keys, in place. A thread has the four logits from 4 tid on of every 4 STH. The loop stays a
+    // loop: the kernel runs once per launch and its code is fetched cold (eight rounds written out took 9200 cycles with penalties, this 6600).
+    unsigned most = 0;  // this thread's largest key
+    static_assert(PIECE % (4 * STH) == 0, "a round lies in one piece");
+#pragma unroll 1
+    for (int base = 0; base < n_loc; base += 4 * STH) {
+        if (bulk && base % PIECE == 0 && base < n4 && !mbar_wait(&bar[base / PIECE], 0) && lane == 0) atomicExch(a.err, 22);
+        const int i4 = base + tid * 4, nv = min(4, n_loc - i4);
+        if (nv <= 0) continue;
+        float v[4];
+        if (bulk && nv == 4) {
+            *reinterpret_cast<float4*>(v) = *reinterpret_cast<const float4*>(vals + i4);
+        } else {
 #pragma unroll
-            for (int b = 0; b < UN; b++) {
-                const int i4 = i0 + b * 4 * STH;
-                f[b] = make_float4(0.f, 0.f, 0.f, 0.f);
-                rw[b] = pw[b] = 0u;
-                if (i4 >= n_loc) continue;
-                if (vec && i4 + 4 <= n_loc) {
-                    f[b] = *reinterpret_cast<const float4*>(L + lo_i + i4);
-                } else {
-                    f[b].x = L[lo_i + i4];
-                    if (i4 + 1 < n_loc) f[b].y = L[lo_i + i4 + 1];
-                    if (i4 + 2 < n_loc) f[b].z = L[lo_i + i4 + 2];
-                    if (i4 + 3 < n_loc) f[b].w = L[lo_i + i4 + 3];
+            for (int e = 0; e < 4; e++) v[e] = L[lo_i + min(i4 + e, n_loc - 1)];  // (past the end: the last one again)
+        }
+        if (penal) {
+            if (DRAFT) {
+                for (int e = 0; e < nv; e++) {
+                    const int x = a.head_ids ? a.head_ids[lo_i + i4 + e] : lo_i + i4 + e;
+                    bool step = false;  // among the chain's drafts before this one
+                    for (int c = 0; c < t; c++) step |= S.chain[c] == x;
+                    if (rep != 1.f && (step || ((sb[x >> 5] >> (x & 31)) & 1))) v[e] = v[e] > 0.f ? v[e] / rep : v[e] * rep;
+                    if (pres != 0.f && (step || ((ob[x >> 5] >> (x & 31)) & 1))) v[e] -= pres;
                 }
-                if (!DRAFT && penal) {
-                    if (rep != 1.f) rw[b] = sb[(lo_i + i4) >> 5];
-                    if (pres != 0.f) pw[b] = ob[(lo_i + i4) >> 5];
-                }
-            }
+            } else {
+                const int bit = i4 & 31;
+                const unsigned r = repbits[i4 >> 5] >> bit & 15u, q = presbits[i4 >> 5] >> bit & 15u;
+                if (r | q) {
 #pragma unroll
-            for (int b = 0; b < UN; b++) {
-                const int i4 = i0 + b * 4 * STH, nv = min(4, n_loc - i4);
-                if (nv <= 0) continue;
-                float v[4] = {f[b].x, f[b].y, f[b].z, f[b].w};
-                if (penal) {
-                    if (DRAFT) {
-                        for (int e = 0; e < nv; e++) {
-                            const int x = a.head_ids ? a.head_ids[lo_i + i4 + e] : lo_i + i4 + e;
-                            bool step = false;  // among the chain's drafts before this one
-                            for (int c = 0; c < t; c++) step |= S.chain[c] == x;
-                            if (rep != 1.f && (step || ((sb[x >> 5] >> (x & 31)) & 1))) v[e] = v[e] > 0.f ? v[e] / rep : v[e] * rep;
-                            if (pres != 0.f && (step || ((ob[x >> 5] >> (x & 31)) & 1))) v[e] -= pres;
-                        }
-                    } else {
-                        const int bit = i4 & 31;
-                        const unsigned st = stepbits[i4 >> 5];
-                        const unsigned r = rep != 1.f ? (rw[b] | st) >> bit : 0u, q = pres != 0.f ? (pw[b] | st) >> bit : 0u;
-                        for (int e = 0; e < nv; e++) {
-                            if ((r >> e) & 1) v[e] = v[e] > 0.f ? v[e] / rep : v[e] * rep;
-                            if ((q >> e) & 1) v[e] -= pres;
-                        }
+                    for (int e = 0; e < 4; e++) {  // (past the end: not used)
+                        if ((r >> e) & 1) v[e] = v[e] > 0.f ? v[e] / rep : v[e] * rep;
+                        if ((q >> e) & 1) v[e] -= pres;
                     }
                 }
-#pragma unroll
-                for (int e = 0; e < 4; e++)
-                    if (e < nv) {
-                        const unsigned u = ordered(v[e]);
-                        vals[i4 + e] = u;
-                        if (!greedy) atomicAdd(&S.hist[((u >> 24) << 5) + lane], 1u);
-                    }
             }
+        }
+        uint4 u = make_uint4(ordered(v[0]), ordered(v[1]), ordered(v[2]), ordered(v[3]));
+        if (nv == 4) {
+            *reinterpret_cast<uint4*>(vals + i4) = u;
+        } else {  // (the keys past the end: the first one again, which changes no maximum)
+            vals[i4] = u.x;
+            if (nv > 1) vals[i4 + 1] = u.y; else u.y = u.x;
+            if (nv > 2) vals[i4 + 2] = u.z; else u.z = u.x;
+            u.w = u.x;
+        }
+        most = max(most, max(max(u.x, u.y), max(u.z, u.w)));
+        if (count) {
+            const unsigned w[4] = {u.x, u.y, u.z, u.w};
+            for (int e = 0; e < nv; e++) atomicAdd(&S.hist[((w[e] >> 24) << 5) + lane], 1u);
         }
     }
     if (tid == 0) { S.sv[3] = 0; S.eq = 0; }
+    if (quick) {
+        unsigned g = max(most, __shfl_xor_sync(0xffffffffu, most, 1));
+        g = max(g, __shfl_xor_sync(0xffffffffu, g, 2));
+        if ((lane & 3) == 0) S.group[tid >> 2] = g;
+    }
     __syncthreads();
+    if (bulk && tid < pieces) asm volatile("mbarrier.inval.shared::cta.b64 [%0];\n" ::"r"(smem_u32(&bar[tid])) : "memory");
 
     // ---- whole-vocabulary rows: the largest value, then the mass of all tokens at the temperature (the blocks' sums
     // added in rank order)
@@ -318,13 +403,92 @@ __global__ void __launch_bounds__(STH, 1) sampler_kernel(const SamplerArgs a) {
         return;
     }
 
+    const uint32_t r_cnt = cluster_map(&S.sv[3], 0), r_cand = cluster_map(&S.cand[0], 0);
+    // every key from `from` on, with its column: to the block's own list, or to the leading block's
+    auto append = [&](unsigned from, bool own) {
+        if (most < from) return;
+        auto add = [&](unsigned u, int i) {
+            if (u < from) return;
+            const unsigned at = own ? atomicAdd(&S.sv[3], 1u) : cluster_atom_add(r_cnt, 1u);
+            const unsigned long long key = ((unsigned long long)u << 32) | (0xffffffffu - (unsigned)(lo_i + i));
+            if (at >= (unsigned)SCAP) return;
+            if (own) S.mine[at] = key;
+            else cluster_st_u64(r_cand + at * 8, key);
+        };
+        // (four at a time: key by key a thread's 31 took 7000 cycles)
+        int i4 = tid * 4;
+#pragma unroll 1
+        for (; i4 < n4; i4 += 4 * STH) {
+            const uint4 u = *reinterpret_cast<const uint4*>(vals + i4);
+            if (max(max(u.x, u.y), max(u.z, u.w)) < from) continue;
+            add(u.x, i4); add(u.y, i4 + 1); add(u.z, i4 + 2); add(u.w, i4 + 3);
+        }
+        for (int i = i4; i < n_loc; i++) add(vals[i], i);  // (at most three, of one thread)
+    };
+    // ---- A bound: in each block the m-th largest of its groups' largest keys has m keys at or above it. So the least of the blocks'
+    // ceil(k / 8)-th ones has k keys at or above it, and so has the greatest of their k-th ones (where the likely tokens sit in one
+    // block); the larger of the two is taken: some 90 candidates for k = 50, 1600 for 1024.
+    bool listed = false;
+    int cnt = 0;
+    if (quick) {
+        if (warp < 2) {  // (their upper 16 bits: two at a time, from the top, the largest that enough of them are at or above)
+            const unsigned want = warp ? (unsigned)k : (unsigned)(k + SCL - 1) / SCL;
+            unsigned g[SGROUPS / 32], b = 0;
+#pragma unroll
+            for (int i = 0; i < SGROUPS / 32; i++) g[i] = S.group[i * 32 + lane];
+#pragma unroll 1
+            for (int bit = 30; bit >= 16; bit -= 2) {
+                const unsigned at1 = b | 1u << bit, at2 = b | 2u << bit, at3 = b | 3u << bit;
+                unsigned n = 0;  // how many are at or above each: ten bits a count
+                static_assert(SGROUPS < 1024, "a count's bits");
+#pragma unroll
+                for (int i = 0; i < SGROUPS / 32; i++) n += (g[i] >= at1 ? 1u : 0u) + (g[i] >= at2 ? 1u << 10 : 0u) + (g[i] >= at3 ? 1u << 20 : 0u);
+                n = __reduce_add_sync(0xffffffffu, n);
+                b = n >> 20 >= want ? at3 : (n >> 10 & 1023u) >= want ? at2 : (n & 1023u) >= want ? at1 : b;
+            }
+            if (lane == 0) S.bound[warp] = b;  // (0 where there are fewer groups than asked for)
+        }
+        cluster_sync();
+        const unsigned least = lane < SCL ? cluster_ld_u32(cluster_map(&S.bound[0], lane)) : 0xffffffffu;
+        const unsigned greatest = lane < SCL ? cluster_ld_u32(cluster_map(&S.bound[1], lane)) : 0u;
+        // (lists of their own, which the leading block then fetches: an atomic in its shared memory for every key took 5000 cycles)
+        append(max(__reduce_min_sync(0xffffffffu, least), __reduce_max_sync(0xffffffffu, greatest)), true);
+        cluster_sync();
+        const unsigned n = lane < SCL ? cluster_ld_u32(cluster_map(&S.sv[3], lane)) : 0u;
+        cnt = (int)__reduce_add_sync(0xffffffffu, n);
+        listed = cnt <= SCAP;
+        if (listed && rank != 0) {
+            cluster_arrive();
+            cluster_wait();  // the leading block has them all
+            return;
+        }
+        if (listed) {
+            int before[SCL + 1] = {0};
+#pragma unroll
+            for (int r = 0; r < SCL; r++) before[r + 1] = before[r] + (int)__shfl_sync(0xffffffffu, n, r);
+            for (int x = tid; x < cnt; x += STH) {
+                int r = 0;
+#pragma unroll
+                for (int b = 1; b < SCL; b++) r += x >= before[b];
+                int first_of = 0;
+#pragma unroll
+                for (int b = 1; b < SCL; b++) first_of = x >= before[b] ? before[b] : first_of;
+                S.cand[x] = cluster_ld_u64(cluster_map(&S.mine[x - first_of], r));
+            }
+            cluster_arrive();
+        } else {
+            cluster_sync();
+            if (rank == 0 && tid == 0) S.sv[3] = 0;  // (the blocks come together again before anything is listed)
+        }
+    }
+
     // ---- radix select: the bin of the k-th largest key, 8 bits per level, until the candidates fit the list
     const int cap = min(SCAP, max(256, 2 * k));
     unsigned prefix = 0, mask = 0, above = 0, in_bin = 0;
     bool fits = false;
-    for (int level = 0; level < 4; level++) {
+    for (int level = 0; level < 4 && !listed; level++) {
         const int shift = 24 - 8 * level;
-        if (level > 0) {  // (the first level was counted with the loads)
+        if (level > 0 || quick) {  // (the first level was counted with the loads)
             for (int w = tid; w < 256 * 32; w += STH) S.hist[w] = 0;
             __syncthreads();
             for (int i = tid; i < n_loc; i += STH) {
@@ -377,18 +541,9 @@ __global__ void __launch_bounds__(STH, 1) sampler_kernel(const SamplerArgs a) {
     }
 
     // ---- candidates to the leading block's list
-    const uint32_t r_cnt = cluster_map(&S.sv[3], 0), r_cand = cluster_map(&S.cand[0], 0);
-    if (fits) {
-        // every key at or above the lower edge of the bin
-        for (int i = tid; i < n_loc; i += STH) {
-            const unsigned u = vals[i];
-            if (u >= prefix) {
-                const unsigned at = cluster_atom_add(r_cnt, 1u);
-                if (at < (unsigned)SCAP)
-                    cluster_st_u64(r_cand + at * 8, ((unsigned long long)u << 32) | (0xffffffffu - (unsigned)(lo_i + i)));
-            }
-        }
-    } else {
+    if (!listed && fits) {
+        append(prefix, false);  // every key at or above the lower edge of the bin
+    } else if (!listed) {
         // more keys equal to the k-th (`prefix`, now exact) than the list holds: the keys above it and, in index
         // order, the first k - above of the equal ones. Blocks own ascending index ranges.
         unsigned mine = 0;
@@ -425,16 +580,14 @@ __global__ void __launch_bounds__(STH, 1) sampler_kernel(const SamplerArgs a) {
             __syncthreads();
         }
     }
-    cluster_sync();
-    if (rank != 0) return;
+    if (!listed) {
+        cluster_sync();
+        if (rank != 0) return;
+    }
 
     // ---- the leading block: sort the candidates (descending by value, ties to the lower index), softmax, cut, draw
-    const int cnt = min((int)S.sv[3], SCAP);
-    int np = 1;
-    while (np < cnt) np <<= 1;
-    for (int i = cnt + tid; i < np; i += STH) S.cand[i] = 0;
-    __syncthreads();
-    bitonic_sort<false>(S.cand, np, tid);
+    if (!listed) cnt = min((int)S.sv[3], SCAP);
+    sort_keys<false>(S.cand, cnt, tid);
     k = min(k, cnt);
     auto column = [&](int r) { return (int)(0xffffffffu - (unsigned)S.cand[r]); };
     auto value = [&](int r) { return unordered((unsigned)(S.cand[r] >> 32)); };
@@ -473,12 +626,8 @@ __global__ void __launch_bounds__(STH, 1) sampler_kernel(const SamplerArgs a) {
         const float prob = tid < keep ? p / mass : 0.f;
         if (tid == (int)S.sv[5]) { a.out_tok[j] = x; a.qtok[q] = x; a.qn[q] = keep; }
         __syncthreads();
-        int nq = 1;
-        while (nq < keep) nq <<= 1;
-        for (int i = keep + tid; i < nq; i += STH) S.cand[i] = ~0ull;
         if (tid < keep) S.cand[tid] = ((unsigned long long)(unsigned)x << 32) | __float_as_uint(prob);
-        __syncthreads();
-        bitonic_sort<true>(S.cand, nq, tid);
+        sort_keys<true>(S.cand, keep, tid);
         if (tid < keep) {
             a.qid[(size_t)q * QCAP + tid] = (int)(S.cand[tid] >> 32);
             a.qp[(size_t)q * QCAP + tid] = __uint_as_float((unsigned)S.cand[tid]);
@@ -548,6 +697,7 @@ int launch_sampler(qb_ctx* ctx, void* stream, SamplerArgs a, int n_out) {
         return QB_ERR_ARG;
     if (n_out == 0) return QB_OK;
     a.slice = ((a.W + SCL - 1) / SCL + 31) / 32 * 32;
+    a.err = ctx->err;
     const size_t smem = sizeof(SamplerSmem) + (size_t)a.slice / 32 * 4 + (size_t)a.slice * 4;
     if (smem > 227 * 1024) return QB_ERR_TOO_LARGE;
     if (int rc = qb::prepare_kernel(ctx->device, (const void*)sampler_kernel<DRAFT>, 227 * 1024)) return rc;

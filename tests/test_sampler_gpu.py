@@ -268,6 +268,39 @@ def test_equal_logits_rank_by_index(ctx):
         assert tok == [t, t] or margin < 1e-5
 
 
+@pytest.mark.parametrize("where", ["anywhere", "one block", "rising", "masked", "few values"])
+def test_the_bound_lets_the_likely_tokens_through(ctx, where):
+    """The candidates are the keys at or above a bound from the blocks' groups: the same draws as the host's wherever the likely tokens sit
+    (in one block's slice; in the last ones of a rising row; ten tokens and the rest masked by the lowest f32 or by -inf; 64 values that
+    tie by the thousand, more than the list holds), for top_k on both sides of the eight blocks, of their 256 groups and of the
+    counting sort's limit. A draw differs from the host's only where its number lies within 1e-5 of a boundary."""
+    g = np.random.default_rng(71)
+    rows = Rows(72, whole=False)
+    lg = (g.standard_normal((2, V)) * 2).astype(F)
+    if where == "one block":
+        lg[:, 93100:93100 + 2000] += 9
+    elif where == "rising":
+        lg = (np.arange(V, dtype=F) * F(1e-4))[None].repeat(2, 0) + lg * F(1e-3)
+    elif where == "masked":
+        keep = g.permutation(V)[:10]
+        full = np.stack([np.full(V, np.finfo(F).min, F), np.full(V, -np.inf, F)])
+        full[:, keep] = lg[:, keep]
+        lg = full
+    elif where == "few values":
+        lg = np.floor(lg * 4).astype(F) / 4
+    rows.logits.copy_(torch.from_numpy(lg))
+    differ = 0
+    for k in (2, 8, 9, 50, 256, 257, 384, 385, 1024):
+        for u in (0.03, 0.4, 0.8, 0.999):
+            params = np.array([[0.9, k, 0.97, 1, u, 0, -1, 0]] * 2, dtype=F)
+            tok, acc = rows.mine(ctx, params)
+            for j in range(2):
+                want = S.sample_row(lg[j], None, None, params[j], want_margin=True)
+                differ += check_host(tok[j], acc[j], want[:2], want[2], f"{where} k {k} u {u}")
+    assert differ <= 2
+    assert ctx.device_error() == 0
+
+
 def test_greedy_rows_with_penalties(ctx, ref):
     rows = Rows(50, whole=True)
     for rep, pres in [(1.0, 0.0), (1.8, 0.0), (1.0, 6.0), (1.5, 3.0)]:
