@@ -36,8 +36,7 @@ constexpr int BH = 128;             // outputs per block
 constexpr int BK = 128;             // k of a group of scales
 constexpr int SG = 2;               // groups per stage
 constexpr int NSTAGE = 4;           // stages in shared memory (words, X): a copy takes some 2000 cycles
-constexpr int NA = 2;               // stages in tensor memory (64 columns per group)
-constexpr int ND = 2;               // accumulators in tensor memory (64 columns per group)
+constexpr int ND = 2;               // stages' accumulators in tensor memory (a column per token and group)
 constexpr int NS = 8;               // stages in the ring of scales: those in shared memory and those being drained
 constexpr int W_BYTES = BH * BK / 2;  // of a group
 constexpr int DQ_WARPS = 8;         // four warps unpack a group of a stage
@@ -50,6 +49,7 @@ struct Cfg {
     static constexpr int DR_WARPS = 4 * (NT / DT);  // a drain warp: 32 outputs x DT tokens
     static constexpr int COPY_WARP = DQ_WARPS + DR_WARPS, MMA_WARP = COPY_WARP + 1, X_WARP = COPY_WARP + 3;
     static constexpr int THREADS = (X_WARP + 1) * 32;  // (NT = 64: 28 warps leave 72 registers a thread, 29 only 64)
+    static constexpr int A_COL = ND * SG * NT, NA = (TMEM_COLS - A_COL) / (BK / 2);  // the groups' weights in tensor memory: 6, 5 or 4 of 64 columns
     static constexpr int XH = NT * 64 * 2, XB = 2 * XH;  // the tokens, 64 of k; a group
     static constexpr int SMEM = NSTAGE * SG * (XB + W_BYTES) + NS * SG * BH * 2 + 1024 + 1024;
     static_assert(XH % 1024 == 0, "swizzled tiles want 1 KB");
@@ -129,7 +129,8 @@ __global__ void __launch_bounds__(Cfg<NT>::THREADS, 1)
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-    const uint32_t tmem = *tmem_slot, tmem_a = tmem + 256;  // accumulators at columns 0, 64, 128 and 192, weights from 256 on
+    const uint32_t tmem = *tmem_slot;  // the accumulators, then the weights
+    constexpr int NA = C::NA;
     pdl_launch_dependents();
 
     // every role walks the same segments (tile, groups [g0, g1)) in stages of two groups, the last of a segment maybe of one; st
@@ -184,16 +185,16 @@ __global__ void __launch_bounds__(Cfg<NT>::THREADS, 1)
             for (int gi = g0; gi < g1; gi += SG, st++) {
                 const int s = (int)(st % NSTAGE);
                 if (!dead) {
-                    // (a lane each; the tensor-memory slot: the products of the stage NA before have read it)
-                    bool ok = true;
-                    if (lane < (st >= NA ? 2 : 1)) ok = mbar_wait(lane ? &empty[(st - NA) % NSTAGE] : &full[s], ((lane ? st - NA : st) / NSTAGE) & 1);
-                    dead = !__all_sync(0xffffffffu, ok);
+                    // (half a warp each; the tensor-memory slot: the products of the group NA before have read it)
+                    const int grp = 2 * (int)st + h, us = (grp - NA) >> 1;
+                    const bool slot = lane >= 16 && grp >= NA;
+                    dead = !warp_wait(slot ? &empty[us % NSTAGE] : &full[s], ((slot ? us : (int)st) / NSTAGE) & 1);
                     if (dead && lane == 0) atomicExch(a.err, 15);
                 }
                 __syncwarp();
                 if (gi + h < g1) {
                     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-                    const uint32_t at = tmem_a + ((int)(st % NA) * SG + h) * (BK / 2);
+                    const uint32_t at = tmem + C::A_COL + (2 * st + h) % NA * (BK / 2);
                     const uint8_t* wp = wsmem + (s * SG + h) * W_BYTES + (q >> 1) * 512 + lane * 16 + (q & 1) * 8;
                     uint2 w[8];
 #pragma unroll
@@ -253,12 +254,12 @@ __global__ void __launch_bounds__(Cfg<NT>::THREADS, 1)
                 // the second group's sums are on their way while the first's are added (in a stage of one group they are whatever the
                 // accumulator holds, and not used)
                 uint32_t v[DT], w[DT];
-                tmem_ld16(tq + p * SG * 64, v);
+                tmem_ld16(tq + p * SG * NT, v);
                 // (the scales landed with the words: the products that made these sums came after)
                 const __half* sp = sc + (int)(st % NS) * SG * BH;
                 const float s0 = __half2float(sp[0]), s1 = __half2float(sp[BH]);
                 asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
-                tmem_ld16(tq + (p * SG + 1) * 64, w);
+                tmem_ld16(tq + (p * SG + 1) * NT, w);
 #pragma unroll
                 for (int j = 0; j < DT; j += 2) fma2(acc[j], acc[j + 1], s0, v[j], v[j + 1]);
                 asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
@@ -360,7 +361,8 @@ __global__ void __launch_bounds__(Cfg<NT>::THREADS, 1)
             for (int gi = g0; gi < g1; gi += SG, st++) {
                 if ((int)(st & 1) != turn) continue;
                 const int s = (int)(st % NSTAGE), p = (int)(st % ND);
-                const uint32_t d = uniform(tm + p * SG * 64), at = uniform(tm + 256 + (int)(st % NA) * SG * (BK / 2)), xa = uniform(xs + s * SG * XB);
+                const uint32_t d = uniform(tm + p * SG * NT), xa = uniform(xs + s * SG * XB);
+                const uint32_t at = uniform(tm + C::A_COL + 2 * st % NA * (BK / 2)), at1 = NA % 2 ? uniform(tm + C::A_COL + (2 * st + 1) % NA * (BK / 2)) : at + BK / 2;
                 // (whole warps check, one barrier after the other: after a branch for some lanes the products are issued in the slow form)
                 if (st >= ND) ok = warp_wait(&dfree[p], ((st / ND) - 1) & 1);
                 ok = ok && warp_wait(&aready[s], (st / NSTAGE) & 1);
@@ -369,8 +371,8 @@ __global__ void __launch_bounds__(Cfg<NT>::THREADS, 1)
                 umma_ts4<1>(d, at, smem_desc(xa), idesc(NT), 0u);
                 umma_ts4<1>(d, at + 32, smem_desc(xa + C::XH), idesc(NT), 1u);
                 if (gi + 1 < g1) {
-                    umma_ts4<1>(d + 64, at + 64, smem_desc(xa + XB), idesc(NT), 0u);
-                    umma_ts4<1>(d + 64, at + 96, smem_desc(xa + XB + C::XH), idesc(NT), 1u);
+                    umma_ts4<1>(d + NT, at1, smem_desc(xa + XB), idesc(NT), 0u);
+                    umma_ts4<1>(d + NT, at1 + 32, smem_desc(xa + XB + C::XH), idesc(NT), 1u);
                 }
                 umma_commit(&empty[s]);
                 umma_commit(&dfull[p]);
