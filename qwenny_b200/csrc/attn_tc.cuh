@@ -49,7 +49,8 @@ __device__ __forceinline__ float ex2(float x) {
     return y;
 }
 
-// A bounded wait that remembers failure: once a wait ran out the role stops waiting and walks on
+// A bounded wait of a whole warp that remembers failure: once a wait ran out the role stops waiting and walks on. All lanes check: a check by
+// one or two of them, with the branch around it, costs more (2048 rows at context 30720 2005 -> 1959 us, 600 at 4000 155.0 -> 151.5)
 struct Waiter {
     int* err;
     int code;
@@ -63,21 +64,17 @@ struct Waiter {
     }
     __device__ __forceinline__ void wait(uint64_t* bar, uint32_t parity, int lane) {
         if (dead) return;
-        bool ok = true;
-        if (lane == 0) ok = sleep(bar, parity);
-        ok = __all_sync(0xffffffffu, ok);  // (the other lanes hold true)
+        const bool ok = __all_sync(0xffffffffu, sleep(bar, parity));
         if (!ok) {
             dead = true;
             if (lane == 0) atomicExch(err, code);
         }
     }
-    // two barriers at once, a lane each: about as long as one wait (2048 rows of prompt attention at context 30720: 1917 us
+    // two barriers at once, half a warp each: about as long as one wait (2048 rows of prompt attention at context 30720: 1917 us
     // without the second wait, 2024 with one after the other, 1930 so)
     __device__ __forceinline__ void wait_both(uint64_t* bar, uint32_t parity, uint64_t* bar1, uint32_t parity1, int lane) {
         if (dead) return;
-        bool ok = true;
-        if (lane < 2) ok = sleep(lane ? bar1 : bar, lane ? parity1 : parity);
-        ok = __all_sync(0xffffffffu, ok);
+        const bool ok = __all_sync(0xffffffffu, sleep(lane & 16 ? bar1 : bar, lane & 16 ? parity1 : parity));
         if (!ok) {
             dead = true;
             if (lane == 0) atomicExch(err, code);
