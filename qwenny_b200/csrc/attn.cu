@@ -2,7 +2,8 @@
 //  attn_prep    per token: sum of the in-projection parts, q/k RMSNorm(1+w), partial RoPE, q scaled to base-2 scores,
 //               sigmoid gate -> out, k and v quantised into the cache in the reference's byte order
 //               (replaces attn_prep + kv_store, kernels/qwen.cu:156-202, kernels/attn.cuh:50-64)
-//  attn_decode  split-K flash-decode: block (segment, kv head, key split) streams its run of keys and values with
+//  attn_decode  split-K flash-decode: a block per (segment, kv head, key split), or with many of those a block per SM that
+//               takes a run of them, streams a split's keys and values with
 //               bulk async copies into a shared-memory ring (keys are [pos][256] and values [pos/16][256][16] bytes
 //               per head, both contiguous per run) while RT x 4 warps compute S = Q K^T and O += P V on tensor cores
 //               with a warp-level base-2 online softmax, straight from the int8 bytes (prmt to 1152 + q halves, the
@@ -434,6 +435,13 @@ attn_decode_kernel(const float* q, const uint8_t* kc, const uint8_t* vc, const f
 // attn_prep and the combine, us, before (a copy warp, maxima in every stage, Q row by row) / now: 5 rows at 100 keys 13.5 / 11.2, at 4000
 // 18.4 / 15.1, at 32000 35.0 / 30.5; 1 row at 32000 26.2 / 24.1; 8 rows 50.6 / 40.2 (registers spilled before); 8 sequences of 4 rows at 972
 // to 7777 66.5 / 59.7, at 4000 to 32000 140 / 128.5.
+// Many splits (MANY): a block per split would pay for each one's start (its segment's tokens, Q, the first stages' way from memory: half of
+// the 11 us that a split of four stages took) and leave the last round of the SMs partly idle. So a block per SM takes a run of them, equal
+// shares of the line on which each split is as long as its stages and SPLIT_COST: Q stays where the run stays with a segment's kv head,
+// and the next split's first stages are under way while the quads merge. The sums of a split are the same in both forms.
+constexpr int DEC_SEGS = 64;         // segments of a step whose splits are dealt out: the table's size
+constexpr unsigned SPLIT_COST = 3;   // what a split costs beside its stages, in stages (measured: 1830 cycles a stage, 5000 a split)
+
 template <int RT, int NQ>
 struct Dec4Cfg {
     static constexpr int QUADS = NQ, CW = 4 * QUADS, THREADS = CW * 32;
@@ -446,15 +454,17 @@ struct Dec4Cfg {
     static constexpr int X_BYTES = X_MAX + 2 * X_P + X_SUM;
     static constexpr int BAR_BYTES = 128;
     static constexpr int SMEM = BAR_BYTES + Q_BYTES + QUADS * X_BYTES + NSTG * STG_BYTES;
+    static constexpr int SMEM_MANY = SMEM + DEC_SEGS * (16 + 8 + 4);  // and the step's segments
     static constexpr int MERGE_BYTES = 8 * 32 * (RT * 8 * 4 + RT * 6) * 4;   // two quads' registers at a time
     static_assert(MERGE_BYTES <= NSTG * STG_BYTES, "the merge buffers reuse the ring");
-    static_assert(SMEM <= 227 * 1024, "shared memory");
+    static constexpr int MERGE_SLOTS = (MERGE_BYTES + STG_BYTES - 1) / STG_BYTES;
+    static_assert(SMEM_MANY <= 227 * 1024, "shared memory");
 };
 
-template <int RT, int NQ>
+template <int RT, int NQ, bool MANY>
 __global__ void __launch_bounds__(Dec4Cfg<RT, NQ>::THREADS, 1)
 attn_dec4_kernel(const float* q, const uint8_t* kc, const uint8_t* vc, const float* ks, const float* vs, const int* dseg,
-                 const int* dtok, const int* tok_slot, const int* tok_pos, int cap, int z, int dsplits, int old_margin,
+                 const int* dtok, const int* tok_slot, const int* tok_pos, int cap, int z, int dsplits, int old_margin, int ndseg,
                  float* part_ml, float* part_acc, float* out, int* err) {
     using C = Dec4Cfg<RT, NQ>;
     constexpr int NSTG = C::NSTG, SK = C::SK, STG_BYTES = C::STG_BYTES;
@@ -465,42 +475,115 @@ attn_dec4_kernel(const float* q, const uint8_t* kc, const uint8_t* vc, const flo
     uint8_t* xch = smem + C::BAR_BYTES + C::Q_BYTES;
     uint8_t* ring = xch + C::QUADS * C::X_BYTES;
 
-    const int seg = blockIdx.x, g = blockIdx.y, s = blockIdx.z, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    if (threadIdx.x == 0) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    int seg = blockIdx.x, g = blockIdx.y, s = blockIdx.z;
+    if (threadIdx.x == 32) {
         for (int i = 0; i < NSTG; i++) { mbar_init(&full[i], 1); issued[i] = 0; }
         mbar_fence_init();
     }
-    __syncthreads();
-    pdl_launch_dependents();
     // The step's token lists are uploaded before its first kernel, so they are read ahead of the kernel before (this
     // step's attn_prep), and so, where the caller vouches for them, are the stages of keys and values that earlier steps wrote: whatever
     // ends `old_margin` positions or more before the segment's last key (0: nothing is read ahead, the first stages are only
     // asked into L2).
-    const int first = dseg[2 * seg], nt = dseg[2 * seg + 1];
-    const int my_tok = dtok[first + min(lane, nt - 1)], my_pos = tok_pos[my_tok];  // lane i: the segment's token i
-    const int tlast = __shfl_sync(0xffffffffu, my_tok, nt - 1), keys = __shfl_sync(0xffffffffu, my_pos, nt - 1) + 1;
-    const int chunk = dec_chunk(keys, dsplits), ns = (keys + chunk - 1) / chunk;
-    if (s >= ns) return;
-    const int kbeg = s * chunk, ke = min(keys, kbeg + chunk), nstg = (ke - kbeg + SK - 1) / SK;
+    int4* segs = (int4*)(ring + NSTG * STG_BYTES);  // MANY: per segment its first token's place, tokens, keys and slot,
+    int2* how = (int2*)(segs + DEC_SEGS);           // keys per split and splits,
+    unsigned* cum = (unsigned*)(how + DEC_SEGS);    // and where its splits end on the line that the blocks share
+    unsigned at = 0, until = 0;                     // where this split begins there, and where the block's share ends
+    if constexpr (MANY) {
+        if (warp == 0) {
+            unsigned sum = 0;
+            for (int i0 = 0; i0 < ndseg; i0 += 32) {
+                const int i = i0 + lane;
+                unsigned c = 0;
+                if (i < ndseg) {
+                    const int first = dseg[2 * i], nt = dseg[2 * i + 1], tlast = dtok[first + nt - 1], keys = tok_pos[tlast] + 1;
+                    segs[i] = make_int4(first, nt, keys, tok_slot[tlast]);
+                    const int chunk = dec_chunk(keys, dsplits), ns = min((keys + chunk - 1) / chunk, z);  // (more: more keys than the caller said)
+                    how[i] = make_int2(chunk, ns);
+                    c = NKV * ((min(keys, ns * chunk) + SK - 1) / SK + SPLIT_COST * ns);
+                }
+#pragma unroll
+                for (int d = 1; d < 32; d <<= 1) {
+                    const unsigned x = __shfl_up_sync(0xffffffffu, c, d);
+                    if (lane >= d) c += x;
+                }
+                if (i < ndseg) cum[i] = sum + c;
+                sum += __shfl_sync(0xffffffffu, c, 31);
+            }
+        }
+        __syncthreads();
+        // the first split that begins in the block's share
+        const unsigned total = cum[ndseg - 1], part = total / gridDim.x, over = total % gridDim.x;
+        const unsigned from = blockIdx.x * part + blockIdx.x * over / gridDim.x;
+        until = (blockIdx.x + 1) * part + (blockIdx.x + 1) * over / gridDim.x;
+        if (from >= total) {  // (fewer units than blocks)
+            pdl_launch_dependents();
+            return;
+        }
+        seg = 0;
+#pragma unroll
+        for (int i0 = 0; i0 < DEC_SEGS; i0 += 32)
+            seg += __popc(__ballot_sync(0xffffffffu, i0 + lane < ndseg && cum[min(i0 + lane, ndseg - 1)] <= from));
+        const unsigned begin_at = seg ? cum[seg - 1] : 0, head = (cum[seg] - begin_at) / NKV, rest = from - begin_at, each = how[seg].x / SK + SPLIT_COST;
+        g = rest / head;
+        s = (rest - g * head + each - 1) / each;
+        if (s >= how[seg].y) { s = 0; g++; }
+        at = begin_at + g * head + s * each;
+        if (g == NKV) { g = 0; seg++; }
+        pdl_launch_dependents();
+        if (at >= until) return;  // (also where seg is ndseg)
+    } else {
+        __syncthreads();
+        pdl_launch_dependents();
+    }
+    int first, nt, my_tok, my_pos, keys, chunk, ns, kbeg, ke, nstg, slot;
+    auto splits = [&]() {  // how the segment is split
+        chunk = MANY ? how[seg].x : dec_chunk(keys, dsplits);
+        ns = MANY ? how[seg].y : (keys + chunk - 1) / chunk;
+    };
+    auto split = [&]() {  // what this split is
+        kbeg = s * chunk;
+        ke = min(keys, kbeg + chunk);
+        nstg = (ke - kbeg + SK - 1) / SK;
+    };
+    if constexpr (MANY) {
+        const int4 x = segs[seg];
+        first = x.x; nt = x.y; keys = x.z; slot = x.w;
+        my_tok = dtok[first + min(lane, nt - 1)];
+        my_pos = tok_pos[my_tok];
+    } else {
+        first = dseg[2 * seg]; nt = dseg[2 * seg + 1];
+        my_tok = dtok[first + min(lane, nt - 1)]; my_pos = tok_pos[my_tok];  // lane i: the segment's token i
+        const int tlast = __shfl_sync(0xffffffffu, my_tok, nt - 1);
+        keys = __shfl_sync(0xffffffffu, my_pos, nt - 1) + 1;
+        slot = tok_slot[tlast];
+    }
+    splits();
+    if (!MANY && s >= ns) return;
+    split();
 
     // ---- the copies of a stage, its keys, values and scales, are shared out among the warps, at the start among all and later among a
     // quad's (by one warp they take 690 cycles, which the others would wait for), behind a barrier of the warps before which the stage's
     // own is armed. (A copy warp would be a third warp of one scheduler, and leave the others 168 registers instead of 255.)
     const int quad = warp >> 2, w = warp & 3, r = lane >> 2, t4 = lane & 3;
     constexpr int NCW = C::THREADS;
-    const int slot = tok_slot[tlast];
+    // (with many splits the slots at the front are those that the quads merge through, and a split's first stages go behind them)
+    constexpr int OFF = MANY ? C::MERGE_SLOTS : 0;
+    int j0 = 0;         // the stages of the block's splits before this one
+    uint32_t pars = 0;  // bit i: the parity that this split's first stage in slot i waits for
+    auto place = [&](int j) { return (j + OFF) % NSTG; };
     const uint64_t pol = policy_evict_first();
     auto copy = [&](int j, int part) {
         const uint8_t* from = part == 0 ? kc + cache_head(slot, g, cap) + (size_t)kbeg * HD : part == 1 ? vc + cache_head(slot, g, cap) + (size_t)kbeg * HD
                               : (const uint8_t*)((part == 2 ? ks : vs) + scale_head(slot, g, cap) + kbeg);
-        const uint32_t bytes = part < 2 ? SK * HD : SK * 4, at = part < 2 ? part * SK * HD : 2 * SK * HD + (part - 2) * SK * 4;
-        bulk_g2s(ring + (j % NSTG) * STG_BYTES + at, from + (size_t)j * bytes, bytes, &full[j % NSTG], pol);
+        const uint32_t bytes = part < 2 ? SK * HD : SK * 4, to = part < 2 ? part * SK * HD : 2 * SK * HD + (part - 2) * SK * 4;
+        bulk_g2s(ring + place(j) * STG_BYTES + to, from + (size_t)j * bytes, bytes, &full[place(j)], pol);
     };
     auto arm = [&](int j) {
-        mbar_expect_tx(&full[j % NSTG], STG_BYTES);
-        issued[j % NSTG] = j;
+        mbar_expect_tx(&full[place(j)], STG_BYTES);
+        issued[place(j)] = j;
     };
-    const int begin = min(nstg, NSTG);
+    int begin = min(nstg, NSTG);
     if (warp < begin && lane == 0) arm(warp);
     named_bar_sync(1, NCW);
     auto ask = [&](bool ahead) {  // the first stages
@@ -521,7 +604,7 @@ attn_dec4_kernel(const float* q, const uint8_t* kc, const uint8_t* vc, const flo
     uint8_t* xp_at = xch + quad * C::X_BYTES + C::X_MAX;             // [2][4][RT][32] x 16 B
     float2* xsum = (float2*)(xch + quad * C::X_BYTES + C::X_MAX + 2 * C::X_P);  // [4][RT][16]
     float* qsum = (float*)(xch + C::X_MAX);  // [RT * 16][2]: where the first quad's P goes later
-    {
+    auto load_q = [&](bool begins) {
         constexpr int PER = RT * 16 * HD / 4 / NCW, RSTEP = NCW / (HD / 4);  // float4 per thread, rows at a time
         const int r0 = threadIdx.x / (HD / 4), d = (threadIdx.x % (HD / 4)) * 4;
         float4 v[PER];
@@ -531,7 +614,7 @@ attn_dec4_kernel(const float* q, const uint8_t* kc, const uint8_t* vc, const flo
             const int t = __shfl_sync(0xffffffffu, my_tok, min(tok, nt - 1));
             v[i] = tok < nt ? *(const float4*)(q + ((size_t)t * NH + g * GROUP + row % GROUP) * HD + d) : make_float4(0.f, 0.f, 0.f, 0.f);
         }
-        ask(false);
+        if (begins) ask(false);
 #pragma unroll
         for (int i = 0; i < PER; i++) {
             const int row = r0 + i * RSTEP;
@@ -541,306 +624,374 @@ attn_dec4_kernel(const float* q, const uint8_t* kc, const uint8_t* vc, const flo
             const float sum = warp_sum((f0.x + f0.y) + (f1.x + f1.y));
             if (lane == 0) qsum[row * 2 + (warp & 1)] = sum;
         }
-    }
-    named_bar_sync(1, NCW);
-    // this lane's rows 16 rt + r and + 8: the keys they may see end at lim; KV_OFF times the sums of their Q
-    int lim[RT][2], all_see = ke;  // (keys below all_see are seen by every row of the segment)
+    };
+    // KV_OFF times the sums of Q of this lane's rows 16 rt + r and + 8
     float qoff[RT][2];
-#pragma unroll
-    for (int rt = 0; rt < RT; rt++)
-#pragma unroll
-        for (int h2 = 0; h2 < 2; h2++) {
-            const int row = rt * 16 + r + 8 * h2, tok = row / GROUP;
-            const float2 x = *(const float2*)&qsum[row * 2];
-            qoff[rt][h2] = KV_OFF * (x.x + x.y);
-            const int p = __shfl_sync(0xffffffffu, my_pos, min(tok, nt - 1));
-            lim[rt][h2] = tok < nt ? min(ke, p + 1) : 0;
-        }
-    all_see = min(all_see, __reduce_min_sync(0xffffffffu, my_pos) + 1);
-    // m: the rows' reference, a power of two that scores are taken from; -inf until a key was seen
-    float m[RT][2], l[RT][2], ps[RT][2], o[RT][8][4];
-#pragma unroll
-    for (int rt = 0; rt < RT; rt++) {
-        m[rt][0] = m[rt][1] = -INFINITY;
-        l[rt][0] = l[rt][1] = ps[rt][0] = ps[rt][1] = 0.f;
-#pragma unroll
-        for (int j = 0; j < 8; j++) o[rt][j][0] = o[rt][j][1] = o[rt][j][2] = o[rt][j][3] = 0.f;
-    }
     uint32_t qa[RT];
 #pragma unroll
     for (int rt = 0; rt < RT; rt++) qa[rt] = smem_u32(qsh + (rt * 16 + (lane & 15)) * SROW + (lane >> 4) * 8);
-    named_bar_sync(1, NCW);  // (the sums of Q have been read)
-
-    bool dead = false;
-    for (int j = quad; j < nstg; j += C::QUADS) {
-        const int sl = j % NSTG;
-        const uint32_t par = (j / NSTG) & 1;
-        if (!dead) {
-            // A slot's stages go to different quads, and a parity says nothing to a waiter that is two phases behind: one whose slot still
-            // waits for its last stage's copies would be let through. A stage is asked for only when that one was consumed.
-            uint32_t polls = 0;
-            if (j >= NSTG)
-                while (issued[sl] != j && polls < WAIT_LIMIT) polls++;
-            dead = polls == WAIT_LIMIT || !mbar_wait(&full[sl], par);
-            if (dead && lane == 0) atomicExch(err, 4);
-        } else {
-            for (int k = 0; k < 1024 && !mbar_try_wait(&full[sl], par); k++) {}
-        }
-        // two quads: the slot of the quad's stage before this one is filled again in the middle of this one
-        const bool refill = C::QUADS == 2 && j >= 2 && j - 2 + NSTG < nstg;
-        if (refill && w == 0 && lane == 0) arm(j - 2 + NSTG);
-        const uint8_t* base = ring + sl * STG_BYTES;
-        const int kb = kbeg + j * SK + 16 * w;  // this warp's 16 keys of the stage
-        const uint8_t* kp = base + (16 * w + r) * HD + 16 * t4;
-        const float* ksc_s = (const float*)(base + 2 * SK * HD) + 16 * w;
-        const float* vsc_s = ksc_s + SK;
-        const bool whole = kbeg + (j + 1) * SK <= all_see;  // every row sees every key of the stage
-        float ksc[2][2], vsc[2][2];
-#pragma unroll
-        for (int nn = 0; nn < 2; nn++)
-#pragma unroll
-            for (int e = 0; e < 2; e++) {
-                const int kk = 8 * nn + 2 * t4 + e;
-                const bool in = kb + kk < ke;
-                ksc[nn][e] = in ? ksc_s[kk] : 0.f;
-                vsc[nn][e] = in ? vsc_s[kk] : 0.f;
-            }
-        // ---- scores: S = Q K^T for every row tile, this warp's 16 keys
-        float v[RT][2][4];
-#pragma unroll
-        for (int rt = 0; rt < RT; rt++)
-#pragma unroll
-            for (int nn = 0; nn < 2; nn++) v[rt][nn][0] = v[rt][nn][1] = v[rt][nn][2] = v[rt][nn][3] = 0.f;
-#pragma unroll
-        for (int b = 0; b < HD / 64; b++) {
-            const uint4 kf0 = *(const uint4*)(kp + 64 * b), kf1 = *(const uint4*)(kp + 8 * HD + 64 * b);
-            const uint32_t w0[4] = {kf0.x, kf0.y, kf0.z, kf0.w}, w1[4] = {kf1.x, kf1.y, kf1.z, kf1.w};
-#pragma unroll
-            for (int st = 0; st < 4; st++) {
-                const uint32_t b00 = kv_half2(w0[st], 0x4140), b01 = kv_half2(w0[st], 0x4342);
-                const uint32_t b10 = kv_half2(w1[st], 0x4140), b11 = kv_half2(w1[st], 0x4342);
-#pragma unroll
-                for (int rt = 0; rt < RT; rt++) {
-                    uint32_t a[4];
-                    ldsm_x4(a[0], a[1], a[2], a[3], qa[rt] + (b * 64 + st * 16) * 2);
-                    mma16816(v[rt][0], a, b00, b01);
-                    mma16816(v[rt][1], a, b10, b11);
-                }
-            }
-        }
-        // ---- the scores proper
-#pragma unroll
-        for (int rt = 0; rt < RT; rt++)
-#pragma unroll
-            for (int nn = 0; nn < 2; nn++)
-#pragma unroll
-                for (int x = 0; x < 4; x++) {
-                    float& sv = v[rt][nn][x];
-                    sv = (sv - qoff[rt][x >> 1]) * ksc[nn][x & 1];
-                    if (!whole && kb + 8 * nn + 2 * t4 + (x & 1) >= lim[rt][x >> 1]) sv = -INFINITY;
-                }
-        // ---- P of this warp's keys (times the value scales, rounded to f16 as the products see it) and its row sums. The first time
-        // with the references as they are; where a row has left its own (P times a value scale near the end of f16, or P past 2^24), and
-        // in the quad's first stage, once more with new ones.
-        uint4* xp = (uint4*)(xp_at + (j / C::QUADS & 1) * C::X_P);  // (a warp may still be reading the stage before's)
-        float sum[RT][2], pr[RT][2];
-#pragma unroll 1
-        for (bool again = false;; again = true) {
-            bool left[RT][2], any_left = j == quad;
-#pragma unroll
-            for (int rt = 0; rt < RT; rt++) {
-                float pv[2][4];
-#pragma unroll
-                for (int h2 = 0; h2 < 2; h2++) {
-                    const float mm = m[rt][h2] == -INFINITY ? 0.f : m[rt][h2];
-                    sum[rt][h2] = 0.f;
-#pragma unroll
-                    for (int nn = 0; nn < 2; nn++)
-#pragma unroll
-                        for (int e = 0; e < 2; e++) {
-                            const float pp = tc::ex2(v[rt][nn][2 * h2 + e] - mm);
-                            sum[rt][h2] += pp;
-                            pv[nn][2 * h2 + e] = pp * vsc[nn][e];
-                        }
-                    left[rt][h2] = fmaxf(fmaxf(pv[0][2 * h2], pv[0][2 * h2 + 1]), fmaxf(pv[1][2 * h2], pv[1][2 * h2 + 1])) > 32768.f || sum[rt][h2] > 0x1p24f;
-                    any_left |= left[rt][h2];
-                }
-                uint4 pa;
-                pa.x = pack_half2(pv[0][0], pv[0][1]); pa.y = pack_half2(pv[0][2], pv[0][3]);
-                pa.z = pack_half2(pv[1][0], pv[1][1]); pa.w = pack_half2(pv[1][2], pv[1][3]);
-                xp[(w * RT + rt) * 32 + lane] = pa;
-                const float2 f0 = __half22float2(*(const __half2*)&pa.x), f1 = __half22float2(*(const __half2*)&pa.y);
-                const float2 f2 = __half22float2(*(const __half2*)&pa.z), f3 = __half22float2(*(const __half2*)&pa.w);
-                pr[rt][0] = f0.x + f0.y + f2.x + f2.y;
-                pr[rt][1] = f1.x + f1.y + f3.x + f3.y;
-            }
-            if (again) {
-                named_bar_sync(2 + quad, 128);
-                break;
-            }
-            if (!named_bar_or(2 + quad, 128, any_left)) break;
+    bool fresh = true, dead = false;  // fresh: these rows' Q is not in place yet
+    for (;;) {  // MANY: the block's splits; else the one
+        if (fresh) {
+            load_q(j0 == 0);
+            named_bar_sync(1, NCW);
 #pragma unroll
             for (int rt = 0; rt < RT; rt++)
 #pragma unroll
                 for (int h2 = 0; h2 < 2; h2++) {
-                    float x = fmaxf(fmaxf(v[rt][0][2 * h2], v[rt][0][2 * h2 + 1]), fmaxf(v[rt][1][2 * h2], v[rt][1][2 * h2 + 1]));
-                    x = fmaxf(x, __shfl_xor_sync(0xffffffffu, x, 1));
-                    x = fmaxf(x, __shfl_xor_sync(0xffffffffu, x, 2));
-                    const bool lf = (__ballot_sync(0xffffffffu, left[rt][h2]) >> (4 * r) & 15) != 0;
-                    if (t4 == 0) xmax[(w * RT + rt) * 16 + r + 8 * h2] = make_float2(x, lf ? 1.f : 0.f);
+                    const float2 x = *(const float2*)&qsum[(rt * 16 + r + 8 * h2) * 2];
+                    qoff[rt][h2] = KV_OFF * (x.x + x.y);
                 }
-            named_bar_sync(2 + quad, 128);
-#pragma unroll
-            for (int rt = 0; rt < RT; rt++) {
-                float corr[2];
-#pragma unroll
-                for (int h2 = 0; h2 < 2; h2++) {
-                    float mn = m[rt][h2];
-                    bool moves = j == quad;
-#pragma unroll
-                    for (int ww = 0; ww < 4; ww++) {
-                        const float2 x = xmax[(ww * RT + rt) * 16 + r + 8 * h2];
-                        mn = fmaxf(mn, x.x);
-                        moves |= x.y != 0.f;
-                    }
-                    moves &= mn > m[rt][h2];  // (it depends on the row's own scores alone, not on what else is in the step)
-                    corr[h2] = moves ? exp2f(m[rt][h2] - mn) : 1.f;
-                    if (moves) m[rt][h2] = mn;
-                    l[rt][h2] *= corr[h2];
-                    ps[rt][h2] *= corr[h2];
-                }
-#pragma unroll
-                for (int jd = 0; jd < 8; jd++) {
-                    o[rt][jd][0] *= corr[0]; o[rt][jd][1] *= corr[0];
-                    o[rt][jd][2] *= corr[1]; o[rt][jd][3] *= corr[1];
-                }
-            }
+            named_bar_sync(1, NCW);  // (the sums of Q have been read)
         }
-        // (a lane sums its own keys; lanes and warps are added up once, after the last stage)
+        // the keys that the rows may see end at lim
+        int lim[RT][2], all_see = ke;  // (keys below all_see are seen by every row of the segment)
 #pragma unroll
         for (int rt = 0; rt < RT; rt++)
 #pragma unroll
             for (int h2 = 0; h2 < 2; h2++) {
-                l[rt][h2] += sum[rt][h2];
-                ps[rt][h2] += pr[rt][h2];
+                const int tok = (rt * 16 + r + 8 * h2) / GROUP;
+                const int p = __shfl_sync(0xffffffffu, my_pos, min(tok, nt - 1));
+                lim[rt][h2] = tok < nt ? min(ke, p + 1) : 0;
             }
-        // (the barrier above: all of the quad is done with its stage before this one, and the slot's barrier is armed)
-        if (refill && lane == 0) copy(j - 2 + NSTG, w);
-        // ---- values: O += P V over the stage's 64 keys, this warp's 64 output dims
+        all_see = min(all_see, __reduce_min_sync(0xffffffffu, my_pos) + 1);
+        // m: the rows' reference, a power of two that scores are taken from; -inf until a key was seen
+        float m[RT][2], l[RT][2], ps[RT][2], o[RT][8][4];
 #pragma unroll
-        for (int kbk = 0; kbk < 4; kbk++) {
-            uint32_t pa[RT][4];
+        for (int rt = 0; rt < RT; rt++) {
+            m[rt][0] = m[rt][1] = -INFINITY;
+            l[rt][0] = l[rt][1] = ps[rt][0] = ps[rt][1] = 0.f;
 #pragma unroll
-            for (int rt = 0; rt < RT; rt++) {
-                const uint4 x = xp[(kbk * RT + rt) * 32 + lane];
-                pa[rt][0] = x.x; pa[rt][1] = x.y; pa[rt][2] = x.z; pa[rt][3] = x.w;
-            }
-            const uint8_t* vp = base + SK * HD + kbk * 16 * HD + (64 * w + r) * 16 + t4 * 4;
-#pragma unroll
-            for (int jd = 0; jd < 8; jd++) {
-                const uint32_t vw = *(const uint32_t*)(vp + jd * 8 * 16);
-                const uint32_t b0 = kv_half2(vw, 0x4140), b1 = kv_half2(vw, 0x4342);
-#pragma unroll
-                for (int rt = 0; rt < RT; rt++) mma16816(o[rt][jd], pa[rt], b0, b1);
-            }
+            for (int j = 0; j < 8; j++) o[rt][j][0] = o[rt][j][1] = o[rt][j][2] = o[rt][j][3] = 0.f;
         }
-        if (C::QUADS > 2 && j + NSTG < nstg) {  // (few stages more than quads: the next stage's barrier would be late)
-            if (w == 0 && lane == 0) arm(j + NSTG);
-            named_bar_sync(2 + quad, 128);
-            if (lane == 0) copy(j + NSTG, w);
-        }
-    }
 
-    // ---- the quads merge pairwise through the ring, which is free (every stage was consumed): 1 -> 0 and 3 -> 2, then
-    // 2 -> 0. A warp's registers go to the warp of the same index in the other quad (same rows, same dims).
-    named_bar_sync(1, NCW);
-    constexpr int MF = RT * 8 * 4 + RT * 6;  // floats per lane
-    for (int round = 1; round < C::QUADS; round <<= 1) {
-        const bool sender = (quad & (2 * round - 1)) == round;
-        const bool receiver = (quad & (2 * round - 1)) == 0 && quad + round < C::QUADS;
-        float* mb = (float*)ring + (size_t)(((quad >> 1) / round % 2) * 4 + w) * 32 * MF + lane;
-        if (sender) {
+        for (int j = quad; j < nstg; j += C::QUADS) {
+            const int sl = place(j);
+            const uint32_t par = ((j / NSTG) ^ (pars >> sl)) & 1;
+            if (!dead) {
+                // A slot's stages go to different quads, and a parity says nothing to a waiter that is two phases behind: one whose slot still
+                // waits for its last stage's copies would be let through. A stage is asked for only when that one was consumed.
+                uint32_t polls = 0;
+                if (j >= NSTG)
+                    while (issued[sl] != j && polls < WAIT_LIMIT) polls++;
+                dead = polls == WAIT_LIMIT || !mbar_wait(&full[sl], par);
+                if (dead && lane == 0) atomicExch(err, 4);
+            } else {
+                for (int k = 0; k < 1024 && !mbar_try_wait(&full[sl], par); k++) {}
+            }
+            // two quads: the slot of the quad's stage before this one is filled again in the middle of this one
+            const bool refill = C::QUADS == 2 && j >= 2 && j - 2 + NSTG < nstg;
+            if (refill && w == 0 && lane == 0) arm(j - 2 + NSTG);
+            const uint8_t* base = ring + sl * STG_BYTES;
+            const int kb = kbeg + j * SK + 16 * w;  // this warp's 16 keys of the stage
+            const uint8_t* kp = base + (16 * w + r) * HD + 16 * t4;
+            const float* ksc_s = (const float*)(base + 2 * SK * HD) + 16 * w;
+            const float* vsc_s = ksc_s + SK;
+            const bool whole = kbeg + (j + 1) * SK <= all_see;  // every row sees every key of the stage
+            float ksc[2][2], vsc[2][2];
 #pragma unroll
-            for (int rt = 0; rt < RT; rt++) {
+            for (int nn = 0; nn < 2; nn++)
 #pragma unroll
-                for (int jd = 0; jd < 8; jd++)
+                for (int e = 0; e < 2; e++) {
+                    const int kk = 8 * nn + 2 * t4 + e;
+                    const bool in = kb + kk < ke;
+                    ksc[nn][e] = in ? ksc_s[kk] : 0.f;
+                    vsc[nn][e] = in ? vsc_s[kk] : 0.f;
+                }
+            // ---- scores: S = Q K^T for every row tile, this warp's 16 keys
+            float v[RT][2][4];
 #pragma unroll
-                    for (int e = 0; e < 4; e++) mb[((rt * 8 + jd) * 4 + e) * 32] = o[rt][jd][e];
+            for (int rt = 0; rt < RT; rt++)
 #pragma unroll
-                for (int h2 = 0; h2 < 2; h2++) {
-                    mb[(RT * 32 + rt * 6 + h2) * 32] = m[rt][h2];
-                    mb[(RT * 32 + rt * 6 + 2 + h2) * 32] = l[rt][h2];
-                    mb[(RT * 32 + rt * 6 + 4 + h2) * 32] = ps[rt][h2];
+                for (int nn = 0; nn < 2; nn++) v[rt][nn][0] = v[rt][nn][1] = v[rt][nn][2] = v[rt][nn][3] = 0.f;
+#pragma unroll
+            for (int b = 0; b < HD / 64; b++) {
+                const uint4 kf0 = *(const uint4*)(kp + 64 * b), kf1 = *(const uint4*)(kp + 8 * HD + 64 * b);
+                const uint32_t w0[4] = {kf0.x, kf0.y, kf0.z, kf0.w}, w1[4] = {kf1.x, kf1.y, kf1.z, kf1.w};
+#pragma unroll
+                for (int st = 0; st < 4; st++) {
+                    const uint32_t b00 = kv_half2(w0[st], 0x4140), b01 = kv_half2(w0[st], 0x4342);
+                    const uint32_t b10 = kv_half2(w1[st], 0x4140), b11 = kv_half2(w1[st], 0x4342);
+#pragma unroll
+                    for (int rt = 0; rt < RT; rt++) {
+                        uint32_t a[4];
+                        ldsm_x4(a[0], a[1], a[2], a[3], qa[rt] + (b * 64 + st * 16) * 2);
+                        mma16816(v[rt][0], a, b00, b01);
+                        mma16816(v[rt][1], a, b10, b11);
+                    }
                 }
             }
-        }
-        named_bar_sync(1, NCW);
-        if (receiver) {
+            // ---- the scores proper
 #pragma unroll
-            for (int rt = 0; rt < RT; rt++) {
-                float c0[2], c1[2];
+            for (int rt = 0; rt < RT; rt++)
+#pragma unroll
+                for (int nn = 0; nn < 2; nn++)
+#pragma unroll
+                    for (int x = 0; x < 4; x++) {
+                        float& sv = v[rt][nn][x];
+                        sv = (sv - qoff[rt][x >> 1]) * ksc[nn][x & 1];
+                        if (!whole && kb + 8 * nn + 2 * t4 + (x & 1) >= lim[rt][x >> 1]) sv = -INFINITY;
+                    }
+            // ---- P of this warp's keys (times the value scales, rounded to f16 as the products see it) and its row sums. The first time
+            // with the references as they are; where a row has left its own (P times a value scale near the end of f16, or P past 2^24), and
+            // in the quad's first stage, once more with new ones.
+            uint4* xp = (uint4*)(xp_at + (j / C::QUADS & 1) * C::X_P);  // (a warp may still be reading the stage before's)
+            float sum[RT][2], pr[RT][2];
+#pragma unroll 1
+            for (bool again = false;; again = true) {
+                bool left[RT][2], any_left = j == quad;
+#pragma unroll
+                for (int rt = 0; rt < RT; rt++) {
+                    float pv[2][4];
+#pragma unroll
+                    for (int h2 = 0; h2 < 2; h2++) {
+                        const float mm = m[rt][h2] == -INFINITY ? 0.f : m[rt][h2];
+                        sum[rt][h2] = 0.f;
+#pragma unroll
+                        for (int nn = 0; nn < 2; nn++)
+#pragma unroll
+                            for (int e = 0; e < 2; e++) {
+                                const float pp = tc::ex2(v[rt][nn][2 * h2 + e] - mm);
+                                sum[rt][h2] += pp;
+                                pv[nn][2 * h2 + e] = pp * vsc[nn][e];
+                            }
+                        left[rt][h2] = fmaxf(fmaxf(pv[0][2 * h2], pv[0][2 * h2 + 1]), fmaxf(pv[1][2 * h2], pv[1][2 * h2 + 1])) > 32768.f || sum[rt][h2] > 0x1p24f;
+                        any_left |= left[rt][h2];
+                    }
+                    uint4 pa;
+                    pa.x = pack_half2(pv[0][0], pv[0][1]); pa.y = pack_half2(pv[0][2], pv[0][3]);
+                    pa.z = pack_half2(pv[1][0], pv[1][1]); pa.w = pack_half2(pv[1][2], pv[1][3]);
+                    xp[(w * RT + rt) * 32 + lane] = pa;
+                    const float2 f0 = __half22float2(*(const __half2*)&pa.x), f1 = __half22float2(*(const __half2*)&pa.y);
+                    const float2 f2 = __half22float2(*(const __half2*)&pa.z), f3 = __half22float2(*(const __half2*)&pa.w);
+                    pr[rt][0] = f0.x + f0.y + f2.x + f2.y;
+                    pr[rt][1] = f1.x + f1.y + f3.x + f3.y;
+                }
+                if (again) {
+                    named_bar_sync(2 + quad, 128);
+                    break;
+                }
+                if (!named_bar_or(2 + quad, 128, any_left)) break;
+#pragma unroll
+                for (int rt = 0; rt < RT; rt++)
+#pragma unroll
+                    for (int h2 = 0; h2 < 2; h2++) {
+                        float x = fmaxf(fmaxf(v[rt][0][2 * h2], v[rt][0][2 * h2 + 1]), fmaxf(v[rt][1][2 * h2], v[rt][1][2 * h2 + 1]));
+                        x = fmaxf(x, __shfl_xor_sync(0xffffffffu, x, 1));
+                        x = fmaxf(x, __shfl_xor_sync(0xffffffffu, x, 2));
+                        const bool lf = (__ballot_sync(0xffffffffu, left[rt][h2]) >> (4 * r) & 15) != 0;
+                        if (t4 == 0) xmax[(w * RT + rt) * 16 + r + 8 * h2] = make_float2(x, lf ? 1.f : 0.f);
+                    }
+                named_bar_sync(2 + quad, 128);
+#pragma unroll
+                for (int rt = 0; rt < RT; rt++) {
+                    float corr[2];
+#pragma unroll
+                    for (int h2 = 0; h2 < 2; h2++) {
+                        float mn = m[rt][h2];
+                        bool moves = j == quad;
+#pragma unroll
+                        for (int ww = 0; ww < 4; ww++) {
+                            const float2 x = xmax[(ww * RT + rt) * 16 + r + 8 * h2];
+                            mn = fmaxf(mn, x.x);
+                            moves |= x.y != 0.f;
+                        }
+                        moves &= mn > m[rt][h2];  // (it depends on the row's own scores alone, not on what else is in the step)
+                        corr[h2] = moves ? exp2f(m[rt][h2] - mn) : 1.f;
+                        if (moves) m[rt][h2] = mn;
+                        l[rt][h2] *= corr[h2];
+                        ps[rt][h2] *= corr[h2];
+                    }
+#pragma unroll
+                    for (int jd = 0; jd < 8; jd++) {
+                        o[rt][jd][0] *= corr[0]; o[rt][jd][1] *= corr[0];
+                        o[rt][jd][2] *= corr[1]; o[rt][jd][3] *= corr[1];
+                    }
+                }
+            }
+            // (a lane sums its own keys; lanes and warps are added up once, after the last stage)
+#pragma unroll
+            for (int rt = 0; rt < RT; rt++)
 #pragma unroll
                 for (int h2 = 0; h2 < 2; h2++) {
-                    const float m1 = mb[(RT * 32 + rt * 6 + h2) * 32], mn = fmaxf(m[rt][h2], m1);
-                    c0[h2] = mn == -INFINITY ? 1.f : exp2f(m[rt][h2] - mn);
-                    c1[h2] = mn == -INFINITY ? 1.f : exp2f(m1 - mn);
-                    m[rt][h2] = mn;
-                    l[rt][h2] = l[rt][h2] * c0[h2] + mb[(RT * 32 + rt * 6 + 2 + h2) * 32] * c1[h2];
-                    ps[rt][h2] = ps[rt][h2] * c0[h2] + mb[(RT * 32 + rt * 6 + 4 + h2) * 32] * c1[h2];
+                    l[rt][h2] += sum[rt][h2];
+                    ps[rt][h2] += pr[rt][h2];
                 }
+            // (the barrier above: all of the quad is done with its stage before this one, and the slot's barrier is armed)
+            if (refill && lane == 0) copy(j - 2 + NSTG, w);
+            // ---- values: O += P V over the stage's 64 keys, this warp's 64 output dims
 #pragma unroll
-                for (int jd = 0; jd < 8; jd++)
+            for (int kbk = 0; kbk < 4; kbk++) {
+                uint32_t pa[RT][4];
 #pragma unroll
-                    for (int e = 0; e < 4; e++)
-                        o[rt][jd][e] = o[rt][jd][e] * c0[e >> 1] + mb[((rt * 8 + jd) * 4 + e) * 32] * c1[e >> 1];
-            }
-        }
-        named_bar_sync(1, NCW);
-    }
-    if (quad != 0) return;
-    // the rows' sums: over a row's four lanes, then over the four warps in order
-#pragma unroll
-    for (int rt = 0; rt < RT; rt++)
-#pragma unroll
-        for (int h2 = 0; h2 < 2; h2++) {
-            float a = l[rt][h2], b = ps[rt][h2];
-            a += __shfl_xor_sync(0xffffffffu, a, 1); b += __shfl_xor_sync(0xffffffffu, b, 1);
-            a += __shfl_xor_sync(0xffffffffu, a, 2); b += __shfl_xor_sync(0xffffffffu, b, 2);
-            if (t4 == 0) xsum[(w * RT + rt) * 16 + r + 8 * h2] = make_float2(a, b);
-        }
-    named_bar_sync(2, 128);
-#pragma unroll
-    for (int rt = 0; rt < RT; rt++)
-#pragma unroll
-        for (int h2 = 0; h2 < 2; h2++) {
-            float L = 0.f, P = 0.f;
-#pragma unroll
-            for (int ww = 0; ww < 4; ww++) {
-                const float2 x = xsum[(ww * RT + rt) * 16 + r + 8 * h2];
-                L += x.x;
-                P += x.y;
-            }
-            const int row = rt * 16 + r + 8 * h2, tok = row / GROUP;
-            if (tok >= nt) continue;
-            const int i = first + tok, t = dtok[i], head = g * GROUP + row % GROUP;
-            if (ns == 1) {
-                const float f = 1.f / L;
-                float* op = out + (size_t)t * MIX + head * HD + 64 * w + 2 * t4;
+                for (int rt = 0; rt < RT; rt++) {
+                    const uint4 x = xp[(kbk * RT + rt) * 32 + lane];
+                    pa[rt][0] = x.x; pa[rt][1] = x.y; pa[rt][2] = x.z; pa[rt][3] = x.w;
+                }
+                const uint8_t* vp = base + SK * HD + kbk * 16 * HD + (64 * w + r) * 16 + t4 * 4;
 #pragma unroll
                 for (int jd = 0; jd < 8; jd++) {
-                    const float2 gt = *(float2*)(op + jd * 8);
-                    *(float2*)(op + jd * 8) = make_float2(gt.x * (o[rt][jd][2 * h2] - KV_OFF * P) * f,
-                                                          gt.y * (o[rt][jd][2 * h2 + 1] - KV_OFF * P) * f);
-                }
-            } else {
-                const size_t pi = ((size_t)i * NH + head) * z + s;
-                float* pp = part_acc + pi * HD + 64 * w + 2 * t4;
+                    const uint32_t vw = *(const uint32_t*)(vp + jd * 8 * 16);
+                    const uint32_t b0 = kv_half2(vw, 0x4140), b1 = kv_half2(vw, 0x4342);
 #pragma unroll
-                for (int jd = 0; jd < 8; jd++)
-                    *(float2*)(pp + jd * 8) = make_float2(o[rt][jd][2 * h2] - KV_OFF * P, o[rt][jd][2 * h2 + 1] - KV_OFF * P);
-                if (w == 0 && t4 == 0) { part_ml[pi * 2] = m[rt][h2]; part_ml[pi * 2 + 1] = L; }
+                    for (int rt = 0; rt < RT; rt++) mma16816(o[rt][jd], pa[rt], b0, b1);
+                }
+            }
+            if (C::QUADS > 2 && j + NSTG < nstg) {  // (few stages more than quads: the next stage's barrier would be late)
+                if (w == 0 && lane == 0) arm(j + NSTG);
+                named_bar_sync(2 + quad, 128);
+                if (lane == 0) copy(j + NSTG, w);
             }
         }
+
+        // ---- the quads merge pairwise through the ring, which is free (every stage was consumed): 1 -> 0 and 3 -> 2, then
+        // 2 -> 0. A warp's registers go to the warp of the same index in the other quad (same rows, same dims).
+        named_bar_sync(1, NCW);
+        // With many splits a quad that has handed its registers over asks for the next one's first stages meanwhile, those that go behind the
+        // slots of the merge; the others when the merge is done, and then it goes on. (Where the results of this one go: `was`.)
+        const int4 was = make_int4(first, nt, g, s);
+        const int was_ns = ns;
+        bool more = false;
+        auto go_on = [&]() {
+            at += nstg + SPLIT_COST;
+            more = at < until;
+            if (!more) return;
+#pragma unroll
+            for (int sl = 0; sl < NSTG; sl++) {
+                const int j = (sl + NSTG - OFF) % NSTG;  // the first stage in this slot
+                if (j < nstg) pars ^= (((nstg - 1 - j) / NSTG + 1) & 1) << sl;
+            }
+            j0 += nstg;
+            fresh = false;
+            if (++s == ns) {
+                s = 0;
+                fresh = true;
+                if (++g == NKV) {
+                    g = 0;
+                    const int4 x = segs[++seg];
+                    first = x.x; nt = x.y; keys = x.z; slot = x.w;
+                    my_tok = dtok[first + min(lane, nt - 1)];
+                    my_pos = tok_pos[my_tok];
+                    splits();
+                }
+            }
+            split();
+            begin = min(nstg, NSTG);
+        };
+        auto begin_with = [&](int a, int b) {  // stages a up to b: a warp of the second quad each
+            const int j = a + w;
+            if (j < min(b, begin) && lane == 0) {
+                arm(j);
+                for (int part = 0; part < 4; part++) copy(j, part);
+            }
+            __syncwarp();
+        };
+        static_assert(!MANY || (NSTG - OFF <= 4 && OFF <= 4), "a warp of a quad per stage");
+        constexpr int MF = RT * 8 * 4 + RT * 6;  // floats per lane
+        for (int round = 1; round < C::QUADS; round <<= 1) {
+            const bool sender = (quad & (2 * round - 1)) == round;
+            const bool receiver = (quad & (2 * round - 1)) == 0 && quad + round < C::QUADS;
+            float* mb = (float*)ring + (size_t)(((quad >> 1) / round % 2) * 4 + w) * 32 * MF + lane;
+            if (sender) {
+#pragma unroll
+                for (int rt = 0; rt < RT; rt++) {
+#pragma unroll
+                    for (int jd = 0; jd < 8; jd++)
+#pragma unroll
+                        for (int e = 0; e < 4; e++) mb[((rt * 8 + jd) * 4 + e) * 32] = o[rt][jd][e];
+#pragma unroll
+                    for (int h2 = 0; h2 < 2; h2++) {
+                        mb[(RT * 32 + rt * 6 + h2) * 32] = m[rt][h2];
+                        mb[(RT * 32 + rt * 6 + 2 + h2) * 32] = l[rt][h2];
+                        mb[(RT * 32 + rt * 6 + 4 + h2) * 32] = ps[rt][h2];
+                    }
+                }
+            }
+            if (MANY && sender) tc::async_proxy_fence();  // (copies are written there next)
+            named_bar_sync(1, NCW);
+            if (MANY && round == 1 && quad == 1) {
+                go_on();
+                if (more) begin_with(0, NSTG - OFF);
+            }
+            if (receiver) {
+#pragma unroll
+                for (int rt = 0; rt < RT; rt++) {
+                    float c0[2], c1[2];
+#pragma unroll
+                    for (int h2 = 0; h2 < 2; h2++) {
+                        const float m1 = mb[(RT * 32 + rt * 6 + h2) * 32], mn = fmaxf(m[rt][h2], m1);
+                        c0[h2] = mn == -INFINITY ? 1.f : exp2f(m[rt][h2] - mn);
+                        c1[h2] = mn == -INFINITY ? 1.f : exp2f(m1 - mn);
+                        m[rt][h2] = mn;
+                        l[rt][h2] = l[rt][h2] * c0[h2] + mb[(RT * 32 + rt * 6 + 2 + h2) * 32] * c1[h2];
+                        ps[rt][h2] = ps[rt][h2] * c0[h2] + mb[(RT * 32 + rt * 6 + 4 + h2) * 32] * c1[h2];
+                    }
+#pragma unroll
+                    for (int jd = 0; jd < 8; jd++)
+#pragma unroll
+                        for (int e = 0; e < 4; e++)
+                            o[rt][jd][e] = o[rt][jd][e] * c0[e >> 1] + mb[((rt * 8 + jd) * 4 + e) * 32] * c1[e >> 1];
+                }
+            }
+            named_bar_sync(1, NCW);
+        }
+        if (MANY && quad == 1 && more) begin_with(NSTG - OFF, NSTG);
+        if (quad == 0) {
+        // the rows' sums: over a row's four lanes, then over the four warps in order
+#pragma unroll
+        for (int rt = 0; rt < RT; rt++)
+#pragma unroll
+            for (int h2 = 0; h2 < 2; h2++) {
+                float a = l[rt][h2], b = ps[rt][h2];
+                a += __shfl_xor_sync(0xffffffffu, a, 1); b += __shfl_xor_sync(0xffffffffu, b, 1);
+                a += __shfl_xor_sync(0xffffffffu, a, 2); b += __shfl_xor_sync(0xffffffffu, b, 2);
+                if (t4 == 0) xsum[(w * RT + rt) * 16 + r + 8 * h2] = make_float2(a, b);
+            }
+        named_bar_sync(2, 128);
+#pragma unroll
+        for (int rt = 0; rt < RT; rt++)
+#pragma unroll
+            for (int h2 = 0; h2 < 2; h2++) {
+                float L = 0.f, P = 0.f;
+#pragma unroll
+                for (int ww = 0; ww < 4; ww++) {
+                    const float2 x = xsum[(ww * RT + rt) * 16 + r + 8 * h2];
+                    L += x.x;
+                    P += x.y;
+                }
+                const int row = rt * 16 + r + 8 * h2, tok = row / GROUP, head = was.z * GROUP + row % GROUP;
+                const bool in = tok < was.y;
+                if (was_ns == 1) {
+                    if (!in) continue;
+                    const float f = 1.f / L;
+                    float* op = out + (size_t)dtok[was.x + tok] * MIX + head * HD + 64 * w + 2 * t4;
+#pragma unroll
+                    for (int jd = 0; jd < 8; jd++) {
+                        const float2 gt = *(float2*)(op + jd * 8);
+                        *(float2*)(op + jd * 8) = make_float2(gt.x * (o[rt][jd][2 * h2] - KV_OFF * P) * f,
+                                                              gt.y * (o[rt][jd][2 * h2 + 1] - KV_OFF * P) * f);
+                    }
+                } else {
+                    // (neighbours swap, so that a lane writes 16 bytes and a row's four 64)
+                    const size_t pi = ((size_t)(was.x + tok) * NH + head) * z + was.w;
+                    float* pp = part_acc + pi * HD + 64 * w + (t4 & 1) * 8 + (t4 & 2) * 2;
+#pragma unroll
+                    for (int jd = 0; jd < 8; jd += 2) {
+                        const bool odd = t4 & 1;
+                        const float2 a = make_float2(o[rt][jd][2 * h2] - KV_OFF * P, o[rt][jd][2 * h2 + 1] - KV_OFF * P);
+                        const float2 b = make_float2(o[rt][jd + 1][2 * h2] - KV_OFF * P, o[rt][jd + 1][2 * h2 + 1] - KV_OFF * P);
+                        const float x = __shfl_xor_sync(0xffffffffu, odd ? a.x : b.x, 1), y = __shfl_xor_sync(0xffffffffu, odd ? a.y : b.y, 1);
+                        if (in) *(float4*)(pp + jd * 8) = odd ? make_float4(x, y, b.x, b.y) : make_float4(a.x, a.y, x, y);
+                    }
+                    if (in && w == 0 && t4 == 0) { part_ml[pi * 2] = m[rt][h2]; part_ml[pi * 2 + 1] = L; }
+                }
+            }
+        }
+        if constexpr (MANY) {
+            if (quad != 1) go_on();
+        }
+        if (!more) return;
+    }
 }
 
 // Merge the ns key splits of one (token, head) in split order; *op *= result (the gate is there); optionally also the
@@ -966,13 +1117,23 @@ int qb_attn_decode_as(qb_ctx* ctx, void* stream, const float* q, const void* kc,
     // (the model's steps have at most 64 decode tokens: whatever lies 64 positions or more before a segment's last key is from
     // earlier steps)
     const int old_margin = ahead && ndec <= 64 ? 64 : 0;
+    // One block per split where they are few; blocks that keep running where they would be more than four rounds of the SMs, or more than
+    // three with the last at most half full, if all sequences were as long as the longest. Block per split against that, us:
+    // 8 sequences x 4 rows, up to context 7777 59.5 / 48.5; 8 x 8 at 8000 99.3 / 90.5; 8 x 1 at 3000 37.0 / 34.0; 4 x 4 up to 8000
+    // (3.4 rounds) 37.0 / 34.4; but 6 x 8 at 3000 (3.9) 44.6 / 47.6, 4 x 4 up to 3000 (2.6) 22.3 / 23.3, 2 x 4 up to 3000 14.4 / 15.4:
+    // the table of the segments costs a microsecond before the first split.
+    const long long most = (long long)ndseg * NKV * dec_splits(max_keys, dsplits);
+    const bool many = ndseg <= DEC_SEGS && (most > 4 * ctx->sms || (most > 3 * ctx->sms && 2 * most <= 7 * ctx->sms));
     int rc;
 #define QB_DEC(RT, NQ)                                                                                          \
     {                                                                                                           \
         using C = Dec4Cfg<RT, NQ>;                                                                              \
-        rc = launch(ctx, attn_dec4_kernel<RT, NQ>, grid, dim3(C::THREADS), C::SMEM, st, q, (const uint8_t*)kc, \
-                    (const uint8_t*)vc, ks, vs, dseg, dtok, tok_slot, tok_pos, cap, z, dsplits, old_margin, part_ml,   \
-                    part_acc, out, ctx->err);                                                                             \
+        rc = many ? launch(ctx, attn_dec4_kernel<RT, NQ, true>, dim3(ctx->sms), dim3(C::THREADS), C::SMEM_MANY, st, q, (const uint8_t*)kc, \
+                           (const uint8_t*)vc, ks, vs, dseg, dtok, tok_slot, tok_pos, cap, z, dsplits, old_margin, ndseg, part_ml,   \
+                           part_acc, out, ctx->err)                                                                             \
+                  : launch(ctx, attn_dec4_kernel<RT, NQ, false>, grid, dim3(C::THREADS), C::SMEM, st, q, (const uint8_t*)kc, \
+                           (const uint8_t*)vc, ks, vs, dseg, dtok, tok_slot, tok_pos, cap, z, dsplits, old_margin, ndseg, part_ml,   \
+                           part_acc, out, ctx->err);                                                                             \
     }
     // quads per block: as many as leave every warp its registers (a warp holds RT x 32 output accumulators per lane);
     // measured at 5 rows with a copy warp beside them: 2 quads 33.4 us, 3 quads (spills) 36.6 us, 4 quads 43.2 us

@@ -338,6 +338,30 @@ def test_attn_decode_of_a_ragged_batch(ctx, rows):
     assert close(full.cpu().numpy(), want).all()
 
 
+@pytest.mark.parametrize("segs,rows", [(64, 1), (33, 3), (40, 7), (65, 1)])
+def test_attn_decode_splits_dealt_out(ctx, segs, rows):
+    """Blocks that take several splits each give every token the bits that its sequence alone gives: more segments than lanes, as many as
+    the table holds and one more, splits of one stage to several, sequences of one key beside long ones."""
+    g = synth.gen(177 + segs)
+    cap = 4480
+    ends = [1, 64, 65, 2048, 4470, 130] + [rows + int(torch.randint(0, 2600, (1,), generator=g)) for _ in range(segs - 6)]
+    cache = make_cache(segs, cap, g, 0)
+    toks = [(0, s, max(0, e - rows) + i) for s, e in enumerate(ends) for i in range(rows)]
+    n = len(toks)
+    q = (torch.randn(n, R.NH, R.HD, generator=g) * QSCALE).cuda()
+    gate = torch.sigmoid(torch.randn(n, R.MIX, generator=g)).cuda()
+    st = R.build_step(toks, list(range(n)), max_dec=n)
+    assert st["ndec"] == n
+    dc = [t.cuda() for t in cache]
+    full = run_decode(ctx, q, gate, dc, st, ref_cuda.upload_step(st), cap, n)
+    for s in (0, 1, 2, 3, 4, 5, 31, 32, segs - 2, segs - 1):
+        a, e = s * rows, (s + 1) * rows
+        st1 = R.build_step(toks[a:e], list(range(rows)))
+        one = run_decode(ctx, q[a:e].contiguous(), gate[a:e].contiguous(), dc, st1, ref_cuda.upload_step(st1), cap, rows)
+        assert torch.equal(one, full[a:e]), s
+    assert ctx.device_error() == 0
+
+
 @pytest.mark.parametrize("lens,pos0,cap,pairs", [
     ((25, 33, 12, 47, 280), (2080, 1700, 1900, 40, 1663), 2112, 1),
     ((50,) * 8, (8000, 30, 7990, 8060, 4000, 64, 8127, 2000), 8192, 1),      # 5 tiles each: runs of 1 to 4 tiles in a pair
