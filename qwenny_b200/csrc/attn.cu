@@ -705,17 +705,26 @@ attn_dec4_kernel(const float* q, const uint8_t* kc, const uint8_t* vc, const flo
 #pragma unroll
                 for (int nn = 0; nn < 2; nn++) v[rt][nn][0] = v[rt][nn][1] = v[rt][nn][2] = v[rt][nn][3] = 0.f;
 #pragma unroll
-            for (int b = 0; b < HD / 64; b++) {
-                const uint4 kf0 = *(const uint4*)(kp + 64 * b), kf1 = *(const uint4*)(kp + 8 * HD + 64 * b);
-                const uint32_t w0[4] = {kf0.x, kf0.y, kf0.z, kf0.w}, w1[4] = {kf1.x, kf1.y, kf1.z, kf1.w};
+            for (int b2 = 0; b2 < HD / 128; b2++) {
+                // Keys are 256 bytes apart, all in the same banks, so the lanes of odd keys read the two halves of 128 dims the other way
+                // round (5 rows at context 32000 30.35 -> 29.67 us; not with one row tile, whose warps have no registers left for it: 8
+                // sequences of one row 42.3 -> 44.8).
+                const bool odd = RT > 1 && (r & 1);
+                const uint8_t* p0 = kp + 128 * b2 + (odd ? 64 : 0);
+                const uint8_t* p1 = kp + 128 * b2 + (odd ? 0 : 64);
+                const uint4 x0 = *(const uint4*)p0, x1 = *(const uint4*)p1, y0 = *(const uint4*)(p0 + 8 * HD), y1 = *(const uint4*)(p1 + 8 * HD);
+                const uint32_t w0[8] = {odd ? x1.x : x0.x, odd ? x1.y : x0.y, odd ? x1.z : x0.z, odd ? x1.w : x0.w,
+                                        odd ? x0.x : x1.x, odd ? x0.y : x1.y, odd ? x0.z : x1.z, odd ? x0.w : x1.w};
+                const uint32_t w1[8] = {odd ? y1.x : y0.x, odd ? y1.y : y0.y, odd ? y1.z : y0.z, odd ? y1.w : y0.w,
+                                        odd ? y0.x : y1.x, odd ? y0.y : y1.y, odd ? y0.z : y1.z, odd ? y0.w : y1.w};
 #pragma unroll
-                for (int st = 0; st < 4; st++) {
+                for (int st = 0; st < 8; st++) {
                     const uint32_t b00 = kv_half2(w0[st], 0x4140), b01 = kv_half2(w0[st], 0x4342);
                     const uint32_t b10 = kv_half2(w1[st], 0x4140), b11 = kv_half2(w1[st], 0x4342);
 #pragma unroll
                     for (int rt = 0; rt < RT; rt++) {
                         uint32_t a[4];
-                        ldsm_x4(a[0], a[1], a[2], a[3], qa[rt] + (b * 64 + st * 16) * 2);
+                        ldsm_x4(a[0], a[1], a[2], a[3], qa[rt] + (b2 * 128 + st * 16) * 2);
                         mma16816(v[rt][0], a, b00, b01);
                         mma16816(v[rt][1], a, b10, b11);
                     }
