@@ -149,13 +149,116 @@ __global__ void __launch_bounds__(128) gemm_f16_wide_kernel(const uint4* __restr
     }
 }
 
+// That, where X lets a row be copied in 16-byte pieces: weights and the block's 32 rows come through shared memory, 64 columns at a time
+// and three such pieces under way in each of three blocks per SM (of registers a warp has room for one k16 step ahead, and 16 steps of it
+// are 16 times the way from L2). Same order of additions per output.
+constexpr int ST_PIECE = 64, ST_NP = 4, ST_ROW = ST_PIECE * 2 + 16;  // columns per piece, pieces, bytes per row of one (no bank conflicts)
+template <int TILES>
+struct StagedCfg {
+    static constexpr int W_BYTES = TILES * 4 * 512, BYTES = W_BYTES + 32 * ST_ROW;
+    static constexpr int RING = ST_NP * BYTES, RED = 3 * TILES * 4 * 32 * 16, SMEM = RING > RED ? RING : RED;
+};
+template <int TILES>
+__global__ void __launch_bounds__(128, 3) gemm_f16_staged_kernel(const uint4* __restrict__ W, const __half* __restrict__ X,
+                                                                 const int* __restrict__ xrows, int K, int ntiles, int n,
+                                                                 int kper, float* __restrict__ Y, int ldy) {
+    using C = StagedCfg<TILES>;
+    constexpr int NTT = 4;
+    extern __shared__ __align__(16) uint8_t st_raw[];
+    pdl_launch_dependents();
+    const int tile0 = blockIdx.x * TILES, split = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int g = lane >> 2, t = lane & 3, tok0 = blockIdx.z * (8 * NTT);
+    const int k0 = split * kper, k1 = min(K, k0 + kper), steps = (k1 - k0) / 16, pieces = (steps + 3) / 4;
+    const uint4* wp = W + ((size_t)tile0 * (K / 16) + k0 / 16 + warp) * 32 + lane;
+    auto fetch_w = [&](int pc) {  // a warp fetches the steps that it will multiply
+        if (pc * 4 + warp < steps)
+#pragma unroll
+            for (int i = 0; i < TILES; i++)
+                cp_async16(st_raw + (pc % ST_NP) * C::BYTES + (i * 4 + warp) * 512 + lane * 16, wp + ((size_t)i * (K / 16) + pc * 4) * 32);
+    };
+    for (int pc = 0; pc < ST_NP - 1; pc++) fetch_w(pc);  // (they do not depend on the kernel before)
+    pdl_wait();
+    const int c = threadIdx.x & 7, r0 = threadIdx.x >> 3;
+    const __half* row[2];  // the thread's 16 bytes of two rows
+#pragma unroll
+    for (int i = 0; i < 2; i++) {
+        const int tok = min(tok0 + r0 + 16 * i, n - 1);  // (a token past the last repeats it and is not written)
+        row[i] = X + (size_t)(xrows ? xrows[tok] : tok) * K + k0 + c * 8;
+    }
+    auto fetch_x = [&](int pc) {
+        if (pc * ST_PIECE + c * 8 < k1 - k0)
+#pragma unroll
+            for (int i = 0; i < 2; i++)
+                cp_async16(st_raw + (pc % ST_NP) * C::BYTES + C::W_BYTES + (r0 + 16 * i) * ST_ROW + c * 16, row[i] + pc * ST_PIECE);
+    };
+    for (int pc = 0; pc < ST_NP - 1; pc++) {
+        fetch_x(pc);
+        cp_async_commit();
+    }
+    float acc[TILES][NTT][4];
+#pragma unroll
+    for (int i = 0; i < TILES; i++)
+#pragma unroll
+        for (int j = 0; j < NTT; j++) acc[i][j][0] = acc[i][j][1] = acc[i][j][2] = acc[i][j][3] = 0.f;
+    const int xat = C::W_BYTES + ((lane & 7) + (lane >> 4) * 8) * ST_ROW + ((lane >> 3) & 1) * 16 + warp * 32;
+    for (int pc = 0; pc < pieces; pc++) {
+        asm volatile("cp.async.wait_group %0;\n" ::"n"(ST_NP - 2) : "memory");
+        __syncthreads();  // (the piece is there, and all are done with the one before it)
+        fetch_w(pc + ST_NP - 1);
+        fetch_x(pc + ST_NP - 1);
+        cp_async_commit();
+        if (pc * 4 + warp < steps) {
+            const uint8_t* base = st_raw + (pc % ST_NP) * C::BYTES;
+            uint32_t b[NTT][2];
+            ldsm_x4(b[0][0], b[0][1], b[1][0], b[1][1], smem_u32(base) + xat);
+            ldsm_x4(b[2][0], b[2][1], b[3][0], b[3][1], smem_u32(base) + xat + 16 * ST_ROW);
+#pragma unroll
+            for (int i = 0; i < TILES; i++) {
+                const uint4 w = *(const uint4*)(base + (i * 4 + warp) * 512 + lane * 16);
+                const uint32_t a[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+                for (int j = 0; j < NTT; j++) mma16816(acc[i][j], a, b[j][0], b[j][1]);
+            }
+        }
+    }
+    cp_async_wait_all();
+    __syncthreads();
+    float4(*red)[TILES][NTT][32] = (float4(*)[TILES][NTT][32])st_raw;
+    if (warp > 0) {
+#pragma unroll
+        for (int i = 0; i < TILES; i++)
+#pragma unroll
+            for (int j = 0; j < NTT; j++)
+                red[warp - 1][i][j][lane] = make_float4(acc[i][j][0], acc[i][j][1], acc[i][j][2], acc[i][j][3]);
+    }
+    __syncthreads();
+    if (warp == 0) {
+        float* y = Y + (size_t)split * n * ldy;
+#pragma unroll
+        for (int i = 0; i < TILES; i++)
+#pragma unroll
+            for (int j = 0; j < NTT; j++) {
+#pragma unroll
+                for (int ww = 0; ww < 3; ww++) {
+                    const float4 v = red[ww][i][j][lane];
+                    acc[i][j][0] += v.x; acc[i][j][1] += v.y; acc[i][j][2] += v.z; acc[i][j][3] += v.w;
+                }
+#pragma unroll
+                for (int e = 0; e < 4; e++) {
+                    const int tok = tok0 + 8 * j + 2 * t + (e & 1), r = (tile0 + i) * 16 + g + (e >> 1) * 8;
+                    if (tok < n) y[(size_t)tok * ldy + r] = acc[i][j][e];
+                }
+            }
+    }
+}
+
 }  // namespace qb
 
 using namespace qb;
 
 // Tiles per block. More than one from the row count on at which one per block fills the SMs (5/6 of a block each): below that, more
-// blocks in flight are worth more than X loaded once. 96 x 5120 in 5 splits, one tile per block against six: 33 rows 5.9 and
-// 7.8 us, 128 rows (120 blocks) 7.1 and 8.0, 160 rows (150) 8.5 and 8.0, 333 rows 11.3 and 8.7, 2048 rows 37.0 and 17.0.
+// blocks in flight are worth more than X loaded once. 96 x 5120 in 5 splits, one tile per block against six (X gathered): 33 rows 5.9
+// and 7.8 us, 128 rows (120 blocks) 7.1 and 8.0, 160 rows (150) 8.5 and 8.0, 333 rows 11.3 and 8.7, 2048 rows 37.0 and 17.0.
 // Six tiles of a split of less than 256 columns leave a warp a few steps: there four blocks of one tile per SM are as good
 // (40 splits, 64 rows, 480 blocks: 3.1 and 3.3 us; 96 rows, 720 blocks: 4.8 and 3.5). Blocks of two save little work each
 // and lose where their second wave is partly filled (5 splits of 1024: 160 outputs, 200 rows, 175 blocks of two 11.4 and
@@ -184,9 +287,16 @@ extern "C" int qb_gemm_f16_plain(qb_ctx* ctx, void* stream, const void* W, const
     const int per = qb_gemm_f16_block_tiles(ntiles, split, kper, n, ctx->sms);
     if (per > 1) {
         grid.x = ntiles / per;
-        if (per == 6) return launch(ctx, gemm_f16_wide_kernel<6>, grid, dim3(128), 0, st, w, x, xrows, K, ntiles, n, kper, Y, ldy);
-        if (per == 4) return launch(ctx, gemm_f16_wide_kernel<4>, grid, dim3(128), 0, st, w, x, xrows, K, ntiles, n, kper, Y, ldy);
-        return launch(ctx, gemm_f16_wide_kernel<2>, grid, dim3(128), 0, st, w, x, xrows, K, ntiles, n, kper, Y, ldy);
+        // X gathered against copied, 96 x 5120 in 5 splits, X from four buffers in turn: 160 rows 8.2 and 7.8 us, 512 9.9 and 8.2, 1024 10.8
+        // and 11.0, 2048 23.7 and 12.3; 160 outputs, 1024 rows 19.8 and 12.5; 768 x 2048 in 2 splits, 1024 rows 19.3 and 20.1.
+        const bool whole = ((uintptr_t)x & 15) == 0;  // (K and kper are multiples of 16)
+#define QB_WIDE(T)                                                                                                                    \
+    return whole ? launch(ctx, gemm_f16_staged_kernel<T>, grid, dim3(128), StagedCfg<T>::SMEM, st, w, x, xrows, K, ntiles, n, kper, Y, ldy) \
+                 : launch(ctx, gemm_f16_wide_kernel<T>, grid, dim3(128), 0, st, w, x, xrows, K, ntiles, n, kper, Y, ldy)
+        if (per == 6) QB_WIDE(6);
+        if (per == 4) QB_WIDE(4);
+        QB_WIDE(2);
+#undef QB_WIDE
     }
     return launch(ctx, gemm_f16_plain_kernel<4>, grid, dim3(128), 0, st, w, x, xrows, K, ntiles, n, kper, Y, ldy);
 }

@@ -152,3 +152,18 @@ def test_gemm_f16_blocks_of_tiles_have_the_bits_of_one_tile(ctx, n, tiles, kper,
     slabs = [ctx.gemm_f16_plain(wp, x, min(32, n - a), K, tiles, kper, xrows=rows[a:a + 32].contiguous()) for a in range(0, n, 32)]
     torch.cuda.synchronize()
     assert torch.equal(y, torch.cat(slabs, 1))
+
+
+@pytest.mark.parametrize("n,tiles,kper", [(700, 6, 256), (1633, 4, 144), (261, 10, 384)])
+def test_gemm_f16_rows_off_16_bytes(ctx, n, tiles, kper):
+    """Rows that start on 16 bytes are copied in such pieces, others gathered: the same bits."""
+    K = 384
+    g = synth.gen(590 + n)
+    wp = torch.from_numpy(R.pack_f16((torch.randn(tiles * 16, K, generator=g) * 0.1).half().numpy())).cuda()
+    x = torch.randn(n, K, generator=g).half().cuda()
+    off = torch.empty(n * K + 2, dtype=torch.half, device="cuda")[2:].view(n, K)
+    off.copy_(x)
+    assert x.data_ptr() % 16 == 0 and off.data_ptr() % 16 == 4
+    a, b = ctx.gemm_f16_plain(wp, x, n, K, tiles, kper), ctx.gemm_f16_plain(wp, off, n, K, tiles, kper)
+    torch.cuda.synchronize()
+    assert torch.equal(a, b)
