@@ -47,6 +47,7 @@ void qb_destroy(qb_ctx* ctx);
  *   11 .. 13 prompt attention on tcgen05 (products, softmax, conversion)
  *   14 .. 17 W4A16 product, 17 to 64 rows (copies, unpacking, draining, products)
  *   20 .. 22 delta rule in chunks (copies, products, state)
+ *   23       sampler (copies of a slice)
  *   99       qb_wait_probe's test */
 int qb_device_error(qb_ctx* ctx);
 int qb_sm_count(const qb_ctx* ctx); /* 0 for a null context */

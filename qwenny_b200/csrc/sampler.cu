@@ -239,7 +239,7 @@ __global__ void __launch_bounds__(STH, 1) sampler_kernel(const SamplerArgs a) {
             if (rank == 0 && tid == 0) a.out_acc[j] = -1;
             if (bulk && tid == 0)  // (its copies do not outlive the block)
                 for (int i = 0; i < pieces; i++)
-                    if (!mbar_wait(&bar[i], 0)) atomicExch(a.err, 22);
+                    if (!mbar_wait(&bar[i], 0)) atomicExch(a.err, 23);
             return;
         }
         k = greedy ? 1 : wide ? min(QCAP, a.W) : min(top_k, a.W);
@@ -284,7 +284,7 @@ __global__ void __launch_bounds__(STH, 1) sampler_kernel(const SamplerArgs a) {
     static_assert(PIECE % (4 * STH) == 0, "a round lies in one piece");
 #pragma unroll 1
     for (int base = 0; base < n_loc; base += 4 * STH) {
-        if (bulk && base % PIECE == 0 && base < n4 && !mbar_wait(&bar[base / PIECE], 0) && lane == 0) atomicExch(a.err, 22);
+        if (bulk && base % PIECE == 0 && base < n4 && !mbar_wait(&bar[base / PIECE], 0) && lane == 0) atomicExch(a.err, 23);
         const int i4 = base + tid * 4, nv = min(4, n_loc - i4);
         if (nv <= 0) continue;
         float v[4];
