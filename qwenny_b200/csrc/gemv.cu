@@ -276,12 +276,12 @@ extern "C" int qb_marlin_gemm(qb_ctx* ctx, void* stream, const void* X, const vo
     if (m > 64 && epi != QB_EPI_ARGMAX && !xrows && !ctx->no_tc)
         return qb_gemm_tc_launch(ctx, st, X, B, Y, S, m, n, k, row0, epi, 0);
     // slabs: 17 .. 64 rows through the tensor-core product for a few rows, up to 16 through the skinny kernel. At 16 rows the
-    // skinny kernel takes 22, 11, 31 and 24 us over the layer's four shapes, at 17 the other 17, 11, 32 and 20 (two skinny
-    // slabs 43, 22, 62 and 48); 40 gathered rows of a 248,320-row output layer take 577 us as three 16-row slabs, 218 so.
+    // skinny kernel takes 22, 10, 30 and 21 us over the layer's four shapes, at 17 the other 16, 11, 30 and 19 (two skinny
+    // slabs 43, 20, 60 and 42); 40 gathered rows of a 248,320-row output layer take 577 us as three 16-row slabs, 207 so.
     // The upper bound is that of its tiles, not where times cross: the prompt-sized product has no gathered and no argmax
     // form, and it rounds each weight to f16, which is exact for bf16 scales only (error against 64 bits 5e-5; with the
     // group's scale applied to the f32 sum 8e-7, as up to 16 rows). At 17 rows it takes 19, 14, 38 and 24 us, at 64 20, 15, 41 and 27
-    // against 20, 14, 36 and 24.
+    // against 20, 14, 37 and 25.
     int mm;
     for (int r = 0; r < m; r += mm) {
         mm = m - r;

@@ -4,13 +4,13 @@
 //
 // A block owns 128 outputs and the weights go from registers to tensor memory in the layout that a Marlin word already has
 // (w4a16_gemm_tc.cu). The floor is the weights' way from HBM (0.52 bytes each, read once): 760 cycles per block and stage, two groups
-// of 128 of k. A stage takes some 1440 (40 rows of a 248,320-output matrix, 262 stages a block): the way of a slot of tensor memory from
-// "free" to "multiplied" (unpacking 680, the issue of 16 products 800, 130 to 150 per check of a barrier, two slots in turn), and 40 KB through
-// shared memory a stage, 24 of them the rows again. What a launch spends beside its stages: 3 us from its first instruction to the
+// of 128 of k. A stage takes some 1350 (40 rows of a 248,320-output matrix, 262 stages a block): the way of a slot of tensor memory from
+// "free" to "multiplied" (unpacking 680, the issue of 16 products 800, 130 to 150 per check of a barrier; a group's slot each, 4 to 6 of
+// them in turn: with a slot per stage, two in turn, a stage took 1440), and 40 KB through shared memory a stage, 24 of them the rows again. What a launch spends beside its stages: 3 us from its first instruction to the
 // first unpacked stage, 3 us from a cut tile's last sum to its result (partial sums 0.2, fence and ticket 1.1, parts 0.6, epilogue 0.7).
-// From a graph, 40 rows: the MLP 60.0 us (one group per stage, a fence per thread and 64-bit divisions before the ticket, one round
-// trip per part, shares whatever the shape: 78.7), 5120 x 6144 12.5 (19.6), the output layer of 248,320 rows 218 (298); 17 and 64 rows of
-// the MLP 55.0 (72) and 64.2 (86.5). What differs from the prompt-sized product:
+// From a graph, 40 rows: the MLP 56.4 us (one group per stage, a fence per thread and 64-bit divisions before the ticket, one round
+// trip per part, shares whatever the shape: 78.7), 5120 x 6144 12.0 (19.6), the output layer of 248,320 rows 207 (298); 17 and 64 rows of
+// the MLP 52.5 (72) and 64.0 (86.5). What differs from the prompt-sized product:
 //   - the weights are the exact integers q - 8; a group of 128 columns is one accumulation, and the drain warps multiply its
 //     f32 sums by the f32 value of the group's scale and add them up in registers (one thread per output, a register
 //     per token): one rounding per group, the arithmetic of the product for up to 16 rows (w4a16_gemv.cuh), where
@@ -20,7 +20,7 @@
 //     the scales and sums took 1000 cycles a group and was what everything waited for)
 //   - a drain warp takes 16 tokens: with 32 its threads held 64 values and spilled
 //   - gathered rows (the output layer) are copied together first, by a launch of their own: gathered by cp.async in every block they slowed
-//     the unpacking from 680 to 1070 cycles a stage (40 rows of 248,320 outputs 269 us against 218, launch included)
+//     the unpacking from 680 to 1070 cycles a stage (40 rows of 248,320 outputs 269 us against 218 at that time, launch included)
 // The (tile, group) list is dealt to at most one block per SM: whole tiles, tiles cut into equal parts, or equal shares; parts of a cut tile are added by its last arriver in
 // block order (the bits repeat). Its ticket is taken behind a barrier by one thread with one fence (a fence per thread: 2 us; a ticket
 // per warp instead of the barriers: the output layer 241 us against 232).
