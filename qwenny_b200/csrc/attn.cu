@@ -579,9 +579,10 @@ attn_dec4_kernel(const float* q, const uint8_t* kc, const uint8_t* vc, const flo
         const uint32_t bytes = part < 2 ? SK * HD : SK * 4, to = part < 2 ? part * SK * HD : 2 * SK * HD + (part - 2) * SK * 4;
         bulk_g2s(ring + place(j) * STG_BYTES + to, from + (size_t)j * bytes, bytes, &full[place(j)], pol);
     };
-    auto arm = [&](int j) {
-        mbar_expect_tx(&full[place(j)], STG_BYTES);
-        issued[place(j)] = j;
+    auto arm = [&](int i) {
+        const int j = j0 + i;  // (counted through the block's splits: a number of the split before says nothing of this one)
+        mbar_expect_tx(&full[place(i)], STG_BYTES);
+        issued[place(i)] = j;
     };
     int begin = min(nstg, NSTG);
     if (warp < begin && lane == 0) arm(warp);
@@ -673,7 +674,7 @@ attn_dec4_kernel(const float* q, const uint8_t* kc, const uint8_t* vc, const flo
                 // waits for its last stage's copies would be let through. A stage is asked for only when that one was consumed.
                 uint32_t polls = 0;
                 if (j >= NSTG)
-                    while (issued[sl] != j && polls < WAIT_LIMIT) polls++;
+                    while (issued[sl] != j0 + j && polls < WAIT_LIMIT) polls++;
                 dead = polls == WAIT_LIMIT || !mbar_wait(&full[sl], par);
                 if (dead && lane == 0) atomicExch(err, 4);
             } else {
