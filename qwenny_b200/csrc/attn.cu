@@ -430,11 +430,11 @@ attn_decode_kernel(const float* q, const uint8_t* kc, const uint8_t* vc, const f
 // The int8 codes go to the tensor cores as 1152 + q halves (one prmt per pair) and the offset is folded out through the
 // row sums, as in the reference (kernels/attn.cuh:38-40,198-234). The quads' partial results meet in shared memory
 // at the end; the block writes one (m, l, acc) partial per row, or the finished rows when the segment has one split.
-// Bound by latency: at 5 rows a quad's stage takes 4400 cycles (scores 1400, softmax and barrier 1050, values 1100, waits and copies 700) with
+// Bound by latency: at 5 rows a quad's stage takes 4100 cycles (scores 1250, softmax and barrier 920, values 1280, waits and copies 650) with
 // two warps per scheduler, and a block 3000 before its first stage behind the kernel before, 3000 after its last. From a graph with
 // attn_prep and the combine, us, before (a copy warp, maxima in every stage, Q row by row) / now: 5 rows at 100 keys 13.5 / 11.2, at 4000
-// 18.4 / 15.1, at 32000 35.0 / 30.5; 1 row at 32000 26.2 / 24.1; 8 rows 50.6 / 40.2 (registers spilled before); 8 sequences of 4 rows at 972
-// to 7777 66.5 / 59.7, at 4000 to 32000 140 / 128.5.
+// 18.4 / 15.1, at 32000 35.0 / 29.6; 1 row at 32000 26.2 / 24.1; 8 rows 50.6 / 39.4 (registers spilled before); 8 sequences of 4 rows at 972
+// to 7777 66.5 / 49.7 (59.7 with a block per split), at 4000 to 32000 140 / 111.9 (128.5).
 // Many splits (MANY): a block per split would pay for each one's start (its segment's tokens, Q, the first stages' way from memory: half of
 // the 11 us that a split of four stages took) and leave the last round of the SMs partly idle. So a block per SM takes a run of them, equal
 // shares of the line on which each split is as long as its stages and SPLIT_COST: Q stays where the run stays with a segment's kv head,

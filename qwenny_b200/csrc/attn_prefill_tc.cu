@@ -11,7 +11,7 @@
 // the int8 -> f16 conversion and the shared memory per block are half of what one block per tile pair needs.
 // Over a pair an instruction takes some 128 cycles whatever its N, so the stage is 128 keys: 2048 rows at context 30720 take 2.79
 // ms with one block per two tiles and 64-key stages, 2.66 as pairs with 64-key stages (S then takes 2000 of 3100 cycles
-// per stage), 2.02 as pairs with 128. The pair passes over its tiles once per run of consecutive tiles of one sequence.
+// per stage), 2.02 as pairs with 128, 1.96 with whole warps at the barriers. The pair passes over its tiles once per run of consecutive tiles of one sequence.
 //   warps 8-15  read the block's share of a stage's int8 keys and values from the cache (128-bit loads, one stage ahead in
 //               registers) and write it as f16 where the tensor core wants it: K as four [64 keys][64 dims] K-major
 //               tiles, V transposed as two [128 dims][64 keys] tiles, with the 128-byte swizzle; the codes are
