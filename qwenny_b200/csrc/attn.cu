@@ -278,13 +278,20 @@ attn_decode_kernel(const float* q, const uint8_t* kc, const uint8_t* vc, const f
             // S = Q K^T
             float sacc[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
 #pragma unroll
-            for (int b = 0; b < HD / 64; b++) {
-                uint4 kf0 = *(const uint4*)(kp + 64 * b), kf1 = *(const uint4*)(kp + 8 * HD + 64 * b);
-                uint32_t w0[4] = {kf0.x, kf0.y, kf0.z, kf0.w}, w1[4] = {kf1.x, kf1.y, kf1.z, kf1.w};
+            for (int b2 = 0; b2 < HD / 128; b2++) {
+                // (odd keys' lanes read the two halves of 128 dims the other way round: attn_dec4_kernel)
+                const bool odd = r & 1;
+                const uint8_t* p0 = kp + 128 * b2 + (odd ? 64 : 0);
+                const uint8_t* p1 = kp + 128 * b2 + (odd ? 0 : 64);
+                const uint4 x0 = *(const uint4*)p0, x1 = *(const uint4*)p1, y0 = *(const uint4*)(p0 + 8 * HD), y1 = *(const uint4*)(p1 + 8 * HD);
+                const uint32_t w0[8] = {odd ? x1.x : x0.x, odd ? x1.y : x0.y, odd ? x1.z : x0.z, odd ? x1.w : x0.w,
+                                        odd ? x0.x : x1.x, odd ? x0.y : x1.y, odd ? x0.z : x1.z, odd ? x0.w : x1.w};
+                const uint32_t w1[8] = {odd ? y1.x : y0.x, odd ? y1.y : y0.y, odd ? y1.z : y0.z, odd ? y1.w : y0.w,
+                                        odd ? y0.x : y1.x, odd ? y0.y : y1.y, odd ? y0.z : y1.z, odd ? y0.w : y1.w};
 #pragma unroll
-                for (int st = 0; st < 4; st++) {
+                for (int st = 0; st < 8; st++) {
                     uint32_t a[4];
-                    ldsm_x4(a[0], a[1], a[2], a[3], qa + (b * 64 + st * 16) * 2);
+                    ldsm_x4(a[0], a[1], a[2], a[3], qa + (b2 * 128 + st * 16) * 2);
                     mma16816(sacc[0], a, kv_half2(w0[st], 0x4140), kv_half2(w0[st], 0x4342));
                     mma16816(sacc[1], a, kv_half2(w1[st], 0x4140), kv_half2(w1[st], 0x4342));
                 }
