@@ -8,7 +8,7 @@ namespace qb {
 constexpr float KV_OFF = 1152.f;
 constexpr int SROW = HD + 8;   // Q row stride in halves (ldmatrix rows on distinct banks)
 constexpr int DSPLITS = 37;    // most key splits of a decode token on a 148-SM part (qb_attn_dec_splits' default)
-constexpr int TSPLITS = 32;    // most key splits of a prompt tile (a power of two)
+constexpr int TSPLITS = 32;    // most key splits of a prompt tile
 
 __host__ __device__ inline size_t cache_head(int slot, int g, int cap) { return ((size_t)slot * NKV + g) * cap * HD; }
 __host__ __device__ inline size_t scale_head(int slot, int g, int cap) { return ((size_t)slot * NKV + g) * cap; }

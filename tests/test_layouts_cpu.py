@@ -226,3 +226,15 @@ def test_form_of_the_prompt_attention():
                  [(500, 4000)] * 4, [(30, 2500)] * 66, [(10, 16000)] * 40 + [(800, 0)]):
         assert pairs(segs) == 0, segs    # 176/295, 540/770, 164/248, 288/401, 542/592, 706/1122, 493/517, 518/543, 1070/1434
     assert pairs([(7, 5)], sms=1) in (0, 1) and lib().qb_attn_tiles_on_pairs(None, 3, None, None, 148) == 0
+
+
+def test_tile_splits_stay_within_the_partials():
+    """Key splits of a few prompt tiles: more than one from 512 keys up to 37 tiles, at most 32, and tiles x splits below 75 (the
+    partials of any step are 740 tokens' at most); no fewer than two blocks per SM and 256 keys per split ask for."""
+    for tiles in range(1, 80):
+        for keys in (1, 255, 511, 512, 513, 1000, 1024, 1025, 2047, 4010, 9012, 9040, 16384, 30010, 32768, 262144):
+            z = lib().qb_attn_tile_splits(tiles, keys)
+            least = 1
+            while least < 32 and tiles * 4 * least * 2 <= 296 and keys // (least * 2) >= 256:
+                least *= 2
+            assert least <= z <= 32 and (z > 1) == (tiles <= 37 and keys >= 512) and (z == 1 or tiles * z < 75), (tiles, keys, z)
