@@ -231,6 +231,7 @@ def test_form_of_the_prompt_attention():
 def test_tile_splits_stay_within_the_partials():
     """Key splits of a few prompt tiles: more than one from 512 keys up to 37 tiles, at most 32, and tiles x splits below 75 (the
     partials of any step are 740 tokens' at most); no fewer than two blocks per SM and 256 keys per split ask for."""
+    from qwenny_b200._lib import lib
     for tiles in range(1, 80):
         for keys in (1, 255, 511, 512, 513, 1000, 1024, 1025, 2047, 4010, 9012, 9040, 16384, 30010, 32768, 262144):
             z = lib().qb_attn_tile_splits(tiles, keys)
