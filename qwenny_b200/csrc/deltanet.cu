@@ -101,7 +101,18 @@ delta_fused_kernel(const float* p, int splits, int n, const float* ba, int ba_sp
     const int cb = blockIdx.x * CH, mm = min(len, CR);
     static_assert(TCH * ((LQKV + 2 * LV_HEADS - 1) / (2 * LV_HEADS)) <= 2 * FNT, "a round's ring share fits 2 values per thread");
 
+    // Every block of the launch counts once, when all of its threads have read the slots' metadata: the last one to get there
+    // records the step in them. The answer is not waited for.
     int tkt = 0;
+    auto count = [&] {
+        if (tid == 0) tkt = atom_add_acq_rel(ticket, 1);  // (ordered: the reads before it, the last block's writes behind it)
+    };
+    if (len <= 0) {  // a segment without tokens: its state as it is becomes the end state
+        st_rows(sbuf(pl.ebuf), S, sub);
+        __syncthreads();
+        count();
+        cluster_wait();
+    }
     bool lp_pending = true;  // a cluster barrier phase this block has arrived at and not yet waited for (the first: it has started)
     for (int c0 = 0; c0 < len; c0 += TCH) {
         const int m = min(TCH, len - c0);
@@ -208,9 +219,7 @@ delta_fused_kernel(const float* p, int splits, int n, const float* ba, int ba_sp
         }
         if (direct) cp_async_wait_all();
         __syncthreads();
-        // (every thread of the block has read the slots' metadata: the launch's last block to get here records the step in them. The
-        // answer is not waited for.)
-        if (c0 == 0 && tid == 0) tkt = atomicAdd(ticket, 1);
+        if (c0 == 0) count();
         // this round's rows of the conv ring (the block's channel share)
 #pragma unroll
         for (int u = 0; u < 2; u++) {
