@@ -445,20 +445,20 @@ attn_decode_kernel(const float* q, const uint8_t* kc, const uint8_t* vc, const f
 // of a stage is dealt so that no byte is converted twice:
 //   scores   warp w multiplies all the rows (RT tiles of 16 (token, head) rows) by the keys 16 w .. 16 w + 15 of the
 //            stage over the whole head dimension: one conversion of a key serves every row tile;
-//   softmax  P = 2^(score - m) for a reference m per row that the quad shares. It moves, to the largest score so far, only when P times
-//            a value's scale comes near the end of f16: the warps tell one another with the barrier that hands over their 16-key slices of P (as f16
-//            mma fragments), so that most stages have one barrier and rescale nothing (maxima exchanged in every stage: two barriers, and
-//            30 rows' accumulators rescaled in nearly all of them). A lane keeps the sums of its own keys to the end;
+//   softmax  the four warps agree on the rows' running maxima through shared memory, so that all of them scale by the same
+//            power of two, and exchange their 16-key slices of P (as f16 mma fragments); a lane keeps the sums of its own keys
+//            to the end. (P relative to a reference that moves only near f16's end: one barrier per stage instead of two, but P
+//            is made twice where it moves and rounded to other values: no faster, 5 rows at 32000 29.4 us, 28.9 so; 8 sequences of 4 rows up to
+//            32000 are the exception, 112.2 and 116.5);
 //   values   warp w accumulates the output dims 64 w .. 64 w + 63 over all 64 keys of the stage (for every row tile),
 //            so the output accumulators of a row are spread over four warps (RT x 32 registers each).
 // The int8 codes go to the tensor cores as 1152 + q halves (one prmt per pair) and the offset is folded out through the
 // row sums, as in the reference (kernels/attn.cuh:38-40,198-234). The quads' partial results meet in shared memory
 // at the end; the block writes one (m, l, acc) partial per row, or the finished rows when the segment has one split.
-// Bound by latency: at 5 rows a quad's stage takes 4100 cycles (scores 1250, softmax and barrier 920, values 1280, waits and copies 650) with
-// two warps per scheduler, and a block 3000 before its first stage behind the kernel before, 3000 after its last. From a graph with
-// attn_prep and the combine, us, before (a copy warp, maxima in every stage, Q row by row) / now: 5 rows at 100 keys 13.5 / 11.2, at 4000
-// 18.4 / 15.1, at 32000 35.0 / 29.6; 1 row at 32000 26.2 / 24.1; 8 rows 50.6 / 39.4 (registers spilled before); 8 sequences of 4 rows at 972
-// to 7777 66.5 / 49.7 (59.7 with a block per split), at 4000 to 32000 140 / 111.9 (128.5).
+// Bound by latency, with two warps per scheduler (four at one row tile). From a graph with attn_prep and the combine, us, before (a copy
+// warp, Q row by row, keys with bank conflicts) / now: 5 rows at 100 keys 13.7 / 11.0, at 4000 18.3 / 14.9, at 32000 34.8 / 28.9; 1 row at
+// 32000 26.3 / 24.3; 8 rows 50.4 / 38.3 (registers spilled before); 8 sequences of 4 rows at 972 to 7777 66.7 / 47.9 (57.7 with a block per
+// split), at 4000 to 32000 139.9 / 116.5 (126.6).
 // Many splits (MANY): a block per split would pay for each one's start (its segment's tokens, Q, the first stages' way from memory: half of
 // the 11 us that a split of four stages took) and leave the last round of the SMs partly idle. So a block per SM takes a run of them, equal
 // shares of the line on which each split is as long as its stages and SPLIT_COST: Q stays where the run stays with a segment's kv head,
@@ -472,10 +472,9 @@ struct Dec4Cfg {
     static constexpr int SK = 64, NSTG = NQ > 2 ? 6 : 5;  // keys per stage, ring depth
     static constexpr int STG_BYTES = SK * HD * 2 + SK * 8;
     static constexpr int Q_BYTES = RT * 16 * SROW * 2;
-    // per quad: the warps' row maxima (and whether a row has left its reference) [4][RT][16], their P fragments, of two stages in turn, [2][4][RT][32 lanes] x 16 B, their (sum,
-    // ps) [4][RT][16][2]
-    static constexpr int X_MAX = 4 * RT * 16 * 8, X_P = 4 * RT * 32 * 16, X_SUM = 4 * RT * 16 * 8;
-    static constexpr int X_BYTES = X_MAX + 2 * X_P + X_SUM;
+    // per quad: the warps' row maxima [4][RT][16], their P fragments [4][RT][32 lanes] x 16 B, their (sum, ps) [4][RT][16][2]
+    static constexpr int X_MAX = 4 * RT * 16 * 4, X_P = 4 * RT * 32 * 16, X_SUM = 4 * RT * 16 * 8;
+    static constexpr int X_BYTES = X_MAX + X_P + X_SUM;
     static constexpr int BAR_BYTES = 128;
     static constexpr int SMEM = BAR_BYTES + Q_BYTES + QUADS * X_BYTES + NSTG * STG_BYTES;
     static constexpr int SMEM_MANY = SMEM + DEC_SEGS * (16 + 8 + 4);  // and the step's segments
@@ -623,12 +622,12 @@ attn_dec4_kernel(const float* q, const uint8_t* kc, const uint8_t* vc, const flo
     else if (warp < begin && lane < 2)
         bulk_prefetch((lane ? vc : kc) + cache_head(slot, g, cap) + (size_t)(kbeg + warp * SK) * HD, SK * HD);
     pdl_wait();  // q, the gates and the step's own keys and values come from its attn_prep
-    // Q of the segment's rows (row = token * GROUP + head) as f16, and KV_OFF times each row's sum of those (a row's 64 threads: two
-    // warps). All of a thread's loads are under way together: one after the other, behind the token's own load, they took 4 us.
-    float2* xmax = (float2*)(xch + quad * C::X_BYTES);               // [4][RT][16]
-    uint8_t* xp_at = xch + quad * C::X_BYTES + C::X_MAX;             // [2][4][RT][32] x 16 B
-    float2* xsum = (float2*)(xch + quad * C::X_BYTES + C::X_MAX + 2 * C::X_P);  // [4][RT][16]
-    float* qsum = (float*)(xch + C::X_MAX);  // [RT * 16][2]: where the first quad's P goes later
+    // Q of the segment's rows (row = token * GROUP + head) as f16, and each row's sum of those. All of a thread's loads are under way
+    // together: one after the other, behind the token's own load, they took 4 us.
+    float* xmax = (float*)(xch + quad * C::X_BYTES);                 // [4][RT][16]
+    uint4* xp = (uint4*)(xch + quad * C::X_BYTES + C::X_MAX);        // [4][RT][32]
+    float2* xsum = (float2*)(xch + quad * C::X_BYTES + C::X_MAX + C::X_P);  // [4][RT][16]
+    float* qsum = (float*)(xch + C::X_BYTES + C::X_MAX + C::X_P);  // [RT * 16], in the second quad's place for sums, which it never uses
     auto load_q = [&](bool begins) {
         constexpr int PER = RT * 16 * HD / 4 / NCW, RSTEP = NCW / (HD / 4);  // float4 per thread, rows at a time
         const int r0 = threadIdx.x / (HD / 4), d = (threadIdx.x % (HD / 4)) * 4;
@@ -641,13 +640,24 @@ attn_dec4_kernel(const float* q, const uint8_t* kc, const uint8_t* vc, const flo
         }
         if (begins) ask(false);
 #pragma unroll
-        for (int i = 0; i < PER; i++) {
-            const int row = r0 + i * RSTEP;
-            const uint2 h = make_uint2(pack_half2(v[i].x, v[i].y), pack_half2(v[i].z, v[i].w));
-            *(uint2*)&qsh[row * SROW + d] = h;
-            const float2 f0 = __half22float2(*(const __half2*)&h.x), f1 = __half22float2(*(const __half2*)&h.y);
-            const float sum = warp_sum((f0.x + f0.y) + (f1.x + f1.y));
-            if (lane == 0) qsum[row * 2 + (warp & 1)] = sum;
+        for (int i = 0; i < PER; i++)
+            *(uint2*)&qsh[(r0 + i * RSTEP) * SROW + d] = make_uint2(pack_half2(v[i].x, v[i].y), pack_half2(v[i].z, v[i].w));
+        named_bar_sync(1, NCW);
+        if (warp < RT) {  // a lane sums half a row
+            const uint4* from = (const uint4*)(qsh + (warp * 16 + (lane & 15)) * SROW + (lane >> 4) * (HD / 2));
+            float sum = 0.f;
+#pragma unroll 4
+            for (int i = 0; i < HD / 16; i++) {
+                const uint4 x = from[i];
+                const uint32_t h[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+                for (int e = 0; e < 4; e++) {
+                    const float2 f = __half22float2(*(const __half2*)&h[e]);
+                    sum += f.x + f.y;
+                }
+            }
+            sum += __shfl_xor_sync(0xffffffffu, sum, 16);
+            if (lane < 16) qsum[warp * 16 + lane] = sum;
         }
     };
     // KV_OFF times the sums of Q of this lane's rows 16 rt + r and + 8
@@ -663,11 +673,7 @@ attn_dec4_kernel(const float* q, const uint8_t* kc, const uint8_t* vc, const flo
 #pragma unroll
             for (int rt = 0; rt < RT; rt++)
 #pragma unroll
-                for (int h2 = 0; h2 < 2; h2++) {
-                    const float2 x = *(const float2*)&qsum[(rt * 16 + r + 8 * h2) * 2];
-                    qoff[rt][h2] = KV_OFF * (x.x + x.y);
-                }
-            named_bar_sync(1, NCW);  // (the sums of Q have been read)
+                for (int h2 = 0; h2 < 2; h2++) qoff[rt][h2] = KV_OFF * qsum[rt * 16 + r + 8 * h2];
         }
         // the keys that the rows may see end at lim
         int lim[RT][2], all_see = ke;  // (keys below all_see are seen by every row of the segment)
@@ -680,7 +686,7 @@ attn_dec4_kernel(const float* q, const uint8_t* kc, const uint8_t* vc, const flo
                 lim[rt][h2] = tok < nt ? min(ke, p + 1) : 0;
             }
         all_see = min(all_see, __reduce_min_sync(0xffffffffu, my_pos) + 1);
-        // m: the rows' reference, a power of two that scores are taken from; -inf until a key was seen
+        // m: the rows' largest score so far; -inf until a key was seen
         float m[RT][2], l[RT][2], ps[RT][2], o[RT][8][4];
 #pragma unroll
         for (int rt = 0; rt < RT; rt++) {
@@ -766,93 +772,73 @@ attn_dec4_kernel(const float* q, const uint8_t* kc, const uint8_t* vc, const flo
                         sv = (sv - qoff[rt][x >> 1]) * ksc[nn][x & 1];
                         if (!whole && kb + 8 * nn + 2 * t4 + (x & 1) >= lim[rt][x >> 1]) sv = -INFINITY;
                     }
-            // ---- P of this warp's keys (times the value scales, rounded to f16 as the products see it) and its row sums. The first time
-            // with the references as they are; where a row has left its own (P times a value scale near the end of f16, or P past 2^24), and
-            // in the quad's first stage, once more with new ones.
-            uint4* xp = (uint4*)(xp_at + (j / C::QUADS & 1) * C::X_P);  // (a warp may still be reading the stage before's)
-            float sum[RT][2], pr[RT][2];
-#pragma unroll 1
-            for (bool again = false;; again = true) {
-                bool left[RT][2], any_left = j == quad;
-#pragma unroll
-                for (int rt = 0; rt < RT; rt++) {
-                    float pv[2][4];
-#pragma unroll
-                    for (int h2 = 0; h2 < 2; h2++) {
-                        const float mm = m[rt][h2] == -INFINITY ? 0.f : m[rt][h2];
-                        sum[rt][h2] = 0.f;
-#pragma unroll
-                        for (int nn = 0; nn < 2; nn++)
-#pragma unroll
-                            for (int e = 0; e < 2; e++) {
-                                const float pp = tc::ex2(v[rt][nn][2 * h2 + e] - mm);
-                                sum[rt][h2] += pp;
-                                pv[nn][2 * h2 + e] = pp * vsc[nn][e];
-                            }
-                        left[rt][h2] = fmaxf(fmaxf(pv[0][2 * h2], pv[0][2 * h2 + 1]), fmaxf(pv[1][2 * h2], pv[1][2 * h2 + 1])) > 32768.f || sum[rt][h2] > 0x1p24f;
-                        any_left |= left[rt][h2];
-                    }
-                    uint4 pa;
-                    pa.x = pack_half2(pv[0][0], pv[0][1]); pa.y = pack_half2(pv[0][2], pv[0][3]);
-                    pa.z = pack_half2(pv[1][0], pv[1][1]); pa.w = pack_half2(pv[1][2], pv[1][3]);
-                    xp[(w * RT + rt) * 32 + lane] = pa;
-                    const float2 f0 = __half22float2(*(const __half2*)&pa.x), f1 = __half22float2(*(const __half2*)&pa.y);
-                    const float2 f2 = __half22float2(*(const __half2*)&pa.z), f3 = __half22float2(*(const __half2*)&pa.w);
-                    pr[rt][0] = f0.x + f0.y + f2.x + f2.y;
-                    pr[rt][1] = f1.x + f1.y + f3.x + f3.y;
-                }
-                if (again) {
-                    named_bar_sync(2 + quad, 128);
-                    break;
-                }
-                if (!named_bar_or(2 + quad, 128, any_left)) break;
-#pragma unroll
-                for (int rt = 0; rt < RT; rt++)
-#pragma unroll
-                    for (int h2 = 0; h2 < 2; h2++) {
-                        float x = fmaxf(fmaxf(v[rt][0][2 * h2], v[rt][0][2 * h2 + 1]), fmaxf(v[rt][1][2 * h2], v[rt][1][2 * h2 + 1]));
-                        x = fmaxf(x, __shfl_xor_sync(0xffffffffu, x, 1));
-                        x = fmaxf(x, __shfl_xor_sync(0xffffffffu, x, 2));
-                        const bool lf = (__ballot_sync(0xffffffffu, left[rt][h2]) >> (4 * r) & 15) != 0;
-                        if (t4 == 0) xmax[(w * RT + rt) * 16 + r + 8 * h2] = make_float2(x, lf ? 1.f : 0.f);
-                    }
-                named_bar_sync(2 + quad, 128);
-#pragma unroll
-                for (int rt = 0; rt < RT; rt++) {
-                    float corr[2];
-#pragma unroll
-                    for (int h2 = 0; h2 < 2; h2++) {
-                        float mn = m[rt][h2];
-                        bool moves = j == quad;
-#pragma unroll
-                        for (int ww = 0; ww < 4; ww++) {
-                            const float2 x = xmax[(ww * RT + rt) * 16 + r + 8 * h2];
-                            mn = fmaxf(mn, x.x);
-                            moves |= x.y != 0.f;
-                        }
-                        moves &= mn > m[rt][h2];  // (it depends on the row's own scores alone, not on what else is in the step)
-                        corr[h2] = moves ? exp2f(m[rt][h2] - mn) : 1.f;
-                        if (moves) m[rt][h2] = mn;
-                        l[rt][h2] *= corr[h2];
-                        ps[rt][h2] *= corr[h2];
-                    }
-#pragma unroll
-                    for (int jd = 0; jd < 8; jd++) {
-                        o[rt][jd][0] *= corr[0]; o[rt][jd][1] *= corr[0];
-                        o[rt][jd][2] *= corr[1]; o[rt][jd][3] *= corr[1];
-                    }
-                }
-            }
-            // (a lane sums its own keys; lanes and warps are added up once, after the last stage)
+            // ---- the rows' maxima over this warp's keys, then over the quad's
 #pragma unroll
             for (int rt = 0; rt < RT; rt++)
 #pragma unroll
                 for (int h2 = 0; h2 < 2; h2++) {
-                    l[rt][h2] += sum[rt][h2];
-                    ps[rt][h2] += pr[rt][h2];
+                    float x = fmaxf(fmaxf(v[rt][0][2 * h2], v[rt][0][2 * h2 + 1]), fmaxf(v[rt][1][2 * h2], v[rt][1][2 * h2 + 1]));
+                    x = fmaxf(x, __shfl_xor_sync(0xffffffffu, x, 1));
+                    x = fmaxf(x, __shfl_xor_sync(0xffffffffu, x, 2));
+                    if (t4 == 0) xmax[(w * RT + rt) * 16 + r + 8 * h2] = x;
                 }
-            // (the barrier above: all of the quad is done with its stage before this one, and the slot's barrier is armed)
+            named_bar_sync(2 + quad, 128);
+            // (all of the quad is done with its stage before this one, and the slot's barrier is armed)
             if (refill && lane == 0) copy(j - 2 + NSTG, w);
+            float corr[RT][2];
+            bool grew = false;
+#pragma unroll
+            for (int rt = 0; rt < RT; rt++)
+#pragma unroll
+                for (int h2 = 0; h2 < 2; h2++) {
+                    float mn = m[rt][h2];
+#pragma unroll
+                    for (int ww = 0; ww < 4; ww++) mn = fmaxf(mn, xmax[(ww * RT + rt) * 16 + r + 8 * h2]);
+                    corr[rt][h2] = mn == -INFINITY ? 1.f : exp2f(m[rt][h2] - mn);
+                    m[rt][h2] = mn;
+                    grew |= corr[rt][h2] != 1.f;
+                }
+            // ---- P of this warp's keys (times the value scales, rounded to f16 as the products see it) and its row sums
+#pragma unroll
+            for (int rt = 0; rt < RT; rt++) {
+                float pv[2][4], sum[2];
+#pragma unroll
+                for (int h2 = 0; h2 < 2; h2++) {
+                    const float mm = m[rt][h2] == -INFINITY ? 0.f : m[rt][h2];
+                    sum[h2] = 0.f;
+#pragma unroll
+                    for (int nn = 0; nn < 2; nn++)
+#pragma unroll
+                        for (int e = 0; e < 2; e++) {
+                            const float pp = tc::ex2(v[rt][nn][2 * h2 + e] - mm);
+                            sum[h2] += pp;
+                            pv[nn][2 * h2 + e] = pp * vsc[nn][e];
+                        }
+                }
+                uint4 pa;
+                pa.x = pack_half2(pv[0][0], pv[0][1]); pa.y = pack_half2(pv[0][2], pv[0][3]);
+                pa.z = pack_half2(pv[1][0], pv[1][1]); pa.w = pack_half2(pv[1][2], pv[1][3]);
+                xp[(w * RT + rt) * 32 + lane] = pa;
+                const float2 f0 = __half22float2(*(const __half2*)&pa.x), f1 = __half22float2(*(const __half2*)&pa.y);
+                const float2 f2 = __half22float2(*(const __half2*)&pa.z), f3 = __half22float2(*(const __half2*)&pa.w);
+                const float pr[2] = {f0.x + f0.y + f2.x + f2.y, f1.x + f1.y + f3.x + f3.y};
+                // (a lane sums its own keys; lanes and warps are added up once, after the last stage)
+#pragma unroll
+                for (int h2 = 0; h2 < 2; h2++) {
+                    l[rt][h2] = fmaf(l[rt][h2], corr[rt][h2], sum[h2]);
+                    ps[rt][h2] = fmaf(ps[rt][h2], corr[rt][h2], pr[h2]);
+                }
+            }
+            named_bar_sync(2 + quad, 128);
+            if (__any_sync(0xffffffffu, grew)) {
+#pragma unroll
+                for (int rt = 0; rt < RT; rt++)
+#pragma unroll
+                    for (int jd = 0; jd < 8; jd++) {
+                        o[rt][jd][0] *= corr[rt][0]; o[rt][jd][1] *= corr[rt][0];
+                        o[rt][jd][2] *= corr[rt][1]; o[rt][jd][3] *= corr[rt][1];
+                    }
+            }
             // ---- values: O += P V over the stage's 64 keys, this warp's 64 output dims
 #pragma unroll
             for (int kbk = 0; kbk < 4; kbk++) {
@@ -1153,9 +1139,9 @@ int qb_attn_decode_as(qb_ctx* ctx, void* stream, const float* q, const void* kc,
     const int old_margin = ahead && ndec <= 64 ? 64 : 0;
     // One block per split where they are few; blocks that keep running where they would be more than four rounds of the SMs, or more than
     // three with the last at most half full, if all sequences were as long as the longest. Block per split against that, us:
-    // 8 sequences x 4 rows, up to context 7777 59.5 / 48.5; 8 x 8 at 8000 99.3 / 90.5; 8 x 1 at 3000 37.0 / 34.0; 4 x 4 up to 8000
-    // (3.4 rounds) 37.0 / 34.4; but 6 x 8 at 3000 (3.9) 44.6 / 47.6, 4 x 4 up to 3000 (2.6) 22.3 / 23.3, 2 x 4 up to 3000 14.4 / 15.4:
-    // the table of the segments costs a microsecond before the first split.
+    // 8 sequences x 4 rows, up to context 7777 57.7 / 47.9; 8 x 8 at 8000 96.0 / 87.1; 8 x 1 at 3000 35.7 / 33.8; 4 x 4 up to 8000
+    // (3.4 rounds) 36.0 / 32.7; but 6 x 8 at 3000 (3.9) 42.5 / 44.5, 4 x 4 up to 3000 (2.6) 21.5 / 22.5, 2 x 4 up to 3000 14.1 / 14.9, 3 x 8 at
+    // 3000 25.0 / 32.2: the table of the segments costs a microsecond before the first split. (Left: 8 x 4 at 2048, 3.7 rounds, 34.1 / 29.1.)
     const long long most = (long long)ndseg * NKV * dec_splits(max_keys, dsplits);
     const bool many = ndseg <= DEC_SEGS && (most > 4 * ctx->sms || (most > 3 * ctx->sms && 2 * most <= 7 * ctx->sms));
     int rc;

@@ -227,14 +227,6 @@ __device__ __forceinline__ void named_bar_sync(int id, int threads) {
     asm volatile("bar.sync %0, %1;\n" ::"r"(id), "r"(threads) : "memory");
 }
 
-// the same barrier, and whether p holds in any of its threads
-__device__ __forceinline__ bool named_bar_or(int id, int threads, bool p) {
-    uint32_t any;
-    asm volatile("{\n.reg .pred p, q;\nsetp.ne.u32 p, %3, 0;\nbar.red.or.pred q, %1, %2, p;\nselp.u32 %0, 1, 0, q;\n}\n"
-                 : "=r"(any) : "r"(id), "r"(threads), "r"((uint32_t)p) : "memory");
-    return any != 0;
-}
-
 __device__ __forceinline__ int atom_add_acq_rel(int* p, int v) {
     int old;
     asm volatile("atom.add.acq_rel.gpu.global.s32 %0, [%1], %2;\n" : "=r"(old) : "l"(p), "r"(v) : "memory");

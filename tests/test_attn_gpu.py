@@ -284,10 +284,10 @@ def test_attn_prefill_runs_of_tiles(ctx, lens, pos0):
 
 @pytest.mark.parametrize("rows,vmax", [(2, 0.05), (5, 0.05), (5, 6.0), (8, 0.05)])
 def test_attn_decode_references_that_move(ctx, rows, vmax):
-    """Splits of several stages whose scores rise from stage to stage for some rows and fall for others (past what a row's reference
-    allows, f16's 2^15 over the value's scale), with value scales of 0 among them and up to 6: the oracle's values, and a
-    row's bits do not depend on the other rows' references (as many row tiles, other rows). P is f16 relative to any reference, so the
-    tolerance is the one of the other cases; its absolute part is for values of scale 0.05 and grows with theirs."""
+    """Splits of several stages whose scores rise from stage to stage for some rows and fall for others, so that a row's running maximum
+    moves often or never, with value scales of 0 among them and up to 6: the oracle's values, and a row's bits do not depend on the other
+    rows' maxima (as many row tiles, other rows). P is f16 relative to the maximum, so the tolerance is the one of the other cases; its
+    absolute part is for values of scale 0.05 and grows with theirs."""
     g = synth.gen(161 + rows)
     cap, pos0 = 16384, 15990
     kc, vc, ks, vs = make_cache(1, cap, g, 0)
