@@ -146,6 +146,8 @@ MEASURE_SIGNATURES = {
     "qb_scratch_chunks": [P, I],
     "qb_attn_tiles_on_pairs": [P, I, P, P, I],
     "qb_gemm_f16_block_tiles": [I, I, I, I, I],
+    "qb_attn_dec_dealt": [I, I, I],
+    "qb_attn_step_form": [I, I, I, I, I],
 }
 _RESTYPE = {"qb_version": C.c_char_p, "qb_destroy": None, "qb_model_destroy": None, "qb_draft_vocab_destroy": None, "qb_model_logits": P,
             "qb_model_hidden": P, "qb_model_xn": P, "qb_model_seen": P, "qb_model_launches": LL, "qb_model_kv_bytes": C.c_size_t,

@@ -1111,6 +1111,22 @@ int qb_attn_dec_splits_sm(int keys, int sms) { return keys > 0 && sms > 0 ? dec_
 
 int qb_attn_dec_grid(int max_keys, int sms) { return max_keys > 0 && sms > 0 ? dec_splits_upto(max_keys, dsplits_for(sms)) : 0; }
 
+// One block per split where they are few; blocks that keep running where they would be more than four rounds of the SMs, or more than
+// three with the last at most half full, if all sequences were as long as the longest. Block per split against that, us:
+// 8 sequences x 4 rows, up to context 7777 57.7 / 47.9; 8 x 8 at 8000 96.0 / 87.1; 8 x 1 at 3000 35.7 / 33.8; 4 x 4 up to 8000
+// (3.4 rounds) 36.0 / 32.7; but 6 x 8 at 3000 (3.9) 42.5 / 44.5, 4 x 4 up to 3000 (2.6) 21.5 / 22.5, 2 x 4 up to 3000 14.1 / 14.9, 3 x 8 at
+// 3000 25.0 / 32.2: the table of the segments costs a microsecond before the first split. (Left: 8 x 4 at 2048, 3.7 rounds, 34.1 / 29.1.)
+int qb_attn_dec_dealt(int ndseg, int max_keys, int sms) {
+    if (ndseg <= 0 || ndseg > DEC_SEGS || max_keys <= 0 || sms <= 0) return 0;
+    const long long most = (long long)ndseg * NKV * dec_splits(max_keys, dsplits_for(sms));
+    return most > 4 * sms || (most > 3 * sms && 2 * most <= 7 * sms);
+}
+
+// (a captured step is replayed for every step that it serves, so whatever the launches are chosen by is here)
+int qb_attn_step_form(int ndseg, int dec_keys, int ntile, int tile_keys, int sms) {
+    return qb_attn_dec_grid(dec_keys, sms) + 128 * (ntile > 0 ? qb_attn_tile_splits(ntile, tile_keys) : 0) + 8192 * qb_attn_dec_dealt(ndseg, dec_keys, sms);
+}
+
 // ndseg short segments (dseg: first index into dtok, token count; at most 8 tokens each), ndec = their tokens in
 // all, dmax = the longest segment's tokens, max_keys = the largest key count among them (sizes the grid).
 int qb_attn_decode(qb_ctx* ctx, void* stream, const float* q, const void* kc, const void* vc, const float* ks,
@@ -1137,13 +1153,7 @@ int qb_attn_decode_as(qb_ctx* ctx, void* stream, const float* q, const void* kc,
     // (the model's steps have at most 64 decode tokens: whatever lies 64 positions or more before a segment's last key is from
     // earlier steps)
     const int old_margin = ahead && ndec <= 64 ? 64 : 0;
-    // One block per split where they are few; blocks that keep running where they would be more than four rounds of the SMs, or more than
-    // three with the last at most half full, if all sequences were as long as the longest. Block per split against that, us:
-    // 8 sequences x 4 rows, up to context 7777 57.7 / 47.9; 8 x 8 at 8000 96.0 / 87.1; 8 x 1 at 3000 35.7 / 33.8; 4 x 4 up to 8000
-    // (3.4 rounds) 36.0 / 32.7; but 6 x 8 at 3000 (3.9) 42.5 / 44.5, 4 x 4 up to 3000 (2.6) 21.5 / 22.5, 2 x 4 up to 3000 14.1 / 14.9, 3 x 8 at
-    // 3000 25.0 / 32.2: the table of the segments costs a microsecond before the first split. (Left: 8 x 4 at 2048, 3.7 rounds, 34.1 / 29.1.)
-    const long long most = (long long)ndseg * NKV * dec_splits(max_keys, dsplits);
-    const bool many = ndseg <= DEC_SEGS && (most > 4 * ctx->sms || (most > 3 * ctx->sms && 2 * most <= 7 * ctx->sms));
+    const bool many = qb_attn_dec_dealt(ndseg, max_keys, ctx->sms);
     int rc;
 #define QB_DEC(RT, NQ)                                                                                          \
     {                                                                                                           \

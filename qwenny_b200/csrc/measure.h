@@ -28,6 +28,10 @@ int qb_gemm_f16_block_tiles(int ntiles, int splits, int kper, int n, int sms);
 /* Host only (host pointers): whether a prompt attention of more than 1664 keys and one key split runs on pairs of blocks (1) or as a
  * block per two tiles (0) on a part with `sms` SMs. qb_marlin_tune with ctas_per_sm 1002 / 1003 forces blocks / pairs. */
 int qb_attn_tiles_on_pairs(const int* h_ptile, int ntile, const int* h_tok_slot, const int* h_tok_pos, int sms);
+/* Host only: whether qb_attn_decode deals a step's splits out to a block per SM (1) or gives each a block (0), and all that the attention
+ * launches of a step are chosen by beside its counts (ndseg or ntile 0: none of that kind), for the key of a captured step. */
+int qb_attn_dec_dealt(int ndseg, int max_keys, int sms);
+int qb_attn_step_form(int ndseg, int dec_keys, int ntile, int tile_keys, int sms);
 /* Tests: the context goes on as one that was created where the prompt-sized kernels' scratch did not fit. */
 int qb_scratch_forget(qb_ctx* ctx);
 /* .. as one where the delta rule's tiles of only so many chunks fit (0: none). */

@@ -187,6 +187,25 @@ def test_decode_attention_grid_holds_every_split():
             assert most <= grid(keys, sms) <= 64
 
 
+def test_a_captured_step_keeps_the_launches_of_the_steps_it_serves():
+    """Steps with the same counts and the same qb_attn_step_form share a captured graph, so the form tells apart every choice that the
+    attention's launches take from the key counts: the decode grid, the blocks that take several splits, the prompt tiles' splits. On 148 SMs
+    eight segments are dealt out at 2048 keys, not at 2112, and again from 2368 on, all with one grid."""
+    from qwenny_b200._lib import lib
+    l = lib()
+    assert [l.qb_attn_dec_dealt(8, k, 148) for k in (2048, 2112, 2368)] == [1, 0, 1]
+    assert len({l.qb_attn_dec_grid(k, 148) for k in (2048, 2112, 2368)}) == 1
+    for sms in (148, 132, 300):
+        for ndseg, ntile in ((1, 0), (8, 1), (16, 3), (64, 0), (65, 0)):
+            seen = {}
+            for keys in list(range(1, 5000, 37)) + list(range(5000, 40000, 1021)):
+                for tile_keys in (0,) if not ntile else (100, 700, 2000, 30000):
+                    tiles = l.qb_attn_tile_splits(ntile, tile_keys) if ntile else 0
+                    how = l.qb_attn_dec_grid(keys, sms), l.qb_attn_dec_dealt(ndseg, keys, sms), tiles
+                    assert seen.setdefault(l.qb_attn_step_form(ndseg, keys, ntile, tile_keys, sms), how) == how
+    assert l.qb_attn_dec_dealt(65, 30000, 148) == 0  # (more segments than the blocks' table holds)
+
+
 def test_tiles_per_block_of_the_16_bit_product():
     """One tile per block while the blocks do not fill the SMs (the DeltaNet gates' 96 x 5120 product in 5 splits up to 128 rows, where
     blocks of six tiles are a third slower), several beyond; never tiles that do not divide."""
