@@ -14,8 +14,7 @@
 // stage beside 65 per product, and the copying lane 70 per copy (64 of k per stage: 600 cycles of the 512 at N = 256).
 //
 // The work is the list of (tile, k block of 128) pairs, tile after tile, on a persistent grid of at most one pair per two SMs. Where whole tiles
-// leave pairs idle the list is dealt out in equal contiguous shares (stream-K; with few tiles each tile is cut into as many equal parts): a
-// pair that ends or starts inside a tile writes that tile's partial accumulators to scratch and takes a ticket; the
+// leave pairs idle the list is dealt out in equal contiguous shares (stream-K): a pair that ends or starts inside a tile writes that tile's partial accumulators to scratch and takes a ticket; the
 // tile's last arriver adds the parts in pair order and runs the epilogue, nobody waits.
 // Per (tile, k block):
 //   warps 0-7   dequantise: lop3 / hsub2 to q - 8, one hfma2 by the f16 group scale (the reference's rounding:
@@ -28,8 +27,8 @@
 //   warp 17     of the pair's first block: issues the products (K = 16 each) as a whole warp, tcgen05.commit hands the stage
 //               back in both blocks when they have read it
 // Bound by the tensor pipe and, where it runs for long, by the power it takes. With the epilogue in the unpacking warps, one block per
-// tile, 4-byte stores and a fence per thread / as it is, us from a graph: 2048 rows of 16384 x 5120 252 / 224, of 34816 x 5120 545 / 500,
-// 333 rows of 5120 x 6144 with zero points 36.3 / 29.3, 100 rows 25.3 / 17.5, 256 rows of 2048 x 2048 41 / 19.4, 100 of 1024 x 1024 18.1 / 9.7.
+// tile, 4-byte stores and a fence per thread / as it is, us from a graph: 2048 rows of 16384 x 5120 243 / 226, of 34816 x 5120 545 / 507,
+// 333 rows of 5120 x 6144 with zero points 36.0 / 29.8, 100 rows 25.4 / 21.0, 256 rows of 2048 x 2048 39.9 / 32.0, 70 of 1024 x 1024 15.6 / 13.1.
 #include "launch.h"
 #include "pair_tc.cuh"
 
@@ -426,38 +425,19 @@ int qb_gemm_tc_launch(qb_ctx* ctx, cudaStream_t st, const void* X, const void* B
     a.S = (const __half*)S; a.Y = Y; a.m = m; a.N = n; a.K = k; a.row0 = row0; a.err = ctx->err;
     a.zp = zp ? 1 : 0; a.part = ctx->tc_part; a.tickets = ctx->tc_tickets; a.iters = (int)tiles * (k / tc::BK);
     a.bt = bt; a.tiles = (int)tiles; a.direct = direct;
-    // How the list is dealt. More tiles than pairs: whole tiles, pair by pair in turn, where they fill five sixths of the rounds, else equal
-    // shares of the list over all pairs (5120 x 6144, 2048 rows, 2.2 rounds: 97 us as shares, 100 as tiles; 1500 rows, 1.6: 74 and 69).
-    // Fewer tiles than pairs: whole ones, or each cut into `cuts` equal parts for as many pairs, or shares, by an estimate in ns of the
-    // stages of the longest part (the products, but no less than unpacking takes) and of what joining the parts costs, more with every part of
-    // a tile (shares: parts of two tiles a pair). Measured at 70 / 256 rows, us: 5120 x 6144 whole 23.1 / 35.9, two parts 17.0 / 28.5,
-    // three 16.1 / 27.2, shares 18.4 / 33.0; 5120 x 17408 56 / 85, 35 / 56, 28.4 / 46, 28.6 / 48; 2048 x 2048 10.8 / 16.9, 10.7 / 17.1, 11.7 /
-    // 19.5, 16.2 / 33; 1024 x 1024 8.1 / 12.3, 8.9 / 14.5, 10.6 / 17.9, 13 / 25; 5120 x 10240 at 333 rows 45 whole, 40.5 as shares.
-    // The tensor core's f32 sums lose some 1.5e-7 per 128 of k, so up to five sixths of the pairs' worth of tiles no part is longer than six
-    // stages or 1.3 shares (2048 x 2048, 1565 rows, 56 tiles: 15 us whole with an error of 2.4e-6 against 64 bits, 26 as shares with 1.4e-6). With zero
-    // points the weights' own rounding, 5e-5, covers it.
-    bool whole;
-    int cuts = 1;
-    if (tiles > pairs) {
-        const long long rounds = (tiles + pairs - 1) / pairs;
-        whole = 6 * tiles > 5 * rounds * pairs;
-    } else {
-        const int nkb = k / tc::BK;
-        const long long stage = 380 + (bt > 128 ? (bt - 128) * 7 / 5 : 0);
-        long long best = a.iters * stage / pairs + 70 * bt;
-        cuts = 0;
-        for (int c = 1; c * tiles <= pairs && c <= nkb; c++) {
-            const long long cost = (nkb + c - 1) / c * stage + (c > 1 ? bt * (10 + 25 * (c - 1) / 2) : 0);
-            const long long longest = (nkb + c - 1) / c;
-            if (!zp && 6 * tiles <= 5 * pairs && longest > 6 && 10 * longest * pairs > 13 * a.iters) continue;
-            if (cost < best) { best = cost; cuts = c; }
-        }
-        whole = cuts == 1;
-    }
-    if (ctx->tune_ctas == 1000) { whole = false; cuts = 0; }  // measurement: shares whatever the shape
-    if (ctx->tune_ctas == 1001) whole = true;                 //              tiles whatever the shape
-    if (!ctx->tc_part) whole = true;                          // a context without the scratch
-    const long long units = whole ? tiles : cuts > 1 ? tiles * cuts : a.iters;
+    // How the list is dealt: whole tiles, pair by pair in turn, where they fill five sixths of the rounds, else equal shares of the list over
+    // all pairs (5120 x 6144, 2048 rows, 2.2 rounds: 97 us as shares, 100 as tiles; 1500 rows, 1.6: 74 and 69; 700 rows, 0.8: 45 and 37).
+    // Not by time alone: the tensor core's f32 sums are cut off, not rounded, and lose 1.5e-7 of the result (2-norm) per 128 of k that an
+    // accumulator runs over. Shares are the shortest parts there are; a tile that is whole where they are the other choice, or cut into
+    // fewer equal parts, is faster with few tiles and further off: 2048 x 2048 at 70 rows 11.3 us and 8.1e-7 in two parts, 15.4 and 3.0e-7 as shares;
+    // 5120 x 6144 at 70 16.1 and 2.4e-6 in three, 18.2 and 1.8e-6, at 700 37 and 7.1e-6 whole, 45 and 4.5e-6; with zero points, whose rounding is
+    // 4.7e-5, at 333 28.6 and 4.78e-5 whole, 29.8 and 4.74e-5. From five sixths on a tile's error is that of its k: 2.4e-6 for 2048, 2.0e-5 for 17408.
+    const long long rounds = (tiles + pairs - 1) / pairs;
+    bool whole = 6 * tiles > 5 * rounds * pairs;
+    if (ctx->tune_ctas == 1000) whole = false;  // measurement: shares whatever the shape
+    if (ctx->tune_ctas == 1001) whole = true;   //              tiles whatever the shape
+    if (!ctx->tc_part) whole = true;            // a context without the scratch
+    const long long units = whole ? tiles : a.iters;
     const int G = (int)(units < pairs ? units : pairs);
     dim3 grid((unsigned)(2 * G));
     if (epi == QB_EPI_SILU)

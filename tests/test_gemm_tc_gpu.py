@@ -98,9 +98,9 @@ def test_shares_of_the_tile_list_repeat_and_agree_with_whole_tiles(ctx, m, rows,
 
 @pytest.mark.parametrize("m,rows,cols,silu", [(65, 256, 4096, False), (70, 512, 6144, True), (100, 5120, 2048, False), (256, 1280, 5248, False),
                                                (300, 9728, 256, True)])
-def test_tiles_cut_into_equal_parts_and_unaligned_results(ctx, m, rows, cols, silu):
-    """Few tiles with a long k are cut into equal parts (up to one per pair of blocks; 5248 columns are 41 groups, which no number of parts
-    divides), many more tiles than pairs are dealt in rounds: the oracle's values and the same bits in a repeated launch. A result that starts off a
+def test_tiles_cut_into_parts_and_unaligned_results(ctx, m, rows, cols, silu):
+    """Few tiles with a long k are cut into parts (down to a stage of 128 per pair of blocks; 5248 columns are 41 stages, which no number
+    of pairs divides), many more tiles than pairs are dealt in rounds: the oracle's values and the same bits in a repeated launch. A result that starts off a
     16-byte boundary takes plain stores: the same bits, and nothing beside it is written. Only the order of the f32 sums over k may differ
     from whole tiles: 2e-4 of the largest value (2e-3 where the result is f16), as above."""
     x, wdq, xd, wd, sd = make(rows, cols, silu, 500 + m, m)
@@ -122,6 +122,30 @@ def test_tiles_cut_into_equal_parts_and_unaligned_results(ctx, m, rows, cols, si
     an, cn = a.float().cpu().numpy(), c.float().cpu().numpy()
     assert close(an, want.astype(np.float32)).all()
     assert np.abs(an - cn).max() <= (2e-3 if silu else 2e-4) * max(1.0, np.abs(want).max())
+
+
+@pytest.mark.parametrize("m,rows,cols,zp", [(70, 1024, 1024, False), (100, 256, 17408, False), (256, 2048, 2048, False), (1565, 2048, 2048, False),
+                                             (2048, 2048, 2048, False), (700, 5120, 6144, False), (1000, 5120, 17408, False), (333, 5120, 6144, True)])
+def test_no_accumulator_runs_longer_than_shares_or_its_tile(ctx, m, rows, cols, zp):
+    """The tensor core cuts its f32 sums off: an accumulator loses 1.5e-7 of the result per stage of 128 columns (measured over 1 to 136 of
+    them), and joining the parts in f32 some 1e-7. So the error against 64 bits tells the longest part: a tile's whole k only where whole tiles
+    fill five sixths of the pairs' rounds, an equal share of all stages elsewhere, with and without zero points."""
+    g = synth.gen(700 + m)
+    pairs = torch.cuda.get_device_properties(0).multi_processor_count // 2
+    tiles, k = rows // 256 * -(-m // 256), cols // 128
+    longest = k if 6 * tiles > 5 * -(-tiles // pairs) * pairs else min(k, -(-tiles * k // pairs))
+    codes, sc = synth.int4_matrix(rows, cols, g)
+    zeros = torch.randint(0, 16, (rows, cols // 128), generator=g, dtype=torch.uint8).numpy() if zp else None
+    words, s16 = host.pack_marlin(codes, sc, zeros=zeros)
+    xd = torch.from_numpy(synth.activations(m, cols, g)).cuda()
+    y = ctx.marlin_gemm(xd, torch.from_numpy(words.view(np.int32)).cuda(), torch.from_numpy(s16.view(np.int16)).cuda().view(torch.float16), zp=zp)
+    s = sc.astype(np.float16)
+    wdq = R.dequant_z(codes, s, ((8.0 - zeros.astype(np.float32)) * sc).astype(np.float16)) if zp else R.dequant(codes, s)
+    wdq = torch.from_numpy(wdq[R.row_order(rows, False)]).cuda().double()  # (as rounded to f16: the sums' error is all there is)
+    want = xd.double() @ wdq.T
+    err = float((y.double() - want).norm() / want.norm())
+    assert err < 1e-7 + 1.7e-7 * longest, (err, longest)
+    assert ctx.device_error() == 0
 
 
 @pytest.mark.parametrize("m,rows,cols", [(17, 256, 128), (32, 512, 384), (33, 256, 640), (40, 1024, 2048), (63, 768, 256),
