@@ -68,7 +68,15 @@ struct Args {
     int unit;            // groups that stay together in a share: 1, or a tile's
 };
 
-// a += s x, two values at a time (each rounded as fmaf rounds it)
+// two values at a time: s x, a + s x (rounded as fmaf rounds it) and a + b
+__device__ __forceinline__ void mul2(float& a0, float& a1, float s, uint32_t x0, uint32_t x1) {
+    asm("{\n.reg .b64 s, x;\nmov.b64 s, {%2, %2};\nmov.b64 x, {%3, %4};\nmul.rn.f32x2 x, s, x;\nmov.b64 {%0, %1}, x;\n}\n"
+        : "=f"(a0), "=f"(a1) : "f"(s), "r"(x0), "r"(x1));
+}
+__device__ __forceinline__ void add2(float& a0, float& a1, float b0, float b1) {
+    asm("{\n.reg .b64 a, b;\nmov.b64 a, {%0, %1};\nmov.b64 b, {%2, %3};\nadd.rn.f32x2 a, a, b;\nmov.b64 {%0, %1}, a;\n}\n"
+        : "+f"(a0), "+f"(a1) : "f"(b0), "f"(b1));
+}
 __device__ __forceinline__ void fma2(float& a0, float& a1, float s, uint32_t x0, uint32_t x1) {
     asm("{\n.reg .b64 a, s, x;\nmov.b64 a, {%0, %1};\nmov.b64 s, {%2, %2};\nmov.b64 x, {%3, %4};\nfma.rn.f32x2 a, s, x, a;\nmov.b64 {%0, %1}, a;\n}\n"
         : "+f"(a0), "+f"(a1) : "f"(s), "r"(x0), "r"(x1));
@@ -251,8 +259,9 @@ __global__ void __launch_bounds__(Cfg<NT>::THREADS, 1)
                     if (dead && lane == 0) atomicExch(a.err, 16);
                 }
                 asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-                // the second group's sums are on their way while the first's are added (in a stage of one group they are whatever the
-                // accumulator holds, and not used)
+                // the second group's sums are on their way while the first's are scaled (in a stage of one group they are whatever the
+                // accumulator holds, and not used). A stage's two groups are added to each other first: half as many sums of full size, so that
+                // a block that walks a whole tile is no further from 64 bits than equal shares were (16384 x 5120: 1.19e-7 group by group)
                 uint32_t v[DT], w[DT];
                 tmem_ld16(tq + p * SG * NT, v);
                 // (the scales landed with the words: the products that made these sums came after)
@@ -260,16 +269,19 @@ __global__ void __launch_bounds__(Cfg<NT>::THREADS, 1)
                 const float s0 = __half2float(sp[0]), s1 = __half2float(sp[BH]);
                 asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
                 tmem_ld16(tq + (p * SG + 1) * NT, w);
+                float t[DT];
 #pragma unroll
-                for (int j = 0; j < DT; j += 2) fma2(acc[j], acc[j + 1], s0, v[j], v[j + 1]);
+                for (int j = 0; j < DT; j += 2) mul2(t[j], t[j + 1], s0, v[j], v[j + 1]);
                 asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
                 asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&dfree[p]);
                 if (gi + 1 < g1) {
 #pragma unroll
-                    for (int j = 0; j < DT; j += 2) fma2(acc[j], acc[j + 1], s1, w[j], w[j + 1]);
+                    for (int j = 0; j < DT; j += 2) fma2(t[j], t[j + 1], s1, w[j], w[j + 1]);
                 }
+#pragma unroll
+                for (int j = 0; j < DT; j += 2) add2(acc[j], acc[j + 1], t[j], t[j + 1]);
             }
             bool finish = !dead;
             if (cut) {
