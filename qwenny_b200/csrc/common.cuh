@@ -227,12 +227,6 @@ __device__ __forceinline__ void named_bar_sync(int id, int threads) {
     asm volatile("bar.sync %0, %1;\n" ::"r"(id), "r"(threads) : "memory");
 }
 
-__device__ __forceinline__ int atom_add_acq_rel(int* p, int v) {
-    int old;
-    asm volatile("atom.add.acq_rel.gpu.global.s32 %0, [%1], %2;\n" : "=r"(old) : "l"(p), "r"(v) : "memory");
-    return old;
-}
-
 // ---------------------------------------------------------------- global loads that bypass L1 (data another CTA
 // wrote during this kernel)
 __device__ __forceinline__ float4 ld_cg4(const float4* p) { return __ldcg(p); }
