@@ -138,9 +138,9 @@ delta_prep_kernel(const float* p, int splits, int n, const float* ba, int ba_spl
 // The same for prompt steps (one part, 16-byte aligned): a block keeps 512 channels and runs along `run` tokens, so that it starts
 // once and reads each row once, and a lane's 16 bytes of the next RUN_ROWS - 1 rows are on their way into shared memory, where they take
 // no registers and no other thread waits for them. grid (LQKV / 512, runs + the gates' blocks of PREP_TOK tokens), block 128.
-// Against the tiles of 8 tokens, us: 128 tokens 6.2 / 5.4, 256 8.4 / 8.5, 333 13.5 / 9.2, 512 16.7 / 12.8, 1024 29.2 / 20.6, 2048 53.2 / 35.2
-// (168 MB: 4.8 TB/s). More rows under way are slower (2048 tokens: 16 rows 39.2, 8 rows 37.0), so are fewer blocks (5 of 8 rows 40.8);
-// 7 or 8 blocks per SM are alike above 700 tokens and worse below (333: 9.7, 10.3).
+// Against the tiles of 8 tokens, us: 128 tokens 6.2 / 5.4, 200 7.6 / 6.1, 220 7.7 / 8.0, 256 8.4 / 8.4, 333 13.4 / 9.1, 512 16.7 / 12.8, 1024
+// 29.2 / 20.5, 2048 53.3 / 35.2 (168 MB: 4.8 TB/s). More rows under way are slower (2048 tokens: 16 rows 39.2, 8 rows 37.0), so are fewer blocks
+// (5 of 8 rows 40.8); 7 or 8 blocks per SM are alike above 700 tokens and worse below (333: 9.7, 10.3).
 constexpr int RUN_ROWS = 4, RUN_PER_SM = 6;
 constexpr int RUN_FROM = 128;  // tokens: a run has four tokens then, and below the tiles fill the SMs as well
 __global__ void __launch_bounds__(128, RUN_PER_SM)

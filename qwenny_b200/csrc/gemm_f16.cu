@@ -287,9 +287,17 @@ extern "C" int qb_gemm_f16_plain(qb_ctx* ctx, void* stream, const void* W, const
     const int per = qb_gemm_f16_block_tiles(ntiles, split, kper, n, ctx->sms);
     if (per > 1) {
         grid.x = ntiles / per;
-        // X gathered against copied, 96 x 5120 in 5 splits, X from four buffers in turn: 160 rows 8.2 and 7.8 us, 512 9.9 and 8.2, 1024 10.8
-        // and 11.0, 2048 23.7 and 12.3; 160 outputs, 1024 rows 19.8 and 12.5; 768 x 2048 in 2 splits, 1024 rows 19.3 and 20.1.
-        const bool whole = ((uintptr_t)x & 15) == 0;  // (K and kper are multiples of 16)
+        // Copied in 16-byte pieces, where X starts on such: three blocks per SM instead of two, but a round of them takes a tenth longer (and
+        // a block on its own a twentieth over a long k). So not where both forms take as many rounds and the last one is fairly full, unless X
+        // no longer stays in L2 beside the rest (from 12 MB on, taken from four buffers in turn). X gathered against copied, us: 96 x 5120 in 5 splits,
+        // 160 rows (25 blocks) 8.1 and 7.8, 512 9.9 and 8.3, 955 (150) 10.4 and 10.0, 1024 (160) 10.8 and 11.0, 2048 (320) 23.7 and 12.3; 160
+        // outputs, 1024 rows (800) 19.8 and 12.6; 384 x 2048 in 2 splits, 640 rows (160) 10.5 and 11.0, 1184 (296) 10.8 and 12.0, 1408 (352)
+        // 18.0 and 11.9; in 4 of 256, 832 rows (208) 5.1 and 4.9, 955 (240) 5.1 and 5.3; 768 x 2048 in 2, 1024 rows (512) 19.3 and 20.0; 768 x
+        // 5120 in one, 160 rows (40) 28.8 and 30.1, 333 (88) 36.9 and 31.5.
+        const long long blocks = (long long)grid.x * grid.y * grid.z, sms = ctx->sms;
+        const bool full = (blocks <= 2 * sms && 20 * blocks > (kper >= 1024 ? 21 : 30) * sms) || (blocks <= 4 * sms && 5 * blocks > 17 * sms) ||
+                          (3 * blocks <= sms && kper >= 4096);
+        const bool whole = ((uintptr_t)x & 15) == 0 && !(full && (long long)n * K <= 6 << 20);  // (K and kper are multiples of 16)
 #define QB_WIDE(T)                                                                                                                    \
     return whole ? launch(ctx, gemm_f16_staged_kernel<T>, grid, dim3(128), StagedCfg<T>::SMEM, st, w, x, xrows, K, ntiles, n, kper, Y, ldy) \
                  : launch(ctx, gemm_f16_wide_kernel<T>, grid, dim3(128), 0, st, w, x, xrows, K, ntiles, n, kper, Y, ldy)

@@ -154,7 +154,7 @@ def test_gemm_f16_blocks_of_tiles_have_the_bits_of_one_tile(ctx, n, tiles, kper,
     assert torch.equal(y, torch.cat(slabs, 1))
 
 
-@pytest.mark.parametrize("n,tiles,kper", [(700, 6, 256), (1633, 4, 144), (261, 10, 384)])
+@pytest.mark.parametrize("n,tiles,kper", [(700, 6, 256), (1633, 4, 144), (1900, 12, 192), (261, 10, 384)])
 def test_gemm_f16_rows_off_16_bytes(ctx, n, tiles, kper):
     """Rows that start on 16 bytes are copied in such pieces, others gathered: the same bits."""
     K = 384
