@@ -128,17 +128,21 @@ __host__ __device__ __forceinline__ int tile_chunk(int keys, int z) { return max
 // single round of blocks can take less (20 rows at context 30000 126 us, 146 so), but of several the shorter ones then leave their SMs early
 // (8 of 20 rows up to 30000 930 us, 761 so), and that the host does not know here. Nor more than a round of blocks of less than 384 keys
 // (100 rows at 1000, 6 splits of 192 52.5 us, 51 with 4 of 320: partials). Where the first rule says one split the tcgen05 forms do the
-// step; tiles x splits stay below 75, which bounds the partials of any step to 740 tokens.
+// step. Tiles x splits stay below 75: with the 64 decode tokens that may stand before a step's tiles (partials are kept by the step's
+// token) that is (64 + 10 tiles) x splits, 2700 partials a head at most. 148 SMs whatever the part: the caller sizes its scratch by this
+// count, and names no device.
 // By the first rule alone / now, one sequence, with attn_prep and the combine, us: 10 rows at context 600 34.7 / 21.0, at 1000 46.5 / 21.4, at
 // 4000 46.1 / 27.1; 20 at 1000 48.4 / 22.4; 40 at 1000 37.2 / 26.3; 64 at 30000 494 / 404; 100 at 4000 153 / 111, at 30000 928 / 574; 200 at 30000
-// 1880 / 1289. Of several sequences of unequal lengths: 3 of 20 rows up to 9000 110 / 103, 6 of 10 up to 30000 302 / 276, 3 of 40 up to 9000 184 / 190.
+// 1880 / 1289. Of several sequences of unequal lengths: 3 of 20 rows up to 9000 111 / 103, 6 of 10 up to 30000 305 / 275, 2 of
+// 100 up to 9000 354 / 279; slower are 3 of 40 up to 9000 188.5 / 189.4, 4 of 30 up to 5000 119.5 / 124.7 (one sequence of 100 rows gains a quarter).
+constexpr int TSMS = 148;
 __host__ inline int tile_splits(int ntile, int max_keys) {
     int z = 1;
-    while (z < TSPLITS && ntile * NKV * z * 2 <= 2 * 148 && max_keys / (z * 2) >= 256) z *= 2;
+    while (z < TSPLITS && ntile * NKV * z * 2 <= 2 * TSMS && max_keys / (z * 2) >= 256) z *= 2;
     int best = z;
     long long least = 0;
     for (int y = z; z > 1 && y <= TSPLITS && ntile * y < 75; y++) {
-        const int chunk = tile_chunk(max_keys, y), ns = (max_keys + chunk - 1) / chunk, rounds = (ntile * NKV * ns + 147) / 148;
+        const int chunk = tile_chunk(max_keys, y), ns = (max_keys + chunk - 1) / chunk, rounds = (ntile * NKV * ns + TSMS - 1) / TSMS;
         const long long cost = rounds * (3000 + 2050ll * (chunk / 32)) + 100 * ns;
         if (y == z) least = cost - cost / 7;
         else if (cost < least && (rounds == 1 || chunk >= 384)) { least = cost; best = y; }

@@ -248,8 +248,8 @@ def test_form_of_the_prompt_attention():
 
 
 def test_tile_splits_stay_within_the_partials():
-    """Key splits of a few prompt tiles: more than one from 512 keys up to 37 tiles, at most 32, and tiles x splits below 75 (the
-    partials of any step are 740 tokens' at most); no fewer than two blocks per SM and 256 keys per split ask for."""
+    """Key splits of a few prompt tiles: more than one from 512 keys up to 37 tiles, at most 32, and tiles x splits below 75, so that
+    (64 decode tokens + 10 a tile) x splits stay within the model's 64 x 128 partials a head; no fewer than two blocks per SM and 256 keys per split ask for."""
     from qwenny_b200._lib import lib
     for tiles in range(1, 80):
         for keys in (1, 255, 511, 512, 513, 1000, 1024, 1025, 2047, 4010, 9012, 9040, 16384, 30010, 32768, 262144):
@@ -257,4 +257,4 @@ def test_tile_splits_stay_within_the_partials():
             least = 1
             while least < 32 and tiles * 4 * least * 2 <= 296 and keys // (least * 2) >= 256:
                 least *= 2
-            assert least <= z <= 32 and (z > 1) == (tiles <= 37 and keys >= 512) and (z == 1 or tiles * z < 75), (tiles, keys, z)
+            assert least <= z <= 32 and (z > 1) == (tiles <= 37 and keys >= 512) and (z == 1 or tiles * z < 75 and (64 + 10 * tiles) * z <= 64 * 128), (tiles, keys, z)
