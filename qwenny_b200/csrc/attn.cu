@@ -118,7 +118,7 @@ attn_prep_kernel(const float* part, int splits, int n, const float* q_norm, cons
     }
 }
 
-// ------------------------------------------------------------------------------------------------ attn_decode
+// ------------------------------------------------------------------------------------------------ prompt tiles
 __device__ __forceinline__ uint32_t kv_half2(uint32_t w, uint32_t sel) { return __byte_perm(w, 0x64646464u, sel); }
 
 // Prompt tiles: z key splits of a whole number of 64-key blocks (z from tile_splits on the host: one value per step).
@@ -152,7 +152,7 @@ __host__ inline int tile_splits(int ntile, int max_keys) {
 
 // RT row tiles of 16 (token, head) rows; KW warps per row tile, one 16-key block of a stage each; NS ring stages
 template <int RT, int KW, int NS>
-struct DecCfg {
+struct TileCfg {
     static constexpr int KWARPS = KW, NSTG = NS;
     static constexpr int SK = 16 * KW;                // keys per ring stage
     static constexpr int STG_BYTES = SK * HD * 2 + SK * 4 * 2;  // keys, values, key scales, value scales
@@ -165,15 +165,27 @@ struct DecCfg {
     static_assert(RT * (KW / 2) * MERGE_FLOATS * 4 <= NS * STG_BYTES, "the merge buffers reuse the ring");
 };
 
-// TILES = false: block (short segment, kv head, key split) of the decode attention (dseg / dtok name the tokens).
-// TILES = true: block (prompt tile, kv head): `dseg` is the host's ptile array (first token, count) of tiles of
-// consecutive tokens, each block takes all the keys of its tile (one split) and finishes its rows.
-template <int RT, int KW, int NS, bool TILES>
-__global__ void __launch_bounds__(DecCfg<RT, KW, NS>::THREADS, 1)
-attn_decode_kernel(const float* q, const uint8_t* kc, const uint8_t* vc, const float* ks, const float* vs,
-                   const int* dseg, const int* dtok, const int* tok_slot, const int* tok_pos, int cap, int z,
-                   float* part_ml, float* part_acc, float* out, __half* mix, int* err) {
-    using C = DecCfg<RT, KW, NS>;
+// 128 dims of two keys, 8 apart, as a lane's words of the key fragments. Keys are 256 bytes apart, all in the same banks, so the lanes of
+// odd keys (odd) read the two halves the other way round.
+__device__ __forceinline__ void key_words(const uint8_t* kp, bool odd, uint32_t* w0, uint32_t* w1) {
+#pragma unroll
+    for (int i = 0; i < 2; i++) {
+        const uint8_t* k = kp + i * 8 * HD;
+        const uint4 a = *(const uint4*)(k + (odd ? 64 : 0)), b = *(const uint4*)(k + (odd ? 0 : 64));
+        const uint4 lo = odd ? b : a, hi = odd ? a : b;
+        uint32_t* w = i ? w1 : w0;
+        w[0] = lo.x; w[1] = lo.y; w[2] = lo.z; w[3] = lo.w;
+        w[4] = hi.x; w[5] = hi.y; w[6] = hi.z; w[7] = hi.w;
+    }
+}
+
+// Block (prompt tile, kv head, key split) of the prompt attention of a few tiles: ptile is the host's array of tiles (first token, count) of
+// consecutive tokens.
+template <int RT, int KW, int NS>
+__global__ void __launch_bounds__(TileCfg<RT, KW, NS>::THREADS, 1)
+attn_tile_kernel(const float* q, const uint8_t* kc, const uint8_t* vc, const float* ks, const float* vs, const int* ptile,
+                 const int* tok_slot, const int* tok_pos, int cap, int z, float* part_ml, float* part_acc, float* out, int* err) {
+    using C = TileCfg<RT, KW, NS>;
     constexpr int KWARPS = C::KWARPS, NSTG = C::NSTG, SK = C::SK, STG_BYTES = C::STG_BYTES;
     constexpr int NTD = HD / 8;  // n8 dim tiles of the output
     extern __shared__ __align__(128) uint8_t smem[];
@@ -182,7 +194,7 @@ attn_decode_kernel(const float* q, const uint8_t* kc, const uint8_t* vc, const f
     __half* qsh = (__half*)(smem + C::BAR_BYTES);
     uint8_t* ring = smem + C::BAR_BYTES + C::Q_BYTES;
 
-    const int seg = TILES ? gridDim.x - 1 - blockIdx.x : blockIdx.x;  // prompt tiles: the longest contexts first
+    const int tile = gridDim.x - 1 - blockIdx.x;  // the longest contexts first
     const int g = blockIdx.y, s = blockIdx.z, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
         for (int i = 0; i < NSTG; i++) { mbar_init(&full[i], 1); mbar_init(&empty[i], C::CW); }
@@ -192,10 +204,9 @@ attn_decode_kernel(const float* q, const uint8_t* kc, const uint8_t* vc, const f
     pdl_launch_dependents();
     pdl_wait();  // the step's own keys and values are written by attn_prep just before
 
-    const int first = dseg[2 * seg], nt = dseg[2 * seg + 1];
-    auto token = [&](int i) { return TILES ? first + i : dtok[first + i]; };
-    const int tlast = token(nt - 1), keys = tok_pos[tlast] + 1;
-    const int chunk = TILES ? tile_chunk(keys, z) : dec_chunk(keys, DSPLITS), ns = (keys + chunk - 1) / chunk;
+    const int first = ptile[2 * tile], nt = ptile[2 * tile + 1];
+    const int tlast = first + nt - 1, keys = tok_pos[tlast] + 1;
+    const int chunk = tile_chunk(keys, z), ns = (keys + chunk - 1) / chunk;
     if (s >= ns) return;
     const int kbeg = s * chunk, ke = min(keys, kbeg + chunk), nstg = (ke - kbeg + SK - 1) / SK;
     const int slot = tok_slot[tlast];
@@ -240,7 +251,7 @@ attn_decode_kernel(const float* q, const uint8_t* kc, const uint8_t* vc, const f
     for (int x = threadIdx.x; x < RT * 16 * HD / 4; x += C::CW * 32) {
         int row = x / (HD / 4), d = (x % (HD / 4)) * 4, tok = row / GROUP;
         float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (tok < nt) v = *(const float4*)(q + ((size_t)token(tok) * NH + g * GROUP + row % GROUP) * HD + d);
+        if (tok < nt) v = *(const float4*)(q + ((size_t)(first + tok) * NH + g * GROUP + row % GROUP) * HD + d);
         *(uint2*)&qsh[row * SROW + d] = make_uint2(pack_half2(v.x, v.y), pack_half2(v.z, v.w));
     }
     named_bar_sync(1, C::CW * 32);
@@ -261,7 +272,7 @@ attn_decode_kernel(const float* q, const uint8_t* kc, const uint8_t* vc, const f
 #pragma unroll
     for (int h2 = 0; h2 < 2; h2++) {
         int tok = (wt * 16 + r + 8 * h2) / GROUP;
-        lim[h2] = tok < nt ? min(ke, tok_pos[token(tok)] + 1) : 0;
+        lim[h2] = tok < nt ? min(ke, tok_pos[first + tok] + 1) : 0;
     }
     float m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f}, ps[2] = {0.f, 0.f}, o[NTD][4];
 #pragma unroll
@@ -300,15 +311,8 @@ attn_decode_kernel(const float* q, const uint8_t* kc, const uint8_t* vc, const f
             float sacc[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
 #pragma unroll
             for (int b2 = 0; b2 < HD / 128; b2++) {
-                // (odd keys' lanes read the two halves of 128 dims the other way round: attn_dec4_kernel)
-                const bool odd = r & 1;
-                const uint8_t* p0 = kp + 128 * b2 + (odd ? 64 : 0);
-                const uint8_t* p1 = kp + 128 * b2 + (odd ? 0 : 64);
-                const uint4 x0 = *(const uint4*)p0, x1 = *(const uint4*)p1, y0 = *(const uint4*)(p0 + 8 * HD), y1 = *(const uint4*)(p1 + 8 * HD);
-                const uint32_t w0[8] = {odd ? x1.x : x0.x, odd ? x1.y : x0.y, odd ? x1.z : x0.z, odd ? x1.w : x0.w,
-                                        odd ? x0.x : x1.x, odd ? x0.y : x1.y, odd ? x0.z : x1.z, odd ? x0.w : x1.w};
-                const uint32_t w1[8] = {odd ? y1.x : y0.x, odd ? y1.y : y0.y, odd ? y1.z : y0.z, odd ? y1.w : y0.w,
-                                        odd ? y0.x : y1.x, odd ? y0.y : y1.y, odd ? y0.z : y1.z, odd ? y0.w : y1.w};
+                uint32_t w0[8], w1[8];
+                key_words(kp + 128 * b2, r & 1, w0, w1);
 #pragma unroll
                 for (int st = 0; st < 8; st++) {
                     uint32_t a[4];
@@ -421,19 +425,17 @@ attn_decode_kernel(const float* q, const uint8_t* kc, const uint8_t* vc, const f
         P += __shfl_xor_sync(0xffffffffu, P, 2);
         int row = wt * 16 + r + 8 * h2, tok = row / GROUP;
         if (tok >= nt) continue;
-        int i = first + tok, t = token(tok), head = g * GROUP + row % GROUP;
+        int t = first + tok, head = g * GROUP + row % GROUP;
         if (ns == 1) {
             float f = 1.f / L;
             float* op = out + (size_t)t * MIX + head * HD + 2 * t4;
 #pragma unroll
             for (int j = 0; j < NTD; j++) {
                 float2 gt = *(float2*)(op + j * 8);
-                float2 res = make_float2(gt.x * (o[j][2 * h2] - KV_OFF * P) * f, gt.y * (o[j][2 * h2 + 1] - KV_OFF * P) * f);
-                *(float2*)(op + j * 8) = res;
-                if (TILES && mix) *(__half2*)(mix + (size_t)t * MIX + head * HD + 2 * t4 + j * 8) = __floats2half2_rn(res.x, res.y);
+                *(float2*)(op + j * 8) = make_float2(gt.x * (o[j][2 * h2] - KV_OFF * P) * f, gt.y * (o[j][2 * h2 + 1] - KV_OFF * P) * f);
             }
         } else {
-            size_t pi = ((size_t)i * NH + head) * z + s;
+            size_t pi = ((size_t)t * NH + head) * z + s;
             float* pp = part_acc + pi * HD + 2 * t4;
 #pragma unroll
             for (int j = 0; j < NTD; j++)
@@ -741,17 +743,10 @@ attn_dec4_kernel(const float* q, const uint8_t* kc, const uint8_t* vc, const flo
                 for (int nn = 0; nn < 2; nn++) v[rt][nn][0] = v[rt][nn][1] = v[rt][nn][2] = v[rt][nn][3] = 0.f;
 #pragma unroll
             for (int b2 = 0; b2 < HD / 128; b2++) {
-                // Keys are 256 bytes apart, all in the same banks, so the lanes of odd keys read the two halves of 128 dims the other way
-                // round (5 rows at context 32000 30.35 -> 29.67 us; not with one row tile, whose warps have no registers left for it: 8
-                // sequences of one row 42.3 -> 44.8).
-                const bool odd = RT > 1 && (r & 1);
-                const uint8_t* p0 = kp + 128 * b2 + (odd ? 64 : 0);
-                const uint8_t* p1 = kp + 128 * b2 + (odd ? 0 : 64);
-                const uint4 x0 = *(const uint4*)p0, x1 = *(const uint4*)p1, y0 = *(const uint4*)(p0 + 8 * HD), y1 = *(const uint4*)(p1 + 8 * HD);
-                const uint32_t w0[8] = {odd ? x1.x : x0.x, odd ? x1.y : x0.y, odd ? x1.z : x0.z, odd ? x1.w : x0.w,
-                                        odd ? x0.x : x1.x, odd ? x0.y : x1.y, odd ? x0.z : x1.z, odd ? x0.w : x1.w};
-                const uint32_t w1[8] = {odd ? y1.x : y0.x, odd ? y1.y : y0.y, odd ? y1.z : y0.z, odd ? y1.w : y0.w,
-                                        odd ? y0.x : y1.x, odd ? y0.y : y1.y, odd ? y0.z : y1.z, odd ? y0.w : y1.w};
+                // (the halves turned round: 5 rows at context 32000 30.35 -> 29.67 us; not with one row tile, whose warps had no registers left
+                // for it: 8 sequences of one row 42.3 -> 44.8)
+                uint32_t w0[8], w1[8];
+                key_words(kp + 128 * b2, RT > 1 && (r & 1), w0, w1);
 #pragma unroll
                 for (int st = 0; st < 8; st++) {
                     const uint32_t b00 = kv_half2(w0[st], 0x4140), b01 = kv_half2(w0[st], 0x4342);
@@ -1255,13 +1250,12 @@ int qb_attn_prefill_as(qb_ctx* ctx, void* stream, const float* q, const void* kc
         if (!rc && form != 1) rc = qb_attn_prefill_short_launch(ctx, st, q, kc, vc, ks, vs, ptile, ntile, tok_slot, tok_pos, cap, out, mix_f16, word);
         return rc;
     }
-    using C = DecCfg<4, 2, 5>;  // 10 tokens x 6 heads = 60 rows: 4 row tiles; 2 warps each; 5 stages of 32 keys
+    using C = TileCfg<4, 2, 5>;  // 10 tokens x 6 heads = 60 rows: 4 row tiles; 2 warps each; 5 stages of 32 keys
     static_assert(PTILE * GROUP <= 64, "a prompt tile fills at most 4 row tiles");
     cudaStream_t st = (cudaStream_t)stream;
-    int rc = launch(ctx, attn_decode_kernel<4, 2, 5, true>, dim3(ntile, NKV, z), dim3(C::THREADS), C::SMEM, st, q,
-                    (const uint8_t*)kc, (const uint8_t*)vc, ks, vs, ptile, (const int*)nullptr, tok_slot, tok_pos, cap, z,
-                    part_ml, part_acc, out, z == 1 ? (__half*)mix_f16 : (__half*)nullptr, ctx->err);
-    if (rc || z == 1) return rc;
+    int rc = launch(ctx, attn_tile_kernel<4, 2, 5>, dim3(ntile, NKV, z), dim3(C::THREADS), C::SMEM, st, q, (const uint8_t*)kc,
+                    (const uint8_t*)vc, ks, vs, ptile, tok_slot, tok_pos, cap, z, part_ml, part_acc, out, ctx->err);
+    if (rc) return rc;
     return launch(ctx, attn_combine_tiles_kernel, dim3(ntile * PTILE, NH), dim3(HD), 0, st, (const float*)part_ml,
                   (const float*)part_acc, ptile, tok_pos, z, out, (__half*)mix_f16);
 }
