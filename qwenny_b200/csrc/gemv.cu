@@ -275,13 +275,16 @@ extern "C" int qb_marlin_gemm(qb_ctx* ctx, void* stream, const void* X, const vo
     // more than 64 rows, plain and SwiGLU epilogues, contiguous: the prompt-sized tensor-core product
     if (m > 64 && epi != QB_EPI_ARGMAX && !xrows && !ctx->no_tc)
         return qb_gemm_tc_launch(ctx, st, X, B, Y, S, m, n, k, row0, epi, 0);
-    // slabs: 17 .. 64 rows through the tensor-core product for a few rows, up to 16 through the skinny kernel. At 16 rows the
-    // skinny kernel takes 22, 10, 30 and 21 us over the layer's four shapes, at 17 the other 16, 11, 30 and 19 (two skinny
-    // slabs 43, 20, 60 and 42); 40 gathered rows of a 248,320-row output layer take 577 us as three 16-row slabs, 207 so.
+    // slabs: 17 .. 64 rows through the tensor-core product for a few rows, up to 16 through the skinny kernel. The line is at 16 because a
+    // row has the same bits alone and among up to 16 (a verify step gives the tokens of one step per token), and the two kernels add in
+    // different orders; by time the other one could take over at 9 rows in two of the layer's shapes: skinny / other, us, at 9 rows 20.9 /
+    // 17.0, 10.0 / 10.7, 30.0 / 30.5 and 20.5 / 19.1, at 16 21.7 / 16.9, 10.3 / 10.5, 30.5 / 29.9 and 20.7 / 19.2, the MLP 52.4 / 52.7, an output
+    // layer of 151,936 rows 146 / 121. At 17 rows two skinny slabs take 43, 20, 60 and 42, the other 16, 11, 30 and 19; 40 gathered rows of a
+    // 248,320-row output layer take 577 us as three 16-row slabs, 211 so.
     // The upper bound is that of its tiles, not where times cross: the prompt-sized product has no gathered and no argmax
     // form, and it rounds each weight to f16, which is exact for bf16 scales only (error against 64 bits 5e-5; with the
-    // group's scale applied to the f32 sum 8e-7, as up to 16 rows). At 17 rows it takes 19, 14, 38 and 24 us, at 64 20, 15, 41 and 27
-    // against 20, 14, 37 and 25.
+    // group's scale applied to the f32 sum 1e-7, up to 16 rows 7e-7). At 17 rows it takes 20, 13, 38 and 22 us, at 64 22, 16, 41 and 26
+    // against 21, 14, 38 and 25.
     int mm;
     for (int r = 0; r < m; r += mm) {
         mm = m - r;

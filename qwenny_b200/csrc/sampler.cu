@@ -122,7 +122,8 @@ __device__ __forceinline__ float scan1024(float v, float* sh) {
     return r;
 }
 
-// c[0 .. n) in order, descending or ascending; no two keys are equal. SCAP entries of c are written.
+// c[0 .. n) in order, descending or ascending; no two keys are equal. Up to SRANK keys only those n entries are written; beyond, the
+// network fills c up to the next power of two, for which it must have room (SCAP at most).
 template <bool ASC>
 __device__ __forceinline__ void sort_keys(unsigned long long* c, int n, int tid) {
     int np = 1;

@@ -4,26 +4,27 @@
 //
 // A block owns 128 outputs and the weights go from registers to tensor memory in the layout that a Marlin word already has
 // (w4a16_gemm_tc.cu). The floor is the weights' way from HBM (0.52 bytes each, read once): 760 cycles per block and stage, two groups
-// of 128 of k. A stage takes some 1350 (40 rows of a 248,320-output matrix, 262 stages a block): the way of a slot of tensor memory from
-// "free" to "multiplied" (unpacking 680, the issue of 16 products 800, 130 to 150 per check of a barrier; a group's slot each, 4 to 6 of
-// them in turn: with a slot per stage, two in turn, a stage took 1440), and 40 KB through shared memory a stage, 24 of them the rows again. What a launch spends beside its stages: 3 us from its first instruction to the
-// first unpacked stage, 3 us from a cut tile's last sum to its result (partial sums 0.2, fence and ticket 1.1, parts 0.6, epilogue 0.7).
-// From a graph, 40 rows: the MLP 56.4 us (one group per stage, a fence per thread and 64-bit divisions before the ticket, one round
-// trip per part, shares whatever the shape: 78.7), 5120 x 6144 12.0 (19.6), the output layer of 248,320 rows 207 (298); 17 and 64 rows of
-// the MLP 52.5 (72) and 64.0 (86.5). What differs from the prompt-sized product:
+// of 128 of k. A stage takes some 1350 (40 rows of a 248,320-output matrix, 262 stages a block): the way of a slot of tensor memory
+// from "free" to "multiplied" (unpacking 680, the issue of 16 products 800, 130 to 150 per check of a barrier; a group's slot each, 4 to
+// 6 of them in turn: with a slot per stage, two in turn, a stage took 1440), and 40 KB through shared memory a stage, 24 of them
+// the rows again. What a launch spends beside its stages: 3 us from its first instruction to the first unpacked stage, 3 us from a cut
+// tile's last sum to its result (partial sums 0.2, fence and ticket 1.1, parts 0.6, epilogue 0.7).
+// From a graph, 40 rows: the MLP 56.5 us (one group per stage, a fence per thread and 64-bit divisions before the ticket, one round
+// trip per part, shares whatever the shape: 78.7), 5120 x 6144 12.1 (19.6), the output layer of 248,320 rows 211 (298); 17 and 64
+// rows of the MLP 52.7 (72) and 65.7 (86.5). What differs from the prompt-sized product:
 //   - the weights are the exact integers q - 8; a group of 128 columns is one accumulation, and the drain warps multiply its
-//     f32 sums by the f32 value of the group's scale and add them up in registers (one thread per output, a register
-//     per token): one rounding per group, the arithmetic of the product for up to 16 rows (w4a16_gemv.cuh), where
-//     f16((q - 8) s) would round every weight. Two pairs of accumulators take turns, so that draining one overlaps the next products,
-//     and two warps issue in turn, so that one's checks overlap the other's products
-//   - a stage is two groups: a role checks its barriers once for both (with one group per stage a drain warp's chain of check, load, check of
-//     the scales and sums took 1000 cycles a group and was what everything waited for)
+//     f32 sums by the f32 value of the group's scale and add them up in registers (one thread per output, a register per token), as
+//     the product for up to 16 rows does (w4a16_gemv.cuh), where f16((q - 8) s) would round every weight. Two pairs of accumulators take
+//     turns, so that draining one overlaps the next products, and two warps issue in turn, so that one's checks overlap the other's
+//     products
+//   - a stage is two groups: a role checks its barriers once for both (with one group per stage a drain warp's chain of check, load,
+//     check of the scales and sums took 1000 cycles a group and was what everything waited for)
 //   - a drain warp takes 16 tokens: with 32 its threads held 64 values and spilled
-//   - gathered rows (the output layer) are copied together first, by a launch of their own: gathered by cp.async in every block they slowed
-//     the unpacking from 680 to 1070 cycles a stage (40 rows of 248,320 outputs 269 us against 218 at that time, launch included)
-// The (tile, group) list is dealt to at most one block per SM: whole tiles, tiles cut into equal parts, or equal shares; parts of a cut tile are added by its last arriver in
-// block order (the bits repeat). Its ticket is taken behind a barrier by one thread with one fence (a fence per thread: 2 us; a ticket
-// per warp instead of the barriers: the output layer 241 us against 232).
+//   - gathered rows (the output layer) are copied together first, by a launch of their own: gathered by cp.async in every block they
+//     slowed the unpacking from 680 to 1070 cycles a stage (40 rows of 248,320 outputs 269 us against 218 at that time, launch included)
+// The (tile, group) list is dealt to at most one block per SM: whole tiles, tiles cut into equal parts, or equal shares; parts of a cut
+// tile are added by its last arriver in block order (the bits repeat). Its ticket is taken behind a barrier by one thread with one fence
+// (a fence per thread: 2 us; a ticket per warp instead of the barriers: the output layer 241 us against 232).
 #include "launch.h"
 #include "pair_tc.cuh"
 
@@ -456,10 +457,13 @@ int qb_gemm_mid_launch(qb_ctx* ctx, cudaStream_t st, const void* X, const void* 
     a.S = (const __half*)S; a.Y = Y; a.keys = keys; a.m = m; a.N = n; a.K = k;
     a.y0 = y0; a.n_valid = n_valid; a.err = ctx->err; a.part = ctx->tc_part;
     a.tickets = ctx->tc_tickets; a.iters = tiles * (k / 128); a.tiles = tiles;
-    // How the list is dealt: whole tiles in rounds, each tile cut into `cuts` equal parts for as many blocks (few tiles), or equal shares of
-    // the list (parts of two tiles a block), by an estimate in ns of the longest block's groups and of joining the parts. Measured
-    // at 40 rows, us: 16384 x 5120 whole 19.2, shares 21.4; 5120 x 6144 in two 14.9, in three 12.5, shares 13.7; 5120 x 17408 in three 23.5,
-    // shares 22.7; 2048 x 2048 whole 9.6, in four 8.1, shares 10.1; 1024 x 1024 whole 6.5, in two 7.3, shares 7.9.
+    // How the list is dealt: whole tiles in rounds, each tile cut into c equal parts for as many blocks (few tiles), or equal shares of
+    // the list (parts of two tiles a block), by an estimate in ns of the longest block's groups and of joining the parts. Measured at 40
+    // rows, us: 16384 x 5120 whole 17.9, shares 20.4; 5120 x 6144 whole 19.3, in two 14.0, in three 12.1, shares 13.3; 5120 x 17408 in
+    // three 22.0, shares 21.4; 2048 x 2048 whole 8.8, in two 8.4, four 7.8, six 8.0, shares 10.1; 1024 x 1024 whole 6.0, in two 7.1, shares
+    // 7.8. Of these forms (and six parts) the choice is the fastest or within 3 % of it at 17, 40 and 64 rows of those and of 14336 x
+    // 5120, 34816 x 5120, 5120 x 10240, 4096 x 4096, 8192 x 2048, 3072 x 8192, 2560 x 5120, 12288 x 4096, 20480 x 2560, 1280 x 17408 and
+    // 7168 x 1024, but for 2048 x 2048 at 17 rows, 7.0 where four parts take 6.6.
     const long long ngr = k / 128, sms = ctx->sms, group = 300 + nt * 6 / 5, rounds = (tiles + sms - 1) / sms;
     long long best = a.iters * group / sms + 2000 + 67 * nt, units = a.iters;
     a.unit = 1;

@@ -13,9 +13,10 @@
 // 1024. A stage is 128 of k because the issuing warps are the next limit: a wait, a commit and their like cost 180 cycles per
 // stage beside 65 per product, and the copying lane 70 per copy (64 of k per stage: 600 cycles of the 512 at N = 256).
 //
-// The work is the list of (tile, k block of 128) pairs, tile after tile, on a persistent grid of at most one pair per two SMs. Where whole tiles
-// leave pairs idle the list is dealt out in equal contiguous shares (stream-K): a pair that ends or starts inside a tile writes that tile's partial accumulators to scratch and takes a ticket; the
-// tile's last arriver adds the parts in pair order and runs the epilogue, nobody waits.
+// The work is the list of (tile, k block of 128) pairs, tile after tile, on a persistent grid of at most one pair per two SMs. Where
+// whole tiles leave pairs idle the list is dealt out in equal contiguous shares (stream-K): a pair that ends or starts inside a tile
+// writes that tile's partial accumulators to scratch and takes a ticket; the tile's last arriver adds the parts in pair order and runs
+// the epilogue, nobody waits.
 // Per (tile, k block):
 //   warps 0-7   dequantise: lop3 / hsub2 to q - 8, one hfma2 by the f16 group scale (the reference's rounding:
 //               w = f16((q - 8) s), kernels/marlin.cuh:100-124), tcgen05.st into the stage's 64 columns
@@ -81,7 +82,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
     uint64_t* done = empty + NSTAGE;            // all products of a segment are done
     uint64_t* accfree = done + 1;               // (first block) both blocks have read the segment's accumulators
     uint32_t* tmem_slot = (uint32_t*)(accfree + 1);
-    int* flag = (int*)(tmem_slot + 1);          // this block finishes its half of the tile (the ticket's answer, for the epilogue warps); the first of the pairs that hold it, how many
+    // this block finishes its half of the tile (the ticket's answer, for the epilogue warps); the first of the pairs that hold it, how many
+    int* flag = (int*)(tmem_slot + 1);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int rank = (int)cluster_ctarank(), pair = blockIdx.x >> 1, G = gridDim.x >> 1;
