@@ -15,6 +15,7 @@
 // The size of a key split is a function of the key count alone (dec_chunk), so a token's sums are the same whether
 // it runs alone or with drafts.
 #include "attn_tc.cuh"
+#include "dec_ring.h"
 #include "launch.h"
 #include "measure.h"
 
@@ -598,20 +599,18 @@ attn_dec4_kernel(const float* q, const uint8_t* kc, const uint8_t* vc, const flo
     constexpr int NCW = C::THREADS;
     // (with many splits the slots at the front are those that the quads merge through, and a split's first stages go behind them)
     constexpr int OFF = MANY ? C::MERGE_SLOTS : 0;
-    int j0 = 0;         // the stages of the block's splits before this one
-    uint32_t pars = 0;  // bit i: the parity that this split's first stage in slot i waits for
-    auto place = [&](int j) { return (j + OFF) % NSTG; };
+    using Ring = DecRing<C::QUADS, NSTG, OFF>;
+    Ring order;
     const uint64_t pol = policy_evict_first();
     auto copy = [&](int j, int part) {
         const uint8_t* from = part == 0 ? kc + cache_head(slot, g, cap) + (size_t)kbeg * HD : part == 1 ? vc + cache_head(slot, g, cap) + (size_t)kbeg * HD
                               : (const uint8_t*)((part == 2 ? ks : vs) + scale_head(slot, g, cap) + kbeg);
         const uint32_t bytes = part < 2 ? SK * HD : SK * 4, to = part < 2 ? part * SK * HD : 2 * SK * HD + (part - 2) * SK * 4;
-        bulk_g2s(ring + place(j) * STG_BYTES + to, from + (size_t)j * bytes, bytes, &full[place(j)], pol);
+        bulk_g2s(ring + Ring::slot(j) * STG_BYTES + to, from + (size_t)j * bytes, bytes, &full[Ring::slot(j)], pol);
     };
-    auto arm = [&](int i) {
-        const int j = j0 + i;  // (counted through the block's splits: a number of the split before says nothing of this one)
-        mbar_expect_tx(&full[place(i)], STG_BYTES);
-        issued[place(i)] = j;
+    auto arm = [&](int j) {
+        mbar_expect_tx(&full[Ring::slot(j)], STG_BYTES);
+        issued[Ring::slot(j)] = order.number(j);
     };
     int begin = min(nstg, NSTG);
     if (warp < begin && lane == 0) arm(warp);
@@ -674,7 +673,7 @@ attn_dec4_kernel(const float* q, const uint8_t* kc, const uint8_t* vc, const flo
     bool fresh = true, dead = false;  // fresh: these rows' Q is not in place yet
     for (;;) {  // MANY: the block's splits; else the one
         if (fresh) {
-            load_q(j0 == 0);
+            load_q(order.j0 == 0);
             named_bar_sync(1, NCW);
 #pragma unroll
             for (int rt = 0; rt < RT; rt++)
@@ -703,22 +702,19 @@ attn_dec4_kernel(const float* q, const uint8_t* kc, const uint8_t* vc, const flo
         }
 
         for (int j = quad; j < nstg; j += C::QUADS) {
-            const int sl = place(j);
-            const uint32_t par = ((j / NSTG) ^ (pars >> sl)) & 1;
+            const int sl = Ring::slot(j);
+            const uint32_t par = order.parity(j);
             if (!dead) {
-                // A slot's stages go to different quads, and a parity says nothing to a waiter that is two phases behind: one whose slot still
-                // waits for its last stage's copies would be let through. A stage is asked for only when that one was consumed.
                 uint32_t polls = 0;
-                if (j >= NSTG)
-                    while (issued[sl] != j0 + j && polls < WAIT_LIMIT) polls++;
+                if (Ring::looks(j))
+                    while (issued[sl] != order.number(j) && polls < WAIT_LIMIT) polls++;
                 dead = polls == WAIT_LIMIT || !mbar_wait(&full[sl], par);
                 if (dead && lane == 0) atomicExch(err, 4);
             } else {
                 for (int k = 0; k < 1024 && !mbar_try_wait(&full[sl], par); k++) {}
             }
-            // two quads: the slot of the quad's stage before this one is filled again in the middle of this one
-            const bool refill = C::QUADS == 2 && j >= 2 && j - 2 + NSTG < nstg;
-            if (refill && w == 0 && lane == 0) arm(j - 2 + NSTG);
+            const int refill = Ring::in_the_middle(j, nstg);  // the slot of the quad's stage before this one is filled again
+            if (refill >= 0 && w == 0 && lane == 0) arm(refill);
             const uint8_t* base = ring + sl * STG_BYTES;
             const int kb = kbeg + j * SK + 16 * w;  // this warp's 16 keys of the stage
             const uint8_t* kp = base + (16 * w + r) * HD + 16 * t4;
@@ -783,7 +779,7 @@ attn_dec4_kernel(const float* q, const uint8_t* kc, const uint8_t* vc, const flo
                 }
             named_bar_sync(2 + quad, 128);
             // (all of the quad is done with its stage before this one, and the slot's barrier is armed)
-            if (refill && lane == 0) copy(j - 2 + NSTG, w);
+            if (refill >= 0 && lane == 0) copy(refill, w);
             float corr[RT][2];
             bool grew = false;
 #pragma unroll
@@ -856,10 +852,11 @@ attn_dec4_kernel(const float* q, const uint8_t* kc, const uint8_t* vc, const flo
                     for (int rt = 0; rt < RT; rt++) mma16816(o[rt][jd], pa[rt], b0, b1);
                 }
             }
-            if (C::QUADS > 2 && j + NSTG < nstg) {  // (few stages more than quads: the next stage's barrier would be late)
-                if (w == 0 && lane == 0) arm(j + NSTG);
+            const int behind = Ring::at_the_end(j, nstg);  // (few stages more than quads: the next stage's barrier would be late)
+            if (behind >= 0) {
+                if (w == 0 && lane == 0) arm(behind);
                 named_bar_sync(2 + quad, 128);
-                if (lane == 0) copy(j + NSTG, w);
+                if (lane == 0) copy(behind, w);
             }
         }
 
@@ -875,12 +872,7 @@ attn_dec4_kernel(const float* q, const uint8_t* kc, const uint8_t* vc, const flo
             at += nstg + SPLIT_COST;
             more = at < until;
             if (!more) return;
-#pragma unroll
-            for (int sl = 0; sl < NSTG; sl++) {
-                const int j = (sl + NSTG - OFF) % NSTG;  // the first stage in this slot
-                if (j < nstg) pars ^= (((nstg - 1 - j) / NSTG + 1) & 1) << sl;
-            }
-            j0 += nstg;
+            order.next_split(nstg);
             fresh = false;
             if (++s == ns) {
                 s = 0;

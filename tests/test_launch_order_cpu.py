@@ -38,13 +38,12 @@ def test_the_first_kernels_of_a_step_wait_before_they_let_others_start():
         assert 0 <= body.find("pdl_wait();") < body.find("pdl_launch_dependents();"), name
 
 
-def test_decode_attention_knows_its_stage_was_asked_for():
-    """The quads of a block share the ring's slots, so a quad may come to a slot whose last stage, another quad's, has not landed: the
-    parity of the stage it wants is then the parity of the phase before that one, and a wait on it ends at once. It looks first
-    whether its stage's copies were asked for (that is done once the slot's last stage has been consumed)."""
+def test_decode_attention_follows_its_rings_order():
+    """The order in which a block's quads share the ring's slots is dec_ring.h's, played through by test_dec_ring_cpu.py; here only that the
+    kernel takes it from there: it looks for its stage's number before it waits, and writes the number behind the slot's barrier."""
     body = {name: body for _, name, body in kernels()}["attn_dec4_kernel"]
-    wait = body.index("mbar_wait(&full[sl]")
-    looks = body.rfind("while (issued[sl] != j", 0, wait)
-    assert looks > 0 and "if (j >= NSTG)" in body[looks - 60:looks]
+    wait = body.index("mbar_wait(&full[sl], par)")
+    looks = body.rfind("while (issued[sl] != order.number(j)", 0, wait)
+    assert looks > 0 and "if (Ring::looks(j))" in body[looks - 60:looks] and "par = order.parity(j)" in body[looks - 400:looks]
     asks = body.index("mbar_expect_tx(")
-    assert re.match(r"mbar_expect_tx\([^;]*\);\s*issued\[[^;]*= j;", body[asks:])
+    assert re.match(r"mbar_expect_tx\([^;]*\);\s*issued\[Ring::slot\(j\)\] = order\.number\(j\);", body[asks:])
