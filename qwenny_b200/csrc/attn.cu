@@ -456,7 +456,7 @@ attn_tile_kernel(const float* q, const uint8_t* kc, const uint8_t* vc, const flo
 //            power of two, and exchange their 16-key slices of P (as f16 mma fragments); a lane keeps the sums of its own keys
 //            to the end. (P relative to a reference that moves only near f16's end: one barrier per stage instead of two, but P
 //            is made twice where it moves and rounded to other values: no faster, 5 rows at 32000 29.4 us, 28.9 so; 8 sequences of 4 rows up to
-//            32000 are the exception, 112.2 and 116.5);
+//            32000 are the exception, 112 and 117);
 //   values   warp w accumulates the output dims 64 w .. 64 w + 63 over all 64 keys of the stage (for every row tile),
 //            so the output accumulators of a row are spread over four warps (RT x 32 registers each).
 // The int8 codes go to the tensor cores as 1152 + q halves (one prmt per pair) and the offset is folded out through the
@@ -464,8 +464,8 @@ attn_tile_kernel(const float* q, const uint8_t* kc, const uint8_t* vc, const flo
 // at the end; the block writes one (m, l, acc) partial per row, or the finished rows when the segment has one split.
 // Bound by latency, with two warps per scheduler (four at one row tile). From a graph with attn_prep and the combine, us, before (a copy
 // warp, Q row by row, keys with bank conflicts) / now: 5 rows at 100 keys 13.7 / 11.0, at 4000 18.3 / 14.9, at 32000 34.8 / 28.9; 1 row at
-// 32000 26.3 / 24.3; 8 rows 50.4 / 38.3 (registers spilled before); 8 sequences of 4 rows at 972 to 7777 66.7 / 47.9 (57.7 with a block per
-// split), at 4000 to 32000 139.9 / 116.5 (126.6).
+// 32000 26.3 / 24.3; 8 rows 50.4 / 38.3 (registers spilled before); 8 sequences of 4 rows at 972 to 7777 66.7 / 47.8 (57.7 with a block per
+// split), at 4000 to 32000 139.9 / 117 (126.6).
 // Many splits (MANY): a block per split would pay for each one's start (its segment's tokens, Q, the first stages' way from memory: half of
 // the 11 us that a split of four stages took) and leave the last round of the SMs partly idle. So a block per SM takes a run of them, equal
 // shares of the line on which each split is as long as its stages and SPLIT_COST: Q stays where the run stays with a segment's kv head,
