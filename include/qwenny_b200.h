@@ -228,7 +228,8 @@ int qb_attn_dec_splits(int keys);
 int qb_attn_dec_splits_sm(int keys, int sms);
 /* The splits that a launch of qb_attn_decode with this max_keys provides for: the most of any key count up to it (a
  * longer range has longer splits: on 148 SMs 3000 keys are 24 splits, 4400 keys 23). A captured launch serves every step
- * with the same value. */
+ * with the same value. (With many segments it deals the splits out to a block per SM or gives each a block, by ndseg and
+ * max_keys: the same results, and a captured launch keeps the form of the step that it was captured at.) */
 int qb_attn_dec_grid(int max_keys, int sms);
 /* qb_attn_prefill  attn_prefill + attn_combine_tiles (+ to_xin when mix_f16 != NULL), kernels/attn.cuh:327-349,351-520,
  *                  as Attn::run launches them (src/cuda/qwen/attn.rs:338-368): ntile tiles (ptile: first token,

@@ -2,6 +2,7 @@
 // two-buffer rollback plan and the gated RMSNorm, which the reference runs as three kernels (kernels/qwen_deltanet.cuh:
 // delta_conv :84-131, delta_rule :172-288, delta_norm :295-315). Steps with longer segments take the three entry points
 // of delta_prompt.cu and delta_rule.cu. Slot memory layout, the plan and the metadata are the reference's (delta_common.cuh).
+#include <climits>
 #include "delta_common.cuh"
 #include "launch.h"
 
